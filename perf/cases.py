@@ -20,6 +20,7 @@ import math
 
 import torch
 import torch.nn.functional as F
+from torch.utils.checkpoint import checkpoint
 
 from aussm_b200 import models, ops, s6, variants
 
@@ -279,3 +280,200 @@ def tolerance(case):
     if kind == "timeseries":
         return {"rel": 4e-5}
     return {"rel": max(1e-4, 5.5e-8 * l)}
+
+
+# ---------------------------------------------------------------------------
+# the same passes in 64 bits, in plain torch
+# ---------------------------------------------------------------------------
+class _LinearRecurrence(torch.autograd.Function):
+    """h_t = a_t h_{t-1} + x_t over the first axis, from zero."""
+
+    @staticmethod
+    def forward(ctx, a, x):
+        h = torch.empty_like(x)
+        h[0] = x[0]
+        for p, q, ai, xi in zip(h[:-1].unbind(0), h[1:].unbind(0), a[1:].unbind(0), x[1:].unbind(0)):
+            torch.addcmul(xi, ai, p, out=q)
+        ctx.save_for_backward(a, h)
+        return h
+
+    @staticmethod
+    def backward(ctx, g):
+        a, h = ctx.saved_tensors
+        e, ac = g.clone(), a.conj().resolve_conj()
+        rows, mult = e.unbind(0), ac.unbind(0)
+        for t in range(len(rows) - 2, -1, -1):
+            rows[t].addcmul_(mult[t + 1], rows[t + 1])
+        ga = torch.zeros_like(a)
+        torch.mul(e[1:], h[:-1].conj(), out=ga[1:])
+        return ga, e
+
+
+def _unitary(theta, drive, coef):
+    """sum_j Re(coef_j h_j) and the last state of h_t = exp(i theta_t) h_{t-1} + drive_t, theta (c, n, l)."""
+    turn = torch.polar(torch.ones_like(theta), torch.cumsum(theta, -1))
+    h = turn * torch.cumsum(turn.conj() * drive, -1)
+    return (coef[:, None] * h).real.sum(-2), h[..., -1]
+
+
+def _polar(r, angle):
+    return torch.polar(r, torch.zeros_like(r)) * torch.polar(torch.ones_like(angle), angle)
+
+
+def _exact_scan(theta_of, u, dt, z, Bc, Cc, D, part):
+    """The unitary operator, `part` channels of one batch entry at a time; theta_of(b, i0, i1) is their phases."""
+    ys, hs = [], []
+    for b in range(u.shape[0]):
+        for i in range(0, u.shape[1], part):
+            def piece(ub, dtb, zb, Db, *own, b=b, i=i):
+                v = F.silu(ub)
+                y, h = _unitary(theta_of(b, i, *own), Bc[:, None] * (dtb * v)[:, None], Cc)
+                return F.silu(zb) * (Db[:, None] * v + y), h
+            own = theta_of.own(b, i, i + part)
+            cut = (u[b, i:i + part], dt[b, i:i + part], z[b, i:i + part], D[i:i + part]) + own
+            y, h = checkpoint(piece, *cut, use_reentrant=False)
+            ys.append(y)
+            hs.append(h)
+    shape = u.shape[:2]
+    return torch.cat(ys).view(*shape, -1), torch.cat(hs).view(*shape, -1)
+
+
+class _Projected:
+    def __init__(self, x, bias, u):
+        self.x, self.bias, self.u = x, bias, u
+
+    def own(self, b, i0, i1):
+        return self.x[i0:i1], self.bias[i0:i1], self.u[b]
+
+    def __call__(self, b, i, x, bias, u):
+        return torch.matmul(x, u) + bias[..., None]
+
+
+class _Given:
+    def __init__(self, theta):
+        self.theta = theta
+
+    def own(self, b, i0, i1):
+        return (self.theta[b, i0:i1],)
+
+    def __call__(self, b, i, theta):
+        return theta
+
+
+def _part(n, l):
+    return max(1, (1 << 26) // (n * l))
+
+
+def _exact_operator(u, dt, x, x_bias, B, C, D, z):
+    Bc, Cc = _polar(F.softplus(B.real), B.imag), _polar(F.softplus(C.real), C.imag)
+    return _exact_scan(_Projected(x, x_bias, u), u, dt, z, Bc, Cc, D, _part(x.shape[1], u.shape[2]))[0]
+
+
+def _exact_decaying(u, a_of, x_of, C, part):
+    """sum_j Re(C_j h_j) of h_t = a_t h_{t-1} + x_t; a_of and x_of give (channels, n, l) from a channel's own rows."""
+    rows = []
+    for b in range(u.shape[0]):
+        for i in range(0, u.shape[1], part):
+            def piece(b=b, i=i):
+                a, x = a_of(b, slice(i, i + part)), x_of(b, slice(i, i + part))
+                h = _LinearRecurrence.apply(a.movedim(-1, 0).contiguous(), x.movedim(-1, 0).contiguous())
+                y = C[b].movedim(-1, 0)[:, None] * h
+                return (y.real if y.is_complex() else y).sum(-1).t()
+            rows.append(checkpoint(piece, use_reentrant=False))
+    return torch.cat(rows).view(u.shape)
+
+
+def _exact_mamba(u, delta, A, B, C, D, z, delta_bias):
+    dl = F.softplus(delta + delta_bias[:, None])
+    y = _exact_decaying(u, lambda b, i: torch.exp(dl[b, i, None] * A[i, :, None]),
+                        lambda b, i: (dl[b, i] * u[b, i])[:, None] * B[b], C, 8 * _part(A.shape[1], u.shape[2]))
+    return F.silu(z) * (y + D[:, None] * u)
+
+
+def _exact_decay(rho, theta, u, dt, z, B_re, B_im, C_re, C_im, D):
+    B, C = (B_re, C_re) if theta is None else (torch.complex(B_re, B_im), torch.complex(C_re, C_im))
+    s = dt * F.silu(u)
+
+    def multiplier(b, i):
+        r = torch.exp(rho[b, i])
+        return r if theta is None else torch.polar(torch.ones_like(r), theta[b, i]) * r
+    y = _exact_decaying(u, multiplier, lambda b, i: s[b, i, None] * B[b], C, 4 * _part(rho.shape[2], u.shape[2]))
+    return F.silu(z) * (D[:, None] * F.silu(u) + y)
+
+
+def _exact_block(kind, p, x):
+    """One mixer; p: its parameters by name; x (b, l, d)."""
+    d = x.shape[-1]
+    inner = p["conv1d.weight"].shape[0]
+    xs, z = (x @ p["in_proj.weight"].t()).transpose(1, 2).split([inner, inner], dim=1)
+    l = x.shape[1]
+    xs = F.conv1d(xs, p["conv1d.weight"], p["conv1d.bias"], padding=p["conv1d.weight"].shape[-1] - 1,
+                  groups=inner)[..., :l]
+    low = p["x_proj.weight"] @ xs
+    rank = p["dt_proj.weight"].shape[1]
+    pre = p["dt_proj.weight"] @ low[:, :rank] + p["dt_proj.bias"][:, None]
+    if kind == "a":
+        n = p["B"].shape[0]
+        y = _exact_operator(xs, F.softplus(pre + p["dt_proj.bias"][:, None]),
+                            p["xA_proj.weight"].view(n, d, d).transpose(0, 1) / math.sqrt(d),
+                            p["xA_proj.bias"].view(n, d).t(), p["B"], p["C"], p["D"], z)
+    else:
+        n = p["A_log"].shape[1]
+        y = _exact_mamba(F.silu(xs), pre, -torch.exp(p["A_log"]), low[:, rank:rank + n], low[:, rank + n:], p["D"], z,
+                         p["dt_proj.bias"])
+    return y.transpose(1, 2) @ p["out_proj.weight"].t()
+
+
+def _exact_model(case, state):
+    def norm(x, w):
+        return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-5) * w
+
+    double = {torch.float32: torch.float64, torch.complex64: torch.complex128}
+    p = {k: v.detach().to(double[v.dtype]).requires_grad_(True) for k, v in state["model"].named_parameters()}
+    if case["kind"] == "timeseries":
+        x = state["x"].double() @ p["embedding.weight"].t() + p["embedding.bias"]
+    else:
+        x = p["embedding.weight"][state["x"]]
+    for k, kind in enumerate(case["layers"].split("|")):
+        pre = "layers.%d." % k
+        mixer = {name[len(pre) + 6:]: t for name, t in p.items() if name.startswith(pre + "mixer.")}
+        x = x + _exact_block(kind, mixer, norm(x, p[pre + "norm.weight"]))
+    if case["kind"] == "classifier":
+        x = x.mean(1)
+    out = norm(x, p["norm_f.weight"]) @ p["output.weight"].t()
+    target = state["target"]
+    loss = F.mse_loss(out, target.double()) if case["kind"] == "timeseries" else F.cross_entropy(out, target)
+    return {"out": out.detach(), "loss": loss.detach(), "grads": dict(zip(p, torch.autograd.grad(loss, list(p.values()))))}
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits; None for the largest cases, whose 64-bit gradients alone fill much of a card,
+    and for Mamba layers in a very long model (a step by step loop)."""
+    kind, states = case["kind"], case["b"] * case["d"] * case["n"] * case["l"]
+    if states > 1 << 30 or (kind == "classifier" and "m" in case["layers"] and case["l"] > 8192):
+        return None
+    state = prepare(case, seed)
+    if kind in ("timeseries", "classifier"):
+        return _exact_model(case, state)
+    double = {torch.float32: torch.float64, torch.complex64: torch.complex128}
+    inputs = {k: None if t is None else t.detach().to(double[t.dtype]).requires_grad_(case["train"])
+              for k, t in state["inputs"].items()}
+    with torch.set_grad_enabled(case["train"]):
+        h = None
+        if kind == "operator":
+            y = _exact_operator(**inputs)
+        elif kind == "scan":
+            i = inputs
+            y, h = _exact_scan(_Given(i["theta"]), i["u"], i["dt"], i["z"], _polar(i["B_r"], i["B_theta"]),
+                               _polar(i["C_r"], i["C_theta"]), i["D"], _part(case["n"], case["l"]))
+        else:
+            y = (_exact_mamba if kind == "mamba" else _exact_decay)(**inputs)
+    result = {"y": y.detach()}
+    if h is not None:
+        result["h_re"], result["h_im"] = h.detach().real, h.detach().imag
+    if not case["train"]:
+        return result if h is not None else result["y"]
+    wanted = {k: t for k, t in inputs.items() if t is not None}
+    grads = torch.autograd.grad(y, list(wanted.values()), state["grad_y"].double())
+    result["grads"] = dict(zip(wanted, grads))
+    return result
