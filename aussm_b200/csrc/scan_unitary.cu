@@ -39,6 +39,8 @@
 //     eta_t = conj(Cc) w_t + exp(-i*theta_{t+1}) eta_{t+1},   w_t = gy_t silu(z_t)
 // so nothing but the inputs and the final state is ever stored.  dtheta is
 // written in place of theta in the stage and leaves with coalesced stores.
+#include <type_traits>
+
 #include "common.cuh"
 #include "scan_unitary.cuh"
 
@@ -175,12 +177,6 @@ __device__ __forceinline__ SegMap seg_map(const P& p) {
 // ---------------------------------------------------------------------------
 // Tile movement
 // ---------------------------------------------------------------------------
-// shared-memory slot of state j of warp-channel c
-template <int NL>
-__device__ __forceinline__ int slot_of(int c, int j) {
-    return (j / NL) * 32 + c * NL + (j % NL);
-}
-
 // Where a warp's rows live in global memory, as seen by one lane: the source
 // of every 16-byte piece this lane copies per tile (at step 0 of the launch).
 template <class C>
@@ -247,29 +243,37 @@ struct TileMap {
     }
 };
 
-// Plain tile load for launches whose rows are not 16-byte aligned: coalesced
-// along time, zero-filled up to a quad, missing rows shadow row 0.
+// Tile copy for launches whose rows are not 16-byte aligned (odd lengths, shifted bases): the same asynchronous
+// ring with 4-byte pieces, one warp-wide instruction per row of 32 steps (consecutive lanes, consecutive words, so
+// the rows' start does not matter).  Missing rows shadow the warp's first row; steps beyond tlen are not written.
+// Four times the copy instructions of the 16-byte path, 1.4 more issue slots per step of about 26; the synchronous
+// loads this replaces exposed the full memory latency of every tile.  B6 D300 N10 L1021, forward + backward through
+// the Python front end: 1238 -> 220 us.
 template <class C>
-__device__ __forceinline__ void plain_load_tile(float* stage, const float* theta_warp, long long ld_theta,
-                                                const float* const* aux_src, long long ld_row, long long ch0,
-                                                int nvalid, int N, long long t0, int tlen, int lane) {
-    float* aux = stage + C::NROWS * C::TP;
-    const int tq = (tlen + 3) & ~3;
-    for (int slot = 0; slot < C::NROWS; ++slot) {
-        const int k = slot / 32, w = slot % 32;
-        const int c = w / C::NL, j = (w % C::NL) + k * C::NL;
-        const long long row = (c < nvalid && j < N) ? (long long)c * N + j : 0;
-        const float* src = theta_warp + row * ld_theta + t0;
-        float* dst = stage + slot * C::TP;
-        for (int t = lane; t < tq; t += 32) dst[t] = t < tlen ? src[t] : 0.f;
+__device__ __forceinline__ void issue_words(float* stage, const float* theta_warp, long long ld_theta,
+                                            const float* const* aux_src, long long aux_row0, long long ld_row,
+                                            int nvalid, int N, long long t0, int tlen, int lane) {
+    static_assert(C::T == 32, "one lane per step");
+    if (lane < tlen) {
+        const float* src = theta_warp + t0 + lane;
+        const uint32_t dst = smem_addr(stage) + (uint32_t)(lane * sizeof(float));
+#pragma unroll
+        for (int slot = 0; slot < C::NROWS; ++slot) {
+            const int c = (slot % 32) / C::NL, j = slot % C::NL + (slot / 32) * C::NL;
+            const long long row = (c < nvalid && j < N) ? (long long)(c * N + j) : 0;
+            cp_async4_s(dst + (uint32_t)(slot * C::TP * sizeof(float)), src + row * ld_theta);
+        }
+        const uint32_t aux = dst + (uint32_t)(C::NROWS * C::TP * sizeof(float));
+#pragma unroll
+        for (int a = 0; a < C::AUX; ++a) {
+            const float* asrc = aux_src[a] + aux_row0 + t0 + lane;
+#pragma unroll
+            for (int cc = 0; cc < C::CPW; ++cc)
+                cp_async4_s(aux + (uint32_t)((cc * C::AUX + a) * C::T * sizeof(float)),
+                            asrc + (cc < nvalid ? cc : 0) * ld_row);
+        }
     }
-    for (int row = 0; row < C::CPW * C::AUX; ++row) {
-        const int cc = row / C::AUX, a = row % C::AUX;
-        const float* src = aux_src[a] + (ch0 + (cc < nvalid ? cc : 0)) * ld_row + t0;
-        float* dst = aux + row * C::T;
-        for (int t = lane; t < tq; t += 32) dst[t] = t < tlen ? src[t] : 0.f;
-    }
-    __syncwarp();
+    cp_async_commit();
 }
 
 // ---------------------------------------------------------------------------
@@ -277,7 +281,8 @@ __device__ __forceinline__ void plain_load_tile(float* stage, const float* theta
 // ---------------------------------------------------------------------------
 // AGG: aggregate mode of the time-axis split - no output row; besides the state, the product of the segment's
 // rotations is carried (as a unit complex number, like the state itself) and returned.
-template <class C, bool ASYNC, bool NORM, bool BIAS, bool AGG>
+// VEC: rows are 16-byte aligned and L is a multiple of 4 (16-byte copies and vector stores).
+template <class C, bool VEC, bool NORM, bool BIAS, bool AGG>
 __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, long long ch0, int nvalid, int lane,
                                          StateConsts (&sc)[C::SPT]) {
     constexpr int NL = C::NL, SPT = C::SPT, T = C::T, TP = C::TP, STAGES = C::STAGES, AUX = C::AUX, VW = C::VW;
@@ -315,29 +320,26 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
     }
 
     TileMap<C> map;
-    if (ASYNC) {
-        map.init(lane, nvalid, N, sm, ch0, aux_src);
-        for (int s = 0; s < STAGES; ++s) {
-            if (s < ntiles)
-                map.issue(wsm + s * C::STAGE_FLOATS, theta_warp, (long long)s * T, min(T, L - s * T), lane);
-            else
-                cp_async_commit();
-        }
+    if (VEC) map.init(lane, nvalid, N, sm, ch0, aux_src);
+    auto fetch = [&](float* stage, const int tile) {
+        const int len = min(T, L - tile * T);
+        if (VEC) map.issue(stage, theta_warp, (long long)tile * T, len, lane);
+        else issue_words<C>(stage, theta_warp, p.ld_theta, aux_src, sm.row(ch0), p.ld_row, nvalid, N, (long long)tile * T,
+                            len, lane);
+    };
+    for (int s = 0; s < STAGES; ++s) {
+        if (s < ntiles) fetch(wsm + s * C::STAGE_FLOATS, s);
+        else cp_async_commit();
     }
 
     for (int tile = 0; tile < ntiles; ++tile) {
-        const int stage = ASYNC ? tile % STAGES : 0;
-        float* th = wsm + stage * C::STAGE_FLOATS;
+        float* th = wsm + (tile % STAGES) * C::STAGE_FLOATS;
         float* aux = th + C::NROWS * TP;
         const long long t0 = (long long)tile * T;
         const int tlen = min(T, L - (int)t0);
         const int nq = (tlen + 3) >> 2;
-        if (ASYNC) {
-            cp_async_wait<STAGES - 1>();
-            __syncwarp();
-        } else {
-            plain_load_tile<C>(th, theta_warp, p.ld_theta, aux_src, p.ld_row, ch0, nvalid, N, t0, tlen, lane);
-        }
+        cp_async_wait<STAGES - 1>();
+        __syncwarp();
 
         // pre-pass: v = silu(u) over the u row, s = dt * v over the dt row
 #pragma unroll
@@ -361,7 +363,7 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
 
         // scan: SPT states per thread, four steps per shared-memory access
         const float* srow = aux + (c * AUX + 1) * T;
-        auto quad = [&](const int q) {
+        auto quad = [&](const int q, auto whole) {
             const float4 s4 = ld_shared_f4(srow + 4 * q);
             const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
             float pacc[4];
@@ -377,7 +379,7 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
                 sincos4(tv, sn, cs);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    if (!ASYNC && 4 * q + e >= tlen) {           // ragged tail (plain path only)
+                    if (!VEC && !whole.value && 4 * q + e >= tlen) {           // ragged tail
                         if (k == 0) pacc[e] = 0.f;
                         continue;
                     }
@@ -403,11 +405,11 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
             }
             if (!AGG) st_shared_f4(th + lane * TP + 4 * q, make_float4(pacc[0], pacc[1], pacc[2], pacc[3]));
         };
-        if (ASYNC && tlen == T) {
+        if (tlen == T) {
 #pragma unroll
-            for (int q = 0; q < T / 4; ++q) quad(q);
+            for (int q = 0; q < T / 4; ++q) quad(q, std::true_type{});
         } else {
-            for (int q = 0; q < nq; ++q) quad(q);
+            for (int q = 0; q < nq; ++q) quad(q, std::false_type{});
         }
         __syncwarp();
 
@@ -431,7 +433,7 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
 #pragma unroll
                     for (int e = 0; e < VW; ++e) acc.v[e] = siluf_(z.v[e]) * fmaf(dval[it], u.v[e], acc.v[e]);
                     float* dst = p.y + ybase[it] + t0 + t;
-                    if (ASYNC) {
+                    if (VEC) {
                         acc.st(dst);      // global pointers take the same vector stores
                     } else {
                         for (int e = 0; e < VW; ++e)
@@ -441,13 +443,10 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
             }
         }
         __syncwarp();
-        if (ASYNC) {
-            const int nt = tile + STAGES;
-            if (nt < ntiles) map.issue(th, theta_warp, (long long)nt * T, min(T, L - nt * T), lane);
-            else cp_async_commit();
-        }
+        if (tile + STAGES < ntiles) fetch(th, tile + STAGES);
+        else cp_async_commit();
     }
-    if (ASYNC) cp_async_wait<0>();
+    cp_async_wait<0>();
 
 #pragma unroll
     for (int k = 0; k < SPT; ++k) {
@@ -469,7 +468,7 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
     }
 }
 
-template <class C, bool ASYNC, bool BIAS, bool AGG>
+template <class C, bool VEC, bool BIAS, bool AGG>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const ScanFwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -495,16 +494,16 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const S
             float a, b;
             normalise_consts(sc[k], a, b);
         }
-        fwd_warp<C, ASYNC, true, BIAS, AGG>(p, wsm, ch0, nvalid, lane, sc);
+        fwd_warp<C, VEC, true, BIAS, AGG>(p, wsm, ch0, nvalid, lane, sc);
     } else {
-        fwd_warp<C, ASYNC, false, BIAS, AGG>(p, wsm, ch0, nvalid, lane, sc);
+        fwd_warp<C, VEC, false, BIAS, AGG>(p, wsm, ch0, nvalid, lane, sc);
     }
 }
 
 // ---------------------------------------------------------------------------
 // Backward
 // ---------------------------------------------------------------------------
-template <class C, bool ASYNC, bool NORM, bool BIAS>
+template <class C, bool VEC, bool NORM, bool BIAS>
 __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, long long ch0, int nvalid, int lane,
                                          StateConsts (&sc)[C::SPT], const float (&ccr)[C::SPT],
                                          const float (&cci)[C::SPT]) {
@@ -564,30 +563,26 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
 
     // r counts tiles in processing order (last tile first)
     TileMap<C> map;
-    if (ASYNC) {
-        map.init(lane, nvalid, N, sm, ch0, aux_src);
-        for (int r = 0; r < STAGES; ++r) {
-            const int tile = ntiles - 1 - r;
-            if (tile >= 0)
-                map.issue(wsm + r * C::STAGE_FLOATS, theta_warp, (long long)tile * T, min(T, L - tile * T), lane);
-            else
-                cp_async_commit();
-        }
+    if (VEC) map.init(lane, nvalid, N, sm, ch0, aux_src);
+    auto fetch = [&](float* stage, const int tile) {
+        const int len = min(T, L - tile * T);
+        if (VEC) map.issue(stage, theta_warp, (long long)tile * T, len, lane);
+        else issue_words<C>(stage, theta_warp, p.ld_theta, aux_src, sm.row(ch0), p.ld_row, nvalid, N, (long long)tile * T,
+                            len, lane);
+    };
+    for (int r = 0; r < STAGES; ++r) {
+        if (r < ntiles) fetch(wsm + r * C::STAGE_FLOATS, ntiles - 1 - r);
+        else cp_async_commit();
     }
 
     for (int r = 0; r < ntiles; ++r) {
         const int tile = ntiles - 1 - r;
-        const int stage = ASYNC ? r % STAGES : 0;
-        float* th = wsm + stage * C::STAGE_FLOATS;
+        float* th = wsm + (r % STAGES) * C::STAGE_FLOATS;
         float* aux = th + C::NROWS * TP;
         const long long t0 = (long long)tile * T;
         const int tlen = min(T, L - (int)t0);
-        if (ASYNC) {
-            cp_async_wait<STAGES - 1>();
-            __syncwarp();
-        } else {
-            plain_load_tile<C>(th, theta_warp, p.ld_theta, aux_src, p.ld_row, ch0, nvalid, N, t0, tlen, lane);
-        }
+        cp_async_wait<STAGES - 1>();
+        __syncwarp();
 
         const int nsb = (tlen + TS - 1) / TS;
         for (int sb = nsb - 1; sb >= 0; --sb) {
@@ -626,7 +621,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
             __syncwarp();
 
             // reverse scan
-            auto quad = [&](const int q) {
+            auto quad = [&](const int q, auto whole) {
                 const float4 s4 = ld_shared_f4(sw + (c * 3 + 0) * TS + 4 * q);
                 const float4 w4 = ld_shared_f4(sw + (c * 3 + 1) * TS + 4 * q);
                 const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
@@ -646,7 +641,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
                     float dth[4];
 #pragma unroll
                     for (int e = 3; e >= 0; --e) {
-                        if (!ASYNC && 4 * q + e >= slen) {
+                        if (!VEC && !whole.value && 4 * q + e >= slen) {
                             dth[e] = 0.f;
                             if (k == 0) { pacc[e] = 0.f; eacc[e] = 0.f; }
                             continue;
@@ -682,11 +677,11 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
                 st_shared_f4(pt + lane * TSP + 4 * q, make_float4(pacc[0], pacc[1], pacc[2], pacc[3]));
                 st_shared_f4(et + lane * TSP + 4 * q, make_float4(eacc[0], eacc[1], eacc[2], eacc[3]));
             };
-            if (ASYNC && slen == TS) {
+            if (slen == TS) {
 #pragma unroll
-                for (int q = TS / 4 - 1; q >= 0; --q) quad(q);
+                for (int q = TS / 4 - 1; q >= 0; --q) quad(q, std::true_type{});
             } else {
-                for (int q = nq - 1; q >= 0; --q) quad(q);
+                for (int q = nq - 1; q >= 0; --q) quad(q, std::false_type{});
             }
             __syncwarp();
 
@@ -720,10 +715,10 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
                         dz.v[e] = g.v[e] * fmaf(dv, v.v[e], P.v[e]) * gz.v[e];
                         ddt.v[e] = E.v[e] * v.v[e];
                         du.v[e] = fmaf(E.v[e], d.v[e], w.v[e] * dv) * gu.v[e];
-                        if (ASYNC || t + e < slen) dacc[it] = fmaf(w.v[e], v.v[e], dacc[it]);
+                        if (VEC || t + e < slen) dacc[it] = fmaf(w.v[e], v.v[e], dacc[it]);
                     }
                     const long long off = obase[it] + t0 + o;
-                    if (ASYNC) {
+                    if (VEC) {
                         du.st(p.du + off);
                         ddt.st(p.ddt + off);
                         dz.st(p.dz + off);
@@ -742,7 +737,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
         }
 
         // dtheta leaves the stage: coalesced 16-byte stores, same piece-to-lane map as the loads
-        if (ASYNC) {
+        if (VEC) {
             constexpr int CPR = C::CHUNKS_PER_ROW, RPI = 32 / CPR;
             const int col = lane % CPR;
             const float* src0 = th + (lane / CPR) * TP + col * 4;
@@ -763,25 +758,20 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
                             ld_shared_f4(src0 + i * RPI * TP);
                 }
             }
-            __syncwarp();
-            const int nr = r + STAGES;
-            if (nr < ntiles) {
-                const int nt = ntiles - 1 - nr;
-                map.issue(th, theta_warp, (long long)nt * T, min(T, L - nt * T), lane);
-            } else {
-                cp_async_commit();
+        } else if (lane < tlen) {                       // one row of 32 steps per instruction
+            float* dst = dtheta_warp + t0 + lane;
+            const float* src = th + lane;
+#pragma unroll
+            for (int slot = 0; slot < C::NROWS; ++slot) {
+                const int cc = (slot % 32) / NL, j = slot % NL + (slot / 32) * NL;
+                if (cc < nvalid && j < N) dst[(long long)(cc * N + j) * p.ld_theta] = src[slot * TP];
             }
-        } else {
-            for (int cc = 0; cc < nvalid; ++cc)
-                for (int j = 0; j < N; ++j) {
-                    float* dst = dtheta_warp + ((long long)cc * N + j) * p.ld_theta + t0;
-                    const float* src = th + slot_of<NL>(cc, j) * TP;
-                    for (int t = lane; t < tlen; t += 32) dst[t] = src[t];
-                }
-            __syncwarp();
         }
+        __syncwarp();
+        if (r + STAGES < ntiles) fetch(th, ntiles - 1 - r - STAGES);
+        else cp_async_commit();
     }
-    if (ASYNC) cp_async_wait<0>();
+    cp_async_wait<0>();
 
     // ---- per-(channel, state) results ----
 #pragma unroll
@@ -838,7 +828,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
     }
 }
 
-template <class C, bool ASYNC, bool BIAS>
+template <class C, bool VEC, bool BIAS>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const ScanBwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -864,9 +854,9 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const S
     if (__all_sync(0xffffffffu, ok)) {
 #pragma unroll
         for (int k = 0; k < C::SPT; ++k) normalise_consts(sc[k], ccr[k], cci[k]);
-        bwd_warp<C, ASYNC, true, BIAS>(p, wsm, ch0, nvalid, lane, sc, ccr, cci);
+        bwd_warp<C, VEC, true, BIAS>(p, wsm, ch0, nvalid, lane, sc, ccr, cci);
     } else {
-        bwd_warp<C, ASYNC, false, BIAS>(p, wsm, ch0, nvalid, lane, sc, ccr, cci);
+        bwd_warp<C, VEC, false, BIAS>(p, wsm, ch0, nvalid, lane, sc, ccr, cci);
     }
 }
 
@@ -1103,9 +1093,9 @@ __global__ void __launch_bounds__(256) reduce_param_grads_kernel(const ReducePar
 // ---------------------------------------------------------------------------
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <class C, bool ASYNC, bool BIAS, bool AGG>
+template <class C, bool VEC, bool BIAS, bool AGG>
 cudaError_t launch_fwd_cfg(const ScanFwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_fwd_kernel<C, ASYNC, BIAS, AGG>;
+    auto kern = scan_unitary_fwd_kernel<C, VEC, BIAS, AGG>;
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1116,9 +1106,9 @@ cudaError_t launch_fwd_cfg(const ScanFwdParams& p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template <class C, bool ASYNC, bool BIAS>
+template <class C, bool VEC, bool BIAS>
 cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_bwd_kernel<C, ASYNC, BIAS>;
+    auto kern = scan_unitary_bwd_kernel<C, VEC, BIAS>;
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1129,12 +1119,12 @@ cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-// Runtime properties -> template parameters.  The plain (unaligned) path is instantiated with the phase
+// Runtime properties -> template parameters.  The kernels for unaligned rows are instantiated with the phase
 // offset always on, to keep the build small.
 template <class C>
-cudaError_t launch_fwd_sel(const ScanFwdParams& p, bool async, cudaStream_t s) {
+cudaError_t launch_fwd_sel(const ScanFwdParams& p, bool vec, cudaStream_t s) {
     const bool bias = p.theta_bias != nullptr;
-    if (!async) return p.nseg > 1 || p.agg_re ? cudaErrorInvalidValue : launch_fwd_cfg<C, false, true, false>(p, s);
+    if (!vec) return p.nseg > 1 || p.agg_re ? cudaErrorInvalidValue : launch_fwd_cfg<C, false, true, false>(p, s);
     if (p.agg_re != nullptr && p.y == nullptr)
         return bias ? launch_fwd_cfg<C, true, true, true>(p, s) : launch_fwd_cfg<C, true, false, true>(p, s);
     return bias ? launch_fwd_cfg<C, true, true, false>(p, s) : launch_fwd_cfg<C, true, false, false>(p, s);
@@ -1157,9 +1147,9 @@ template <int NL, int SPT, int T, int STAGES, int WARPS>
 using EtaCfg = Cfg<NL, SPT, T, T, STAGES, WARPS, 4, false>;
 
 template <class C>
-cudaError_t launch_bwd_sel(const ScanBwdParams& p, bool async, cudaStream_t s) {
+cudaError_t launch_bwd_sel(const ScanBwdParams& p, bool vec, cudaStream_t s) {
     const bool bias = p.theta_bias != nullptr || p.part_rowsum != nullptr;
-    if (!async) return p.nseg > 1 ? cudaErrorInvalidValue : launch_bwd_cfg<C, false, true>(p, s);
+    if (!vec) return p.nseg > 1 ? cudaErrorInvalidValue : launch_bwd_cfg<C, false, true>(p, s);
     return bias ? launch_bwd_cfg<C, true, true>(p, s) : launch_bwd_cfg<C, true, false>(p, s);
 }
 
@@ -1175,16 +1165,16 @@ cudaError_t launch_scan_unitary_fwd(const ScanFwdParams& p_, cudaStream_t stream
     ScanFwdParams p = p_;
     p.status = device_status_ptr();
     if (!p.status) return cudaErrorInvalidSymbol;
-    const bool async = (p.L % 4 == 0) && (p.ld_theta % 4 == 0) && (p.ld_row % 4 == 0) && aligned16(p.theta) &&
+    const bool vec = (p.L % 4 == 0) && (p.ld_theta % 4 == 0) && (p.ld_row % 4 == 0) && aligned16(p.theta) &&
                        aligned16(p.u) && aligned16(p.dt) && aligned16(p.z) && (p.y == nullptr || aligned16(p.y)) &&
                        offsets_fit(p.ld_theta, 128);
     const int N = p.N;
-    if (N <= 4) return launch_fwd_sel<FwdCfg<4, 1, 32, 2, 4>>(p, async, stream);
-    if (N <= 8) return launch_fwd_sel<FwdCfg<8, 1, 32, 2, 4>>(p, async, stream);
-    if (N <= 16) return launch_fwd_sel<FwdCfg<16, 1, 32, 2, 4>>(p, async, stream);
-    if (N <= 32) return launch_fwd_sel<FwdCfg<32, 1, 32, 2, 4>>(p, async, stream);
-    if (N <= 64) return launch_fwd_sel<FwdCfg<32, 2, 32, 2, 4>>(p, async, stream);
-    if (N <= 128) return launch_fwd_sel<FwdCfg<32, 4, 32, 2, 2>>(p, async, stream);
+    if (N <= 4) return launch_fwd_sel<FwdCfg<4, 1, 32, 2, 4>>(p, vec, stream);
+    if (N <= 8) return launch_fwd_sel<FwdCfg<8, 1, 32, 2, 4>>(p, vec, stream);
+    if (N <= 16) return launch_fwd_sel<FwdCfg<16, 1, 32, 2, 4>>(p, vec, stream);
+    if (N <= 32) return launch_fwd_sel<FwdCfg<32, 1, 32, 2, 4>>(p, vec, stream);
+    if (N <= 64) return launch_fwd_sel<FwdCfg<32, 2, 32, 2, 4>>(p, vec, stream);
+    if (N <= 128) return launch_fwd_sel<FwdCfg<32, 4, 32, 2, 2>>(p, vec, stream);
     return cudaErrorInvalidValue;
 }
 
@@ -1194,13 +1184,13 @@ cudaError_t launch_scan_unitary_bwd(const ScanBwdParams& p_, cudaStream_t stream
     p.status = device_status_ptr();
     if (!p.status) return cudaErrorInvalidSymbol;
     if (p.ld_dtheta != p.ld_theta) return cudaErrorInvalidValue;
-    const bool async = (p.L % 4 == 0) && (p.ld_theta % 4 == 0) && (p.ld_row % 4 == 0) && aligned16(p.theta) &&
+    const bool vec = (p.L % 4 == 0) && (p.ld_theta % 4 == 0) && (p.ld_row % 4 == 0) && aligned16(p.theta) &&
                        aligned16(p.dtheta) && aligned16(p.u) && aligned16(p.dt) && aligned16(p.z) &&
                        aligned16(p.gy) && aligned16(p.du) && aligned16(p.ddt) && aligned16(p.dz) &&
                        offsets_fit(p.ld_theta, 128);
     const int N = p.N;
     if (p.eta_only) {
-        if (!async || !p.dh0_re) return cudaErrorInvalidValue;
+        if (!vec || !p.dh0_re) return cudaErrorInvalidValue;
         const bool bias = p.theta_bias != nullptr;
 #define AUSSM_ETA(...) (bias ? launch_eta_cfg<__VA_ARGS__, true>(p, stream) : launch_eta_cfg<__VA_ARGS__, false>(p, stream))
         if (N <= 4) return AUSSM_ETA(EtaCfg<4, 1, 32, 2, 4>);
@@ -1212,13 +1202,13 @@ cudaError_t launch_scan_unitary_bwd(const ScanBwdParams& p_, cudaStream_t stream
 #undef AUSSM_ETA
         return cudaErrorInvalidValue;
     }
-    if (N <= 4) return launch_bwd_sel<BwdCfg<4, 1, 32, 32, 2, 2>>(p, async, stream);
-    if (N <= 8) return launch_bwd_sel<BwdCfg<8, 1, 32, 32, 2, 2>>(p, async, stream);
+    if (N <= 4) return launch_bwd_sel<BwdCfg<4, 1, 32, 32, 2, 2>>(p, vec, stream);
+    if (N <= 8) return launch_bwd_sel<BwdCfg<8, 1, 32, 32, 2, 2>>(p, vec, stream);
     // one-warp blocks: a finished warp is replaced at once (measured 9.55 ms against 10.2 ms with two-warp blocks)
-    if (N <= 16) return launch_bwd_sel<BwdCfg<16, 1, 32, 32, 2, 1>>(p, async, stream);
-    if (N <= 32) return launch_bwd_sel<BwdCfg<32, 1, 32, 32, 2, 2>>(p, async, stream);
-    if (N <= 64) return launch_bwd_sel<BwdCfg<32, 2, 32, 32, 2, 2>>(p, async, stream);
-    if (N <= 128) return launch_bwd_sel<BwdCfg<32, 4, 32, 32, 2, 2>>(p, async, stream);
+    if (N <= 16) return launch_bwd_sel<BwdCfg<16, 1, 32, 32, 2, 1>>(p, vec, stream);
+    if (N <= 32) return launch_bwd_sel<BwdCfg<32, 1, 32, 32, 2, 2>>(p, vec, stream);
+    if (N <= 64) return launch_bwd_sel<BwdCfg<32, 2, 32, 32, 2, 2>>(p, vec, stream);
+    if (N <= 128) return launch_bwd_sel<BwdCfg<32, 4, 32, 32, 2, 2>>(p, vec, stream);
     return cudaErrorInvalidValue;
 }
 
