@@ -79,6 +79,8 @@ struct GemmKernelParams {
     int kbatches;      // batch entries summed inside the K loop (1 when batches are independent)
     int a_batched;     // 0: operand shared by all batch entries (batch coordinate 0)
     int b_batched;
+    int ksplit;        // partial outputs per output (runs of the contraction), c_part_stride floats apart
+    long long c_part_stride;
     int beta;
     int* status;
     const unsigned* amax_a;   // FP16 parts: bit patterns of max|a|, max|b| (the parts are scaled by a power of two)
@@ -246,7 +248,11 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
     const int tiles_mn = p.tiles_m * p.tiles_n;
     constexpr int CHUNK_KB = 256 / BK;                         // K blocks per accumulation chunk (256 values)
     const int kblocks = (p.K + BK - 1) / BK;
-    const int total = kblocks * p.kbatches;
+    const int blocks_all = kblocks * p.kbatches;
+    // tile t: which output, which run of its contraction (K blocks [begin, begin + total) of blocks_all)
+    auto tile_batch = [&](int t) { return (t / tiles_mn) / p.ksplit; };
+    auto tile_run = [&](int t) { return (t / tiles_mn) % p.ksplit; };
+    auto run_begin = [&](int run) { return (int)((long long)blocks_all * run / p.ksplit); };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -277,7 +283,9 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
         int g = 0;                                       // K blocks copied by this CTA so far
         bool okp = true;
         for (int t = blockIdx.x; t < p.ntiles && okp; t += gridDim.x) {
-        const int zb = t / tiles_mn, m0 = ((t % tiles_mn) % p.tiles_m) * BM, n0 = ((t % tiles_mn) / p.tiles_m) * BN;
+        const int zb = tile_batch(t), run = tile_run(t);
+        const int m0 = ((t % tiles_mn) % p.tiles_m) * BM, n0 = ((t % tiles_mn) / p.tiles_m) * BN;
+        const int begin = run_begin(run), total = run_begin(run + 1) - begin;
         for (int it = 0; it < total; ++it, ++g) {
             const int s = g % STAGES;
             const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
@@ -289,8 +297,8 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
             }
             w = __shfl_sync(0xffffffffu, w, 0);          // also orders the copies after the arming of the barrier
             if (!w) { okp = false; break; }
-            const int kb = it % kblocks;
-            const int batch = zb * p.kbatches + it / kblocks;
+            const int kb = (begin + it) % kblocks;
+            const int batch = zb * p.kbatches + (begin + it) / kblocks;
             const int ba = p.a_batched ? batch : 0, bb = p.b_batched ? batch : 0;
             uint8_t* st = smem + s * STAGE_BYTES;
             const int k0 = kb * BK;
@@ -309,7 +317,8 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
             bool ok = true;
             int ch[2] = {0, 0};                       // chunks finished per column half
             int g = 0;                                // K blocks consumed so far
-            for (int t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x)
+            for (int t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
+            const int run = tile_run(t), total = run_begin(run + 1) - run_begin(run);
             for (int it = 0; it < total && ok; ++it, ++g) {
                 const int s = g % STAGES;
                 if (!mbar_wait_bounded(&full_bar[s], (uint32_t)(g / STAGES) & 1u, p.status)) { failed = 1; ok = false; break; }
@@ -344,6 +353,7 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                 }
                 umma_commit(&empty_bar[s]);                 // frees the stage when these MMAs have read it
             }
+            }
         }
     } else {
         // ---- accumulate + epilogue: warps 2..9; TMEM lane quarter = warp % 4, column half = (warp - 2) / 4.
@@ -363,7 +373,8 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
         const int rsub = lane >> 3, c4 = (lane & 7) * 4;           // coalesced phase: 4 rows x 8 quads per instruction
         const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * 2 * MMA_N);
         for (int t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
-            const int zb = t / tiles_mn, m0 = ((t % tiles_mn) % p.tiles_m) * BM, n0 = ((t % tiles_mn) / p.tiles_m) * BN;
+            const int zb = tile_batch(t), run = tile_run(t), total = run_begin(run + 1) - run_begin(run);
+            const int m0 = ((t % tiles_mn) % p.tiles_m) * BM, n0 = ((t % tiles_mn) / p.tiles_m) * BN;
 #pragma unroll
             for (int i = 0; i < MMA_N; ++i) acc[i] = 0.f;
             for (int it = 0; it < total; ++it) {
@@ -389,7 +400,7 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
             // The 32 x 32 blocks of the warp turn through the staging tile: lane = row on the way in, 4 rows x 128
             // bytes per instruction on the way out.
             if (ok && !failed) {
-                float* cbase = p.C + (long long)zb * p.c_batch_stride;
+                float* cbase = p.C + (long long)zb * p.c_batch_stride + (long long)run * p.c_part_stride;
 #pragma unroll
                 for (int blk = 0; blk < MMA_N / 32; ++blk) {
 #pragma unroll
@@ -646,12 +657,34 @@ int sm_count() {
 
 bool gemm_split3_supported(const SplitOperand& A, const SplitOperand& B, const float* C, const GemmShape& s) {
     if (s.M <= 0 || s.N <= 0 || s.K <= 0 || s.batches <= 0 || !C) return false;
-    if (s.reduce_batches < 0 || (s.reduce_batches > 0 && s.batches % s.reduce_batches)) return false;
     if (!A.amax || !B.amax) return false;
     // the parts are rows of halves whose pitch is a multiple of 16 bytes (split_f16 writes them that way)
     if (A.ld % 8 || B.ld % 8 || A.batch_stride % 8 || B.batch_stride % 8) return false;
     if (!ok16(A.hi) || !ok16(A.lo) || !ok16(B.hi) || !ok16(B.lo)) return false;
     return encode_fn() != nullptr;
+}
+
+long long gemm_split3_blocks(const GemmShape& s) {
+    return (long long)((s.K + BK - 1) / BK) * (s.reduce_batches ? s.batches : 1);
+}
+
+int gemm_split3_runs(long long M, long long N, long long K, int batches, bool reduce_batches, int most) {
+    constexpr long long SMS = 148;          // fixed, so that a workspace sized with it always fits
+    const long long outputs = reduce_batches ? 1 : batches;
+    const long long tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * outputs;
+    const long long blocks = ((K + BK - 1) / BK) * (reduce_batches ? batches : 1);
+    const double part = 8.0 * (double)M * (double)N * (double)outputs / 7.8e6;
+    int best = 1;
+    double best_cost = 0.0;
+    for (int g = 1; g <= most && (g == 1 || blocks / g >= 4); ++g) {
+        const double waves = (double)((tiles * g + SMS - 1) / SMS);
+        const double cost = waves * ((double)((blocks + g - 1) / g) + 6.0) + (g > 1 ? 2.0 + part * g : 0.0);
+        if (g == 1 || cost < 0.97 * best_cost) {
+            best = g;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 int gemm_split3(const SplitOperand& A, const SplitOperand& B, float* C, const GemmShape& s, cudaStream_t stream) {
@@ -668,13 +701,15 @@ int gemm_split3(const SplitOperand& A, const SplitOperand& B, float* C, const Ge
     GemmKernelParams kp;
     kp.C = C; kp.ldc = s.ldc; kp.c_batch_stride = s.c_batch_stride;
     kp.M = s.M; kp.N = s.N; kp.K = s.K;
-    kp.kbatches = s.reduce_batches ? s.batches / s.reduce_batches : 1;
+    kp.kbatches = s.reduce_batches ? s.batches : 1;
+    kp.ksplit = std::max(1, std::min(s.ksplit, (s.K + BK - 1) / BK * kp.kbatches));
+    kp.c_part_stride = s.c_part_stride;
     kp.beta = s.beta;
     kp.a_batched = A.batch_stride != 0;
     kp.b_batched = B.batch_stride != 0;
     kp.amax_a = A.amax;
     kp.amax_b = B.amax;
-    kp.c_vec = (ok16(C) && s.ldc % 4 == 0 && s.c_batch_stride % 4 == 0) ? 1 : 0;
+    kp.c_vec = (ok16(C) && s.ldc % 4 == 0 && s.c_batch_stride % 4 == 0 && s.c_part_stride % 4 == 0) ? 1 : 0;
     kp.status = device_status_ptr();
     if (!kp.status) {
         set_error("gemm_split3: device status word unavailable");
@@ -682,7 +717,7 @@ int gemm_split3(const SplitOperand& A, const SplitOperand& B, float* C, const Ge
     }
     kp.tiles_m = (s.M + BM - 1) / BM;
     kp.tiles_n = (s.N + BN - 1) / BN;
-    kp.ntiles = kp.tiles_m * kp.tiles_n * (s.reduce_batches ? s.reduce_batches : s.batches);
+    kp.ntiles = kp.tiles_m * kp.tiles_n * (s.reduce_batches ? 1 : s.batches) * kp.ksplit;
     const dim3 grid((unsigned)std::min(kp.ntiles, sm_count()), 1, 1);     // one persistent CTA per SM
     if (A.mn_major) return B.mn_major ? launch<1, 1>(maps, kp, grid, stream) : launch<1, 0>(maps, kp, grid, stream);
     return B.mn_major ? launch<0, 1>(maps, kp, grid, stream) : launch<0, 0>(maps, kp, grid, stream);

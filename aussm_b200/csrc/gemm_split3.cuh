@@ -29,12 +29,22 @@ struct SplitOperand {
 struct GemmShape {
     int M, N, K;
     int batches;          // number of operand batch entries
-    int reduce_batches;   // 0: one output per batch entry; g >= 1: the batch entries are summed in g groups of
-                          // batches / g consecutive entries, one output per group (g = 1: C = sum over all)
+    int reduce_batches;   // 0: one output per batch entry; 1: C = sum over the batch entries
     int beta;             // 0: overwrite C, 1: add to C
     long long ldc;        // floats; any value (rows that are not 16-byte aligned take scalar stores)
     long long c_batch_stride;
+    int ksplit;           // 0 or 1: whole contraction per tile; g > 1: the contraction (all K blocks of all summed
+                          // batch entries) is cut into g nearly equal runs, each a partial output of its own at
+                          // C + run * c_part_stride, to be added by the caller
+    long long c_part_stride;
 };
+
+long long gemm_split3_blocks(const GemmShape& s);      // K blocks of one output: no more runs than these are made
+// How many runs to cut a contraction into: few output tiles leave most SMs without work, and the time of a launch is
+// its number of tile waves times the K blocks of a tile.  Counted in K blocks (64 values, about 1.3 us of a tile):
+// a tile costs its blocks + 6 for its epilogue, and g > 1 adds the writing and reading of g partial outputs
+// (8 bytes an element at 6 TB/s) and a launch (2 blocks).  A run keeps at least 4 blocks (one accumulation chunk).
+int gemm_split3_runs(long long M, long long N, long long K, int batches, bool reduce_batches, int most);
 
 // Halves to reserve for one part of a split operand that holds `halves` values: rounded up to 256 bytes, with
 // room for the up to 63 halves that the last copy of an MN-major operand reads past the end of its last row.

@@ -1,10 +1,12 @@
 """Kernel variants and dispatch rules at the sizes where they can go wrong, against the float64 oracle."""
+import math
+
 import pytest
 import torch
 
 import aussm_b200
 from oracle import unitary as O
-from tests.helpers import scaled_error, scan_core_inputs
+from tests.helpers import NAMES, model_like_inputs, scaled_error, scan_core_inputs
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +49,32 @@ def test_scan_rows_that_start_anywhere(n, l):
     errors = scan_errors(b, d, n, l, 1000 + 10 * n + l)
     assert aussm_b200.device_status() == 0
     check_scan(errors, b, d, n, l)
+
+
+# The phases come from a product over d terms held to 2^-22 each: another 2.4e-7 sqrt(d) per step at worst.
+def operator_bound(b, d, n, l):
+    return scan_bound(b, d, n, l) + 2.4e-7 * math.sqrt(d) * l
+
+
+def operator_errors(b, d, n, l, seed):
+    inp = model_like_inputs(seed, b, d, n, l)
+    results = []
+    for dev, real, cplx, fn in (("cpu", torch.float64, torch.complex128, O.interface_unitary),
+                                ("cuda", torch.float32, torch.complex64, aussm_b200.ssm_adaptive_interface)):
+        a = [inp[k].to(dev, cplx if inp[k].is_complex() else real).clone().requires_grad_(True) for k in NAMES]
+        y = fn(*a)
+        (y * inp["gy"].to(dev, real)).sum().backward()
+        results.append({"y": y.detach()} | {"grad_" + k: t.grad for k, t in zip(NAMES, a)})
+    truth, got = results
+    view = lambda t: torch.view_as_real(t.cpu()) if t.is_complex() else t.cpu()
+    return {k: scaled_error(view(got[k]), view(truth[k])) for k in truth}
+
+
+# One output tile and a long contraction (many runs), runs that do not divide the K blocks, tiles that do not divide
+# the output, d that is no multiple of 4 (scalar stores of the partial outputs), no split at all.
+@pytest.mark.parametrize("shape", [(8, 16, 4, 256), (3, 37, 9, 200), (2, 130, 10, 500), (1, 65, 32, 96), (1, 8, 1, 16)])
+def test_operator_adjoints_summed_in_runs(shape):
+    errors = operator_errors(*shape, 3000 + sum(shape))
+    assert aussm_b200.device_status() == 0
+    bound = operator_bound(*shape)
+    assert max(errors.values()) < 10 * bound, (errors, bound)
