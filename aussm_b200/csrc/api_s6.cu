@@ -44,9 +44,11 @@ size_t aussm_b200_selective_scan_ckpt_floats(int B, int D, int N, int L) {
 }
 
 size_t aussm_b200_selective_scan_bwd_workspace_bytes(int B, int D, int N, int L) {
-    (void)L;
     if (B <= 0 || D <= 0 || N <= 0) return 0;
-    return up256(((size_t)B * D * N + 2 * (size_t)B * D) * sizeof(float));
+    // per-channel partials, one set per segment; a split adds the gradients between segments and their step sizes
+    const size_t nseg = L > 0 ? s6_split_plan(B, D, N, L, true).nseg : 1, nch = (size_t)B * D;
+    const size_t split = nseg > 1 ? nch * nseg * (N + 1) : 0;
+    return up256((nch * nseg * (N + 2) + split) * sizeof(float));
 }
 
 int aussm_b200_selective_scan_fwd(const float* u, const float* delta, const float* A, const float* Bm,
@@ -98,8 +100,9 @@ int aussm_b200_selective_scan_bwd(const float* gout, const float* u, const float
     cudaStream_t stream = (cudaStream_t)stream_;
     const long long nch = (long long)B * D;
     float* part_A = static_cast<float*>(workspace);
-    float* part_D = part_A + nch * N;
-    float* part_bias = part_D + nch;
+    const S6Plan plan = s6_split_plan(B, D, N, L, true);
+    float* part_D = part_A + nch * plan.nseg * N;
+    float* part_bias = part_D + nch * plan.nseg;
     // dB and dC are accumulated with atomics: they start from zero
     cudaError_t e = cudaMemsetAsync(dB, 0, (size_t)B * N * L * sizeof(float), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(dC, 0, (size_t)B * N * L * sizeof(float), stream);
@@ -112,12 +115,15 @@ int aussm_b200_selective_scan_bwd(const float* gout, const float* u, const float
     p.delta_bias = delta_bias; p.ckpt = ckpt; p.du = du; p.ddelta = ddelta; p.dz = dz; p.dB = dB; p.dC = dC;
     p.part_A = part_A; p.part_D = part_D; p.part_bias = part_bias; p.delta_softplus = delta_softplus;
     p.nch = (int)nch; p.Dmod = D; p.N = N; p.L = L;
+    p.nseg = plan.nseg; p.seg_tiles = plan.seg_tiles;
+    p.seg_grad = part_bias + nch * plan.nseg;
+    p.seg_delta = p.seg_grad + nch * plan.nseg * N;
     e = s6_wide(N) ? launch_s6_wide_bwd(p, stream) : launch_s6_bwd(p, stream);
     if (e != cudaSuccess) {
         set_error("selective_scan_bwd launch: %s", cudaGetErrorString(e));
         return AUSSM_ECUDA;
     }
-    S6ReduceParams r = {part_A, part_D, part_bias, dA, dD, ddelta_bias, B, D, N};
+    S6ReduceParams r = {part_A, part_D, part_bias, dA, dD, ddelta_bias, B * plan.nseg, D, N};
     e = launch_s6_reduce(r, stream);
     if (e != cudaSuccess) {
         set_error("selective_scan_bwd reduction launch: %s", cudaGetErrorString(e));

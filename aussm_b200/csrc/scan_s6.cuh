@@ -31,6 +31,9 @@ struct S6FwdParams {
     float* last_state;        // (nch, N) or nullptr
     int delta_softplus;
     int nch, Dmod, N, L;
+    // Time-axis split (N <= kS6WideStates, filled in by the launcher): nseg > 1 segments of seg_tiles tiles side by
+    // side.  The start state of a segment is the record's entry of its first tile.
+    int nseg, seg_tiles;
 };
 
 struct S6BwdParams {
@@ -49,11 +52,14 @@ struct S6BwdParams {
     float* dz;                // (nch, L) or nullptr when z is nullptr
     float* dB;                // (batch, N, L), zeroed by the launcher, accumulated with float atomics
     float* dC;
-    float* part_A;            // (nch, N) per-channel partial of dA
-    float* part_D;            // (nch,)
-    float* part_bias;         // (nch,)
+    float* part_A;            // (batch, nseg, D, N) partials of dA
+    float* part_D;            // (batch, nseg, D)
+    float* part_bias;         // (batch, nseg, D)
     int delta_softplus;
     int nch, Dmod, N, L;
+    int nseg, seg_tiles;      // time-axis split (nseg <= 1: none)
+    float* seg_grad;          // (nch, nseg, N): gradient of the state after every segment
+    float* seg_delta;         // (nch, nseg): sum of the segment's step sizes
 };
 
 struct S6ReduceParams {
@@ -72,6 +78,12 @@ inline long long s6_ntiles(long long L, int N) {
     const int t = s6_wide(N) ? kS6WideTile : kS6Tile;
     return (L + t - 1) / t;
 }
+
+// Time-axis split of the wide kernels' launches (nseg == 1: none)
+struct S6Plan {
+    int nseg, seg_tiles;
+};
+S6Plan s6_split_plan(long long batches, int D, int N, int L, bool bwd);
 
 cudaError_t launch_s6_fwd(const S6FwdParams& p, cudaStream_t stream);
 cudaError_t launch_s6_bwd(const S6BwdParams& p, cudaStream_t stream);

@@ -26,6 +26,8 @@
 // MambaBlock.ssm_mamba, ai-modules/wavesAI/model/aussm.py:771-805); that file serves 16 < N <= 32.
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "host_common.cuh"
 #include "scan_s6.cuh"
@@ -148,13 +150,16 @@ __global__ void __launch_bounds__(32) s6w_fwd_kernel(const S6FwdParams p) {
     const int lane = threadIdx.x;
     const int c = lane / LPC, k = lane % LPC;
     const int tasks_per_batch = (p.Dmod + CPW - 1) / CPW;
-    const int b = blockIdx.x / tasks_per_batch, i0 = (blockIdx.x % tasks_per_batch) * CPW;
+    const int tasks = tasks_per_batch * (p.nch / p.Dmod);
+    const int seg = (int)(blockIdx.x / tasks), task = blockIdx.x % tasks;
+    const int b = task / tasks_per_batch, i0 = (task % tasks_per_batch) * CPW;
     const int nvalid = min(CPW, p.Dmod - i0);
     const bool act = c < nvalid;
     const int i = i0 + min(c, nvalid - 1);
     const long long ch0 = (long long)b * p.Dmod + i0, ch = (long long)b * p.Dmod + i;
     const int N = p.N, L = p.L;
     const int ntiles = (L + WT - 1) / WT;
+    const int first = seg * p.seg_tiles, last = p.nseg > 1 ? min(ntiles, first + p.seg_tiles) : ntiles;   // tiles
 
     float A2[SPT], h[SPT];
 #pragma unroll
@@ -175,12 +180,18 @@ __global__ void __launch_bounds__(32) s6w_fwd_kernel(const S6FwdParams p) {
     WMap<C> map;
     map.init(lane, nvalid, N, L, p.Bm + (long long)b * N * L, p.Cm + (long long)b * N * L, ch0);
     for (int s = 0; s < WSTAGES; ++s) {
-        if (s < ntiles) map.issue(smem + s * C::STAGE_FLOATS, aux_src, (long long)s * WT, min(WT, L - s * WT), lane);
+        const int t = first + s;
+        if (t < last) map.issue(smem + (t % WSTAGES) * C::STAGE_FLOATS, aux_src, (long long)t * WT, min(WT, L - t * WT), lane);
         else cp_async_commit();
     }
     float* ck = p.ckpt ? p.ckpt + ch * ntiles * N : nullptr;
+    if (seg > 0) {                                          // left there by the segment chain
+#pragma unroll
+        for (int jj = 0; jj < SPT; ++jj)
+            if (jj * LPC + k < N) h[jj] = ck[(long long)first * N + jj * LPC + k];
+    }
 
-    for (int tile = 0; tile < ntiles; ++tile) {
+    for (int tile = first; tile < last; ++tile) {
         float* st = smem + (tile % WSTAGES) * C::STAGE_FLOATS;
         float* urow = st + C::BC_FLOATS + c * WTP;
         float* drow = urow + C::AUX_FLOATS;
@@ -249,11 +260,11 @@ __global__ void __launch_bounds__(32) s6w_fwd_kernel(const S6FwdParams p) {
         map.store(st + C::BC_FLOATS, p.out, t0, tlen, lane);
         __syncwarp();
         const int nt = tile + WSTAGES;
-        if (nt < ntiles) map.issue(st, aux_src, (long long)nt * WT, min(WT, L - nt * WT), lane);
+        if (nt < last) map.issue(st, aux_src, (long long)nt * WT, min(WT, L - nt * WT), lane);
         else cp_async_commit();
     }
     cp_async_wait<0>();
-    if (act && p.last_state) {
+    if (act && p.last_state && last == ntiles) {
 #pragma unroll
         for (int jj = 0; jj < SPT; ++jj)
             if (jj * LPC + k < N) p.last_state[ch * N + jj * LPC + k] = h[jj];
@@ -276,13 +287,16 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
     const int lane = threadIdx.x;
     const int c = lane / LPC, k = lane % LPC;
     const int tasks_per_batch = (p.Dmod + CPW - 1) / CPW;
-    const int b = blockIdx.x / tasks_per_batch, i0 = (blockIdx.x % tasks_per_batch) * CPW;
+    const int tasks = tasks_per_batch * (p.nch / p.Dmod);
+    const int seg = (int)(blockIdx.x / tasks), task = blockIdx.x % tasks;
+    const int b = task / tasks_per_batch, i0 = (task % tasks_per_batch) * CPW;
     const int nvalid = min(CPW, p.Dmod - i0);
     const bool act = c < nvalid;
     const int i = i0 + min(c, nvalid - 1);
     const long long ch0 = (long long)b * p.Dmod + i0, ch = (long long)b * p.Dmod + i;
     const int N = p.N, L = p.L;
     const int ntiles = (L + WT - 1) / WT;
+    const int first = seg * p.seg_tiles, last = p.nseg > 1 ? min(ntiles, first + p.seg_tiles) : ntiles;   // tiles
 
     float* sub = smem + WSTAGES * C::STAGE_FLOATS;          // [NQ][SPT][32]
     float* red = sub + C::SUB_FLOATS;                       // [2 NS][RP] float4: gB rows, then gC rows
@@ -292,7 +306,7 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
     for (int jj = 0; jj < SPT; ++jj) {
         const int j = jj * LPC + k;
         A2[jj] = j < N ? p.A[(long long)i * N + j] * kLog2e : 0.f;
-        eps[jj] = 0.f;       // a_{t+1} eta_{t+1}
+        eps[jj] = (p.nseg > 1 && act && j < N) ? p.seg_grad[(ch * p.nseg + seg) * N + j] : 0.f;       // a_{t+1} eta_{t+1}
         dA[jj] = 0.f;
     }
     const float dskip = p.Dskip ? p.Dskip[i] : 0.f;
@@ -307,8 +321,8 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
     WMap<C> map;
     map.init(lane, nvalid, N, L, p.Bm + (long long)b * N * L, p.Cm + (long long)b * N * L, ch0);
     for (int r = 0; r < WSTAGES; ++r) {
-        const int tile = ntiles - 1 - r;
-        if (tile >= 0)
+        const int tile = last - 1 - r;
+        if (tile >= first)
             map.issue(smem + r * C::STAGE_FLOATS, aux_src, (long long)tile * WT, min(WT, L - tile * WT), lane);
         else cp_async_commit();
     }
@@ -316,14 +330,14 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
     float hn[SPT];                                          // state at the start of the tile taken next
 #pragma unroll
     for (int jj = 0; jj < SPT; ++jj)
-        hn[jj] = jj * LPC + k < N ? ck[(long long)(ntiles - 1) * N + jj * LPC + k] : 0.f;
+        hn[jj] = jj * LPC + k < N ? ck[(long long)(last - 1) * N + jj * LPC + k] : 0.f;
     // lane r of the channel-sum pass owns row r of the tile: dB of state r (r < NS) or dC of state r - NS
     const int rj = lane % NS;
     float* red_dst = (lane < NS ? p.dB : p.dC) + ((long long)b * N + min(rj, N - 1)) * L;
     const bool red_on = lane < 2 * NS && rj < N;
 
-    for (int r = 0; r < ntiles; ++r) {
-        const int tile = ntiles - 1 - r;
+    for (int r = 0; r < last - first; ++r) {
+        const int tile = last - 1 - r;
         float* st = smem + (r % WSTAGES) * C::STAGE_FLOATS;
         float* urow = st + C::BC_FLOATS + c * WTP;
         float* drow = urow + C::AUX_FLOATS;
@@ -335,7 +349,7 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
         float h[SPT];
 #pragma unroll
         for (int jj = 0; jj < SPT; ++jj) h[jj] = hn[jj];
-        if (tile > 0) {
+        if (tile > first) {
 #pragma unroll
             for (int jj = 0; jj < SPT; ++jj)
                 hn[jj] = jj * LPC + k < N ? ck[(long long)(tile - 1) * N + jj * LPC + k] : 0.f;
@@ -476,8 +490,8 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
         if (gate) map.store(st + C::BC_FLOATS + 2 * C::AUX_FLOATS, p.dz, t0, tlen, lane);
         __syncwarp();
         const int nr = r + WSTAGES;
-        if (nr < ntiles) {
-            const int nt = ntiles - 1 - nr;
+        if (nr < last - first) {
+            const int nt = last - 1 - nr;
             map.issue(st, aux_src, (long long)nt * WT, min(WT, L - nt * WT), lane);
         } else {
             cp_async_commit();
@@ -485,13 +499,232 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
     }
     cp_async_wait<0>();
     if (act) {
+        const long long o = ((long long)b * max(1, p.nseg) + seg) * p.Dmod + i;
 #pragma unroll
         for (int jj = 0; jj < SPT; ++jj)
-            if (jj * LPC + k < N) p.part_A[ch * N + jj * LPC + k] = dA[jj];
+            if (jj * LPC + k < N) p.part_A[o * N + jj * LPC + k] = dA[jj];
         if (k == 0) {
-            p.part_D[ch] = dD_acc;
-            p.part_bias[ch] = db_acc;
+            p.part_D[o] = dD_acc;
+            p.part_bias[o] = db_acc;
         }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Time-axis split: the segments' summaries and the chain through them.  With S the sum of a segment's step sizes its
+// multipliers' product is exp(A S), so a segment is summed up by S and
+//     forward    e = its end state from zero                     (the recurrence without the output)
+//     backward   l = sum_t exp(A S_t) C_t w_t                    (S_t the sum up to step t, w = gout silu(z)): the
+//                    gradient its outputs send to the state before it; no recurrence, 3 operations and one exponential
+// Forward: e of segment s lies in the state record where segment s + 1 starts and S one tile into segment s (two
+// entries that the real pass overwrites), the chain turns the e's into true start states in place.
+// ---------------------------------------------------------------------------
+template <int NS, int LPC>
+__global__ void __launch_bounds__(32) s6w_fwd_summary_kernel(const S6FwdParams p) {
+    using C = WCfg<NS, LPC, false>;
+    constexpr int SPT = C::SPT, CPW = C::CPW;
+    extern __shared__ __align__(128) float smem[];
+    const int lane = threadIdx.x;
+    const int c = lane / LPC, k = lane % LPC;
+    const int tasks_per_batch = (p.Dmod + CPW - 1) / CPW;
+    const int tasks = tasks_per_batch * (p.nch / p.Dmod);
+    const int seg = (int)(blockIdx.x / tasks), task = blockIdx.x % tasks;
+    const int b = task / tasks_per_batch, i0 = (task % tasks_per_batch) * CPW;
+    const int nvalid = min(CPW, p.Dmod - i0);
+    const bool act = c < nvalid;
+    const int i = i0 + min(c, nvalid - 1);
+    const long long ch0 = (long long)b * p.Dmod + i0, ch = (long long)b * p.Dmod + i;
+    const int N = p.N, L = p.L, ntiles = (L + WT - 1) / WT;
+    const int first = seg * p.seg_tiles, last = first + p.seg_tiles;      // never the last segment: whole tiles
+    float A2[SPT], h[SPT], S = 0.f;
+#pragma unroll
+    for (int jj = 0; jj < SPT; ++jj) {
+        const int j = jj * LPC + k;
+        A2[jj] = j < N ? p.A[(long long)i * N + j] * kLog2e : 0.f;
+        h[jj] = 0.f;
+    }
+    const float bias = p.delta_bias ? p.delta_bias[i] : 0.f;
+    const bool softplus = p.delta_softplus != 0;
+    for (int x = lane; x < WSTAGES * C::STAGE_FLOATS; x += 32) smem[x] = 0.f;
+    __syncwarp();
+    const float* aux_src[C::AUX] = {p.u, p.delta, nullptr};
+    WMap<C> map;
+    map.init(lane, nvalid, N, L, p.Bm + (long long)b * N * L, p.Cm + (long long)b * N * L, ch0);
+    for (int s = 0; s < WSTAGES; ++s) {
+        const int t = first + s;
+        if (t < last) map.issue(smem + (t % WSTAGES) * C::STAGE_FLOATS, aux_src, (long long)t * WT, WT, lane);
+        else cp_async_commit();
+    }
+    for (int tile = first; tile < last; ++tile) {
+        float* st = smem + (tile % WSTAGES) * C::STAGE_FLOATS;
+        float* urow = st + C::BC_FLOATS + c * WTP;
+        float* drow = urow + C::AUX_FLOATS;
+        cp_async_wait<WSTAGES - 1>();
+        __syncwarp();
+#pragma unroll
+        for (int x = 0; x < C::PRE_STEPS; x += 4) {
+            const int t = k * C::PRE_STEPS + x;
+            const float4 d4 = ld_shared_f4(drow + t);
+            float dv[4] = AUSSM_F4(d4);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                dv[e] += bias;
+                if (softplus) dv[e] = softplus_(dv[e]);
+                S += dv[e];
+            }
+            st_shared_f4(drow + t, make_float4(dv[0], dv[1], dv[2], dv[3]));
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const float4 u4 = ld_shared_f4(urow + 4 * q), d4 = ld_shared_f4(drow + 4 * q);
+            const float uv[4] = AUSSM_F4(u4), dlt[4] = AUSSM_F4(d4);
+#pragma unroll
+            for (int jj = 0; jj < SPT; ++jj) {
+                const float4 b4 = ld_shared_f4(st + (jj * LPC + k) * WTP + 4 * q);
+                const float bv[4] = AUSSM_F4(b4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) h[jj] = fmaf(ex2_ftz(dlt[e] * A2[jj]), h[jj], dlt[e] * uv[e] * bv[e]);
+            }
+        }
+        __syncwarp();
+        const int nt = tile + WSTAGES;
+        if (nt < last) map.issue(st, aux_src, (long long)nt * WT, WT, lane);
+        else cp_async_commit();
+    }
+    cp_async_wait<0>();
+    S = channel_sum<LPC>(S);
+    if (act) {
+        float* ck = p.ckpt + ch * ntiles * N;
+#pragma unroll
+        for (int jj = 0; jj < SPT; ++jj)
+            if (jj * LPC + k < N) ck[(long long)last * N + jj * LPC + k] = h[jj];
+        if (k == 0) ck[(long long)(first + 1) * N] = S;
+    }
+}
+
+template <int NS, int LPC>
+__global__ void __launch_bounds__(32) s6w_bwd_summary_kernel(const S6BwdParams p) {
+    using C = WCfg<NS, LPC, false>;                       // rows: delta, z, gout
+    constexpr int SPT = C::SPT, CPW = C::CPW;
+    extern __shared__ __align__(128) float smem[];
+    const int lane = threadIdx.x;
+    const int c = lane / LPC, k = lane % LPC;
+    const int tasks_per_batch = (p.Dmod + CPW - 1) / CPW;
+    const int tasks = tasks_per_batch * (p.nch / p.Dmod);
+    const int seg = 1 + (int)(blockIdx.x / tasks), task = blockIdx.x % tasks;
+    const int b = task / tasks_per_batch, i0 = (task % tasks_per_batch) * CPW;
+    const int nvalid = min(CPW, p.Dmod - i0);
+    const bool act = c < nvalid;
+    const int i = i0 + min(c, nvalid - 1);
+    const long long ch0 = (long long)b * p.Dmod + i0, ch = (long long)b * p.Dmod + i;
+    const int N = p.N, L = p.L, ntiles = (L + WT - 1) / WT;
+    const int first = seg * p.seg_tiles, last = min(ntiles, first + p.seg_tiles);     // never segment 0
+    float A2[SPT], l[SPT], S = 0.f;
+#pragma unroll
+    for (int jj = 0; jj < SPT; ++jj) {
+        const int j = jj * LPC + k;
+        A2[jj] = j < N ? p.A[(long long)i * N + j] * kLog2e : 0.f;
+        l[jj] = 0.f;
+    }
+    const float bias = p.delta_bias ? p.delta_bias[i] : 0.f;
+    const bool softplus = p.delta_softplus != 0, gate = p.z != nullptr;
+    for (int x = lane; x < WSTAGES * C::STAGE_FLOATS; x += 32) smem[x] = 0.f;
+    __syncwarp();
+    const float* aux_src[C::AUX] = {p.delta, p.z, p.gout};
+    WMap<C> map;
+    map.init(lane, nvalid, N, L, p.Bm + (long long)b * N * L, p.Cm + (long long)b * N * L, ch0);
+    for (int s = 0; s < WSTAGES; ++s) {
+        const int t = first + s;
+        if (t < last) map.issue(smem + (t % WSTAGES) * C::STAGE_FLOATS, aux_src, (long long)t * WT, min(WT, L - t * WT), lane);
+        else cp_async_commit();
+    }
+    for (int tile = first; tile < last; ++tile) {
+        float* st = smem + (tile % WSTAGES) * C::STAGE_FLOATS;
+        float* drow = st + C::BC_FLOATS + c * WTP;
+        float* zrow = drow + C::AUX_FLOATS;
+        float* grow = zrow + C::AUX_FLOATS;
+        const int tlen = min(WT, L - tile * WT);
+        cp_async_wait<WSTAGES - 1>();
+        __syncwarp();
+#pragma unroll
+        for (int x = 0; x < C::PRE_STEPS; x += 4) {
+            const int t = k * C::PRE_STEPS + x;
+            const float4 d4 = ld_shared_f4(drow + t);
+            float dv[4] = AUSSM_F4(d4);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                dv[e] += bias;
+                if (softplus) dv[e] = softplus_(dv[e]);
+            }
+            st_shared_f4(drow + t, make_float4(dv[0], dv[1], dv[2], dv[3]));
+            if (gate) {
+                const float4 z4 = ld_shared_f4(zrow + t), g4 = ld_shared_f4(grow + t);
+                st_shared_f4(grow + t, make_float4(g4.x * siluf_(z4.x), g4.y * siluf_(z4.y), g4.z * siluf_(z4.z),
+                                                   g4.w * siluf_(z4.w)));
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            if (4 * q >= tlen) break;
+            const float4 d4 = ld_shared_f4(drow + 4 * q), w4 = ld_shared_f4(grow + 4 * q);
+            const float w[4] = AUSSM_F4(w4);
+            const float at[4] = {S + d4.x, S + d4.x + d4.y, S + d4.x + d4.y + d4.z, S + d4.x + d4.y + d4.z + d4.w};
+            S = at[3];
+#pragma unroll
+            for (int jj = 0; jj < SPT; ++jj) {
+                const float4 c4 = ld_shared_f4(st + (NS + jj * LPC + k) * WTP + 4 * q);
+                const float cv[4] = AUSSM_F4(c4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) l[jj] = fmaf(ex2_ftz(at[e] * A2[jj]), cv[e] * w[e], l[jj]);
+            }
+        }
+        __syncwarp();
+        const int nt = tile + WSTAGES;
+        if (nt < last) map.issue(st, aux_src, (long long)nt * WT, min(WT, L - nt * WT), lane);
+        else cp_async_commit();
+    }
+    cp_async_wait<0>();
+    if (act) {
+        const long long o = ch * p.nseg + seg;
+#pragma unroll
+        for (int jj = 0; jj < SPT; ++jj)
+            if (jj * LPC + k < N) p.seg_grad[o * N + jj * LPC + k] = l[jj];
+        if (k == 0) p.seg_delta[o] = S;
+    }
+}
+
+// one thread per (channel, state): start states in place of the end states from zero
+__global__ void __launch_bounds__(128) s6w_fwd_chain_kernel(const S6FwdParams p, int ntiles) {
+    const long long id = (long long)blockIdx.x * 128 + threadIdx.x;
+    if (id >= (long long)p.nch * p.N) return;
+    const long long ch = id / p.N;
+    const int j = (int)(id % p.N);
+    const float A2 = p.A[(ch % p.Dmod) * p.N + j] * kLog2e;
+    float* ck = p.ckpt + ch * ntiles * p.N;
+    float h = 0.f;
+    for (int seg = 0; seg + 1 < p.nseg; ++seg) {
+        const float S = ck[((long long)seg * p.seg_tiles + 1) * p.N];
+        float* at = ck + (long long)(seg + 1) * p.seg_tiles * p.N + j;
+        h = fmaf(ex2_ftz(A2 * S), h, *at);
+        *at = h;
+    }
+}
+
+// one thread per (channel, state): seg_grad of segment s turns from l_s into the gradient of the state after s
+__global__ void __launch_bounds__(128) s6w_bwd_chain_kernel(const S6BwdParams p) {
+    const long long id = (long long)blockIdx.x * 128 + threadIdx.x;
+    if (id >= (long long)p.nch * p.N) return;
+    const long long ch = id / p.N;
+    const int j = (int)(id % p.N);
+    const float A2 = p.A[(ch % p.Dmod) * p.N + j] * kLog2e;
+    float g = 0.f;
+    for (int seg = p.nseg - 1; seg >= 0; --seg) {
+        const long long o = ch * p.nseg + seg;
+        const float l = seg > 0 ? p.seg_grad[o * p.N + j] : 0.f, S = seg > 0 ? p.seg_delta[o] : 0.f;
+        p.seg_grad[o * p.N + j] = g;
+        g = fmaf(ex2_ftz(A2 * S), g, l);
     }
 }
 
@@ -517,32 +750,55 @@ int lanes_per_channel(long long batches, int D, int NS, bool bwd) {
     return lpc;
 }
 
+template <class C, class K, class P>
+cudaError_t launch_w(K kern, const P& p, int segments, cudaStream_t stream) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    const long long tasks = (long long)(p.nch / p.Dmod) * ((p.Dmod + C::CPW - 1) / C::CPW);
+    kern<<<(unsigned)(tasks * segments), 32, C::SMEM_BYTES, stream>>>(p);
+    count_launch();
+    return cudaGetLastError();
+}
+
+unsigned chain_blocks(long long nch, int N) { return (unsigned)((nch * N + 127) / 128); }
+
 template <int NS, int LPC>
 cudaError_t launch_w_fwd(const S6FwdParams& p, cudaStream_t stream) {
     using C = WCfg<NS, LPC, false>;
-    auto kern = s6w_fwd_kernel<NS, LPC>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    const long long blocks = (long long)(p.nch / p.Dmod) * ((p.Dmod + C::CPW - 1) / C::CPW);
-    kern<<<(unsigned)blocks, 32, C::SMEM_BYTES, stream>>>(p);
-    count_launch();
-    return cudaGetLastError();
+    return launch_w<C>(s6w_fwd_kernel<NS, LPC>, p, p.nseg > 1 ? p.nseg : 1, stream);
 }
 
 template <int NS, int LPC>
 cudaError_t launch_w_bwd(const S6BwdParams& p, cudaStream_t stream) {
     using C = WCfg<NS, LPC, true>;
-    auto kern = s6w_bwd_kernel<NS, LPC>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
+    return launch_w<C>(s6w_bwd_kernel<NS, LPC>, p, p.nseg > 1 ? p.nseg : 1, stream);
+}
+
+template <int NS>
+cudaError_t launch_w_fwd_split(const S6FwdParams& p, cudaStream_t stream) {
+    using C = WCfg<NS, 2, false>;
+    cudaError_t e = launch_w<C>(s6w_fwd_summary_kernel<NS, 2>, p, p.nseg - 1, stream);
     if (e != cudaSuccess) return e;
-    const long long blocks = (long long)(p.nch / p.Dmod) * ((p.Dmod + C::CPW - 1) / C::CPW);
-    kern<<<(unsigned)blocks, 32, C::SMEM_BYTES, stream>>>(p);
+    s6w_fwd_chain_kernel<<<chain_blocks(p.nch, p.N), 128, 0, stream>>>(p, (p.L + WT - 1) / WT);
     count_launch();
-    return cudaGetLastError();
+    e = cudaGetLastError();
+    return e != cudaSuccess ? e : launch_w_fwd<NS, 2>(p, stream);
+}
+
+template <int NS>
+cudaError_t launch_w_bwd_split(const S6BwdParams& p, cudaStream_t stream) {
+    using C = WCfg<NS, 2, false>;
+    cudaError_t e = launch_w<C>(s6w_bwd_summary_kernel<NS, 2>, p, p.nseg - 1, stream);
+    if (e != cudaSuccess) return e;
+    s6w_bwd_chain_kernel<<<chain_blocks(p.nch, p.N), 128, 0, stream>>>(p);
+    count_launch();
+    e = cudaGetLastError();
+    return e != cudaSuccess ? e : launch_w_bwd<NS, 2>(p, stream);
 }
 
 template <int NS>
 cudaError_t launch_w_fwd_ns(const S6FwdParams& p, cudaStream_t stream) {
+    if (p.nseg > 1) return launch_w_fwd_split<NS>(p, stream);
     switch (lanes_per_channel(p.nch / p.Dmod, p.Dmod, NS, false)) {
         case 4: return launch_w_fwd<NS, 4>(p, stream);
         case 2: return launch_w_fwd<NS, 2>(p, stream);
@@ -552,14 +808,43 @@ cudaError_t launch_w_fwd_ns(const S6FwdParams& p, cudaStream_t stream) {
 
 template <int NS>
 cudaError_t launch_w_bwd_ns(const S6BwdParams& p, cudaStream_t stream) {
+    if (p.nseg > 1) return launch_w_bwd_split<NS>(p, stream);
     if (lanes_per_channel(p.nch / p.Dmod, p.Dmod, NS, true) == 4) return launch_w_bwd<NS, 4>(p, stream);
     return launch_w_bwd<NS, 2>(p, stream);
 }
 
 }  // namespace
 
-cudaError_t launch_s6_wide_fwd(const S6FwdParams& p, cudaStream_t stream) {
-    if (p.nch <= 0 || p.L <= 0) return cudaSuccess;
+// A launch whose channels give few warps (two lanes per channel) is cut along the time axis.  The backward kernel
+// holds 8 warps per SM (shared memory) and its summary pass costs an eighth of it: worth it below 4 warps per SM, as
+// many segments as fill one wave.  The forward summary costs two thirds of the real pass, which reaches its rate at
+// about 7 warps per SM: worth it below 3.  A segment keeps at least 64 steps; short sequences stay whole (the two
+// extra launches cost what they save).  N = 16, forward + backward, whole -> split: B1 D512 L8192 3357 -> 368 us (forward
+// alone 767 -> 140), B2 D1024 L2048 898 -> 348 us, B4 D512 L1024 487 -> 260 us, B4 D2048 L4096 (3.5 warps per SM)
+// 2067 -> 1863 us; B2 D256 N4 L300 216 -> 224 us (bound by the host).
+S6Plan s6_split_plan(long long batches, int D, int N, int L, bool bwd) {
+    S6Plan plan = {1, (L + WT - 1) / WT};
+    if (!s6_wide(N) || L < 256 || !time_split_option()) return plan;
+    constexpr long long SMS = 148;                          // fixed: a workspace sized with the plan always fits
+    const long long warps = batches * ((D + 15) / 16);
+    if (warps >= (bwd ? 4 : 3) * SMS) return plan;
+    const long long want = std::min<long long>((bwd ? 8 : 14) * SMS / warps, L / 64);
+    if (want < 2) return plan;
+    const int tiles = plan.seg_tiles;
+    plan.seg_tiles = (int)((tiles + want - 1) / want);
+    plan.nseg = (tiles + plan.seg_tiles - 1) / plan.seg_tiles;
+    return plan;
+}
+
+cudaError_t launch_s6_wide_fwd(const S6FwdParams& p_, cudaStream_t stream) {
+    if (p_.nch <= 0 || p_.L <= 0) return cudaSuccess;
+    S6FwdParams p = p_;
+    p.nseg = 1;
+    if (p.ckpt) {                                           // the split hands states on through the record
+        const S6Plan plan = s6_split_plan(p.nch / p.Dmod, p.Dmod, p.N, p.L, false);
+        p.nseg = plan.nseg;
+        p.seg_tiles = plan.seg_tiles;
+    }
     if (p.N <= 4) return launch_w_fwd_ns<4>(p, stream);
     if (p.N <= 8) return launch_w_fwd_ns<8>(p, stream);
     if (p.N <= 16) return launch_w_fwd_ns<16>(p, stream);

@@ -5,7 +5,9 @@ import pytest
 import torch
 
 import aussm_b200
+from aussm_b200.s6 import selective_scan_fn
 from oracle import unitary as O
+from oracle.s6 import selective_scan_ref
 from tests.helpers import NAMES, model_like_inputs, scaled_error, scan_core_inputs
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +80,34 @@ def test_operator_adjoints_summed_in_runs(shape):
     assert aussm_b200.device_status() == 0
     bound = operator_bound(*shape)
     assert max(errors.values()) < 10 * bound, (errors, bound)
+
+
+S6_KEYS = ["u", "delta", "A", "B", "C", "D", "z", "delta_bias"]
+
+
+# A step of the contracting recurrence costs two roundings and the exponential's 2^-22; earlier errors decay, but at
+# worst (A near 0) stay.  Sums over states, channels and steps add an ulp per term at worst.
+@pytest.mark.parametrize("shape", [(1, 5, 16, 256), (2, 33, 4, 300), (1, 16, 7, 1028), (3, 40, 12, 516), (1, 1, 1, 4096)])
+@pytest.mark.parametrize("full", [True, False])
+def test_selective_scan_cut_into_segments(shape, full):
+    b, d, n, l = shape
+    g = torch.Generator().manual_seed(4000 + sum(shape))
+    r = lambda *s: torch.randn(*s, generator=g)
+    inp = dict(u=r(b, d, l), delta=r(b, d, l) * 0.5 - 1.0, A=-torch.exp(r(d, n)), B=r(b, n, l) / math.sqrt(n),
+               C=r(b, n, l) / math.sqrt(n), D=r(d), z=r(b, d, l), delta_bias=r(d) * 0.5)
+    gy = r(b, d, l)
+    if not full:
+        inp["z"] = inp["D"] = inp["delta_bias"] = None
+        inp["delta"] = torch.nn.functional.softplus(inp["delta"])
+    results = []
+    for dev, dtype, fn in (("cpu", torch.float64, selective_scan_ref), ("cuda", torch.float32, selective_scan_fn)):
+        a = [None if inp[k] is None else inp[k].to(dev, dtype).clone().requires_grad_(True) for k in S6_KEYS]
+        y, last = fn(*a, delta_softplus=full, return_last_state=True)
+        (y * gy.to(dev, dtype)).sum().backward()
+        results.append({"y": y.detach(), "last": last.detach()} |
+                       {k: t.grad for k, t in zip(S6_KEYS, a) if t is not None})
+    assert aussm_b200.device_status() == 0
+    truth, got = results
+    bound = 4.5e-7 * l + 1.2e-7 * (n + b * d)
+    for k in truth:
+        assert scaled_error(got[k].cpu(), truth[k]) < bound, k
