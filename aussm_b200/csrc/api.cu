@@ -71,7 +71,7 @@ struct Plan {
     int window;          // steps per window
     long long ldw;       // row pitch of the window (floats)
     size_t off_theta, off_h, off_gh, off_part, off_proj, off_split, total;   // byte offsets
-    int nseg_fwd, nseg_bwd;   // time-axis split of the scans inside a window (1: none)
+    SegPlan seg_fwd, seg_bwd;   // time-axis split of the scans inside a window
 };
 
 Plan make_plan(int B, int D, int N, int L, int window_steps = window_steps_option()) {
@@ -97,23 +97,28 @@ Plan make_plan(int B, int D, int N, int L, int window_steps = window_steps_optio
     off = align_up(off + (size_t)p.rows * 2 * 4, 256);
     p.off_gh = off;      // re, im
     off = align_up(off + (size_t)p.rows * 2 * 4, 256);
-    // Few channels (small batch x d_inner) leave most of the GPU idle in a scan that is sequential in time:
-    // the scans of a window are then cut into segments (only when all windows have the same length, so that
-    // the per-segment partial sums of the backward pass line up from window to window).
+    // Few channels (small batch x d_inner) leave most of the GPU idle in a scan that is sequential in time: the
+    // scans of a window are then cut into segments (see scan_split_plan).
     const long long nch = (long long)B * D;
-    const bool equal_windows = (L % p.window) == 0;
-    p.nseg_fwd = equal_windows ? scan_split_segments(nch, N, p.window, false) : 1;
-    p.nseg_bwd = equal_windows ? scan_split_segments(nch, N, p.window, true) : 1;
+    p.seg_fwd = scan_split_plan(nch, N, p.window, false);
+    p.seg_bwd = scan_split_plan(nch, N, p.window, true);
     p.off_part = off;
-    off = align_up(off + scan_bwd_partial_floats(nch * p.nseg_bwd, N) * 4, 256);
+    off = align_up(off + scan_bwd_partial_floats(nch * p.seg_bwd.nseg, N) * 4, 256);
     p.off_proj = off;    // FP16 hi/lo parts of x, of the u window and of the dtheta window
     off = align_up(off + proj_scratch_bytes(B, D, (long long)D * N, p.ldw), 256);
     p.off_split = off;
-    const size_t split_floats = std::max(p.nseg_fwd > 1 ? scan_split_fwd_scratch_floats(nch, p.nseg_fwd, N) : 0,
-                                         p.nseg_bwd > 1 ? scan_split_bwd_scratch_floats(nch, p.nseg_bwd, N) : 0);
+    const size_t split_floats = std::max(p.seg_fwd.nseg > 1 ? scan_split_fwd_scratch_floats(nch, p.seg_fwd.nseg, N) : 0,
+                                         p.seg_bwd.nseg > 1 ? scan_split_bwd_scratch_floats(nch, p.seg_bwd.nseg, N) : 0);
     off = align_up(off + split_floats * 4, 256);
     p.total = off;
     return p;
+}
+
+// the plan of a full window applied to one of tl steps: segments of the same length, fewer of them
+SegPlan window_segments(const SegPlan& full, int tl) {
+    SegPlan s = full;
+    s.nseg = (tl + full.seg_len - 1) / full.seg_len;
+    return s;
 }
 
 // The layout of a kept-phase buffer (window length and row pitch) follows from the plan of the forward call,
@@ -202,8 +207,8 @@ int run_unitary_fwd(const OpArgs& a, const float* h0_re, const float* h0_im, flo
         sp.ld_theta = pl.ldw;
         sp.ld_row = a.L;
         cudaError_t e;
-        if (pl.nseg_fwd > 1 && scan_split_allowed(sp))
-            e = scan_unitary_fwd_split(sp, pl.nseg_fwd, reinterpret_cast<float*>(ws + pl.off_split), stream);
+        const SegPlan seg = window_segments(pl.seg_fwd, tl);
+        if (seg.nseg > 1) e = scan_unitary_fwd_split(sp, seg, reinterpret_cast<float*>(ws + pl.off_split), stream);
         else
             e = launch_scan_unitary_fwd(sp, stream);
         if (e != cudaSuccess) return cuda_fail(e, "unitary scan forward launch");
@@ -271,7 +276,7 @@ int aussm_b200_scan_unitary_fwd(const float* theta, const float* u, const float*
 
 size_t aussm_b200_scan_unitary_fwd_workspace_bytes(int B, int D, int N, int L) {
     if (B <= 0 || D <= 0 || N <= 0 || L <= 0) return 0;
-    const int nseg = scan_split_segments((long long)B * D, N, L, false);
+    const int nseg = scan_split_plan((long long)B * D, N, L, false).nseg;
     return nseg > 1 ? align_up(scan_split_fwd_scratch_floats((long long)B * D, nseg, N) * sizeof(float), 256) : 0;
 }
 
@@ -303,24 +308,18 @@ int aussm_b200_scan_unitary_fwd_ws(const float* theta, const float* u, const flo
     p.B_r = B_r; p.B_theta = B_theta; p.C_r = C_r; p.C_theta = C_theta; p.Dskip = Dskip;
     p.h0_re = h0_re; p.h0_im = h0_im; p.y = y; p.h1_re = h1_re; p.h1_im = h1_im;
     p.nch = B * D; p.Dmod = D; p.N = N; p.L = L; p.ld_theta = L; p.ld_row = L;
-    const int nseg = scan_split_segments((long long)B * D, N, L, false);
-    cudaError_t e = scan_split_allowed(p) ? scan_unitary_fwd_split(p, nseg, static_cast<float*>(workspace),
-                                                                   (cudaStream_t)stream)
-                                          : launch_scan_unitary_fwd(p, (cudaStream_t)stream);
+    cudaError_t e = scan_unitary_fwd_split(p, scan_split_plan((long long)B * D, N, L, false),
+                                           static_cast<float*>(workspace), (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "unitary scan forward launch");
     return AUSSM_OK;
 }
 
 // backward workspace: the per-channel partial sums (one set per segment when the time axis is split), then
 // the scratch of the split
-namespace {
-int bwd_segments(int B, int D, int N, int L) { return scan_split_segments((long long)B * D, N, L, true); }
-}  // namespace
-
 size_t aussm_b200_scan_unitary_bwd_workspace_bytes(int B, int D, int N, int L) {
     if (B <= 0 || D <= 0 || N <= 0) return 0;
     const long long nch = (long long)B * D;
-    const int nseg = L > 0 ? bwd_segments(B, D, N, L) : 1;
+    const int nseg = scan_split_plan(nch, N, L, true).nseg;
     size_t bytes = align_up(scan_bwd_partial_floats(nch * nseg, N) * sizeof(float), 256);
     if (nseg > 1) bytes += align_up(scan_split_bwd_scratch_floats(nch, nseg, N) * sizeof(float), 256);
     return bytes;
@@ -353,12 +352,12 @@ int aussm_b200_scan_unitary_bwd(const float* grad_y, const float* gh1_re, const 
     ScanBwdParams p = {};
     p.theta = theta; p.dtheta = dtheta; p.u = u; p.dt = dt; p.z = z; p.gy = grad_y; p.du = du; p.ddt = ddt; p.dz = dz;
     p.L = L; p.ld_theta = L; p.ld_dtheta = L; p.ld_row = L;
-    int nseg = bwd_segments(B, D, N, L);
-    if (nseg > 1 && !scan_split_allowed(p)) nseg = 1;
+    const SegPlan seg = scan_split_plan(nch, N, L, true);
+    const int nseg = seg.nseg;
     float* part_bc = static_cast<float*>(workspace);
     float* part_d = part_bc + nch * nseg * N * 4;
     float* split_scratch = reinterpret_cast<float*>(
-        static_cast<char*>(workspace) + align_up(scan_bwd_partial_floats(nch * bwd_segments(B, D, N, L), N) * sizeof(float), 256));
+        static_cast<char*>(workspace) + align_up(scan_bwd_partial_floats(nch * nseg, N) * sizeof(float), 256));
     p.theta = theta; p.theta_bias = nullptr; p.u = u; p.dt = dt; p.z = z; p.gy = grad_y;
     p.B_r = B_r; p.B_theta = B_theta; p.C_r = C_r; p.C_theta = C_theta; p.Dskip = Dskip;
     p.h1_re = h1_re; p.h1_im = h1_im; p.gh1_re = gh1_re; p.gh1_im = gh1_im;
@@ -366,7 +365,7 @@ int aussm_b200_scan_unitary_bwd(const float* grad_y, const float* gh1_re, const 
     p.h0_re = nullptr; p.h0_im = nullptr;
     p.part_bc = part_bc; p.part_d = part_d; p.part_rowsum = nullptr; p.accumulate = 0;
     p.nch = (int)nch; p.Dmod = D; p.N = N; p.L = L; p.ld_theta = L; p.ld_dtheta = L; p.ld_row = L;
-    cudaError_t e = nseg > 1 ? scan_unitary_bwd_split(p, nseg, split_scratch, (cudaStream_t)stream)
+    cudaError_t e = nseg > 1 ? scan_unitary_bwd_split(p, seg, split_scratch, (cudaStream_t)stream)
                              : launch_scan_unitary_bwd(p, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "unitary scan backward launch");
     ReduceParams r = {};
@@ -559,12 +558,9 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
     float* g_re = reinterpret_cast<float*>(ws + pl.off_gh);
     float* g_im = g_re + pl.rows;
     const long long nch = (long long)B * D;
-    // time-axis split of the backward scans: decided once per call (the partial sums of all windows share one
-    // layout); it needs the bulk-copy path, i.e. 16-byte aligned rows
-    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
-    const bool rows_aligned = (L % 4 == 0) && al16(u) && al16(dt) && al16(z) && al16(grad_y) && al16(du) && al16(ddt) &&
-                              al16(dz);
-    const int nseg_b = (pl.nseg_bwd > 1 && rows_aligned) ? pl.nseg_bwd : 1;
+    // the partial sums of all windows share one layout: as many entries per channel as a full window has segments.
+    // The last window in time comes first and may have fewer, so then the sums start from zero.
+    const int nseg_b = pl.seg_bwd.nseg;
     const long long nvirt = nch * nseg_b;
     float* part_bc = reinterpret_cast<float*>(ws + pl.off_part);
     float* part_d = part_bc + nvirt * N * 4;
@@ -587,6 +583,11 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
     }
 
     const int nwin = (L + pl.window - 1) / pl.window;
+    const bool zeroed = nseg_b > 1 && L % pl.window != 0;
+    if (zeroed) {
+        cudaError_t ez = cudaMemsetAsync(part_bc, 0, scan_bwd_partial_floats(nvirt, N) * sizeof(float), stream);
+        if (ez != cudaSuccess) return cuda_fail(ez, "clearing the partial sums");
+    }
     for (int w = nwin - 1; w >= 0; --w) {
         const long long t0 = (long long)w * pl.window;
         const int tl = (int)std::min<long long>(pl.window, L - t0);
@@ -614,7 +615,8 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
         p.h0_re = final_ ? nullptr : cur_re;
         p.h0_im = final_ ? nullptr : cur_im;
         p.part_bc = part_bc; p.part_d = part_d; p.part_rowsum = part_rowsum;
-        p.accumulate = first ? 0 : 1;
+        p.accumulate = first && !zeroed ? 0 : 1;
+        p.part_nseg = nseg_b;
         p.nch = (int)nch; p.Dmod = D; p.N = N; p.L = tl;
         p.ld_theta = pl.ldw; p.ld_dtheta = pl.ldw; p.ld_row = L;
         // the scan leaves max|dtheta| of the window behind for the FP16 split of the adjoint GEMMs
@@ -622,12 +624,9 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
         if (em != cudaSuccess) return cuda_fail(em, "clearing the dtheta maximum");
         p.dtheta_amax = ps.amax + 2;
         cudaError_t e;
-        if (nseg_b > 1) {
-            if (!scan_split_allowed(p)) {
-                set_error("unitary_bwd: window rows lost their 16-byte alignment (t0=%lld)", t0);
-                return AUSSM_EINVAL;
-            }
-            e = scan_unitary_bwd_split(p, nseg_b, reinterpret_cast<float*>(ws + pl.off_split), stream);
+        const SegPlan seg = window_segments(pl.seg_bwd, tl);
+        if (seg.nseg > 1) {
+            e = scan_unitary_bwd_split(p, seg, reinterpret_cast<float*>(ws + pl.off_split), stream);
         } else {
             e = launch_scan_unitary_bwd(p, stream);
         }

@@ -39,6 +39,7 @@
 //     eta_t = conj(Cc) w_t + exp(-i*theta_{t+1}) eta_{t+1},   w_t = gy_t silu(z_t)
 // so nothing but the inputs and the final state is ever stored.  dtheta is
 // written in place of theta in the stage and leaves with coalesced stores.
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -154,24 +155,28 @@ __device__ __forceinline__ void cdiv(float ar, float ai, float kr, float ki, flo
     qi = ti * ur - tr * ui;
 }
 
-// Where the rows of a (virtual) channel start.  Without a time-axis split channel v owns rows v; with nseg
-// segments virtual channel v = ch * nseg + s owns steps [s L, (s+1) L) of the rows of channel ch.
-struct SegMap {
-    int nseg, N;
-    long long seg_len, ld_theta, ld_row;
-    __device__ __forceinline__ long long chan(long long v) const { return nseg <= 1 ? v : v / nseg; }
-    // offset (floats) of the per-channel rows (u, dt, z, y, ...)
-    __device__ __forceinline__ long long row(long long v) const {
-        return nseg <= 1 ? v * ld_row : (v / nseg) * ld_row + (v % nseg) * seg_len;
-    }
-    // offset (floats) of the theta row of state 0
-    __device__ __forceinline__ long long theta(long long v) const {
-        return nseg <= 1 ? v * N * ld_theta : (v / nseg) * N * ld_theta + (v % nseg) * seg_len;
-    }
+// A warp's work: CPW consecutive channels and, when the time axis is split, one segment of it.  The segments are
+// seg_len steps (a multiple of the tile), the last one what is left; all channels of a warp share the segment.
+struct WarpTask {
+    long long ch0;      // first channel
+    int nvalid;         // channels that exist
+    int seg, nseg;      // segment and number of segments (1: no split)
+    long long t0;       // first step of the segment
+    int L;              // its steps
+    // entry of the per-segment state arrays that belongs to channel ch0 + c
+    __device__ __forceinline__ long long entry(int c) const { return (ch0 + c) * nseg + seg; }
 };
-template <class P>
-__device__ __forceinline__ SegMap seg_map(const P& p) {
-    return SegMap{p.nseg, p.N, (long long)p.L, p.ld_theta, p.ld_row};
+template <int CPW, class P>
+__device__ __forceinline__ bool warp_task(const P& p, long long task, WarpTask& w) {
+    const long long groups = ((long long)p.nch + CPW - 1) / CPW;
+    w.nseg = p.nseg > 1 ? p.nseg : 1;
+    if (task >= groups * w.nseg) return false;
+    w.seg = w.nseg > 1 ? (int)(task / groups) : 0;
+    w.ch0 = (task - w.seg * groups) * CPW;
+    w.nvalid = (int)min((long long)CPW, (long long)p.nch - w.ch0);
+    w.t0 = (long long)w.seg * p.seg_len;
+    w.L = w.nseg > 1 ? (int)min((long long)p.seg_len, (long long)p.L - w.t0) : p.L;
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -184,9 +189,8 @@ struct TileMap {
     unsigned theta_off[C::NCH_THETA];     // byte offset from the warp's first theta row (32 bits: base + offset addressing)
     const float* aux_ptr[C::NCH_AUX];     // per-channel rows (nullptr: this lane has no piece)
 
-    __device__ __forceinline__ void init(int lane, int nvalid, int N, const SegMap& sm, long long ch0,
-                                         const float* const* aux_src) {
-        const long long base0 = sm.theta(ch0);
+    __device__ __forceinline__ void init(int lane, int nvalid, int N, long long ld_theta, const float* const* aux_src,
+                                         long long aux_row0, long long ld_row) {
 #pragma unroll
         for (int i = 0; i < C::NCH_THETA; ++i) {
             const int id = i * 32 + lane;
@@ -195,7 +199,7 @@ struct TileMap {
             const int c = w / C::NL, j = (w % C::NL) + k * C::NL;
             const bool ok = c < nvalid && j < N;
             // missing rows shadow the warp's first row
-            const long long row = ok ? (sm.theta(ch0 + c) - base0) + (long long)j * sm.ld_theta : 0;
+            const long long row = ok ? (long long)(c * N + j) * ld_theta : 0;
             theta_off[i] = (unsigned)((row + col * 4) * (long long)sizeof(float));
         }
 #pragma unroll
@@ -205,8 +209,7 @@ struct TileMap {
             aux_ptr[i] = nullptr;
             if (row < C::CPW * C::AUX) {
                 const int cc = row / C::AUX, a = row % C::AUX;
-                const long long ch = ch0 + (cc < nvalid ? cc : 0);
-                aux_ptr[i] = aux_src[a] + sm.row(ch) + col * 4;
+                aux_ptr[i] = aux_src[a] + aux_row0 + (cc < nvalid ? cc : 0) * ld_row + col * 4;
             }
         }
     }
@@ -279,23 +282,18 @@ __device__ __forceinline__ void issue_words(float* stage, const float* theta_war
 // ---------------------------------------------------------------------------
 // Forward
 // ---------------------------------------------------------------------------
-// AGG: aggregate mode of the time-axis split - no output row; besides the state, the product of the segment's
-// rotations is carried (as a unit complex number, like the state itself) and returned.
 // VEC: rows are 16-byte aligned and L is a multiple of 4 (16-byte copies and vector stores).
-template <class C, bool VEC, bool NORM, bool BIAS, bool AGG>
-__device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, long long ch0, int nvalid, int lane,
+template <class C, bool VEC, bool NORM, bool BIAS>
+__device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, const WarpTask& wt, int lane,
                                          StateConsts (&sc)[C::SPT]) {
     constexpr int NL = C::NL, SPT = C::SPT, T = C::T, TP = C::TP, STAGES = C::STAGES, AUX = C::AUX, VW = C::VW;
     const int c = lane / NL, jl = lane % NL;
-    const long long ch = ch0 + c;
-    const int N = p.N, L = p.L;
+    const long long ch = wt.entry(c);
+    const int N = p.N, L = wt.L, nvalid = wt.nvalid;
     const int ntiles = (L + T - 1) / T;
-    const SegMap sm = seg_map(p);
-    const float* theta_warp = p.theta + sm.theta(ch0);
+    const float* theta_warp = p.theta + wt.ch0 * N * p.ld_theta + wt.t0;
+    const long long row0 = wt.ch0 * p.ld_row + wt.t0;           // this warp's first row of u, dt, z, y
     const float* aux_src[AUX] = {p.u, p.dt, p.z};
-    float ar[SPT], ai[SPT];     // product of the rotations so far (aggregate mode)
-#pragma unroll
-    for (int k = 0; k < SPT; ++k) { ar[k] = 1.f; ai[k] = 0.f; }
 
     float hr[SPT], hi[SPT];
 #pragma unroll
@@ -315,17 +313,17 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
 #pragma unroll
     for (int it = 0; it < C::ITERS; ++it) {
         const int cc = ((lane + 32 * it) * VW) / T;
-        dval[it] = cc < nvalid ? p.Dskip[sm.chan(ch0 + cc) % p.Dmod] : 0.f;
-        ybase[it] = sm.row(ch0 + (cc < nvalid ? cc : 0));
+        dval[it] = cc < nvalid ? p.Dskip[(wt.ch0 + cc) % p.Dmod] : 0.f;
+        ybase[it] = row0 + (cc < nvalid ? cc : 0) * p.ld_row;
     }
 
     TileMap<C> map;
-    if (VEC) map.init(lane, nvalid, N, sm, ch0, aux_src);
+    if (VEC) map.init(lane, nvalid, N, p.ld_theta, aux_src, row0, p.ld_row);
     auto fetch = [&](float* stage, const int tile) {
         const int len = min(T, L - tile * T);
         if (VEC) map.issue(stage, theta_warp, (long long)tile * T, len, lane);
-        else issue_words<C>(stage, theta_warp, p.ld_theta, aux_src, sm.row(ch0), p.ld_row, nvalid, N, (long long)tile * T,
-                            len, lane);
+        else issue_words<C>(stage, theta_warp, p.ld_theta, aux_src, row0, p.ld_row, nvalid, N, (long long)tile * T, len,
+                            lane);
     };
     for (int s = 0; s < STAGES; ++s) {
         if (s < ntiles) fetch(wsm + s * C::STAGE_FLOATS, s);
@@ -393,17 +391,11 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
                     }
                     hr[k] = nr;
                     hi[k] = ni;
-                    if (AGG) {
-                        const float qr = fmaf(cs[e], ar[k], -sn[e] * ai[k]);
-                        ai[k] = fmaf(cs[e], ai[k], sn[e] * ar[k]);
-                        ar[k] = qr;
-                    } else {
-                        pacc[e] = (k == 0) ? fmaf(sc[k].mr, nr, -sc[k].mi * ni)
-                                           : fmaf(sc[k].mr, nr, fmaf(-sc[k].mi, ni, pacc[e]));
-                    }
+                    pacc[e] = (k == 0) ? fmaf(sc[k].mr, nr, -sc[k].mi * ni)
+                                       : fmaf(sc[k].mr, nr, fmaf(-sc[k].mi, ni, pacc[e]));
                 }
             }
-            if (!AGG) st_shared_f4(th + lane * TP + 4 * q, make_float4(pacc[0], pacc[1], pacc[2], pacc[3]));
+            st_shared_f4(th + lane * TP + 4 * q, make_float4(pacc[0], pacc[1], pacc[2], pacc[3]));
         };
         if (tlen == T) {
 #pragma unroll
@@ -414,7 +406,7 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
         __syncwarp();
 
         // post-pass: one lane = one channel and VW steps
-        if (!AGG && p.y) {
+        if (p.y) {
 #pragma unroll
             for (int it = 0; it < C::ITERS; ++it) {
                 const int e0 = (lane + 32 * it) * VW;
@@ -460,24 +452,19 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, lon
             p.h1_re[ch * N + j] = orr;
             p.h1_im[ch * N + j] = oi;
         }
-        if (AGG && sc[k].act && p.agg_re) {
-            const int j = jl + k * NL;
-            p.agg_re[ch * N + j] = ar[k];
-            p.agg_im[ch * N + j] = ai[k];
-        }
     }
 }
 
-template <class C, bool VEC, bool BIAS, bool AGG>
+template <class C, bool VEC, bool BIAS>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const ScanFwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long ch0 = ((long long)blockIdx.x * C::WARPS + warp) * C::CPW;
-    if (ch0 >= p.nch) return;   // warps never meet at a block barrier
-    const int nvalid = (int)min((long long)C::CPW, (long long)p.nch - ch0);
+    WarpTask wt;
+    if (!warp_task<C::CPW>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;   // no block barriers
+    const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / C::NL, jl = lane % C::NL;
-    const int i = (int)(seg_map(p).chan(ch0 + min(c, nvalid - 1)) % p.Dmod);
+    const int i = (int)((wt.ch0 + min(c, nvalid - 1)) % p.Dmod);
     StateConsts sc[C::SPT];
     bool ok = true;
 #pragma unroll
@@ -494,9 +481,9 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const S
             float a, b;
             normalise_consts(sc[k], a, b);
         }
-        fwd_warp<C, VEC, true, BIAS, AGG>(p, wsm, ch0, nvalid, lane, sc);
+        fwd_warp<C, VEC, true, BIAS>(p, wsm, wt, lane, sc);
     } else {
-        fwd_warp<C, VEC, false, BIAS, AGG>(p, wsm, ch0, nvalid, lane, sc);
+        fwd_warp<C, VEC, false, BIAS>(p, wsm, wt, lane, sc);
     }
 }
 
@@ -504,18 +491,18 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const S
 // Backward
 // ---------------------------------------------------------------------------
 template <class C, bool VEC, bool NORM, bool BIAS>
-__device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, long long ch0, int nvalid, int lane,
+__device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, const WarpTask& wt, int lane,
                                          StateConsts (&sc)[C::SPT], const float (&ccr)[C::SPT],
                                          const float (&cci)[C::SPT]) {
     constexpr int NL = C::NL, SPT = C::SPT, T = C::T, TS = C::TS, TP = C::TP, TSP = C::TSP, STAGES = C::STAGES,
                   AUX = C::AUX, VW = C::VW;
     const int c = lane / NL, jl = lane % NL;
-    const long long ch = ch0 + c;
-    const int N = p.N, L = p.L;
+    const long long ch = wt.entry(c);
+    const int N = p.N, L = wt.L, nvalid = wt.nvalid;
     const int ntiles = (L + T - 1) / T;
-    const SegMap sm = seg_map(p);
-    const float* theta_warp = p.theta + sm.theta(ch0);
-    float* dtheta_warp = p.dtheta + sm.theta(ch0);              // launcher guarantees equal pitches
+    const float* theta_warp = p.theta + wt.ch0 * N * p.ld_theta + wt.t0;
+    float* dtheta_warp = p.dtheta + wt.ch0 * N * p.ld_theta + wt.t0;      // launcher guarantees equal pitches
+    const long long row0 = wt.ch0 * p.ld_row + wt.t0;
 
     float* scratch = wsm + STAGES * C::STAGE_FLOATS;
     float* pt = scratch;                    // [32][TSP] projections, summed over a thread's states
@@ -555,20 +542,20 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
 #pragma unroll
     for (int it = 0; it < C::ITERS; ++it) {
         const int cc = ((lane + 32 * it) * VW) / TS;
-        dval[it] = cc < nvalid ? p.Dskip[sm.chan(ch0 + cc) % p.Dmod] : 0.f;
+        dval[it] = cc < nvalid ? p.Dskip[(wt.ch0 + cc) % p.Dmod] : 0.f;
         dacc[it] = 0.f;
-        obase[it] = sm.row(ch0 + (cc < nvalid ? cc : 0));
+        obase[it] = row0 + (cc < nvalid ? cc : 0) * p.ld_row;
     }
     const float* aux_src[AUX] = {p.u, p.dt, p.z, p.gy};
 
     // r counts tiles in processing order (last tile first)
     TileMap<C> map;
-    if (VEC) map.init(lane, nvalid, N, sm, ch0, aux_src);
+    if (VEC) map.init(lane, nvalid, N, p.ld_theta, aux_src, row0, p.ld_row);
     auto fetch = [&](float* stage, const int tile) {
         const int len = min(T, L - tile * T);
         if (VEC) map.issue(stage, theta_warp, (long long)tile * T, len, lane);
-        else issue_words<C>(stage, theta_warp, p.ld_theta, aux_src, sm.row(ch0), p.ld_row, nvalid, N, (long long)tile * T,
-                            len, lane);
+        else issue_words<C>(stage, theta_warp, p.ld_theta, aux_src, row0, p.ld_row, nvalid, N, (long long)tile * T, len,
+                            lane);
     };
     for (int r = 0; r < STAGES; ++r) {
         if (r < ntiles) fetch(wsm + r * C::STAGE_FLOATS, ntiles - 1 - r);
@@ -778,7 +765,8 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
     for (int k = 0; k < SPT; ++k) {
         if (!sc[k].act) continue;
         const int j = jl + k * NL;
-        const long long o = ch * N + j;
+        const long long o = ch * N + j;                                          // states and their gradients
+        const long long po = ((wt.ch0 + c) * p.part_nseg + wt.seg) * N + j;      // partial sums
         float dbr, dbi, dcr, dci, d0r, d0i, s0r, s0i;
         if (NORM) {
             const float kr = sc[k].kr, ki = sc[k].ki;
@@ -798,13 +786,13 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
             dcr = gmr[k]; dci = gmi[k]; dbr = sbr[k]; dbi = sbi[k];
             d0r = er[k]; d0i = ei[k]; s0r = hr[k]; s0i = hi[k];
         }
-        float4* pb = reinterpret_cast<float4*>(p.part_bc) + o;
+        float4* pb = reinterpret_cast<float4*>(p.part_bc) + po;
         if (p.accumulate) {
             const float4 old = *pb;
             dbr += old.x; dbi += old.y; dcr += old.z; dci += old.w;
         }
         *pb = make_float4(dbr, dbi, dcr, dci);
-        if (BIAS && p.part_rowsum) p.part_rowsum[o] = rsum[k] + (p.accumulate ? p.part_rowsum[o] : 0.f);
+        if (BIAS && p.part_rowsum) p.part_rowsum[po] = rsum[k] + (p.accumulate ? p.part_rowsum[po] : 0.f);
         if (p.dh0_re) { p.dh0_re[o] = d0r; p.dh0_im[o] = d0i; }
         if (p.h0_re) { p.h0_re[o] = s0r; p.h0_im[o] = s0i; }
     }
@@ -823,7 +811,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, lon
         float acc = 0.f;
         for (int idx = 0; idx < 32 * C::ITERS; ++idx)
             if ((idx * VW) / TS == lane) acc += pt[idx];
-        const long long o = ch0 + lane;
+        const long long o = (wt.ch0 + lane) * p.part_nseg + wt.seg;
         p.part_d[o] = acc + (p.accumulate ? p.part_d[o] : 0.f);
     }
 }
@@ -832,12 +820,12 @@ template <class C, bool VEC, bool BIAS>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const ScanBwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long ch0 = ((long long)blockIdx.x * C::WARPS + warp) * C::CPW;
-    if (ch0 >= p.nch) return;
-    const int nvalid = (int)min((long long)C::CPW, (long long)p.nch - ch0);
+    WarpTask wt;
+    if (!warp_task<C::CPW>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;
+    const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / C::NL, jl = lane % C::NL;
-    const int i = (int)(seg_map(p).chan(ch0 + min(c, nvalid - 1)) % p.Dmod);
+    const int i = (int)((wt.ch0 + min(c, nvalid - 1)) % p.Dmod);
     StateConsts sc[C::SPT];
     float ccr[C::SPT], cci[C::SPT];
     bool ok = true;
@@ -854,32 +842,34 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const S
     if (__all_sync(0xffffffffu, ok)) {
 #pragma unroll
         for (int k = 0; k < C::SPT; ++k) normalise_consts(sc[k], ccr[k], cci[k]);
-        bwd_warp<C, VEC, true, BIAS>(p, wsm, ch0, nvalid, lane, sc, ccr, cci);
+        bwd_warp<C, VEC, true, BIAS>(p, wsm, wt, lane, sc, ccr, cci);
     } else {
-        bwd_warp<C, VEC, false, BIAS>(p, wsm, ch0, nvalid, lane, sc, ccr, cci);
+        bwd_warp<C, VEC, false, BIAS>(p, wsm, wt, lane, sc, ccr, cci);
     }
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint-only reverse pass (time-axis split): for every (virtual) channel the gradient that the segment's own
-// grad_y sends to the state before the segment, from a zero gradient after it:
-//     e <- conj(lambda_t) (e + conj(Cc) w_t),  t = L-1 .. 0,   w_t = gy_t silu(z_t)
-// (general representation, no state regeneration, nothing else produced).
+// Segment summary of the time-axis split: what a segment does to the state and to the adjoint, from its inputs alone.
+// With a_t the product of the segment's rotations up to step t (|a_t| = 1, so conj(a_t) is its inverse)
+//     end state from zero          e = a_end Bc sum_t conj(a_t) s_t
+//     gradient sent to its start   l = conj(Cc) sum_t conj(a_t) w_t          (BWD; w_t = gy_t silu(z_t))
+// so one forward walk gives a_end and both sums: 8 multiply-adds per step after the sine and cosine, against two
+// walks over theta (aggregate and adjoint) before.  Bound by the FP32 pipe and the loads' latency about equally: 1023 us
+// for the two passes of B1 D512 N16 L65536 (2 x 2.1 GB of phases, 0.62 of the copy bandwidth), where the two aggregate
+// passes and the adjoint pass took 1710 us.
 // ---------------------------------------------------------------------------
-template <class C, bool BIAS>
-__global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_eta_kernel(const ScanBwdParams p) {
+template <class C, bool VEC, bool BIAS, bool BWD>
+__global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_summary_kernel(const SegSummaryParams p) {
     constexpr int NL = C::NL, SPT = C::SPT, T = C::T, TP = C::TP, STAGES = C::STAGES, AUX = C::AUX, VW = C::VW;
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long ch0 = ((long long)blockIdx.x * C::WARPS + warp) * C::CPW;
-    if (ch0 >= p.nch) return;
-    const int nvalid = (int)min((long long)C::CPW, (long long)p.nch - ch0);
+    WarpTask wt;
+    if (!warp_task<C::CPW>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;
+    const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / NL, jl = lane % NL;
-    const SegMap sm = seg_map(p);
-    const int i = (int)(sm.chan(ch0 + min(c, nvalid - 1)) % p.Dmod);
-    const long long ch = ch0 + c;
-    const int N = p.N, L = p.L;
+    const int i = (int)((wt.ch0 + min(c, nvalid - 1)) % p.Dmod);
+    const int N = p.N, L = wt.L;
     const int ntiles = (L + T - 1) / T;
     StateConsts sc[SPT];
 #pragma unroll
@@ -888,44 +878,66 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_eta_kernel(const S
         load_state_consts(sc[k], c < nvalid && jl + k * NL < N, jl + k * NL, i, N, p.B_r, p.B_theta, p.C_r, p.C_theta,
                           BIAS ? p.theta_bias : nullptr, okk);      // mr, mi hold Cc
     }
-    const float* theta_warp = p.theta + sm.theta(ch0);
-    const float* aux_src[AUX] = {p.u, p.dt, p.z, p.gy};
-    float er[SPT], ei[SPT];
+    const float* theta_warp = p.theta + wt.ch0 * N * p.ld_theta + wt.t0;
+    const long long row0 = wt.ch0 * p.ld_row + wt.t0;
+    const float* aux_src[4] = {p.u, p.dt, p.z, p.gy};
+    float ar[SPT], ai[SPT], hr[SPT], hi[SPT], gr[SPT], gi[SPT];
 #pragma unroll
-    for (int k = 0; k < SPT; ++k) er[k] = ei[k] = 0.f;
+    for (int k = 0; k < SPT; ++k) {
+        ar[k] = 1.f;
+        ai[k] = hr[k] = hi[k] = gr[k] = gi[k] = 0.f;
+    }
     TileMap<C> map;
-    map.init(lane, nvalid, N, sm, ch0, aux_src);
-    for (int r = 0; r < STAGES; ++r) {
-        const int tile = ntiles - 1 - r;
-        if (tile >= 0) map.issue(wsm + r * C::STAGE_FLOATS, theta_warp, (long long)tile * T, min(T, L - tile * T), lane);
+    if (VEC) map.init(lane, nvalid, N, p.ld_theta, aux_src, row0, p.ld_row);
+    auto fetch = [&](float* stage, const int tile) {
+        const int len = min(T, L - tile * T);
+        if (VEC) map.issue(stage, theta_warp, (long long)tile * T, len, lane);
+        else issue_words<C>(stage, theta_warp, p.ld_theta, aux_src, row0, p.ld_row, nvalid, N, (long long)tile * T, len,
+                            lane);
+    };
+    for (int s = 0; s < STAGES; ++s) {
+        if (s < ntiles) fetch(wsm + s * C::STAGE_FLOATS, s);
         else cp_async_commit();
     }
-    for (int r = 0; r < ntiles; ++r) {
-        const int tile = ntiles - 1 - r;
-        float* th = wsm + (r % STAGES) * C::STAGE_FLOATS;
+    for (int tile = 0; tile < ntiles; ++tile) {
+        float* th = wsm + (tile % STAGES) * C::STAGE_FLOATS;
         float* aux = th + C::NROWS * TP;
         const int tlen = min(T, L - tile * T);
+        // conj(a) stands for 1/a below: bring |a| back to 1 (one Newton step; 32 roundings move it by about 1e-6)
+#pragma unroll
+        for (int k = 0; k < SPT; ++k) {
+            const float r = fmaf(-0.5f, fmaf(ar[k], ar[k], ai[k] * ai[k]), 1.5f);
+            ar[k] *= r;
+            ai[k] *= r;
+        }
         cp_async_wait<STAGES - 1>();
         __syncwarp();
-        // pre-pass: w = gy silu(z) replaces gy
+        // pre-pass: s = dt silu(u) replaces dt, w = gy silu(z) replaces gy
 #pragma unroll
         for (int it = 0; it < C::ITERS; ++it) {
             const int e0 = (lane + 32 * it) * VW;
             const int cc = e0 / T, t = e0 % T;
             if (t < tlen) {
-                Vec<VW> z, g;
-                z.ld(aux + (cc * AUX + 2) * T + t);
-                g.ld(aux + (cc * AUX + 3) * T + t);
+                Vec<VW> a, b;
+                a.ld(aux + (cc * AUX + 0) * T + t);
+                b.ld(aux + (cc * AUX + 1) * T + t);
 #pragma unroll
-                for (int e = 0; e < VW; ++e) g.v[e] *= siluf_(z.v[e]);
-                g.st(aux + (cc * AUX + 3) * T + t);
+                for (int e = 0; e < VW; ++e) b.v[e] *= siluf_(a.v[e]);
+                b.st(aux + (cc * AUX + 1) * T + t);
+                if (BWD) {
+                    a.ld(aux + (cc * AUX + 2) * T + t);
+                    b.ld(aux + (cc * AUX + 3) * T + t);
+#pragma unroll
+                    for (int e = 0; e < VW; ++e) b.v[e] *= siluf_(a.v[e]);
+                    b.st(aux + (cc * AUX + 3) * T + t);
+                }
             }
         }
         __syncwarp();
-        const float* wrow = aux + (c * AUX + 3) * T;
-        for (int q = (tlen >> 2) - 1; q >= 0; --q) {
-            const float4 w4 = ld_shared_f4(wrow + 4 * q);
-            const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
+        auto quad = [&](const int q, auto whole) {
+            const float4 s4 = ld_shared_f4(aux + (c * AUX + 1) * T + 4 * q);
+            const float4 w4 = BWD ? ld_shared_f4(aux + (c * AUX + 3) * T + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float sv[4] = {s4.x, s4.y, s4.z, s4.w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
             for (int k = 0; k < SPT; ++k) {
                 const float4 t4 = ld_shared_f4(th + (k * 32 + lane) * TP + 4 * q);
@@ -937,99 +949,111 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_eta_kernel(const S
                 float sn[4], cs[4];
                 sincos4(tv, sn, cs);
 #pragma unroll
-                for (int e = 3; e >= 0; --e) {
-                    const float nr = fmaf(sc[k].mr, wv[e], er[k]);
-                    const float ni = fmaf(-sc[k].mi, wv[e], ei[k]);
-                    er[k] = fmaf(cs[e], nr, sn[e] * ni);
-                    ei[k] = fmaf(cs[e], ni, -sn[e] * nr);
+                for (int e = 0; e < 4; ++e) {
+                    if (!VEC && !whole.value && 4 * q + e >= tlen) continue;           // ragged tail
+                    const float nr = fmaf(cs[e], ar[k], -sn[e] * ai[k]);
+                    ai[k] = fmaf(cs[e], ai[k], sn[e] * ar[k]);
+                    ar[k] = nr;
+                    hr[k] = fmaf(ar[k], sv[e], hr[k]);
+                    hi[k] = fmaf(-ai[k], sv[e], hi[k]);
+                    if (BWD) {
+                        gr[k] = fmaf(ar[k], wv[e], gr[k]);
+                        gi[k] = fmaf(-ai[k], wv[e], gi[k]);
+                    }
                 }
             }
+        };
+        if (tlen == T) {
+#pragma unroll
+            for (int q = 0; q < T / 4; ++q) quad(q, std::true_type{});
+        } else {
+            for (int q = 0; q < (tlen + 3) >> 2; ++q) quad(q, std::false_type{});
         }
         __syncwarp();
-        const int nr2 = r + STAGES;
-        if (nr2 < ntiles) {
-            const int nt = ntiles - 1 - nr2;
-            map.issue(th, theta_warp, (long long)nt * T, min(T, L - nt * T), lane);
-        } else {
-            cp_async_commit();
-        }
+        if (tile + STAGES < ntiles) fetch(th, tile + STAGES);
+        else cp_async_commit();
     }
     cp_async_wait<0>();
 #pragma unroll
     for (int k = 0; k < SPT; ++k) {
-        if (sc[k].act) {
-            const long long o = ch * N + jl + k * NL;
-            p.dh0_re[o] = er[k];
-            p.dh0_im[o] = ei[k];
+        if (!sc[k].act) continue;
+        const long long o = wt.entry(c) * N + jl + k * NL;
+        p.a_re[o] = ar[k];
+        p.a_im[o] = ai[k];
+        const float br = sc[k].br * hr[k] - sc[k].bi * hi[k], bi = sc[k].br * hi[k] + sc[k].bi * hr[k];
+        p.e_re[o] = ar[k] * br - ai[k] * bi;
+        p.e_im[o] = ar[k] * bi + ai[k] * br;
+        if (BWD) {
+            p.l_re[o] = sc[k].mr * gr[k] + sc[k].mi * gi[k];
+            p.l_im[o] = sc[k].mr * gi[k] - sc[k].mi * gr[k];
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// Segment chains of the time-axis split: one thread per (channel, state) walks the nseg segments.
+// Segment chains of the time-axis split: one thread per (channel, state) walks the nseg segments.  The loads do not
+// depend on the chain, so a few segments of them are in flight.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) segment_states_fwd_kernel(const float* e_re, const float* e_im,
-                                                                 const float* a_re, const float* a_im,
-                                                                 const float* start_re, const float* start_im,
-                                                                 float* before_re, float* before_im, float* final_re,
-                                                                 float* final_im, long long total, int nseg, int N) {
-    const long long id = (long long)blockIdx.x * 256 + threadIdx.x;      // ch * N + j
-    if (id >= total) return;
-    const long long ch = id / N, j = id % N;
-    float cr = start_re ? start_re[id] : 0.f, ci = start_im ? start_im[id] : 0.f;
-    for (int s = 0; s < nseg; ++s) {
-        const long long o = (ch * nseg + s) * N + j;
-        before_re[o] = cr;
-        before_im[o] = ci;
-        const float ar = a_re[o], ai = a_im[o];
-        const float nr = fmaf(ar, cr, fmaf(-ai, ci, e_re[o]));
-        ci = fmaf(ar, ci, fmaf(ai, cr, e_im[o]));
+struct SegChainParams {
+    const float *e_re, *e_im, *a_re, *a_im;
+    const float *l_re, *l_im;           // backward
+    const float *from_re, *from_im;     // forward: state before segment 0 (or nullptr = 0); backward: the final state
+    const float *gh_re, *gh_im;         // backward: gradient of the final state, or nullptr
+    float *at_re, *at_im;               // forward: state before every segment; backward: state after it
+    float *g_re, *g_im;                 // backward: gradient of the state after every segment
+    float *end_re, *end_im;             // forward: final state; backward: state before segment 0 (or nullptr)
+    float *dh0_re, *dh0_im;             // backward: gradient of that state (or nullptr)
+    long long total;
+    int nseg, N;
+};
+
+__global__ void __launch_bounds__(128) segment_states_fwd_kernel(const SegChainParams p) {
+    const long long id = (long long)blockIdx.x * 128 + threadIdx.x;      // ch * N + j
+    if (id >= p.total) return;
+    const float *__restrict__ e_re = p.e_re, *__restrict__ e_im = p.e_im;
+    const float *__restrict__ a_re = p.a_re, *__restrict__ a_im = p.a_im;
+    float *__restrict__ at_re = p.at_re, *__restrict__ at_im = p.at_im;
+    float cr = p.from_re ? p.from_re[id] : 0.f, ci = p.from_im ? p.from_im[id] : 0.f;
+    long long o = (id / p.N) * p.nseg * p.N + id % p.N;
+#pragma unroll 4
+    for (int s = 0; s < p.nseg; ++s, o += p.N) {
+        const float ar = a_re[o], ai = a_im[o], er = e_re[o], ei = e_im[o];
+        at_re[o] = cr;
+        at_im[o] = ci;
+        const float nr = fmaf(ar, cr, fmaf(-ai, ci, er));               // c_{s+1} = e_s + a_s c_s
+        ci = fmaf(ar, ci, fmaf(ai, cr, ei));
         cr = nr;
     }
-    if (final_re) { final_re[id] = cr; final_im[id] = ci; }
+    if (p.end_re) { p.end_re[id] = cr; p.end_im[id] = ci; }
 }
 
-__global__ void __launch_bounds__(256) segment_states_bwd_kernel(const float* e_re, const float* e_im,
-                                                                 const float* a_re, const float* a_im,
-                                                                 const float* final_re, const float* final_im,
-                                                                 float* after_re, float* after_im, float* first_re,
-                                                                 float* first_im, long long total, int nseg, int N) {
-    const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (id >= total) return;
-    const long long ch = id / N, j = id % N;
-    float cr = final_re[id], ci = final_im[id];
-    for (int s = nseg - 1; s >= 0; --s) {
-        const long long o = (ch * nseg + s) * N + j;
-        after_re[o] = cr;
-        after_im[o] = ci;
-        // the rotations have modulus one: the state before the segment is conj(a) (c - e)
-        const float dr = cr - e_re[o], di = ci - e_im[o];
-        const float ar = a_re[o], ai = a_im[o];
+// walking back from the final state: c_s = conj(a_s) (c_{s+1} - e_s) (|a_s| = 1) and g_s = l_s + conj(a_s) g_{s+1}
+__global__ void __launch_bounds__(128) segment_states_bwd_kernel(const SegChainParams p) {
+    const long long id = (long long)blockIdx.x * 128 + threadIdx.x;
+    if (id >= p.total) return;
+    const float *__restrict__ e_re = p.e_re, *__restrict__ e_im = p.e_im, *__restrict__ l_re = p.l_re;
+    const float *__restrict__ a_re = p.a_re, *__restrict__ a_im = p.a_im, *__restrict__ l_im = p.l_im;
+    float *__restrict__ at_re = p.at_re, *__restrict__ at_im = p.at_im;
+    float *__restrict__ g_re = p.g_re, *__restrict__ g_im = p.g_im;
+    float cr = p.from_re[id], ci = p.from_im[id];
+    float gr = p.gh_re ? p.gh_re[id] : 0.f, gi = p.gh_im ? p.gh_im[id] : 0.f;
+    long long o = ((id / p.N) * p.nseg + p.nseg - 1) * p.N + id % p.N;
+#pragma unroll 4
+    for (int s = 0; s < p.nseg; ++s, o -= p.N) {
+        const float ar = a_re[o], ai = a_im[o], er = e_re[o], ei = e_im[o], lr = l_re[o], li = l_im[o];
+        at_re[o] = cr;
+        at_im[o] = ci;
+        g_re[o] = gr;
+        g_im[o] = gi;
+        const float dr = cr - er, di = ci - ei;
         cr = fmaf(ar, dr, ai * di);
         ci = fmaf(ar, di, -ai * dr);
-    }
-    if (first_re) { first_re[id] = cr; first_im[id] = ci; }
-}
-
-__global__ void __launch_bounds__(256) segment_adjoints_kernel(const float* l_re, const float* l_im, const float* a_re,
-                                                               const float* a_im, const float* last_re,
-                                                               const float* last_im, float* after_re, float* after_im,
-                                                               float* first_re, float* first_im, long long total,
-                                                               int nseg, int N) {
-    const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (id >= total) return;
-    const long long ch = id / N, j = id % N;
-    float gr = last_re ? last_re[id] : 0.f, gi = last_im ? last_im[id] : 0.f;
-    for (int s = nseg - 1; s >= 0; --s) {
-        const long long o = (ch * nseg + s) * N + j;
-        after_re[o] = gr;
-        after_im[o] = gi;
-        const float ar = a_re[o], ai = a_im[o];
-        const float nr = fmaf(ar, gr, fmaf(ai, gi, l_re[o]));          // l + conj(a) g
-        gi = fmaf(ar, gi, fmaf(-ai, gr, l_im[o]));
+        const float nr = fmaf(ar, gr, fmaf(ai, gi, lr));
+        gi = fmaf(ar, gi, fmaf(-ai, gr, li));
         gr = nr;
     }
-    if (first_re) { first_re[id] = gr; first_im[id] = gi; }
+    if (p.end_re) { p.end_re[id] = cr; p.end_im[id] = ci; }
+    if (p.dh0_re) { p.dh0_re[id] = gr; p.dh0_im[id] = gi; }
 }
 
 // ---------------------------------------------------------------------------
@@ -1093,14 +1117,19 @@ __global__ void __launch_bounds__(256) reduce_param_grads_kernel(const ReducePar
 // ---------------------------------------------------------------------------
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <class C, bool VEC, bool BIAS, bool AGG>
+// warp tasks of a launch: channel groups times segments
+template <class C, class P>
+long long warp_tasks(const P& p) {
+    return (((long long)p.nch + C::CPW - 1) / C::CPW) * (p.nseg > 1 ? p.nseg : 1);
+}
+
+template <class C, bool VEC, bool BIAS>
 cudaError_t launch_fwd_cfg(const ScanFwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_fwd_kernel<C, VEC, BIAS, AGG>;
+    auto kern = scan_unitary_fwd_kernel<C, VEC, BIAS>;
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const long long tasks = ((long long)p.nch + C::CPW - 1) / C::CPW;
-    const long long blocks = (tasks + C::WARPS - 1) / C::WARPS;
+    const long long blocks = (warp_tasks<C>(p) + C::WARPS - 1) / C::WARPS;
     kern<<<(unsigned)blocks, C::WARPS * 32, smem, stream>>>(p);
     count_launch();
     return cudaGetLastError();
@@ -1112,8 +1141,7 @@ cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const long long tasks = ((long long)p.nch + C::CPW - 1) / C::CPW;
-    const long long blocks = (tasks + C::WARPS - 1) / C::WARPS;
+    const long long blocks = (warp_tasks<C>(p) + C::WARPS - 1) / C::WARPS;
     kern<<<(unsigned)blocks, C::WARPS * 32, smem, stream>>>(p);
     count_launch();
     return cudaGetLastError();
@@ -1123,34 +1151,35 @@ cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
 // offset always on, to keep the build small.
 template <class C>
 cudaError_t launch_fwd_sel(const ScanFwdParams& p, bool vec, cudaStream_t s) {
-    const bool bias = p.theta_bias != nullptr;
-    if (!vec) return p.nseg > 1 || p.agg_re ? cudaErrorInvalidValue : launch_fwd_cfg<C, false, true, false>(p, s);
-    if (p.agg_re != nullptr && p.y == nullptr)
-        return bias ? launch_fwd_cfg<C, true, true, true>(p, s) : launch_fwd_cfg<C, true, false, true>(p, s);
-    return bias ? launch_fwd_cfg<C, true, true, false>(p, s) : launch_fwd_cfg<C, true, false, false>(p, s);
+    if (!vec) return launch_fwd_cfg<C, false, true>(p, s);
+    return p.theta_bias != nullptr ? launch_fwd_cfg<C, true, true>(p, s) : launch_fwd_cfg<C, true, false>(p, s);
 }
 
-template <class C, bool BIAS>
-cudaError_t launch_eta_cfg(const ScanBwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_eta_kernel<C, BIAS>;
+template <class C>
+cudaError_t launch_bwd_sel(const ScanBwdParams& p, bool vec, cudaStream_t s) {
+    const bool bias = p.theta_bias != nullptr || p.part_rowsum != nullptr;
+    if (!vec) return launch_bwd_cfg<C, false, true>(p, s);
+    return bias ? launch_bwd_cfg<C, true, true>(p, s) : launch_bwd_cfg<C, true, false>(p, s);
+}
+
+template <class C, bool VEC, bool BIAS, bool BWD>
+cudaError_t launch_summary_cfg(const SegSummaryParams& p, cudaStream_t stream) {
+    auto kern = scan_unitary_summary_kernel<C, VEC, BIAS, BWD>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    const long long tasks = ((long long)p.nch + C::CPW - 1) / C::CPW;
-    const long long blocks = (tasks + C::WARPS - 1) / C::WARPS;
+    const long long blocks = (warp_tasks<C>(p) + C::WARPS - 1) / C::WARPS;
     kern<<<(unsigned)blocks, C::WARPS * 32, C::SMEM_BYTES, stream>>>(p);
     count_launch();
     return cudaGetLastError();
 }
 
-// the adjoint-only pass stages (u, dt, z, gy) like the backward kernel but keeps no column-sum tiles
+// the summary pass stages (u, dt) or (u, dt, z, gy) and keeps no column-sum tiles
 template <int NL, int SPT, int T, int STAGES, int WARPS>
-using EtaCfg = Cfg<NL, SPT, T, T, STAGES, WARPS, 4, false>;
-
-template <class C>
-cudaError_t launch_bwd_sel(const ScanBwdParams& p, bool vec, cudaStream_t s) {
-    const bool bias = p.theta_bias != nullptr || p.part_rowsum != nullptr;
-    if (!vec) return p.nseg > 1 ? cudaErrorInvalidValue : launch_bwd_cfg<C, false, true>(p, s);
-    return bias ? launch_bwd_cfg<C, true, true>(p, s) : launch_bwd_cfg<C, true, false>(p, s);
+cudaError_t launch_summary_sel(const SegSummaryParams& p, bool vec, cudaStream_t s) {
+    using F = Cfg<NL, SPT, T, T, STAGES, WARPS, 2, false>;
+    using B = Cfg<NL, SPT, T, T, STAGES, WARPS, 4, false>;
+    if (p.gy) return vec ? launch_summary_cfg<B, true, true, true>(p, s) : launch_summary_cfg<B, false, true, true>(p, s);
+    return vec ? launch_summary_cfg<F, true, true, false>(p, s) : launch_summary_cfg<F, false, true, false>(p, s);
 }
 
 // a warp's rows must be addressable with 32-bit byte offsets from its first row
@@ -1184,24 +1213,12 @@ cudaError_t launch_scan_unitary_bwd(const ScanBwdParams& p_, cudaStream_t stream
     p.status = device_status_ptr();
     if (!p.status) return cudaErrorInvalidSymbol;
     if (p.ld_dtheta != p.ld_theta) return cudaErrorInvalidValue;
+    if (p.part_nseg <= 0) p.part_nseg = p.nseg > 1 ? p.nseg : 1;
     const bool vec = (p.L % 4 == 0) && (p.ld_theta % 4 == 0) && (p.ld_row % 4 == 0) && aligned16(p.theta) &&
                        aligned16(p.dtheta) && aligned16(p.u) && aligned16(p.dt) && aligned16(p.z) &&
                        aligned16(p.gy) && aligned16(p.du) && aligned16(p.ddt) && aligned16(p.dz) &&
                        offsets_fit(p.ld_theta, 128);
     const int N = p.N;
-    if (p.eta_only) {
-        if (!vec || !p.dh0_re) return cudaErrorInvalidValue;
-        const bool bias = p.theta_bias != nullptr;
-#define AUSSM_ETA(...) (bias ? launch_eta_cfg<__VA_ARGS__, true>(p, stream) : launch_eta_cfg<__VA_ARGS__, false>(p, stream))
-        if (N <= 4) return AUSSM_ETA(EtaCfg<4, 1, 32, 2, 4>);
-        if (N <= 8) return AUSSM_ETA(EtaCfg<8, 1, 32, 2, 4>);
-        if (N <= 16) return AUSSM_ETA(EtaCfg<16, 1, 32, 2, 4>);
-        if (N <= 32) return AUSSM_ETA(EtaCfg<32, 1, 32, 2, 4>);
-        if (N <= 64) return AUSSM_ETA(EtaCfg<32, 2, 32, 2, 4>);
-        if (N <= 128) return AUSSM_ETA(EtaCfg<32, 4, 32, 2, 2>);
-#undef AUSSM_ETA
-        return cudaErrorInvalidValue;
-    }
     if (N <= 4) return launch_bwd_sel<BwdCfg<4, 1, 32, 32, 2, 2>>(p, vec, stream);
     if (N <= 8) return launch_bwd_sel<BwdCfg<8, 1, 32, 32, 2, 2>>(p, vec, stream);
     // one-warp blocks: a finished warp is replaced at once (measured 9.55 ms against 10.2 ms with two-warp blocks)
@@ -1212,123 +1229,116 @@ cudaError_t launch_scan_unitary_bwd(const ScanBwdParams& p_, cudaStream_t stream
     return cudaErrorInvalidValue;
 }
 
-int scan_split_segments(long long nch, int N, int L, bool bwd) {
-    if (nch <= 0 || L <= 0 || N <= 0 || N > 128 || !time_split_option()) return 1;
-    // warps the launch has and warps the GPU holds (148 SMs; 20 resident forward warps per SM, 10 backward:
-    // shared memory limits both)
-    const int nl = N <= 4 ? 4 : N <= 8 ? 8 : N <= 16 ? 16 : 32;
-    const long long warps = (nch + (32 / nl) - 1) / (32 / nl);
-    const long long slots = 148LL * (bwd ? 10 : 20);
-    // a split doubles the work (an aggregate pass before the real one), and an SM with a third of its warps
-    // resident is already more than half busy, so it pays only when the launch fills less than a quarter
-    if (warps * 4 > slots) return 1;
-    int best = 1;
-    for (int s = 2; s <= 64; s *= 2) {
-        if (L % s != 0 || (L / s) % 32 != 0 || L / s < 256) break;
-        best = s;
-        if (warps * s >= slots) break;
-    }
-    return best;
+namespace {
+cudaError_t launch_summary(const SegSummaryParams& p, cudaStream_t stream) {
+    const bool vec = (p.L % 4 == 0) && (p.ld_theta % 4 == 0) && (p.ld_row % 4 == 0) && aligned16(p.theta) &&
+                     aligned16(p.u) && aligned16(p.dt) && (!p.gy || (aligned16(p.z) && aligned16(p.gy))) &&
+                     offsets_fit(p.ld_theta, 128);
+    if (p.N <= 4) return launch_summary_sel<4, 1, 32, 2, 4>(p, vec, stream);
+    if (p.N <= 8) return launch_summary_sel<8, 1, 32, 2, 4>(p, vec, stream);
+    if (p.N <= 16) return launch_summary_sel<16, 1, 32, 2, 4>(p, vec, stream);
+    if (p.N <= 32) return launch_summary_sel<32, 1, 32, 2, 4>(p, vec, stream);
+    if (p.N <= 64) return launch_summary_sel<32, 2, 32, 2, 4>(p, vec, stream);
+    if (p.N <= 128) return launch_summary_sel<32, 4, 32, 2, 2>(p, vec, stream);
+    return cudaErrorInvalidValue;
 }
 
-namespace {
-unsigned seg_blocks(long long total) { return (unsigned)((total + 255) / 256); }
+unsigned chain_blocks(long long total) { return (unsigned)((total + 127) / 128); }
+
+// warps of a kernel that an SM holds: shared memory limits them (228 KB, 1 KB of it per block reserved)
+template <class C>
+constexpr long long warps_per_sm() {
+    return (228 * 1024 / (long long)(C::SMEM_BYTES + 1024)) * C::WARPS;
+}
 }  // namespace
 
-cudaError_t launch_segment_states_fwd(const float* e_re, const float* e_im, const float* a_re, const float* a_im,
-                                      const float* start_re, const float* start_im, float* before_re,
-                                      float* before_im, float* final_re, float* final_im, long long nch, int nseg,
-                                      int N, cudaStream_t stream) {
-    const long long total = nch * N;
-    segment_states_fwd_kernel<<<seg_blocks(total), 256, 0, stream>>>(e_re, e_im, a_re, a_im, start_re, start_im,
-                                                                      before_re, before_im, final_re, final_im, total,
-                                                                      nseg, N);
-    count_launch();
-    return cudaGetLastError();
+SegPlan scan_split_plan(long long nch, int N, int L, bool bwd) {
+    SegPlan plan = {1, L};
+    if (nch <= 0 || L <= 0 || N <= 0 || N > 128 || !time_split_option()) return plan;
+    const int nl = N <= 4 ? 4 : N <= 8 ? 8 : N <= 16 ? 16 : 32;
+    const long long warps = (nch + (32 / nl) - 1) / (32 / nl);
+    long long per_sm = 0;
+#define AUSSM_SLOTS(FWD, BWD) per_sm = bwd ? warps_per_sm<BWD>() : warps_per_sm<FWD>()
+    using F4 = FwdCfg<4, 1, 32, 2, 4>; using B4 = BwdCfg<4, 1, 32, 32, 2, 2>;
+    using F8 = FwdCfg<8, 1, 32, 2, 4>; using B8 = BwdCfg<8, 1, 32, 32, 2, 2>;
+    using F16 = FwdCfg<16, 1, 32, 2, 4>; using B16 = BwdCfg<16, 1, 32, 32, 2, 1>;
+    using F32 = FwdCfg<32, 1, 32, 2, 4>; using B32 = BwdCfg<32, 1, 32, 32, 2, 2>;
+    using F64 = FwdCfg<32, 2, 32, 2, 4>; using B64 = BwdCfg<32, 2, 32, 32, 2, 2>;
+    using F128 = FwdCfg<32, 4, 32, 2, 2>; using B128 = BwdCfg<32, 4, 32, 32, 2, 2>;
+    if (N <= 4) AUSSM_SLOTS(F4, B4);
+    else if (N <= 8) AUSSM_SLOTS(F8, B8);
+    else if (N <= 16) AUSSM_SLOTS(F16, B16);
+    else if (N <= 32) AUSSM_SLOTS(F32, B32);
+    else if (N <= 64) AUSSM_SLOTS(F64, B64);
+    else AUSSM_SLOTS(F128, B128);
+#undef AUSSM_SLOTS
+    // A split doubles the work (a summary pass before the real one), and an SM with a third of its warps resident is
+    // already more than half busy, so it pays only when the launch fills less than a quarter.  As many segments as
+    // fill a wave, and 32 of at least 256 steps where that is more: several waves of short segments keep the SMs
+    // evenly busy to the end.  N = 16, 256 warps, L = 16384, forward + backward (device time): 1535 us whole, 850 with
+    // 11 / 5 segments (one wave), 765 with 11, 738 with 16, 734 with 32, 772 with 64, 866 with 128; L = 65536: 3233 us
+    // with 11 / 5, 2648 with 64; L = 3000 (150 warps): 292 whole, 131 with 11, 149 with 64.  Below 1024 steps a call is
+    // bound by the host and two more launches cost more than the shorter chains save (B1 D64 L600: 204 us whole, 224
+    // split).
+    const long long slots = 148 * per_sm;
+    if (warps * 4 > slots) return plan;
+    const long long want = std::min<long long>(std::max<long long>(slots / warps, std::min(32, L / 256)), L / 128);
+    if (want < 8) return plan;
+    plan.seg_len = (int)(((L + want - 1) / want + 31) / 32 * 32);
+    plan.nseg = (L + plan.seg_len - 1) / plan.seg_len;
+    return plan;
 }
 
-cudaError_t launch_segment_states_bwd(const float* e_re, const float* e_im, const float* a_re, const float* a_im,
-                                      const float* final_re, const float* final_im, float* after_re, float* after_im,
-                                      float* first_re, float* first_im, long long nch, int nseg, int N,
-                                      cudaStream_t stream) {
-    const long long total = nch * N;
-    segment_states_bwd_kernel<<<seg_blocks(total), 256, 0, stream>>>(e_re, e_im, a_re, a_im, final_re, final_im,
-                                                                      after_re, after_im, first_re, first_im, total,
-                                                                      nseg, N);
-    count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_segment_adjoints(const float* l_re, const float* l_im, const float* a_re, const float* a_im,
-                                    const float* last_re, const float* last_im, float* after_re, float* after_im,
-                                    float* first_re, float* first_im, long long nch, int nseg, int N,
-                                    cudaStream_t stream) {
-    const long long total = nch * N;
-    segment_adjoints_kernel<<<seg_blocks(total), 256, 0, stream>>>(l_re, l_im, a_re, a_im, last_re, last_im, after_re,
-                                                                    after_im, first_re, first_im, total, nseg, N);
-    count_launch();
-    return cudaGetLastError();
-}
-
-bool scan_split_allowed(const ScanFwdParams& p) {
-    return (p.L % 4 == 0) && (p.ld_theta % 4 == 0) && (p.ld_row % 4 == 0) && aligned16(p.theta) && aligned16(p.u) &&
-           aligned16(p.dt) && aligned16(p.z) && (p.y == nullptr || aligned16(p.y)) && offsets_fit(p.ld_theta, 128);
-}
-
-bool scan_split_allowed(const ScanBwdParams& p) {
-    return (p.L % 4 == 0) && (p.ld_theta % 4 == 0) && (p.ld_row % 4 == 0) && p.ld_dtheta == p.ld_theta &&
-           aligned16(p.theta) && aligned16(p.dtheta) && aligned16(p.u) && aligned16(p.dt) && aligned16(p.z) &&
-           aligned16(p.gy) && aligned16(p.du) && aligned16(p.ddt) && aligned16(p.dz) && offsets_fit(p.ld_theta, 128);
-}
-
-// Forward with the time axis cut into nseg segments per channel: (A) every segment from a zero state, without
-// output: its end state e and the product a of its rotations; (B) the chain c_{s+1} = e_s + a_s c_s gives the
-// state before every segment; (C) the real pass, every segment from its true initial state.
-cudaError_t scan_unitary_fwd_split(const ScanFwdParams& p, int nseg, float* scratch, cudaStream_t stream) {
-    const long long V = (long long)p.nch * nseg, VN = V * p.N;
+// Forward with the time axis cut into segments: (A) every segment's summary: its end state from zero, e, and the
+// product of its rotations, a; (B) the chain c_{s+1} = e_s + a_s c_s gives the state before every segment; (C) the
+// real pass, every segment from its true initial state.
+cudaError_t scan_unitary_fwd_split(const ScanFwdParams& p, const SegPlan& plan, float* scratch, cudaStream_t stream) {
+    const long long VN = (long long)p.nch * plan.nseg * p.N;
     float *e_re = scratch, *e_im = e_re + VN, *a_re = e_im + VN, *a_im = a_re + VN, *b_re = a_im + VN,
           *b_im = b_re + VN;
+    const SegSummaryParams sum = {p.theta, p.theta_bias, p.u, p.dt, nullptr, nullptr, p.B_r, p.B_theta, p.C_r, p.C_theta,
+                                  e_re, e_im, a_re, a_im, nullptr, nullptr, p.nch, p.Dmod, p.N, p.L, p.ld_theta,
+                                  p.ld_row, plan.nseg, plan.seg_len};
+    cudaError_t err = launch_summary(sum, stream);
+    if (err != cudaSuccess) return err;
+    SegChainParams c = {};
+    c.e_re = e_re; c.e_im = e_im; c.a_re = a_re; c.a_im = a_im; c.from_re = p.h0_re; c.from_im = p.h0_im;
+    c.at_re = b_re; c.at_im = b_im; c.end_re = p.h1_re; c.end_im = p.h1_im;
+    c.total = (long long)p.nch * p.N; c.nseg = plan.nseg; c.N = p.N;
+    segment_states_fwd_kernel<<<chain_blocks(c.total), 128, 0, stream>>>(c);
+    count_launch();
+    err = cudaGetLastError();
+    if (err != cudaSuccess || !p.y) return err;         // state-only call: the chain already gave the final state
     ScanFwdParams q = p;
-    q.nch = (int)V; q.L = p.L / nseg; q.nseg = nseg;
-    q.y = nullptr; q.h0_re = q.h0_im = nullptr; q.h1_re = e_re; q.h1_im = e_im; q.agg_re = a_re; q.agg_im = a_im;
-    cudaError_t err = launch_scan_unitary_fwd(q, stream);
-    if (err != cudaSuccess) return err;
-    err = launch_segment_states_fwd(e_re, e_im, a_re, a_im, p.h0_re, p.h0_im, b_re, b_im, p.h1_re, p.h1_im, p.nch, nseg,
-                                    p.N, stream);
-    if (err != cudaSuccess) return err;
-    if (!p.y) return cudaSuccess;                       // state-only call: the chain already gave the final state
-    q.y = p.y; q.h0_re = b_re; q.h0_im = b_im; q.h1_re = q.h1_im = nullptr; q.agg_re = q.agg_im = nullptr;
+    q.nseg = plan.nseg; q.seg_len = plan.seg_len;
+    q.h0_re = b_re; q.h0_im = b_im; q.h1_re = q.h1_im = nullptr;
     return launch_scan_unitary_fwd(q, stream);
 }
 
-// Backward with the same cut: (A) the forward aggregates again; (B) the state after every segment, walking
-// back from the final state (the rotations are invertible); (C) every segment's own contribution to the
-// gradient of the state before it; (D) the chain g_s = l_s + conj(a_s) g_{s+1} gives the gradient after every
-// segment; (E) the real backward pass, every segment with its true end state and incoming gradient.
-cudaError_t scan_unitary_bwd_split(const ScanBwdParams& p, int nseg, float* scratch, cudaStream_t stream) {
-    const long long V = (long long)p.nch * nseg, VN = V * p.N;
+// Backward with the same cut: (A) the summaries, now with every segment's own contribution l to the gradient of the
+// state before it; (B) one chain walks back from the final state and its gradient (the rotations are invertible);
+// (C) the real backward pass, every segment with its true end state and incoming gradient.
+cudaError_t scan_unitary_bwd_split(const ScanBwdParams& p, const SegPlan& plan, float* scratch, cudaStream_t stream) {
+    const long long VN = (long long)p.nch * plan.nseg * p.N;
     float *e_re = scratch, *e_im = e_re + VN, *a_re = e_im + VN, *a_im = a_re + VN, *s_re = a_im + VN,
           *s_im = s_re + VN, *l_re = s_im + VN, *l_im = l_re + VN, *g_re = l_im + VN, *g_im = g_re + VN;
-    ScanFwdParams f = {};
-    f.theta = p.theta; f.theta_bias = p.theta_bias; f.u = p.u; f.dt = p.dt; f.z = p.z;
-    f.B_r = p.B_r; f.B_theta = p.B_theta; f.C_r = p.C_r; f.C_theta = p.C_theta; f.Dskip = p.Dskip;
-    f.h1_re = e_re; f.h1_im = e_im; f.agg_re = a_re; f.agg_im = a_im;
-    f.nch = (int)V; f.Dmod = p.Dmod; f.N = p.N; f.L = p.L / nseg; f.ld_theta = p.ld_theta; f.ld_row = p.ld_row;
-    f.nseg = nseg;
-    cudaError_t err = launch_scan_unitary_fwd(f, stream);
+    const SegSummaryParams sum = {p.theta, p.theta_bias, p.u, p.dt, p.z, p.gy, p.B_r, p.B_theta, p.C_r, p.C_theta,
+                                  e_re, e_im, a_re, a_im, l_re, l_im, p.nch, p.Dmod, p.N, p.L, p.ld_theta, p.ld_row,
+                                  plan.nseg, plan.seg_len};
+    cudaError_t err = launch_summary(sum, stream);
     if (err != cudaSuccess) return err;
-    err = launch_segment_states_bwd(e_re, e_im, a_re, a_im, p.h1_re, p.h1_im, s_re, s_im, p.h0_re, p.h0_im, p.nch, nseg,
-                                    p.N, stream);
+    SegChainParams c = {};
+    c.e_re = e_re; c.e_im = e_im; c.a_re = a_re; c.a_im = a_im; c.l_re = l_re; c.l_im = l_im;
+    c.from_re = p.h1_re; c.from_im = p.h1_im; c.gh_re = p.gh1_re; c.gh_im = p.gh1_im;
+    c.at_re = s_re; c.at_im = s_im; c.g_re = g_re; c.g_im = g_im;
+    c.end_re = p.h0_re; c.end_im = p.h0_im; c.dh0_re = p.dh0_re; c.dh0_im = p.dh0_im;
+    c.total = (long long)p.nch * p.N; c.nseg = plan.nseg; c.N = p.N;
+    segment_states_bwd_kernel<<<chain_blocks(c.total), 128, 0, stream>>>(c);
+    count_launch();
+    err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     ScanBwdParams q = p;
-    q.nch = (int)V; q.L = p.L / nseg; q.nseg = nseg;
-    q.eta_only = 1; q.dh0_re = l_re; q.dh0_im = l_im;
-    err = launch_scan_unitary_bwd(q, stream);
-    if (err != cudaSuccess) return err;
-    err = launch_segment_adjoints(l_re, l_im, a_re, a_im, p.gh1_re, p.gh1_im, g_re, g_im, p.dh0_re, p.dh0_im, p.nch,
-                                  nseg, p.N, stream);
-    if (err != cudaSuccess) return err;
-    q.eta_only = 0;
+    q.nseg = plan.nseg; q.seg_len = plan.seg_len;
     q.h1_re = s_re; q.h1_im = s_im; q.gh1_re = g_re; q.gh1_im = g_im;
     q.dh0_re = q.dh0_im = nullptr; q.h0_re = q.h0_im = nullptr;
     return launch_scan_unitary_bwd(q, stream);

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import aussm_b200
+from aussm_b200 import _lib
 from aussm_b200.s6 import selective_scan_fn
 from oracle import unitary as O
 from oracle.s6 import selective_scan_ref
@@ -53,6 +54,16 @@ def test_scan_rows_that_start_anywhere(n, l):
     check_scan(errors, b, d, n, l)
 
 
+@pytest.mark.parametrize("shape", [(1, 3, 16, 1024), (1, 2, 5, 1029), (2, 5, 4, 1533), (1, 2, 33, 1280),
+                                   (1, 1, 128, 1100), (1, 1, 1, 2047), (3, 7, 10, 1027)])
+def test_scan_cut_into_unequal_segments(shape):
+    """Few channels: as many segments as a wave holds, the last one what is left, at any length and alignment."""
+    assert _lib.load().aussm_b200_scan_unitary_fwd_workspace_bytes(*shape) > 0, "this shape should be split"
+    errors = scan_errors(*shape, 2000 + sum(shape))
+    assert aussm_b200.device_status() == 0
+    check_scan(errors, *shape)
+
+
 # The phases come from a product over d terms held to 2^-22 each: another 2.4e-7 sqrt(d) per step at worst.
 def operator_bound(b, d, n, l):
     return scan_bound(b, d, n, l) + 2.4e-7 * math.sqrt(d) * l
@@ -82,12 +93,25 @@ def test_operator_adjoints_summed_in_runs(shape):
     assert max(errors.values()) < 10 * bound, (errors, bound)
 
 
+@pytest.mark.parametrize("steps", [576, 640, 2000])
+def test_operator_windows_of_unequal_length_split_in_time(steps):
+    """2000 steps in windows of 576 (the last one shorter than a segment), 640 and one: same result."""
+    b, d, n, l = 1, 5, 6, 2000
+    try:
+        _lib.set_option("window_steps", steps)
+        errors = operator_errors(b, d, n, l, 3100)
+    finally:
+        _lib.set_option("window_steps", 0)
+    assert aussm_b200.device_status() == 0
+    assert max(errors.values()) < operator_bound(b, d, n, l), errors
+
+
 S6_KEYS = ["u", "delta", "A", "B", "C", "D", "z", "delta_bias"]
 
 
 # A step of the contracting recurrence costs two roundings and the exponential's 2^-22; earlier errors decay, but at
 # worst (A near 0) stay.  Sums over states, channels and steps add an ulp per term at worst.
-@pytest.mark.parametrize("shape", [(1, 5, 16, 256), (2, 33, 4, 300), (1, 16, 7, 1028), (3, 40, 12, 516), (1, 1, 1, 4096)])
+@pytest.mark.parametrize("shape", [(1, 5, 16, 512), (2, 33, 4, 516), (1, 16, 7, 1028), (3, 40, 12, 516), (1, 1, 1, 4096)])
 @pytest.mark.parametrize("full", [True, False])
 def test_selective_scan_cut_into_segments(shape, full):
     b, d, n, l = shape
