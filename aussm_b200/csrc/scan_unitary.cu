@@ -1060,21 +1060,33 @@ __global__ void __launch_bounds__(128) segment_states_bwd_kernel(const SegChainP
 // Second stage: fixed-order sums of the per-channel partials (deterministic)
 // and the polar chain rule  dr = Re(conj(G) e^{i phi}),  dphi = -Im(conj(G) w).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) reduce_param_grads_kernel(const ReduceParams p) {
-    __shared__ float4 red[256];
+// One block per state walks that state's partials of all channels.  There are only N such blocks, so what bounds them is
+// the latency of their loads: 1024 threads with four loads in flight each (16384 channels, N = 16: 30 us with 256
+// threads and one).
+constexpr int REDUCE_THREADS = 1024;
+__global__ void __launch_bounds__(REDUCE_THREADS) reduce_param_grads_kernel(const ReduceParams p) {
+    __shared__ float4 red[REDUCE_THREADS];
     const int tid = threadIdx.x;
     const int nseg = p.nseg > 1 ? p.nseg : 1;               // partial arrays: nseg entries per channel
     const long long nch = (long long)p.batch * p.D * nseg;
     if (blockIdx.x < p.N) {
         const int j = blockIdx.x;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (long long ch = tid; ch < nch; ch += 256) {
-            const float4 v = reinterpret_cast<const float4*>(p.part_bc)[ch * p.N + j];
-            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        for (long long ch = tid; ch < nch; ch += 4 * REDUCE_THREADS) {
+            float4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const long long at = ch + (long long)k * REDUCE_THREADS;
+                v[k] = at < nch ? reinterpret_cast<const float4*>(p.part_bc)[at * p.N + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                acc.x += v[k].x; acc.y += v[k].y; acc.z += v[k].z; acc.w += v[k].w;
+            }
         }
         red[tid] = acc;
         __syncthreads();
-        for (int s = 128; s > 0; s >>= 1) {
+        for (int s = REDUCE_THREADS / 2; s > 0; s >>= 1) {
             if (tid < s) {
                 float4 a = red[tid], b = red[tid + s];
                 red[tid] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
@@ -1095,7 +1107,7 @@ __global__ void __launch_bounds__(256) reduce_param_grads_kernel(const ReducePar
         return;
     }
     // remaining blocks: dD (D values) then dx_bias (D*N values), one thread per output
-    const long long o = (long long)(blockIdx.x - p.N) * 256 + tid;
+    const long long o = (long long)(blockIdx.x - p.N) * REDUCE_THREADS + tid;
     if (o < p.D) {
         float acc = 0.f;
         for (int b = 0; b < p.batch; ++b)
@@ -1346,8 +1358,8 @@ cudaError_t scan_unitary_bwd_split(const ScanBwdParams& p, const SegPlan& plan, 
 
 cudaError_t launch_reduce_param_grads(const ReduceParams& p, cudaStream_t stream) {
     const long long tail = (long long)p.D + (p.dx_bias ? (long long)p.D * p.N : 0);
-    const unsigned blocks = (unsigned)(p.N + (tail + 255) / 256);
-    reduce_param_grads_kernel<<<blocks, 256, 0, stream>>>(p);
+    const unsigned blocks = (unsigned)(p.N + (tail + REDUCE_THREADS - 1) / REDUCE_THREADS);
+    reduce_param_grads_kernel<<<blocks, REDUCE_THREADS, 0, stream>>>(p);
     count_launch();
     return cudaGetLastError();
 }
