@@ -89,7 +89,7 @@ struct CMap {
             const int c = w / C::NL, j = w % C::NL;
             const float* base = row < 32 ? rho_b : theta_b;        // rows of this batch entry
             const bool ok = c < nvalid && j < N;
-            own_ptr[i] = base ? base + ((long long)(i0 + (ok ? c : 0)) * N + (ok ? j : 0)) * ld_lam + col * 4 : nullptr;
+            own_ptr[i] = base && ok ? base + ((long long)(i0 + c) * N + j) * ld_lam + col * 4 : nullptr;
         }
 #pragma unroll
         for (int i = 0; i < C::NCH_BC; ++i) {
@@ -99,7 +99,7 @@ struct CMap {
             if (row < C::BC_ROWS) {
                 const int which = (C::REAL ? 2 : 1) * (row / C::NL), j = row % C::NL;
                 const float* base = bc_src[which];
-                bc_ptr[i] = base ? base + (long long)(j < N ? j : 0) * ld_row + col * 4 : nullptr;
+                bc_ptr[i] = base && j < N ? base + (long long)j * ld_row + col * 4 : nullptr;
             }
         }
 #pragma unroll
@@ -135,7 +135,9 @@ struct CMap {
     }
 };
 
-// rows that are never copied (null inputs) must read as zero
+// Rows that are never copied must read as zero: those of null inputs, and those of lanes without a state or channel.
+// Such a lane then has lambda = 1 and, with B = C = 0, a state, an adjoint and contributions to its channel's sums
+// that stay zero, so the loops over the steps need no selects (24 per four steps in the backward kernel).
 template <class C>
 __device__ __forceinline__ void zero_stages(float* bc_ring, float* wsm, int lane) {
     for (int i = threadIdx.x; i < STAGES * C::BC_FLOATS; i += C::WARPS * 32) bc_ring[i] = 0.f;
@@ -270,7 +272,7 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     hr = fmaf(ex2_ftz(rv[e] * kLog2e), hr, sv[e] * brv[e]);
-                    pv[e] = act ? crv[e] * hr : 0.f;
+                    pv[e] = crv[e] * hr;
                 }
             } else {
                 const float4 bi4 = ld_shared_f4(bc + (1 * NL + j) * TP + 4 * q);
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
                     const float ni = fmaf(lr[e], hi, fmaf(li[e], hr, sv[e] * biv[e]));
                     hr = nr;
                     hi = ni;
-                    pv[e] = act ? fmaf(crv[e], nr, -civ[e] * ni) : 0.f;
+                    pv[e] = fmaf(crv[e], nr, -civ[e] * ni);
                 }
             }
             st_shared_f4(pt + lane * TP + 4 * q, make_float4(pv[0], pv[1], pv[2], pv[3]));
@@ -333,6 +335,32 @@ __device__ __forceinline__ void red_add_v4c(float* addr, const float (&v)[4]) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]),
                  "f"(v[3])
                  : "memory");
+}
+
+// Sums of four steps' dB and dC contributions over the channels of a warp (lanes NL apart).  With two or more channels
+// the first exchange leaves the lower half-warp with B and the upper with C (in `b`): half the shuffles, and every
+// lane's atomics carry one of the two (B8 D2048 N16 L4096 backward: see the comment at the kernel).
+template <int NL>
+__device__ __forceinline__ void add_channels(float (&b)[4], const float (&c)[4]) {
+    if (NL == 32) return;
+    const bool upper = (threadIdx.x & 16) != 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float other = __shfl_xor_sync(0xffffffffu, upper ? b[e] : c[e], 16);
+        b[e] = (upper ? c[e] : b[e]) + other;
+    }
+#pragma unroll
+    for (int off = NL; off < 16; off <<= 1) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) b[e] += __shfl_xor_sync(0xffffffffu, b[e], off);
+    }
+}
+// a warp with fewer channels than lanes for them: the missing ones add nothing to dB and dC
+__device__ __forceinline__ void drop_if(bool drop, float (&a)[4], float (&b)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (drop) a[e] = b[e] = 0.f;
+    }
 }
 
 template <int NL, bool REAL>
@@ -401,6 +429,10 @@ cplx_bwd_kernel(const CplxBwdParams p) {
         else cp_async_commit();
     }
     float2 h_next = act ? rec[ntiles - 1] : make_float2(0.f, 0.f);
+    // dB / dC: the lanes of a warp's first channel (of each half-warp) add, the lower half dB, the upper dC
+    const bool upper = (lane & 16) != 0;
+    const bool grad_lane = (NL == 32 || (lane & 15) < NL) && j < N && nvalid > 0;
+    const long long grad_off = bo + (long long)j * p.ld_row;
 
     for (int r = 0; r < ntiles; ++r) {
         const int tile = ntiles - 1 - r;
@@ -499,27 +531,25 @@ cplx_bwd_kernel(const CplxBwdParams p) {
                 const float htr = fmaf(sv[e], brv[e], ar);
                 const float nr = fmaf(crv[e], wv[e], er);         // eta_t = carry + C w
                 dr[e] = nr * ar;
-                E[e] = act ? nr * brv[e] : 0.f;
-                P[e] = act ? crv[e] * htr : 0.f;
-                gBr[e] = act ? nr * sv[e] : 0.f;
-                gCr[e] = act ? wv[e] * htr : 0.f;
+                E[e] = nr * brv[e];
+                P[e] = crv[e] * htr;
+                gBr[e] = nr * sv[e];
+                gCr[e] = wv[e] * htr;
                 er = lr[e] * nr;
             }
             st_shared_f4(st + lane * TP + 4 * q, make_float4(dr[0], dr[1], dr[2], dr[3]));
             st_shared_f4(et + lane * TP + 4 * q, make_float4(E[0], E[1], E[2], E[3]));
             st_shared_f4(pt + lane * TP + 4 * q, make_float4(P[0], P[1], P[2], P[3]));
-#pragma unroll
-            for (int off = NL; off < 32; off <<= 1) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    gBr[e] += __shfl_xor_sync(0xffffffffu, gBr[e], off);
-                    gCr[e] += __shfl_xor_sync(0xffffffffu, gCr[e], off);
+            if (nvalid < CPW) drop_if(!act, gBr, gCr);
+            add_channels<NL>(gBr, gCr);
+            const long long o = grad_off + t0 + 4 * q;
+            if (NL == 32) {
+                if (grad_lane) {
+                    red_add_v4c(p.dB_re + o, gBr);
+                    red_add_v4c(p.dC_re + o, gCr);
                 }
-            }
-            if (c == 0 && j < N && nvalid > 0) {
-                const long long o = bo + (long long)j * p.ld_row + t0 + 4 * q;
-                red_add_v4c(p.dB_re + o, gBr);
-                red_add_v4c(p.dC_re + o, gCr);
+            } else if (grad_lane) {
+                red_add_v4c((upper ? p.dC_re : p.dB_re) + o, gBr);
             }
         };
         // reverse pass
@@ -551,12 +581,12 @@ cplx_bwd_kernel(const CplxBwdParams p) {
                 const float nr = fmaf(crv[e], wv[e], er), ni = fmaf(-civ[e], wv[e], ei);
                 dr[e] = fmaf(nr, ar, ni * ai);            // Re(conj(eta) a)
                 dth[e] = fmaf(ni, ar, -nr * ai);          // -Im(conj(eta) a)
-                E[e] = act ? fmaf(nr, brv[e], ni * biv[e]) : 0.f;
-                P[e] = act ? fmaf(crv[e], htr, -civ[e] * hti) : 0.f;
-                gBr[e] = act ? nr * sv[e] : 0.f;
-                gBi[e] = act ? ni * sv[e] : 0.f;
-                gCr[e] = act ? wv[e] * htr : 0.f;
-                gCi[e] = act ? -wv[e] * hti : 0.f;
+                E[e] = fmaf(nr, brv[e], ni * biv[e]);
+                P[e] = fmaf(crv[e], htr, -civ[e] * hti);
+                gBr[e] = nr * sv[e];
+                gBi[e] = ni * sv[e];
+                gCr[e] = wv[e] * htr;
+                gCi[e] = -wv[e] * hti;
                 er = fmaf(lr[e], nr, li[e] * ni);         // conj(lambda) eta
                 ei = fmaf(lr[e], ni, -li[e] * nr);
             }
@@ -567,28 +597,25 @@ cplx_bwd_kernel(const CplxBwdParams p) {
                                                                   : make_float4(0.f, 0.f, 0.f, 0.f));
             st_shared_f4(et + lane * TP + 4 * q, make_float4(E[0], E[1], E[2], E[3]));
             st_shared_f4(pt + lane * TP + 4 * q, make_float4(P[0], P[1], P[2], P[3]));
-#pragma unroll
-            for (int off = NL; off < 32; off <<= 1) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    gBr[e] += __shfl_xor_sync(0xffffffffu, gBr[e], off);
-                    gCr[e] += __shfl_xor_sync(0xffffffffu, gCr[e], off);
-                }
-                if (p.dB_im) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) gBi[e] += __shfl_xor_sync(0xffffffffu, gBi[e], off);
-                }
-                if (p.dC_im) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) gCi[e] += __shfl_xor_sync(0xffffffffu, gCi[e], off);
-                }
+            if (nvalid < CPW) {
+                drop_if(!act, gBr, gCr);
+                drop_if(!act, gBi, gCi);
             }
-            if (c == 0 && j < N && nvalid > 0) {
-                const long long o = bo + (long long)j * p.ld_row + t0 + 4 * q;
-                red_add_v4c(p.dB_re + o, gBr);
-                red_add_v4c(p.dC_re + o, gCr);
-                if (p.dB_im) red_add_v4c(p.dB_im + o, gBi);
-                if (p.dC_im) red_add_v4c(p.dC_im + o, gCi);
+            add_channels<NL>(gBr, gCr);
+            const bool imag = p.dB_im || p.dC_im;
+            if (imag) add_channels<NL>(gBi, gCi);
+            const long long o = grad_off + t0 + 4 * q;
+            if (NL == 32) {
+                if (grad_lane) {
+                    red_add_v4c(p.dB_re + o, gBr);
+                    red_add_v4c(p.dC_re + o, gCr);
+                    if (p.dB_im) red_add_v4c(p.dB_im + o, gBi);
+                    if (p.dC_im) red_add_v4c(p.dC_im + o, gCi);
+                }
+            } else if (grad_lane) {
+                red_add_v4c((upper ? p.dC_re : p.dB_re) + o, gBr);
+                float* im = upper ? p.dC_im : p.dB_im;
+                if (im) red_add_v4c(im + o, gBi);
             }
         };
 #pragma unroll
