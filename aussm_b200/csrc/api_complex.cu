@@ -89,9 +89,11 @@ size_t aussm_b200_scan_complex_states_floats(int B, int D, int N, int L) {
 }
 
 size_t aussm_b200_scan_complex_bwd_workspace_bytes(int B, int D, int N, int L) {
-    (void)N; (void)L;
     if (B <= 0 || D <= 0) return 0;
-    return ((size_t)B * D * sizeof(float) + 255) / 256 * 256;
+    // a split launch: the gradients between segments and the segments' multipliers; always: dD per channel (and segment)
+    const size_t nseg = N > 0 && L > 0 ? cplx_split_plan(B, D, N, L, true).nseg : 1, nch = (size_t)B * D;
+    const size_t split = nseg > 1 ? 4 * nch * nseg * N : 0;
+    return ((split + nch * nseg) * sizeof(float) + 255) / 256 * 256;
 }
 
 int aussm_b200_scan_complex_fwd(const float* rho, const float* theta, const float* u, const float* dt,
@@ -113,6 +115,10 @@ int aussm_b200_scan_complex_fwd(const float* rho, const float* theta, const floa
     p.C_im = C_im; p.Dskip = Dskip; p.y = y; p.states = states; p.states_stride = cplx_ntiles(L) + 1; p.tile0 = 0;
     p.nch = B * D; p.Dmod = D; p.N = N; p.L = L;
     p.ld_lam = L; p.lam_batch_stride = (long long)D * N * L; p.ld_row = L;
+    if (states) {                                           // the split hands states on through the record
+        const CplxPlan plan = cplx_split_plan(B, D, N, L, false);
+        p.nseg = plan.nseg; p.seg_tiles = plan.seg_tiles;
+    }
     cudaError_t e = launch_cplx_fwd(p, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "scan_complex_fwd launch");
     return AUSSM_OK;
@@ -156,9 +162,17 @@ int aussm_b200_scan_complex_bwd(const float* gy, const float* gstates, const flo
     p.dB_im = B_im ? dB_im : nullptr; p.dC_re = dC_re; p.dC_im = C_im ? dC_im : nullptr;
     p.part_D = static_cast<float*>(workspace); p.eta_in = nullptr; p.eta_out = nullptr; p.accumulate = 0;
     p.nch = B * D; p.Dmod = D; p.N = N; p.L = L;
+    const CplxPlan plan = cplx_split_plan(B, D, N, L, true);
+    p.nseg = 1;
+    if (plan.nseg > 1 && (reinterpret_cast<uintptr_t>(workspace) & 7u) == 0) {
+        p.nseg = plan.nseg; p.seg_tiles = plan.seg_tiles;
+        p.seg_eta = static_cast<float*>(workspace);
+        p.seg_mul = p.seg_eta + 2 * (size_t)B * D * plan.nseg * N;
+        p.part_D = p.seg_mul + 2 * (size_t)B * D * plan.nseg * N;
+    }
     p.ld_lam = L; p.lam_batch_stride = (long long)D * N * L; p.ld_row = L;
     e = launch_cplx_bwd(p, stream);
-    if (e == cudaSuccess) e = launch_cplx_reduce_D(p.part_D, dD, B, D, stream);
+    if (e == cudaSuccess) e = launch_cplx_reduce_D(p.part_D, dD, B * p.nseg, D, stream);
     if (e != cudaSuccess) return cuda_fail(e, "scan_complex_bwd launch");
     return AUSSM_OK;
 }

@@ -26,6 +26,8 @@
 
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace aussm {
@@ -174,7 +176,10 @@ __device__ __forceinline__ void lambda4(const float4 r4, const float4 t4, float 
 // ---------------------------------------------------------------------------
 // REAL: no angle stream and real B, C - the state, the multiplier and every product are real (the positive-real
 // operator); the imaginary halves of the arithmetic and the sine / cosine are compiled out.
-template <int NL, bool REAL>
+// SUM: summary of a segment of the time-axis split - from a zero state and without output: the end state goes to the
+// record's entry of the next segment's first tile, the product of the multipliers one tile into this segment (both
+// are overwritten by the real pass).
+template <int NL, bool REAL, bool SUM>
 __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(const CplxFwdParams p) {
     using C = CCfg<NL, false, REAL>;
     constexpr int CPW = C::CPW, AUX = C::AUX, VW = C::VW;
@@ -184,8 +189,10 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
     // shadows it (it takes part in the copies of the shared tile and in the barriers, and stores nothing)
     const int tasks_per_batch = (p.Dmod + CPW - 1) / CPW;
     const int blocks_per_batch = (tasks_per_batch + C::WARPS - 1) / C::WARPS;
-    const int b = blockIdx.x / blocks_per_batch;
-    const int tw_raw = (blockIdx.x % blocks_per_batch) * C::WARPS + warp;
+    const int blocks = blocks_per_batch * (p.nch / p.Dmod);
+    const int seg = blockIdx.x / blocks, block = blockIdx.x % blocks;
+    const int b = block / blocks_per_batch;
+    const int tw_raw = (block % blocks_per_batch) * C::WARPS + warp;
     const int tw = min(tw_raw, tasks_per_batch - 1);
     const int i0 = tw * CPW;
     const int nvalid = tw_raw < tasks_per_batch ? min(CPW, p.Dmod - i0) : 0;
@@ -196,6 +203,7 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
     const bool act = c < nvalid && j < p.N;
     const int N = p.N, L = p.L;
     const int ntiles = (L + T - 1) / T;
+    const int first = seg * p.seg_tiles, last = p.nseg > 1 ? min(ntiles, first + p.seg_tiles) : ntiles;   // tiles
     const long long ch = ch0 + c;
 
     float* srow = smem + STAGES * C::STAGE_FLOATS;          // [CPW][T]: s = dt silu(u)
@@ -204,9 +212,9 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
 
     float2* rec = (p.states && act) ? reinterpret_cast<float2*>(p.states) + (ch * N + j) * p.states_stride + p.tile0
                                     : nullptr;
-    float hr = 0.f, hi = 0.f;
-    if (rec && p.tile0 > 0) {
-        const float2 h0 = rec[0];
+    float hr = 0.f, hi = 0.f, ar = 1.f, ai = 0.f;
+    if (!SUM && rec && p.tile0 + first > 0) {              // later segments: left there by the segment chain
+        const float2 h0 = rec[first];
         hr = h0.x;
         hi = h0.y;
     }
@@ -224,13 +232,14 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
     map.init(lane, warp, nvalid, N, p.rho ? p.rho + lam_b : nullptr, p.theta ? p.theta + lam_b : nullptr, p.ld_lam,
              i0, bc_src, aux_src, ch0, p.ld_row);
     for (int s = 0; s < STAGES; ++s) {
-        if (s < ntiles)
-            map.issue(smem + s * C::STAGE_FLOATS, bc_ring + s * C::BC_FLOATS, (long long)s * T, min(T, L - s * T), lane,
-                      warp);
+        const int t = first + s;
+        if (t < last)
+            map.issue(smem + (t % STAGES) * C::STAGE_FLOATS, bc_ring + (t % STAGES) * C::BC_FLOATS, (long long)t * T,
+                      min(T, L - t * T), lane, warp);
         else cp_async_commit();
     }
 
-    for (int tile = 0; tile < ntiles; ++tile) {
+    for (int tile = first; tile < last; ++tile) {
         float* st = smem + (tile % STAGES) * C::STAGE_FLOATS;
         float* bc = bc_ring + (tile % STAGES) * C::BC_FLOATS;
         float* aux = st + C::OWN_ROWS * TP;
@@ -238,7 +247,7 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
         const int tlen = min(T, L - (int)t0);
         cp_async_wait<STAGES - 1>();
         block_sync<C>();                                    // every warp's share of the B / C tile has landed
-        if (rec) rec[tile] = make_float2(hr, hi);
+        if (!SUM && rec) rec[tile] = make_float2(hr, hi);
         // pre-pass: silu(u) replaces u, s = dt silu(u)
 #pragma unroll
         for (int it = 0; it < C::ITERS; ++it) {
@@ -271,8 +280,10 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
                 const float rv[4] = AUSSM_F4(r4);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    hr = fmaf(ex2_ftz(rv[e] * kLog2e), hr, sv[e] * brv[e]);
+                    const float lr = ex2_ftz(rv[e] * kLog2e);
+                    hr = fmaf(lr, hr, sv[e] * brv[e]);
                     pv[e] = crv[e] * hr;
+                    if (SUM) ar *= lr;
                 }
             } else {
                 const float4 bi4 = ld_shared_f4(bc + (1 * NL + j) * TP + 4 * q);
@@ -287,9 +298,14 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
                     hr = nr;
                     hi = ni;
                     pv[e] = fmaf(crv[e], nr, -civ[e] * ni);
+                    if (SUM) {
+                        const float qr = fmaf(lr[e], ar, -li[e] * ai);
+                        ai = fmaf(lr[e], ai, li[e] * ar);
+                        ar = qr;
+                    }
                 }
             }
-            st_shared_f4(pt + lane * TP + 4 * q, make_float4(pv[0], pv[1], pv[2], pv[3]));
+            if (!SUM) st_shared_f4(pt + lane * TP + 4 * q, make_float4(pv[0], pv[1], pv[2], pv[3]));
         };
         if (tlen == T) {
 #pragma unroll
@@ -303,7 +319,7 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
         for (int it = 0; it < C::ITERS; ++it) {
             const int e0 = (lane + 32 * it) * VW;
             const int cc = e0 / T, t = e0 % T;
-            if (e0 < C::ELEMS && t < tlen && cc < nvalid) {
+            if (!SUM && e0 < C::ELEMS && t < tlen && cc < nvalid) {
                 Vec<VW> acc, v, z;
                 acc.ld(pt + cc * NL * TP + t);
 #pragma unroll
@@ -321,11 +337,18 @@ __global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_fwd_kernel(c
         }
         block_sync<C>();                                    // nobody reads this stage's B / C tile any more
         const int nt = tile + STAGES;
-        if (nt < ntiles) map.issue(st, bc, (long long)nt * T, min(T, L - nt * T), lane, warp);
+        if (nt < last) map.issue(st, bc, (long long)nt * T, min(T, L - nt * T), lane, warp);
         else cp_async_commit();
     }
     cp_async_wait<0>();
-    if (rec) rec[ntiles] = make_float2(hr, hi);
+    if (SUM) {
+        if (rec) {
+            rec[last] = make_float2(hr, hi);
+            rec[first + 1] = make_float2(ar, ai);
+        }
+    } else if (rec && last == ntiles) {
+        rec[ntiles] = make_float2(hr, hi);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -372,8 +395,10 @@ cplx_bwd_kernel(const CplxBwdParams p) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tasks_per_batch = (p.Dmod + CPW - 1) / CPW;
     const int blocks_per_batch = (tasks_per_batch + C::WARPS - 1) / C::WARPS;
-    const int b = blockIdx.x / blocks_per_batch;
-    const int tw_raw = (blockIdx.x % blocks_per_batch) * C::WARPS + warp;
+    const int blocks = blocks_per_batch * (p.nch / p.Dmod);
+    const int seg = blockIdx.x / blocks, block = blockIdx.x % blocks;
+    const int b = block / blocks_per_batch;
+    const int tw_raw = (block % blocks_per_batch) * C::WARPS + warp;
     const int tw = min(tw_raw, tasks_per_batch - 1);          // warps beyond the last task shadow it
     const int i0 = tw * CPW;
     const int nvalid = tw_raw < tasks_per_batch ? min(CPW, p.Dmod - i0) : 0;
@@ -384,6 +409,7 @@ cplx_bwd_kernel(const CplxBwdParams p) {
     const bool act = c < nvalid && j < p.N;
     const int N = p.N, L = p.L;
     const int ntiles = (L + T - 1) / T;
+    const int first = seg * p.seg_tiles, last = p.nseg > 1 ? min(ntiles, first + p.seg_tiles) : ntiles;   // tiles
     const long long ch = ch0 + c;
     const bool has_rho = p.rho != nullptr, has_theta = p.theta != nullptr;
 
@@ -397,7 +423,11 @@ cplx_bwd_kernel(const CplxBwdParams p) {
     const float2* grec = (p.gstates && act) ? reinterpret_cast<const float2*>(p.gstates) + rec_off : nullptr;
     float er = 0.f, ei = 0.f;       // conj(lambda_{t+1}) eta_{t+1}: the gradient that reaches h_t from later steps
     if (act) {
-        if (p.eta_in) {
+        if (p.nseg > 1) {
+            const float2 e0 = reinterpret_cast<const float2*>(p.seg_eta)[(ch * p.nseg + seg) * N + j];
+            er = e0.x;
+            ei = e0.y;
+        } else if (p.eta_in) {
             const float2 e0 = reinterpret_cast<const float2*>(p.eta_in)[ch * N + j];
             er = e0.x;
             ei = e0.y;
@@ -422,20 +452,20 @@ cplx_bwd_kernel(const CplxBwdParams p) {
     map.init(lane, warp, nvalid, N, has_rho ? p.rho + lam_b : nullptr, has_theta ? p.theta + lam_b : nullptr,
              p.ld_lam, i0, bc_src, aux_src, ch0, p.ld_row);
     for (int r = 0; r < STAGES; ++r) {
-        const int tile = ntiles - 1 - r;
-        if (tile >= 0)
+        const int tile = last - 1 - r;
+        if (tile >= first)
             map.issue(smem + r * C::STAGE_FLOATS, bc_ring + r * C::BC_FLOATS, (long long)tile * T,
                       min(T, L - tile * T), lane, warp);
         else cp_async_commit();
     }
-    float2 h_next = act ? rec[ntiles - 1] : make_float2(0.f, 0.f);
+    float2 h_next = act ? rec[last - 1] : make_float2(0.f, 0.f);
     // dB / dC: the lanes of a warp's first channel (of each half-warp) add, the lower half dB, the upper dC
     const bool upper = (lane & 16) != 0;
     const bool grad_lane = (NL == 32 || (lane & 15) < NL) && j < N && nvalid > 0;
     const long long grad_off = bo + (long long)j * p.ld_row;
 
-    for (int r = 0; r < ntiles; ++r) {
-        const int tile = ntiles - 1 - r;
+    for (int r = 0; r < last - first; ++r) {
+        const int tile = last - 1 - r;
         float* st = smem + (r % STAGES) * C::STAGE_FLOATS;
         float* bc = bc_ring + (r % STAGES) * C::BC_FLOATS;
         float* aux = st + C::OWN_ROWS * TP;
@@ -443,7 +473,7 @@ cplx_bwd_kernel(const CplxBwdParams p) {
         const int tlen = min(T, L - (int)t0);
         const int nq = tlen >> 2;
         float hr = h_next.x, hi = h_next.y;                 // state before the tile's first step
-        if (tile > 0 && act) h_next = rec[tile - 1];
+        if (tile > first && act) h_next = rec[tile - 1];
         cp_async_wait<STAGES - 1>();
         block_sync<C>();                                    // every warp's share of the B / C tile has landed
 
@@ -690,15 +720,15 @@ cplx_bwd_kernel(const CplxBwdParams p) {
         }
         block_sync<C>();                                    // nobody reads this stage's B / C tile any more
         const int nr = r + STAGES;
-        if (nr < ntiles) {
-            const int nt = ntiles - 1 - nr;
+        if (nr < last - first) {
+            const int nt = last - 1 - nr;
             map.issue(st, bc, (long long)nt * T, min(T, L - nt * T), lane, warp);
         } else {
             cp_async_commit();
         }
     }
     cp_async_wait<0>();
-    if (act && p.eta_out) reinterpret_cast<float2*>(p.eta_out)[ch * N + j] = make_float2(er, ei);
+    if (act && p.eta_out && seg == 0) reinterpret_cast<float2*>(p.eta_out)[ch * N + j] = make_float2(er, ei);
 
     __syncwarp();
 #pragma unroll
@@ -708,7 +738,163 @@ cplx_bwd_kernel(const CplxBwdParams p) {
         float aD = 0.f;
         for (int idx = 0; idx < 32 * C::ITERS; ++idx)
             if (idx * VW < C::ELEMS && (idx * VW) / T == lane) aD += et[idx];
-        p.part_D[ch0 + lane] = aD + (p.accumulate ? p.part_D[ch0 + lane] : 0.f);
+        const long long o = ((long long)b * max(1, p.nseg) + seg) * p.Dmod + i0 + lane;
+        p.part_D[o] = aD + (p.accumulate ? p.part_D[o] : 0.f);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Time-axis split, backward: what the outputs (and the gradients of the state record) of a segment send to the state
+// before it.  With a_t the product of the segment's multipliers up to step t
+//     l = sum_t conj(a_t C_t) w_t + sum over tiles conj(a before the tile) gstates[tile],   w = gy silu(z)
+// a forward walk; the segment's whole product goes along for the chain.
+// ---------------------------------------------------------------------------
+template <int NL, bool REAL>
+__global__ void __launch_bounds__(CCfg<NL, false>::WARPS * 32) cplx_bwd_summary_kernel(const CplxBwdParams p) {
+    using C = CCfg<NL, false, REAL>;                         // rows: z, gy, (unused)
+    constexpr int CPW = C::CPW, AUX = C::AUX, VW = C::VW;
+    extern __shared__ __align__(128) float smem_all[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tasks_per_batch = (p.Dmod + CPW - 1) / CPW;
+    const int blocks_per_batch = (tasks_per_batch + C::WARPS - 1) / C::WARPS;
+    const int blocks = blocks_per_batch * (p.nch / p.Dmod);
+    const int seg = 1 + blockIdx.x / blocks, block = blockIdx.x % blocks;      // segment 0 has nothing before it
+    const int b = block / blocks_per_batch;
+    const int tw_raw = (block % blocks_per_batch) * C::WARPS + warp;
+    const int tw = min(tw_raw, tasks_per_batch - 1);
+    const int i0 = tw * CPW;
+    const int nvalid = tw_raw < tasks_per_batch ? min(CPW, p.Dmod - i0) : 0;
+    const long long ch0 = (long long)b * p.Dmod + i0;
+    float* bc_ring = smem_all;
+    float* smem = smem_all + STAGES * C::BC_FLOATS + warp * C::WARP_FLOATS;
+    const int c = lane / NL, j = lane % NL;
+    const bool act = c < nvalid && j < p.N;
+    const int N = p.N, L = p.L;
+    const int ntiles = (L + T - 1) / T;
+    const int first = seg * p.seg_tiles, last = min(ntiles, first + p.seg_tiles);
+    const long long ch = ch0 + c;
+    float* wrow = smem + STAGES * C::STAGE_FLOATS;           // [CPW][T]: w
+    zero_stages<C>(bc_ring, smem, lane);
+    const float2* grec = (p.gstates && act)
+                             ? reinterpret_cast<const float2*>(p.gstates) + (ch * N + j) * p.states_stride + p.tile0
+                             : nullptr;
+    const long long bo = (long long)b * N * p.ld_row;
+    const float* bc_src[4] = {p.B_re + bo, p.B_im ? p.B_im + bo : nullptr, p.C_re + bo, p.C_im ? p.C_im + bo : nullptr};
+    const float* aux_src[AUX] = {p.z, p.gy, p.z};
+    const long long lam_b = (long long)b * p.lam_batch_stride;
+    CMap<C> map;
+    map.init(lane, warp, nvalid, N, p.rho ? p.rho + lam_b : nullptr, p.theta ? p.theta + lam_b : nullptr, p.ld_lam, i0,
+             bc_src, aux_src, ch0, p.ld_row);
+    for (int s = 0; s < STAGES; ++s) {
+        const int t = first + s;
+        if (t < last)
+            map.issue(smem + (t % STAGES) * C::STAGE_FLOATS, bc_ring + (t % STAGES) * C::BC_FLOATS, (long long)t * T,
+                      min(T, L - t * T), lane, warp);
+        else cp_async_commit();
+    }
+    float ar = 1.f, ai = 0.f, gr = 0.f, gi = 0.f;
+    for (int tile = first; tile < last; ++tile) {
+        float* st = smem + (tile % STAGES) * C::STAGE_FLOATS;
+        float* bc = bc_ring + (tile % STAGES) * C::BC_FLOATS;
+        float* aux = st + C::OWN_ROWS * TP;
+        const int tlen = min(T, L - tile * T);
+        if (grec) {
+            const float2 g = grec[tile];
+            gr += fmaf(ar, g.x, ai * g.y);
+            gi += fmaf(ar, g.y, -ai * g.x);
+        }
+        cp_async_wait<STAGES - 1>();
+        block_sync<C>();
+#pragma unroll
+        for (int it = 0; it < C::ITERS; ++it) {
+            const int e0 = (lane + 32 * it) * VW;
+            const int cc = e0 / T, t = e0 % T;
+            if (e0 < C::ELEMS && t < tlen) {
+                Vec<VW> z, g;
+                z.ld(aux + (cc * AUX + 0) * T + t);
+                g.ld(aux + (cc * AUX + 1) * T + t);
+#pragma unroll
+                for (int e = 0; e < VW; ++e) g.v[e] *= siluf_(z.v[e]);
+                g.st(wrow + cc * T + t);
+            }
+        }
+        __syncwarp();
+        auto quad = [&](const int q) {
+            const float4 w4 = ld_shared_f4(wrow + c * T + 4 * q);
+            const float4 r4 = ld_shared_f4(st + lane * TP + 4 * q);
+            const float4 cr4 = ld_shared_f4(bc + (C::CROW * NL + j) * TP + 4 * q);
+            const float wv[4] = AUSSM_F4(w4), crv[4] = AUSSM_F4(cr4);
+            if (REAL) {
+                const float rv[4] = AUSSM_F4(r4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    ar *= ex2_ftz(rv[e] * kLog2e);
+                    gr = fmaf(ar, crv[e] * wv[e], gr);
+                }
+                return;
+            }
+            const float4 ci4 = ld_shared_f4(bc + (3 * NL + j) * TP + 4 * q);
+            const float civ[4] = AUSSM_F4(ci4);
+            float lr[4], li[4];
+            lambda4(r4, ld_shared_f4(st + (32 + lane) * TP + 4 * q), lr, li);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float qr = fmaf(lr[e], ar, -li[e] * ai);
+                ai = fmaf(lr[e], ai, li[e] * ar);
+                ar = qr;
+                const float cr = crv[e] * wv[e], ci = civ[e] * wv[e];
+                gr = fmaf(ar, cr, fmaf(-ai, ci, gr));
+                gi = fmaf(-ar, ci, fmaf(-ai, cr, gi));
+            }
+        };
+        if (tlen == T) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) quad(q);
+        } else {
+            for (int q = 0; q < (tlen >> 2); ++q) quad(q);
+        }
+        block_sync<C>();
+        const int nt = tile + STAGES;
+        if (nt < last) map.issue(st, bc, (long long)nt * T, min(T, L - nt * T), lane, warp);
+        else cp_async_commit();
+    }
+    cp_async_wait<0>();
+    if (act) {
+        const long long o = (ch * p.nseg + seg) * N + j;
+        reinterpret_cast<float2*>(p.seg_eta)[o] = make_float2(gr, gi);
+        reinterpret_cast<float2*>(p.seg_mul)[o] = make_float2(ar, ai);
+    }
+}
+
+// one thread per (channel, state): true start states in place of the end states from zero
+__global__ void __launch_bounds__(128) cplx_fwd_chain_kernel(const CplxFwdParams p) {
+    const long long id = (long long)blockIdx.x * 128 + threadIdx.x;
+    if (id >= (long long)p.nch * p.N) return;
+    float2* rec = reinterpret_cast<float2*>(p.states) + id * p.states_stride + p.tile0;
+    float2 h = p.tile0 > 0 ? rec[0] : make_float2(0.f, 0.f);
+    for (int seg = 0; seg + 1 < p.nseg; ++seg) {
+        const float2 a = rec[seg * p.seg_tiles + 1], e = rec[(seg + 1) * p.seg_tiles];
+        h = make_float2(fmaf(a.x, h.x, fmaf(-a.y, h.y, e.x)), fmaf(a.x, h.y, fmaf(a.y, h.x, e.y)));
+        rec[(seg + 1) * p.seg_tiles] = h;
+    }
+}
+
+// one thread per (channel, state): seg_eta of segment s turns from l_s into the gradient of the state after s
+__global__ void __launch_bounds__(128) cplx_bwd_chain_kernel(const CplxBwdParams p) {
+    const long long id = (long long)blockIdx.x * 128 + threadIdx.x;
+    if (id >= (long long)p.nch * p.N) return;
+    const long long ch = id / p.N, j = id % p.N;
+    float2 g = make_float2(0.f, 0.f);
+    if (p.eta_in) g = reinterpret_cast<const float2*>(p.eta_in)[id];
+    else if (p.gstates)
+        g = reinterpret_cast<const float2*>(p.gstates)[id * p.states_stride + p.tile0 + (p.L + T - 1) / T];
+    float2* eta = reinterpret_cast<float2*>(p.seg_eta);
+    const float2* mul = reinterpret_cast<const float2*>(p.seg_mul);
+    for (int seg = p.nseg - 1; seg >= 0; --seg) {
+        const long long o = (ch * p.nseg + seg) * p.N + j;
+        const float2 l = seg > 0 ? eta[o] : make_float2(0.f, 0.f), a = seg > 0 ? mul[o] : make_float2(0.f, 0.f);
+        eta[o] = g;
+        g = make_float2(fmaf(a.x, g.x, fmaf(a.y, g.y, l.x)), fmaf(a.x, g.y, fmaf(-a.y, g.x, l.y)));   // l + conj(a) g
     }
 }
 
@@ -720,50 +906,92 @@ __global__ void __launch_bounds__(256) cplx_reduce_D_kernel(const float* part_D,
     dD[i] = acc;
 }
 
-template <int NL, bool BWD, bool REAL, class Kern, class Params>
-cudaError_t launch_nl(Kern kern, const Params& p, cudaStream_t stream) {
-    using C = CCfg<NL, BWD, REAL>;
+template <class C, class Kern, class Params>
+cudaError_t launch_nl(Kern kern, const Params& p, int segments, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     const long long tasks = (p.Dmod + C::CPW - 1) / C::CPW;
-    const long long blocks = (long long)(p.nch / p.Dmod) * ((tasks + C::WARPS - 1) / C::WARPS);
+    const long long blocks = (long long)(p.nch / p.Dmod) * ((tasks + C::WARPS - 1) / C::WARPS) * segments;
     kern<<<(unsigned)blocks, C::WARPS * 32, C::SMEM_BYTES, stream>>>(p);
     count_launch();
     return cudaGetLastError();
 }
 
+unsigned chain_blocks(long long nch, int N) { return (unsigned)((nch * N + 127) / 128); }
+
+template <int NL, bool REAL>
+cudaError_t launch_fwd(const CplxFwdParams& p, cudaStream_t stream) {
+    using C = CCfg<NL, false, REAL>;
+    if (p.nseg <= 1) return launch_nl<C>(cplx_fwd_kernel<NL, REAL, false>, p, 1, stream);
+    cudaError_t e = launch_nl<C>(cplx_fwd_kernel<NL, REAL, true>, p, p.nseg - 1, stream);
+    if (e != cudaSuccess) return e;
+    cplx_fwd_chain_kernel<<<chain_blocks(p.nch, p.N), 128, 0, stream>>>(p);
+    count_launch();
+    e = cudaGetLastError();
+    return e != cudaSuccess ? e : launch_nl<C>(cplx_fwd_kernel<NL, REAL, false>, p, p.nseg, stream);
+}
+
+template <int NL, bool REAL>
+cudaError_t launch_bwd(const CplxBwdParams& p, cudaStream_t stream) {
+    using C = CCfg<NL, true, REAL>;
+    if (p.nseg <= 1) return launch_nl<C>(cplx_bwd_kernel<NL, REAL>, p, 1, stream);
+    cudaError_t e = launch_nl<CCfg<NL, false, REAL>>(cplx_bwd_summary_kernel<NL, REAL>, p, p.nseg - 1, stream);
+    if (e != cudaSuccess) return e;
+    cplx_bwd_chain_kernel<<<chain_blocks(p.nch, p.N), 128, 0, stream>>>(p);
+    count_launch();
+    e = cudaGetLastError();
+    return e != cudaSuccess ? e : launch_nl<C>(cplx_bwd_kernel<NL, REAL>, p, p.nseg, stream);
+}
+
+template <bool REAL>
+cudaError_t launch_fwd_n(const CplxFwdParams& p, cudaStream_t stream) {
+    if (p.N <= 4) return launch_fwd<4, REAL>(p, stream);
+    if (p.N <= 8) return launch_fwd<8, REAL>(p, stream);
+    if (p.N <= 16) return launch_fwd<16, REAL>(p, stream);
+    if (p.N <= 32) return launch_fwd<32, REAL>(p, stream);
+    return cudaErrorInvalidValue;
+}
+
+template <bool REAL>
+cudaError_t launch_bwd_n(const CplxBwdParams& p, cudaStream_t stream) {
+    if (p.N <= 4) return launch_bwd<4, REAL>(p, stream);
+    if (p.N <= 8) return launch_bwd<8, REAL>(p, stream);
+    if (p.N <= 16) return launch_bwd<16, REAL>(p, stream);
+    if (p.N <= 32) return launch_bwd<32, REAL>(p, stream);
+    return cudaErrorInvalidValue;
+}
+
 }  // namespace
+
+// A launch with few warps per SM (12 fit forward, 8 backward at N = 16: shared memory) is cut along the time axis.
+// The summary passes cost about two thirds of the forward and a third of the backward kernel, so a split pays below 3
+// and 4 warps per SM; two waves of segments even out their ends.  A segment keeps at least 128 steps; below 768 a call is
+// bound by the host.  Whole -> split, N = 16, forward + backward: B1 D512 L8192 1952 -> 1190 us (forward alone 556 ->
+// 380), B2 D256 L2048 548 -> 413 us, N = 4 B4 D512 L1024 364 -> 289 us; B2 D512 L4096 (3.5 warps per SM) 1097 -> 1087 us.
+CplxPlan cplx_split_plan(long long batches, int D, int N, int L, bool bwd) {
+    CplxPlan plan = {1, (L + T - 1) / T};
+    if (N > 32 || L < 512 || !time_split_option()) return plan;
+    constexpr long long SMS = 148;                          // fixed: a workspace sized with the plan always fits
+    const int per_warp = 32 / (N <= 4 ? 4 : N <= 8 ? 8 : N <= 16 ? 16 : 32);
+    const long long warps = batches * ((D + per_warp - 1) / per_warp);
+    if (warps >= (bwd ? 4 : 3) * SMS) return plan;
+    const long long want = std::min<long long>(2 * (bwd ? 8 : 12) * SMS / warps, L / 128);
+    if (want < 6) return plan;
+    const int tiles = plan.seg_tiles;
+    plan.seg_tiles = (int)((tiles + want - 1) / want);
+    plan.nseg = (tiles + plan.seg_tiles - 1) / plan.seg_tiles;
+    return plan;
+}
 
 cudaError_t launch_cplx_fwd(const CplxFwdParams& p, cudaStream_t stream) {
     if (p.nch <= 0 || p.L <= 0) return cudaSuccess;
-    if (!p.theta && !p.B_im && !p.C_im) {          // everything real
-        if (p.N <= 4) return launch_nl<4, false, true>(cplx_fwd_kernel<4, true>, p, stream);
-        if (p.N <= 8) return launch_nl<8, false, true>(cplx_fwd_kernel<8, true>, p, stream);
-        if (p.N <= 16) return launch_nl<16, false, true>(cplx_fwd_kernel<16, true>, p, stream);
-        if (p.N <= 32) return launch_nl<32, false, true>(cplx_fwd_kernel<32, true>, p, stream);
-        return cudaErrorInvalidValue;
-    }
-    if (p.N <= 4) return launch_nl<4, false, false>(cplx_fwd_kernel<4, false>, p, stream);
-    if (p.N <= 8) return launch_nl<8, false, false>(cplx_fwd_kernel<8, false>, p, stream);
-    if (p.N <= 16) return launch_nl<16, false, false>(cplx_fwd_kernel<16, false>, p, stream);
-    if (p.N <= 32) return launch_nl<32, false, false>(cplx_fwd_kernel<32, false>, p, stream);
-    return cudaErrorInvalidValue;
+    return !p.theta && !p.B_im && !p.C_im ? launch_fwd_n<true>(p, stream) : launch_fwd_n<false>(p, stream);
 }
 
 cudaError_t launch_cplx_bwd(const CplxBwdParams& p, cudaStream_t stream) {
     if (p.nch <= 0 || p.L <= 0) return cudaSuccess;
-    if (!p.theta && !p.B_im && !p.C_im && !p.dB_im && !p.dC_im) {
-        if (p.N <= 4) return launch_nl<4, true, true>(cplx_bwd_kernel<4, true>, p, stream);
-        if (p.N <= 8) return launch_nl<8, true, true>(cplx_bwd_kernel<8, true>, p, stream);
-        if (p.N <= 16) return launch_nl<16, true, true>(cplx_bwd_kernel<16, true>, p, stream);
-        if (p.N <= 32) return launch_nl<32, true, true>(cplx_bwd_kernel<32, true>, p, stream);
-        return cudaErrorInvalidValue;
-    }
-    if (p.N <= 4) return launch_nl<4, true, false>(cplx_bwd_kernel<4, false>, p, stream);
-    if (p.N <= 8) return launch_nl<8, true, false>(cplx_bwd_kernel<8, false>, p, stream);
-    if (p.N <= 16) return launch_nl<16, true, false>(cplx_bwd_kernel<16, false>, p, stream);
-    if (p.N <= 32) return launch_nl<32, true, false>(cplx_bwd_kernel<32, false>, p, stream);
-    return cudaErrorInvalidValue;
+    const bool real = !p.theta && !p.B_im && !p.C_im && !p.dB_im && !p.dC_im;
+    return real ? launch_bwd_n<true>(p, stream) : launch_bwd_n<false>(p, stream);
 }
 
 cudaError_t launch_cplx_reduce_D(const float* part_D, float* dD, int batch, int D, cudaStream_t stream) {

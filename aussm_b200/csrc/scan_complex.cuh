@@ -43,6 +43,7 @@ struct CplxFwdParams {
     int tile0;
     int nch, Dmod, N, L;
     long long ld_lam, lam_batch_stride, ld_row;
+    int nseg, seg_tiles;      // time-axis split into nseg segments of seg_tiles tiles (<= 1: none; needs states)
 };
 
 struct CplxBwdParams {
@@ -70,13 +71,22 @@ struct CplxBwdParams {
     float* dB_im;             // or nullptr
     float* dC_re;
     float* dC_im;             // or nullptr
-    float* part_D;            // (nch,)
+    float* part_D;            // (batch, nseg, D)
     const float* eta_in;      // (nch, N, 2) adjoint state handed over by the launch of the following window, or nullptr (= 0)
     float* eta_out;           // adjoint state for the launch of the preceding window, or nullptr (may alias eta_in)
     int accumulate;           // 1: add to part_D instead of overwriting it
     int nch, Dmod, N, L;
     long long ld_lam, lam_batch_stride, ld_row;
+    int nseg, seg_tiles;      // time-axis split (<= 1: none)
+    float* seg_eta;           // (nch, nseg, N, 2): gradient of the state after every segment
+    float* seg_mul;           // (nch, nseg, N, 2): product of a segment's multipliers
 };
+
+// Time-axis split of a launch that covers whole sequences (nseg == 1: none)
+struct CplxPlan {
+    int nseg, seg_tiles;
+};
+CplxPlan cplx_split_plan(long long batches, int D, int N, int L, bool bwd);
 
 inline long long cplx_ntiles(long long L) { return (L + kCplxTile - 1) / kCplxTile; }
 

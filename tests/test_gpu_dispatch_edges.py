@@ -3,12 +3,14 @@ import math
 
 import pytest
 import torch
+import torch.nn.functional as F
 
 import aussm_b200
-from aussm_b200 import _lib
+from aussm_b200 import _lib, variants
 from aussm_b200.s6 import selective_scan_fn
 from oracle import unitary as O
 from oracle.s6 import selective_scan_ref
+from oracle.variants import scan_complex_ref
 from tests.helpers import NAMES, model_like_inputs, scaled_error, scan_core_inputs
 
 pytestmark = pytest.mark.gpu
@@ -135,3 +137,60 @@ def test_selective_scan_cut_into_segments(shape, full):
     bound = 4.5e-7 * l + 1.2e-7 * (n + b * d)
     for k in truth:
         assert scaled_error(got[k].cpu(), truth[k]) < bound, k
+
+
+# Channels that do not fill a warp, states that do not fill their lanes, whole and cut into segments (from 768 steps).
+# Per step the multiplier (exponential, sine, cosine) and the products cost 4e-7 of the magnitude; with rho = 0 errors
+# stay, otherwise they decay.
+DECAY_SHAPES = [(2, 3, 4, 40), (1, 5, 8, 36), (1, 3, 10, 52), (2, 1, 16, 16), (1, 3, 20, 44), (1, 3, 16, 768),
+                (2, 5, 3, 900), (1, 1, 32, 1028), (1, 7, 9, 2048)]
+
+
+def decay_inputs(shape, angle, seed):
+    b, d, n, l = shape
+    g = torch.Generator().manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g)
+    return dict(rho=-F.softplus(r(b, d, n, l)), theta=3 * r(b, d, n, l) if angle else None, u=r(b, d, l),
+                dt=F.softplus(r(b, d, l)), z=r(b, d, l), B_re=r(b, n, l), B_im=r(b, n, l) if angle else None,
+                C_re=r(b, n, l), C_im=r(b, n, l) if angle else None, D=r(d)), r(b, d, l)
+
+
+@pytest.mark.parametrize("shape", DECAY_SHAPES)
+@pytest.mark.parametrize("angle", [True, False])
+def test_decaying_scan_partial_warps_and_segments(shape, angle):
+    b, d, n, l = shape
+    inp, gy = decay_inputs(shape, angle, 7000 + sum(shape))
+    results = []
+    for dev, dtype in (("cpu", torch.float64), ("cuda", torch.float32)):
+        a = {k: None if t is None else t.to(dev, dtype).requires_grad_(True) for k, t in inp.items()}
+        if dev == "cpu":
+            pair = (lambda x, y: torch.complex(x, y)) if angle else (lambda x, y: x)
+            y = scan_complex_ref(a["rho"], a["theta"], a["u"], a["dt"], a["z"], pair(a["B_re"], a["B_im"]),
+                                 pair(a["C_re"], a["C_im"]), a["D"])
+        else:
+            y = variants.scan_complex(**a)
+        (y * gy.to(dev, dtype)).sum().backward()
+        results.append({"y": y.detach()} | {k: t.grad for k, t in a.items() if t is not None})
+    assert aussm_b200.device_status() == 0
+    for k, t in results[0].items():
+        assert scaled_error(results[1][k].cpu(), t) < 8e-7 * l + 1.2e-7 * (n + b * d), k
+
+
+@pytest.mark.parametrize("shape", [(1, 3, 16, 768), (1, 2, 5, 1040)])
+@pytest.mark.parametrize("angle", [True, False])
+def test_decaying_scan_state_record_does_not_depend_on_the_segments(shape, angle):
+    """The record of the states and gradients that arrive through it, cut into segments and whole."""
+    inp, gy = decay_inputs(shape, angle, 7100 + sum(shape))
+    results = []
+    try:
+        for split in (1, 0):
+            _lib.set_option("time_split", split)
+            a = {k: None if t is None else t.cuda().requires_grad_(True) for k, t in inp.items()}
+            y, states = variants.scan_complex(**a, return_states=True)
+            weight = torch.linspace(-1, 1, states.numel(), device="cuda").view_as(states)
+            ((y * gy.cuda()).sum() + (states * weight).sum()).backward()
+            results.append({"y": y.detach(), "states": states.detach()} | {k: t.grad for k, t in a.items() if t is not None})
+    finally:
+        _lib.set_option("time_split", 1)
+    for k, t in results[1].items():
+        assert scaled_error(results[0][k], t) < 8e-7 * shape[3], k
