@@ -50,6 +50,9 @@ SIGNATURES = {
     "aussm_b200_softplus_bias_fwd": (_I, [_P, _P, ctypes.c_float, _P] + [_I] * 3 + [_P]),
     "aussm_b200_softplus_bias_bwd_workspace_bytes": (_Z, [_I] * 2),
     "aussm_b200_softplus_bias_bwd": (_I, [_P, _P, ctypes.c_float, _P, _P] + [_I] * 3 + [_P, _Z, _P]),
+    "aussm_b200_rms_norm_fwd": (_I, [_P, _P, ctypes.c_float, _P, _P, _LL, _I, _P]),
+    "aussm_b200_rms_norm_bwd_workspace_bytes": (_Z, [_LL, _I]),
+    "aussm_b200_rms_norm_bwd": (_I, [_P] * 7 + [_LL, _I, _P, _Z, _P]),
     "aussm_b200_unitary_fwd": (_I, [_P] * 15 + [_I] * 4 + [_P, _Z, _P]),
     "aussm_b200_unitary_bwd": (_I, [_P] * 29 + [_I] * 4 + [_P, _Z, _P]),
     "aussm_b200_unitary_keep_bytes": (_Z, [_I] * 4),

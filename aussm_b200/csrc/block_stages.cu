@@ -211,6 +211,140 @@ __global__ void __launch_bounds__(256) bias_reduce_kernel(const float* __restric
     dbias[i] = scale * s;
 }
 
+// ---- RMS norm over the channels of token-major rows ---------------------------------------------
+// y = x rstd w,  rstd = rsqrt(mean(x^2) + eps);  one warp per row, the row in registers (d <= 128 V, d a multiple of
+// 4), so x is read once.  Bound by HBM: 8 bytes per element forward, 12 backward (16 with `extra`); as separate
+// torch passes (square, mean, scale, weight and their adjoints) the block's norm moved about 24 and 60.
+constexpr int NORM_WARPS = 8;
+
+template <int V>
+__device__ __forceinline__ void load_row(const float* row, int d4, int lane, float4 (&v)[V]) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+        const int q = k * 32 + lane;
+        v[k] = q < d4 ? reinterpret_cast<const float4*>(row)[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+__device__ __forceinline__ float dot4(const float4& a, const float4& b) {
+    return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w)));
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+template <int V>
+__global__ void __launch_bounds__(32 * NORM_WARPS) rms_norm_fwd_kernel(const float* __restrict__ x,
+                                                                       const float* __restrict__ w, float eps,
+                                                                       float* __restrict__ y,
+                                                                       float* __restrict__ rstd, long long rows, int d) {
+    const int lane = threadIdx.x & 31, d4 = d / 4;
+    float4 wv[V];
+    load_row<V>(w, d4, lane, wv);
+    for (long long r = (long long)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * NORM_WARPS) {
+        float4 xv[V];
+        load_row<V>(x + r * d, d4, lane, xv);
+        float ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < V; ++k) ss += dot4(xv[k], xv[k]);
+        const float rs = rsqrtf(warp_sum(ss) / (float)d + eps);
+        if (lane == 0) rstd[r] = rs;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const int q = k * 32 + lane;
+            if (q < d4)
+                reinterpret_cast<float4*>(y + r * d)[q] =
+                    make_float4(xv[k].x * rs * wv[k].x, xv[k].y * rs * wv[k].y, xv[k].z * rs * wv[k].z,
+                                xv[k].w * rs * wv[k].w);
+        }
+    }
+}
+
+// dx = rstd (g w - x rstd^2 mean(g w x)) [+ extra];  partial[block][c] = sum over the block's rows of g x rstd
+template <int V>
+__global__ void __launch_bounds__(32 * NORM_WARPS) rms_norm_bwd_kernel(const float* __restrict__ g,
+                                                                       const float* __restrict__ extra,
+                                                                       const float* __restrict__ x,
+                                                                       const float* __restrict__ w,
+                                                                       const float* __restrict__ rstd,
+                                                                       float* __restrict__ dx,
+                                                                       float* __restrict__ partial, long long rows,
+                                                                       int d) {
+    __shared__ float4 sums[NORM_WARPS][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d4 = d / 4;
+    float4 wv[V], acc[V];
+    load_row<V>(w, d4, lane, wv);
+#pragma unroll
+    for (int k = 0; k < V; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (long long r = (long long)blockIdx.x * NORM_WARPS + warp; r < rows; r += (long long)gridDim.x * NORM_WARPS) {
+        float4 xv[V], gv[V];
+        load_row<V>(x + r * d, d4, lane, xv);
+        load_row<V>(g + r * d, d4, lane, gv);
+        const float rs = rstd[r];
+        float dot = 0.f;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            acc[k].x = fmaf(gv[k].x, xv[k].x * rs, acc[k].x);
+            acc[k].y = fmaf(gv[k].y, xv[k].y * rs, acc[k].y);
+            acc[k].z = fmaf(gv[k].z, xv[k].z * rs, acc[k].z);
+            acc[k].w = fmaf(gv[k].w, xv[k].w * rs, acc[k].w);
+            gv[k] = make_float4(gv[k].x * wv[k].x, gv[k].y * wv[k].y, gv[k].z * wv[k].z, gv[k].w * wv[k].w);
+            dot += dot4(gv[k], xv[k]);
+        }
+        const float m = warp_sum(dot) / (float)d * rs * rs;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const int q = k * 32 + lane;
+            if (q >= d4) continue;
+            float4 o = make_float4(rs * fmaf(-xv[k].x, m, gv[k].x), rs * fmaf(-xv[k].y, m, gv[k].y),
+                                   rs * fmaf(-xv[k].z, m, gv[k].z), rs * fmaf(-xv[k].w, m, gv[k].w));
+            if (extra) {
+                const float4 e = reinterpret_cast<const float4*>(extra + r * d)[q];
+                o.x += e.x; o.y += e.y; o.z += e.z; o.w += e.w;
+            }
+            reinterpret_cast<float4*>(dx + r * d)[q] = o;
+        }
+    }
+    // the block's warps in a fixed order
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+        __syncthreads();
+        sums[warp][lane] = acc[k];
+        __syncthreads();
+        if (warp == 0 && k * 32 + lane < d4) {
+            float4 s = sums[0][lane];
+#pragma unroll
+            for (int v = 1; v < NORM_WARPS; ++v) {
+                const float4 a = sums[v][lane];
+                s.x += a.x; s.y += a.y; s.z += a.z; s.w += a.w;
+            }
+            reinterpret_cast<float4*>(partial + (long long)blockIdx.x * d)[k * 32 + lane] = s;
+        }
+    }
+}
+
+// dw[c] = sum over blocks: one warp per 32 columns and 8 strands of blocks, strands added in order
+__global__ void __launch_bounds__(256) norm_weight_reduce_kernel(const float* __restrict__ partial,
+                                                                 float* __restrict__ dw, int blocks, int d) {
+    __shared__ float sums[8][32];
+    const int c = blockIdx.x * 32 + (threadIdx.x & 31), strand = threadIdx.x >> 5;
+    float s = 0.f;
+    if (c < d)
+        for (int b = strand; b < blocks; b += 8) s += partial[(long long)b * d + c];
+    sums[strand][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (strand == 0 && c < d) {
+        for (int k = 1; k < 8; ++k) s += sums[k][threadIdx.x];
+        dw[c] = s;
+    }
+}
+
+// four resident blocks per SM, fewer when there are fewer rows
+unsigned norm_blocks(long long rows) {
+    return (unsigned)std::min<long long>((rows + NORM_WARPS - 1) / NORM_WARPS, 148LL * 4);
+}
+
 bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 int stage_dims_ok(const char* who, int B, int D, int L) {
@@ -326,6 +460,65 @@ int aussm_b200_softplus_bias_bwd(const float* ddt, const float* dt, float scale,
         return launch_ok("softplus_bias_bwd reduction");
     }
     return AUSSM_OK;
+}
+
+static int norm_ok(const char* who, const void* a, const void* b, const void* c, long long rows, int d) {
+    if (rows <= 0 || d <= 0 || d % 4 || d > AUSSM_MAX_NORM_CHANNELS) {
+        set_error("%s: rows=%lld must be positive and d=%d a multiple of 4 up to %d", who, rows, d, AUSSM_MAX_NORM_CHANNELS);
+        return AUSSM_EINVAL;
+    }
+    if (!a || !b || !c || !al16(a) || !al16(b) || !al16(c)) {
+        set_error("%s: null or misaligned (16 bytes) pointer", who);
+        return AUSSM_EINVAL;
+    }
+    return AUSSM_OK;
+}
+
+#define AUSSM_NORM(KERNEL, ...)                                                                        \
+    do {                                                                                               \
+        const dim3 grid(norm_blocks(rows)), block(32 * NORM_WARPS);                                    \
+        if (d <= 128) KERNEL<1><<<grid, block, 0, (cudaStream_t)stream>>>(__VA_ARGS__);                \
+        else if (d <= 256) KERNEL<2><<<grid, block, 0, (cudaStream_t)stream>>>(__VA_ARGS__);           \
+        else if (d <= 512) KERNEL<4><<<grid, block, 0, (cudaStream_t)stream>>>(__VA_ARGS__);           \
+        else KERNEL<8><<<grid, block, 0, (cudaStream_t)stream>>>(__VA_ARGS__);                         \
+        count_launch();                                                                                \
+    } while (0)
+
+int aussm_b200_rms_norm_fwd(const float* x, const float* w, float eps, float* y, float* rstd, long long rows, int d,
+                            aussm_stream_t stream) {
+    if (int rc = norm_ok("rms_norm_fwd", x, w, y, rows, d)) return rc;
+    if (!rstd) {
+        set_error("rms_norm_fwd: null pointer");
+        return AUSSM_EINVAL;
+    }
+    AUSSM_NORM(rms_norm_fwd_kernel, x, w, eps, y, rstd, rows, d);
+    return launch_ok("rms_norm_fwd");
+}
+
+size_t aussm_b200_rms_norm_bwd_workspace_bytes(long long rows, int d) {
+    if (rows <= 0 || d <= 0) return 0;
+    return ((size_t)norm_blocks(rows) * d * sizeof(float) + 255) / 256 * 256;
+}
+
+int aussm_b200_rms_norm_bwd(const float* g, const float* extra, const float* x, const float* w, const float* rstd,
+                            float* dx, float* dw, long long rows, int d, void* workspace, size_t workspace_bytes,
+                            aussm_stream_t stream) {
+    if (int rc = norm_ok("rms_norm_bwd", x, w, dx, rows, d)) return rc;
+    if (!g || !rstd || !dw || !al16(g) || !al16(extra)) {
+        set_error("rms_norm_bwd: null or misaligned (16 bytes) pointer");
+        return AUSSM_EINVAL;
+    }
+    const size_t need = aussm_b200_rms_norm_bwd_workspace_bytes(rows, d);
+    if (!workspace || workspace_bytes < need || !al16(workspace)) {
+        set_error("rms_norm_bwd: workspace of %zu bytes (16-byte aligned) required, got %zu", need, workspace_bytes);
+        return AUSSM_EWORKSPACE;
+    }
+    float* partial = static_cast<float*>(workspace);
+    AUSSM_NORM(rms_norm_bwd_kernel, g, extra, x, w, rstd, dx, partial, rows, d);
+    if (int rc = launch_ok("rms_norm_bwd")) return rc;
+    norm_weight_reduce_kernel<<<(d + 31) / 32, 256, 0, (cudaStream_t)stream>>>(partial, dw, (int)norm_blocks(rows), d);
+    count_launch();
+    return launch_ok("rms_norm_bwd reduction");
 }
 
 }  // extern "C"

@@ -34,7 +34,7 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(d_model))
 
     def forward(self, x):
-        return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + self.eps) * self.weight
+        return stages.rms_norm(x, self.weight, self.eps)
 
 
 def _causal_depthwise_conv(conv: nn.Conv1d, x_bld: torch.Tensor) -> torch.Tensor:
@@ -166,6 +166,14 @@ class MambaBlock(nn.Module):
         return stages.project_back(self.out_proj.weight, y, self.out_proj.bias)
 
 
+def _has_hooks(m: nn.Module) -> bool:
+    from torch.nn.modules import module as hooks
+    return bool(type(m) is not RMSNorm or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks
+                or m._backward_hooks or m._backward_pre_hooks or hooks._global_forward_hooks
+                or hooks._global_forward_pre_hooks or hooks._global_backward_hooks
+                or hooks._global_backward_pre_hooks)
+
+
 class ResidualBlock(nn.Module):
     """x + mixer(norm(x))."""
 
@@ -175,7 +183,10 @@ class ResidualBlock(nn.Module):
         self.norm = RMSNorm(d_model)
 
     def forward(self, x):
-        return self.mixer(self.norm(x)) + x
+        if _has_hooks(self.norm):              # somebody watches the norm: call it as a module
+            return self.mixer(self.norm(x)) + x
+        normed, residual = stages.rms_norm_residual(x, self.norm.weight, self.norm.eps)
+        return self.mixer(normed) + residual
 
 
 def _build_layers(layers: str, d_model, d_state, mamba_expand, dt_rank, d_conv, conv_bias, bias, ssmau_conv_1d):

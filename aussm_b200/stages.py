@@ -23,7 +23,8 @@ from . import _lib
 from .ops import _f32c, _ptr, _stream, _workspace
 from .variants import _gemm
 
-__all__ = ["causal_conv_bias", "softplus_bias", "project_tokens", "project_channels", "project_back"]
+__all__ = ["causal_conv_bias", "softplus_bias", "project_tokens", "project_channels", "project_back", "rms_norm",
+           "rms_norm_residual"]
 
 # Below this many floating-point operations a product runs on torch.matmul (over views: still no copies); the
 # split GEMM spends two passes over each operand on its FP16 parts before the product starts.
@@ -110,6 +111,90 @@ def softplus_bias(pre: Tensor, bias: Tensor = None, scale: float = 1.0) -> Tenso
     (aussm.py:878-880, where dt_proj's bias enters a second time) in one pass."""
     b, d, l = pre.shape
     return _SoftplusBias.apply(_f32c("pre", pre, (b, d, l)), None if bias is None else _f32c("bias", bias, (d,)), scale)
+
+
+# ---------------------------------------------------------------------------
+# RMS norm
+# ---------------------------------------------------------------------------
+MAX_NORM_CHANNELS = 1024
+
+
+def _rms_norm_ops(x: Tensor, weight: Tensor, eps: float) -> Tensor:
+    return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * weight
+
+
+def _norm_kernel_takes(x: Tensor, weight: Tensor) -> bool:
+    """The kernels serve whole rows of quads in eager mode; everything else (other types and devices, odd widths,
+    function transforms, forward-mode differentiation, tracing) takes the plain operations."""
+    return (x.is_cuda and x.dtype == torch.float32 and weight.dtype == torch.float32 and weight.device == x.device
+            and weight.dim() == 1 and x.dim() >= 1 and x.shape[-1] == weight.shape[0] and x.numel() > 0
+            and x.shape[-1] % 4 == 0 and x.shape[-1] <= MAX_NORM_CHANNELS
+            and type(x) is Tensor and isinstance(weight, Tensor)
+            and not torch._C._are_functorch_transforms_active()
+            and torch.autograd.forward_ad._current_level < 0 and not torch.compiler.is_compiling())
+
+
+def _aligned(t: Tensor) -> Tensor:
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+class _RMSNorm(torch.autograd.Function):
+    """(norm(x), x): the second output carries the residual branch, whose gradient joins in the same pass."""
+
+    @staticmethod
+    def forward(ctx, x, weight, eps):
+        xc, w = _aligned(x), _aligned(weight)
+        d = xc.shape[-1]
+        rows = xc.numel() // d
+        y = torch.empty_like(xc)
+        rstd = torch.empty(rows, device=xc.device, dtype=torch.float32)
+        with torch.cuda.device(xc.device):
+            rc = _lib.load().aussm_b200_rms_norm_fwd(_ptr(xc), _ptr(w), eps, _ptr(y), _ptr(rstd), rows, d, _stream(xc))
+        _lib.check(rc, "rms_norm")
+        ctx.save_for_backward(x, weight, rstd)
+        ctx.eps = eps
+        ctx.set_materialize_grads(False)
+        return y, x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, g, extra):
+        x, weight, rstd = ctx.saved_tensors
+        if g is None:
+            return extra, None, None
+        if torch.is_grad_enabled():                    # a graph of the gradient is wanted: differentiable operations
+            r = torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + ctx.eps)
+            gw = g * weight
+            dx = r * gw - x * r.pow(3) * (gw * x).mean(-1, keepdim=True)
+            dw = (g * x * r).reshape(-1, x.shape[-1]).sum(0)
+            return dx if extra is None else dx + extra, dw, None
+        lib = _lib.load()
+        xc, w, gc = _aligned(x), _aligned(weight), _aligned(g)
+        ec = None if extra is None else _aligned(extra)
+        d = xc.shape[-1]
+        rows = xc.numel() // d
+        dx, dw = torch.empty_like(xc), torch.empty(d, device=xc.device, dtype=torch.float32)
+        with torch.cuda.device(xc.device):
+            ws = _workspace(lib.aussm_b200_rms_norm_bwd_workspace_bytes(rows, d), xc.device)
+            rc = lib.aussm_b200_rms_norm_bwd(_ptr(gc), _ptr(ec), _ptr(xc), _ptr(w), _ptr(rstd), _ptr(dx), _ptr(dw), rows, d,
+                                             _ptr(ws), ws.numel(), _stream(xc))
+        _lib.check(rc, "rms_norm backward")
+        return dx, dw, None
+
+
+def rms_norm(x: Tensor, weight: Tensor, eps: float = 1e-5) -> Tensor:
+    """``x * rsqrt(mean(x^2, -1) + eps) * weight`` (the reference's RMSNorm, aussm.py:905-916) in one pass."""
+    if not _norm_kernel_takes(x, weight):
+        return _rms_norm_ops(x, weight, eps)
+    return _RMSNorm.apply(x, weight, float(eps))[0]
+
+
+def rms_norm_residual(x: Tensor, weight: Tensor, eps: float = 1e-5):
+    """``(rms_norm(x), x)``: the pair a residual block needs; adding the second to the mixer's output lets the two
+    gradients of x meet in the norm's backward pass instead of in a pass of their own."""
+    if not _norm_kernel_takes(x, weight):
+        return _rms_norm_ops(x, weight, eps), x
+    return _RMSNorm.apply(x, weight, float(eps))
 
 
 # ---------------------------------------------------------------------------

@@ -346,6 +346,17 @@ int aussm_b200_softplus_bias_bwd(const float* ddt, const float* dt, float scale,
                                  float* dbias, /* may be NULL */
                                  int B, int D, int L, void* workspace, size_t workspace_bytes, aussm_stream_t stream);
 
+/* RMS norm over the last axis of x (rows, d), d a multiple of 4 up to AUSSM_MAX_NORM_CHANNELS, all pointers 16-byte
+ * aligned:  y = x rstd w,  rstd (rows) = rsqrt(mean(x^2) + eps).  Backward: g is the gradient of y; `extra` (rows, d),
+ * when not NULL, is added to dx (a residual branch's gradient). */
+#define AUSSM_MAX_NORM_CHANNELS 1024
+int aussm_b200_rms_norm_fwd(const float* x, const float* w, float eps, float* y, float* rstd, long long rows, int d,
+                            aussm_stream_t stream);
+size_t aussm_b200_rms_norm_bwd_workspace_bytes(long long rows, int d);
+int aussm_b200_rms_norm_bwd(const float* g, const float* extra, /* may be NULL */
+                            const float* x, const float* w, const float* rstd, float* dx, float* dw, long long rows,
+                            int d, void* workspace, size_t workspace_bytes, aussm_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -6,7 +6,7 @@ import torch
 import torch.nn.functional as F
 
 import aussm_b200
-from aussm_b200 import _lib, variants
+from aussm_b200 import _lib, stages, variants
 from aussm_b200.s6 import selective_scan_fn
 from oracle import unitary as O
 from oracle.s6 import selective_scan_ref
@@ -194,3 +194,30 @@ def test_decaying_scan_state_record_does_not_depend_on_the_segments(shape, angle
         _lib.set_option("time_split", 1)
     for k, t in results[1].items():
         assert scaled_error(results[0][k], t) < 8e-7 * shape[3], k
+
+
+# A row's mean square sums d products (a lane d / 32 of them in a chain, then five additions), the rest is a handful
+# of roundings; the weight's gradient sums over the rows.
+@pytest.mark.parametrize("rows,d", [(1, 4), (3, 128), (9, 132), (7, 252), (1300, 516), (5000, 1024), (2, 1028), (4, 30)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_rms_norm_and_its_residual(rows, d, shift):
+    g = torch.Generator().manual_seed(5000 + rows + d)
+    r = lambda *s: torch.randn(*s, generator=g)
+    x, w, gy, gr = r(rows, d) * 3, r(d), r(rows, d), r(rows, d)
+    results = []
+    for dev, dtype in (("cpu", torch.float64), ("cuda", torch.float32)):
+        flat = torch.zeros(rows * d + shift, device=dev, dtype=dtype)      # shift: rows that are not 16-byte aligned
+        flat[shift:] = x.to(dev, dtype).reshape(-1)
+        xs = flat[shift:].view(rows, d).requires_grad_(True)
+        ws = w.to(dev, dtype).requires_grad_(True)
+        if dev == "cpu":
+            y, res = xs * torch.rsqrt(xs.pow(2).mean(-1, keepdim=True) + 1e-5) * ws, xs
+        else:
+            y, res = stages.rms_norm_residual(xs, ws)
+        loss = (y * gy.to(dev, dtype)).sum() + (res * gr.to(dev, dtype)).sum()
+        dx, dw = torch.autograd.grad(loss, (xs, ws), create_graph=True)
+        (ddx,) = torch.autograd.grad((dx * gy.to(dev, dtype)).sum(), xs)
+        plain = torch.autograd.grad((stages.rms_norm(xs, ws) * gy.to(dev, dtype)).sum(), (xs, ws))
+        results.append([y, dx, dw, ddx, *plain])
+    for t, o in zip(*results):
+        assert scaled_error(o.detach().cpu(), t.detach()) < 1.2e-7 * (16 + d / 16 + (rows if t.dim() == 1 else 0))
