@@ -53,6 +53,8 @@ SIGNATURES = {
     "aussm_b200_rms_norm_fwd": (_I, [_P, _P, ctypes.c_float, _P, _P, _LL, _I, _P]),
     "aussm_b200_rms_norm_bwd_workspace_bytes": (_Z, [_LL, _I]),
     "aussm_b200_rms_norm_bwd": (_I, [_P] * 7 + [_LL, _I, _P, _Z, _P]),
+    "aussm_b200_polar_params_fwd": (_I, [_P] * 3 + [_I, _P]),
+    "aussm_b200_polar_params_bwd": (_I, [_P] * 8 + [_I, _P]),
     "aussm_b200_unitary_fwd": (_I, [_P] * 15 + [_I] * 4 + [_P, _Z, _P]),
     "aussm_b200_unitary_bwd": (_I, [_P] * 29 + [_I] * 4 + [_P, _Z, _P]),
     "aussm_b200_unitary_keep_bytes": (_Z, [_I] * 4),

@@ -340,6 +340,34 @@ __global__ void __launch_bounds__(256) norm_weight_reduce_kernel(const float* __
     }
 }
 
+// ---- polar form of the operator's B and C -------------------------------------------------------
+// r = softplus(re) (re above 20 passes through, as torch's softplus), angle = im; both parameters in one launch each
+// way: the views, softplus, copies and their adjoints were 16 launches of a training call (B8 D16 N4 L256: 41 -> 23
+// launches with the zero states gone too).
+__global__ void __launch_bounds__(128) polar_params_fwd_kernel(const float2* __restrict__ B, const float2* __restrict__ C,
+                                                               float* __restrict__ out, int N) {
+    const int j = blockIdx.x * 128 + threadIdx.x;
+    if (j >= 2 * N) return;
+    const float2 v = j < N ? B[j] : C[j - N];
+    float* o = out + (j < N ? j : N + j);                     // rows B_r, B_theta, C_r, C_theta
+    o[0] = v.x > 20.f ? v.x : log1pf(expf(v.x));
+    o[N] = v.y;
+}
+
+__global__ void __launch_bounds__(128) polar_params_bwd_kernel(const float* __restrict__ dBr, const float* __restrict__ dBt,
+                                                               const float* __restrict__ dCr, const float* __restrict__ dCt,
+                                                               const float2* __restrict__ B, const float2* __restrict__ C,
+                                                               float2* __restrict__ dB, float2* __restrict__ dC, int N) {
+    const int j = blockIdx.x * 128 + threadIdx.x;
+    if (j >= 2 * N) return;
+    const bool b = j < N;
+    const int i = b ? j : j - N;
+    const float x = b ? B[i].x : C[i].x;
+    const float *gr = b ? dBr : dCr, *gt = b ? dBt : dCt;
+    const float e = expf(x), g = gr ? gr[i] : 0.f;
+    (b ? dB : dC)[i] = make_float2(x > 20.f ? g : g * e / (e + 1.f), gt ? gt[i] : 0.f);
+}
+
 // four resident blocks per SM, fewer when there are fewer rows
 unsigned norm_blocks(long long rows) {
     return (unsigned)std::min<long long>((rows + NORM_WARPS - 1) / NORM_WARPS, 148LL * 4);
@@ -472,6 +500,30 @@ static int norm_ok(const char* who, const void* a, const void* b, const void* c,
         return AUSSM_EINVAL;
     }
     return AUSSM_OK;
+}
+
+int aussm_b200_polar_params_fwd(const float* B, const float* C, float* out, int N, aussm_stream_t stream) {
+    if (N <= 0 || N > 0x3fffffff || !B || !C || !out) {
+        set_error("polar_params_fwd: null pointer or N=%d out of range", N);
+        return AUSSM_EINVAL;
+    }
+    polar_params_fwd_kernel<<<(2 * N + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
+        reinterpret_cast<const float2*>(B), reinterpret_cast<const float2*>(C), out, N);
+    count_launch();
+    return launch_ok("polar_params_fwd");
+}
+
+int aussm_b200_polar_params_bwd(const float* dB_r, const float* dB_theta, const float* dC_r, const float* dC_theta,
+                                const float* B, const float* C, float* dB, float* dC, int N, aussm_stream_t stream) {
+    if (N <= 0 || N > 0x3fffffff || !B || !C || !dB || !dC) {
+        set_error("polar_params_bwd: null pointer or N=%d out of range", N);
+        return AUSSM_EINVAL;
+    }
+    polar_params_bwd_kernel<<<(2 * N + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
+        dB_r, dB_theta, dC_r, dC_theta, reinterpret_cast<const float2*>(B), reinterpret_cast<const float2*>(C),
+        reinterpret_cast<float2*>(dB), reinterpret_cast<float2*>(dC), N);
+    count_launch();
+    return launch_ok("polar_params_bwd");
 }
 
 #define AUSSM_NORM(KERNEL, ...)                                                                        \

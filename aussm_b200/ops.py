@@ -101,7 +101,8 @@ def _check_op_inputs(u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, D, z, h_re, h
             u, _f32c("dt", dt, (b, d, l)), _f32c("x", x, (d, n, d)), _f32c("x_bias", x_bias, (d, n)),
             _f32c("B_r", B_r, (n,)), _f32c("B_theta", B_theta, (n,)), _f32c("C_r", C_r, (n,)),
             _f32c("C_theta", C_theta, (n,)), _f32c("D", D, (d,)), _f32c("z", z, (b, d, l)),
-            _f32c("prev_hid_real", h_re, (b, d, n)), _f32c("prev_hid_imag", h_im, (b, d, n)))
+            None if h_re is None else _f32c("prev_hid_real", h_re, (b, d, n)),        # no state: zero
+            None if h_im is None else _f32c("prev_hid_imag", h_im, (b, d, n)))
 
 
 def _unitary_forward(u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, D, z, h_re, h_im):
@@ -136,7 +137,7 @@ def _unitary_backward(grad_y, g_re, g_im, u, dt, x, x_bias, B_r, B_theta, C_r, C
     g_re = None if g_re is None else _f32c("grad_next_hid_real", g_re, (b, d, n))
     g_im = None if g_im is None else _f32c("grad_next_hid_imag", g_im, (b, d, n))
     if (g_re is None) != (g_im is None):
-        zero = torch.zeros_like(h_re)
+        zero = torch.zeros_like(g_re if g_im is None else g_im)
         g_re = zero if g_re is None else g_re
         g_im = zero if g_im is None else g_im
     f_re = f_im = None
@@ -147,7 +148,7 @@ def _unitary_backward(grad_y, g_re, g_im, u, dt, x, x_bias, B_r, B_theta, C_r, C
     dx, dxb = torch.empty_like(x), torch.empty_like(x_bias)
     dBr, dBt, dCr, dCt = (torch.empty_like(B_r) for _ in range(4))
     dD = torch.empty_like(D)
-    dh_re, dh_im = torch.empty_like(h_re), torch.empty_like(h_im)
+    dh_re, dh_im = (None, None) if h_re is None else (torch.empty_like(h_re), torch.empty_like(h_im))
     if l == 0 or b == 0:
         for t in (du, ddt, dz, dx, dxb, dBr, dBt, dCr, dCt, dD):
             t.zero_()
@@ -212,7 +213,7 @@ def _fits_a_quarter(nbytes: int, device) -> bool:
 
 def _want_keep(inputs, b, d, n, l) -> int:
     """Size of the phase buffer to keep for this call, or 0 for the recomputing path."""
-    if keep_phases is False or not torch.is_grad_enabled() or not any(t.requires_grad for t in inputs):
+    if keep_phases is False or not torch.is_grad_enabled() or not any(t is not None and t.requires_grad for t in inputs):
         return 0
     if b == 0 or l == 0:
         return 0
@@ -229,7 +230,8 @@ class _UnitaryKeep(torch.autograd.Function):
     def forward(ctx, keep_bytes, *inputs):
         (b, d, n, l, u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, D, z, h_re, h_im) = _check_op_inputs(*inputs)
         lib = _lib.load()
-        y, o_re, o_im = torch.empty_like(u), torch.empty_like(h_re), torch.empty_like(h_im)
+        y = torch.empty_like(u)
+        o_re, o_im = (torch.empty(b, d, n, device=u.device, dtype=torch.float32) for _ in range(2))
         keep = torch.empty(keep_bytes, dtype=torch.uint8, device=u.device)
         with torch.cuda.device(u.device):
             ws = _workspace(lib.aussm_b200_unitary_workspace_bytes(b, d, n, l), u.device)
@@ -240,6 +242,7 @@ class _UnitaryKeep(torch.autograd.Function):
         _lib.check(rc, "ssm_adaptive_unitary (phases kept)")
         _poll_status("ssm_adaptive_unitary (phases kept)", u.device)
         ctx.save_for_backward(u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, D, z, h_re, h_im, o_re, o_im)
+        ctx.set_materialize_grads(False)       # the states' gradients are mostly absent: no zeros for them
         ctx.keep = keep
         return y, o_re, o_im
 
@@ -256,12 +259,16 @@ class _UnitaryKeep(torch.autograd.Function):
 def ssm_adaptive_unitary(u: Tensor, dt: Tensor, x: Tensor, x_bias: Tensor, B_r: Tensor, B_theta: Tensor,
                          C_r: Tensor, C_theta: Tensor, D: Tensor, z: Tensor, prev_hidden_state_real: Tensor,
                          prev_hidden_state_imag: Tensor) -> Tuple[Tensor, Tensor, Tensor]:
-    """The operator call of the reference (ops.py:97-105): returns (y, next_hid_real, next_hid_imag)."""
+    """The operator call of the reference (ops.py:97-105): returns (y, next_hid_real, next_hid_imag).  Both previous
+    states may be None (zero)."""
     inputs = (u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, D, z, prev_hidden_state_real, prev_hidden_state_imag)
     if u.is_cuda and u.dim() == 3 and x.dim() == 3:
         keep_bytes = _want_keep(inputs, u.shape[0], u.shape[1], x.shape[1], u.shape[2])
         if keep_bytes:
             return _UnitaryKeep.apply(keep_bytes, *inputs)
+    if prev_hidden_state_real is None and prev_hidden_state_imag is None:      # the op's schema has no optional state
+        zeros = torch.zeros((u.shape[0], u.shape[1], x.shape[1]), device=u.device, dtype=torch.float32)
+        inputs = inputs[:10] + (zeros, zeros.clone())
     return torch.ops.extension_cpp.ssm_adaptive_unitary.default(*inputs)
 
 
@@ -292,6 +299,50 @@ def _backward(ctx, grad_y, grad_next_hid_real, grad_next_hid_imag):
 torch.library.register_autograd("extension_cpp::ssm_adaptive_unitary", _backward, setup_context=_setup_context)
 
 
+class _PolarParams(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, B, C):
+        Bc, Cc = (t.resolve_conj().contiguous() for t in (B, C))
+        n = Bc.shape[0]
+        out = torch.empty(4, n, device=B.device, dtype=torch.float32)
+        with torch.cuda.device(B.device):
+            rc = _lib.load().aussm_b200_polar_params_fwd(_ptr(Bc), _ptr(Cc), _ptr(out), n, _stream(out))
+        _lib.check(rc, "polar parameters")
+        ctx.save_for_backward(B, C)
+        ctx.set_materialize_grads(False)
+        return tuple(out.unbind(0))
+
+    @staticmethod
+    def backward(ctx, *g):
+        B, C = ctx.saved_tensors
+        if torch.is_grad_enabled():                    # a graph of the gradient is wanted: differentiable operations
+            zero = torch.zeros_like(B.real)
+            gBr, gBt, gCr, gCt = (zero if t is None else t for t in g)
+            return (torch.complex(gBr * torch.sigmoid(B.real), gBt), torch.complex(gCr * torch.sigmoid(C.real), gCt))
+        Bc, Cc = (t.resolve_conj().contiguous() for t in (B, C))
+        g = [None if t is None else t.contiguous() for t in g]
+        dB, dC = torch.empty_like(Bc), torch.empty_like(Cc)
+        with torch.cuda.device(B.device):
+            rc = _lib.load().aussm_b200_polar_params_bwd(*(_ptr(t) for t in g), _ptr(Bc), _ptr(Cc), _ptr(dB), _ptr(dC),
+                                                         Bc.shape[0], _stream(Bc))
+        _lib.check(rc, "polar parameters backward")
+        return dB, dC
+
+
+def _eager() -> bool:
+    """No function transform, forward-mode differentiation or tracing around this call."""
+    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+                or torch.compiler.is_compiling())
+
+
+def _polar_params(B: Tensor, C: Tensor):
+    """(B_r, B_theta, C_r, C_theta) with radius softplus(real part) and angle imaginary part."""
+    if (B.is_cuda and C.device == B.device and B.dtype == C.dtype == torch.complex64 and B.dim() == 1
+            and B.shape == C.shape and B.numel() > 0 and _eager()):
+        return _PolarParams.apply(B, C)
+    return (F.softplus(B.real).contiguous(), B.imag.contiguous(), F.softplus(C.real).contiguous(), C.imag.contiguous())
+
+
 def pad_to_multiple_of(tensor: Tensor, multiple_of: int) -> Tensor:
     """Zero-pad the last axis up to a multiple (reference: ops.py:21-25)."""
     pad = (-tensor.shape[-1]) % multiple_of
@@ -319,17 +370,14 @@ def ssm_adaptive_interface(u: Tensor, dt: Tensor, x: Tensor, x_bias: Tensor, B: 
     dt = pad_to_multiple_of(dt, 16).contiguous()
     z = pad_to_multiple_of(z, 16).contiguous()
     l = u.shape[-1]
-    B_r = F.softplus(B.real).contiguous()
-    B_theta = B.imag.contiguous()
-    C_r = F.softplus(C.real).contiguous()
-    C_theta = C.imag.contiguous()
-    h_re = torch.zeros((b, d, n), device=u.device, dtype=torch.float32)
-    h_im = torch.zeros((b, d, n), device=u.device, dtype=torch.float32)
+    B_r, B_theta, C_r, C_theta = _polar_params(B, C)
     chunk = l if max_parallel_length is None or max_parallel_length >= 2048 else int(max_parallel_length)
     if chunk >= l:
         out, _, _ = ssm_adaptive_unitary(u, dt, x.contiguous(), x_bias.contiguous(), B_r, B_theta, C_r, C_theta,
-                                         D.contiguous(), z, h_re, h_im)
+                                         D.contiguous(), z, None, None)
     else:
+        h_re = torch.zeros((b, d, n), device=u.device, dtype=torch.float32)
+        h_im = torch.zeros((b, d, n), device=u.device, dtype=torch.float32)
         pieces = []
         for s in range(0, l, chunk):
             e = min(s + chunk, l)
@@ -370,6 +418,7 @@ class _ScanUnitary(torch.autograd.Function):
                 0 if ws is None else ws.numel(), _stream(u))
         _lib.check(rc, "scan_unitary forward")
         ctx.save_for_backward(theta, u, dt, z, B_r, B_theta, C_r, C_theta, D, h_re, h_im)
+        ctx.set_materialize_grads(False)       # the states' gradients are mostly absent: no zeros for them
         ctx.has_h0 = h0_re is not None
         return y, h_re, h_im
 

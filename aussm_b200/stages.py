@@ -20,7 +20,7 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from .ops import _f32c, _ptr, _stream, _workspace
+from .ops import _eager, _f32c, _ptr, _stream, _workspace
 from .variants import _gemm
 
 __all__ = ["causal_conv_bias", "softplus_bias", "project_tokens", "project_channels", "project_back", "rms_norm",
@@ -130,8 +130,7 @@ def _norm_kernel_takes(x: Tensor, weight: Tensor) -> bool:
             and weight.dim() == 1 and x.dim() >= 1 and x.shape[-1] == weight.shape[0] and x.numel() > 0
             and x.shape[-1] % 4 == 0 and x.shape[-1] <= MAX_NORM_CHANNELS
             and type(x) is Tensor and isinstance(weight, Tensor)
-            and not torch._C._are_functorch_transforms_active()
-            and torch.autograd.forward_ad._current_level < 0 and not torch.compiler.is_compiling())
+            and _eager())
 
 
 def _aligned(t: Tensor) -> Tensor:

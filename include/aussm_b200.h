@@ -346,6 +346,12 @@ int aussm_b200_softplus_bias_bwd(const float* ddt, const float* dt, float scale,
                                  float* dbias, /* may be NULL */
                                  int B, int D, int L, void* workspace, size_t workspace_bytes, aussm_stream_t stream);
 
+/* Polar form of the operator's complex parameters: B, C are N interleaved (re, im) pairs; out receives the rows B_r,
+ * B_theta, C_r, C_theta (N each) with r = softplus(re), theta = im.  Backward: a NULL gradient row counts as zero. */
+int aussm_b200_polar_params_fwd(const float* B, const float* C, float* out, int N, aussm_stream_t stream);
+int aussm_b200_polar_params_bwd(const float* dB_r, const float* dB_theta, const float* dC_r, const float* dC_theta,
+                                const float* B, const float* C, float* dB, float* dC, int N, aussm_stream_t stream);
+
 /* RMS norm over the last axis of x (rows, d), d a multiple of 4 up to AUSSM_MAX_NORM_CHANNELS, all pointers 16-byte
  * aligned:  y = x rstd w,  rstd (rows) = rsqrt(mean(x^2) + eps).  Backward: g is the gradient of y; `extra` (rows, d),
  * when not NULL, is added to dx (a residual branch's gradient). */

@@ -6,7 +6,7 @@ import torch
 import torch.nn.functional as F
 
 import aussm_b200
-from aussm_b200 import _lib, stages, variants
+from aussm_b200 import _lib, ops, stages, variants
 from aussm_b200.s6 import selective_scan_fn
 from oracle import unitary as O
 from oracle.s6 import selective_scan_ref
@@ -221,3 +221,22 @@ def test_rms_norm_and_its_residual(rows, d, shift):
         results.append([y, dx, dw, ddx, *plain])
     for t, o in zip(*results):
         assert scaled_error(o.detach().cpu(), t.detach()) < 1.2e-7 * (16 + d / 16 + (rows if t.dim() == 1 else 0))
+
+
+# exp, log1p and the quotient to a few ulp each
+@pytest.mark.parametrize("n", [1, 5, 64, 128])
+def test_polar_parameters(n):
+    g = torch.Generator().manual_seed(6000 + n)
+    B, C = (torch.complex(torch.randn(n, generator=g) * s, torch.randn(n, generator=g)) for s in (1.0, 30.0))
+    weights = [torch.randn(n, generator=g) for _ in range(4)]
+    results = []
+    for dev, cplx, real in (("cpu", torch.complex128, torch.float64), ("cuda", torch.complex64, torch.float32)):
+        b, c = B.to(dev, cplx).requires_grad_(True), C.conj().to(dev, cplx).requires_grad_(True)
+        if dev == "cpu":
+            out = (F.softplus(b.real), b.imag, F.softplus(c.conj().real), c.conj().imag)
+        else:
+            out = ops._polar_params(b, c.conj())
+        loss = sum((o * w.to(dev, real)).sum() for o, w in zip(out, weights))
+        results.append([*out, *(torch.stack([t.real, t.imag]) for t in torch.autograd.grad(loss, (b, c)))])
+    for t, o in zip(*results):
+        assert scaled_error(o.detach().cpu(), t.detach()) < 1e-6
