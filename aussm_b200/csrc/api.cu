@@ -486,7 +486,7 @@ static int unitary_fwd_impl(const float* u, const float* dt, const float* x, con
     const OpArgs a = {u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, Dskip, z, B, D, N, L};
     ProjScratch ps;
     proj_scratch_bind(ps, ws + pl.off_proj, B, D, (long long)D * N, pl.ldw);
-    if (int rc = proj_begin(D, (long long)D * N, x, ps, (cudaStream_t)stream)) return rc;
+    proj_begin(x, ps);
     if (keep) keep_note_layout(keep, pl);
     return run_unitary_fwd(a, h0_re, h0_im, y, h1_re ? h1_re : cur_re, h1_im ? h1_im : cur_re + pl.rows, ws, pl, ps,
                            (cudaStream_t)stream, static_cast<float*>(keep));
@@ -571,7 +571,7 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
     }
     ProjScratch ps;
     proj_scratch_bind(ps, ws + pl.off_proj, B, D, (long long)D * N, pl.ldw);
-    if (int rc = proj_begin(D, (long long)D * N, x, ps, stream)) return rc;
+    proj_begin(x, ps);
 
     // final state: given by the caller, or recomputed by a state-only forward sweep
     const float* hend_re = h1_re;
@@ -619,9 +619,8 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
         p.part_nseg = nseg_b;
         p.nch = (int)nch; p.Dmod = D; p.N = N; p.L = tl;
         p.ld_theta = pl.ldw; p.ld_dtheta = pl.ldw; p.ld_row = L;
-        // the scan leaves max|dtheta| of the window behind for the FP16 split of the adjoint GEMMs
-        cudaError_t em = cudaMemsetAsync(ps.amax + 2, 0, sizeof(unsigned), stream);
-        if (em != cudaSuccess) return cuda_fail(em, "clearing the dtheta maximum");
+        // the scan leaves max|dtheta| of the window behind for the FP16 split of the adjoint GEMMs (cleared with the
+        // split of u)
         p.dtheta_amax = ps.amax + 2;
         cudaError_t e;
         const SegPlan seg = window_segments(pl.seg_bwd, tl);

@@ -208,7 +208,7 @@ int aussm_b200_complex_fwd(const float* u, const float* dt, const float* x, int 
     float* lam = reinterpret_cast<float*>(ws + pl.off_lam);
     ProjScratch ps;
     proj_scratch_bind(ps, ws + pl.off_proj, B, D, pl.M, pl.ldw);
-    if (int rc = proj_begin(D, pl.M, x, ps, stream)) return rc;
+    proj_begin(x, ps);
     const long long DN = (long long)D * N;
     const int nwin = (L + pl.window - 1) / pl.window;
     for (int w = 0; w < nwin; ++w) {
@@ -266,7 +266,7 @@ int aussm_b200_complex_bwd(const float* gy, const float* gstates, const float* u
     if (e != cudaSuccess) return cuda_fail(e, "complex_bwd: clearing dB/dC");
     ProjScratch ps;
     proj_scratch_bind(ps, ws + pl.off_proj, B, D, pl.M, pl.ldw);
-    if (int rc = proj_begin(D, pl.M, x, ps, stream)) return rc;
+    proj_begin(x, ps);
     const long long DN = (long long)D * N;
     const int nwin = (L + pl.window - 1) / pl.window;
     for (int w = nwin - 1; w >= 0; --w) {

@@ -466,8 +466,8 @@ __device__ __forceinline__ float4 load_quad(const float* row, long long c, long 
 struct QuadWalk {
     unsigned r, q;           // row, quad of the row
     unsigned dr, dq, nq;
-    __device__ __forceinline__ explicit QuadWalk(unsigned quads) : nq(quads) {
-        const unsigned first = blockIdx.x * 256u + threadIdx.x, step = gridDim.x * 256u;
+    __device__ __forceinline__ QuadWalk(unsigned quads, unsigned block, unsigned blocks) : nq(quads) {
+        const unsigned first = block * 256u + threadIdx.x, step = blocks * 256u;
         r = first / nq;
         q = first % nq;
         dr = step / nq;
@@ -481,14 +481,19 @@ struct QuadWalk {
 };
 constexpr int QUADS_IN_FLIGHT = 4;
 
+// The sources of a launch: source k owns blocks_of[k] consecutive blocks per batch entry.
+struct SplitLaunch {
+    SplitSource s[kSplitSources];
+    unsigned blocks_of[kSplitSources];
+    int vec[kSplitSources];
+    unsigned second;             // first block of the second source
+};
+
 template <bool VEC>
-__global__ void __launch_bounds__(256) absmax_kernel(const float* __restrict__ src, long long ld_src,
-                                                     long long src_bs, unsigned rows, unsigned cols,
-                                                     unsigned* __restrict__ amax) {
-    __shared__ float warp_max[8];
-    src += blockIdx.z * src_bs;
+__device__ __forceinline__ float quads_absmax(const float* __restrict__ src, long long ld_src, unsigned rows,
+                                              unsigned cols, unsigned block, unsigned blocks) {
     float m = 0.f;
-    for (QuadWalk w((cols + 3) / 4); w.r < rows;) {
+    for (QuadWalk w((cols + 3) / 4, block, blocks); w.r < rows;) {
         float4 v[QUADS_IN_FLIGHT];
 #pragma unroll
         for (int k = 0; k < QUADS_IN_FLIGHT; ++k) {
@@ -499,6 +504,17 @@ __global__ void __launch_bounds__(256) absmax_kernel(const float* __restrict__ s
         for (int k = 0; k < QUADS_IN_FLIGHT; ++k)
             m = fmaxf(fmaxf(fmaxf(m, fabsf(v[k].x)), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
     }
+    return m;
+}
+
+__global__ void __launch_bounds__(256) absmax_kernel(const SplitLaunch p) {
+    __shared__ float warp_max[8];
+    const int k = blockIdx.x >= p.second ? 1 : 0;
+    const SplitSource& s = p.s[k];
+    const unsigned id = blockIdx.x - (k ? p.second : 0u), blocks = p.blocks_of[k];
+    const float* src = s.src + (id / blocks) * s.src_batch_stride;
+    float m = p.vec[k] ? quads_absmax<true>(src, s.ld_src, (unsigned)s.rows, (unsigned)s.cols, id % blocks, blocks)
+                       : quads_absmax<false>(src, s.ld_src, (unsigned)s.rows, (unsigned)s.cols, id % blocks, blocks);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
@@ -507,22 +523,16 @@ __global__ void __launch_bounds__(256) absmax_kernel(const float* __restrict__ s
 #pragma unroll
         for (int w = 1; w < 8; ++w) m = fmaxf(m, warp_max[w]);
         // non-negative floats order like their bit patterns; NaN / inf would only spoil a result that is spoilt anyway
-        if (m > 0.f) atomicMax(amax, __float_as_uint(fminf(m, 3.0e38f)));
+        if (m > 0.f) atomicMax(s.amax, __float_as_uint(fminf(m, 3.0e38f)));
     }
 }
 
 template <bool VEC>
-__global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ src, long long ld_src,
-                                                        long long src_bs, __half* __restrict__ hi,
-                                                        __half* __restrict__ lo, long long ld_dst, long long dst_bs,
-                                                        unsigned rows, unsigned cols,
-                                                        const unsigned* __restrict__ amax) {
-    src += blockIdx.z * src_bs;
-    hi += blockIdx.z * dst_bs;
-    lo += blockIdx.z * dst_bs;
-    const float S = pow2f(scale_exponent(*amax));
+__device__ __forceinline__ void quads_split(const float* __restrict__ src, long long ld_src, __half* __restrict__ hi,
+                                            __half* __restrict__ lo, long long ld_dst, unsigned rows, unsigned cols,
+                                            float S, unsigned block, unsigned blocks) {
     const float up = pow2f(LO_SHIFT);
-    for (QuadWalk w((cols + 3) / 4); w.r < rows;) {
+    for (QuadWalk w((cols + 3) / 4, block, blocks); w.r < rows;) {
         float4 v[QUADS_IN_FLIGHT];
         long long at[QUADS_IN_FLIGHT];
 #pragma unroll
@@ -552,6 +562,19 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
             }
         }
     }
+}
+
+__global__ void __launch_bounds__(256) split_f16_kernel(const SplitLaunch p) {
+    const int k = blockIdx.x >= p.second ? 1 : 0;
+    const SplitSource& s = p.s[k];
+    const unsigned id = blockIdx.x - (k ? p.second : 0u), blocks = p.blocks_of[k];
+    const long long b = id / blocks;
+    const float* src = s.src + b * s.src_batch_stride;
+    __half* hi = static_cast<__half*>(s.hi) + b * s.dst_batch_stride;
+    __half* lo = static_cast<__half*>(s.lo) + b * s.dst_batch_stride;
+    const float S = pow2f(scale_exponent(*s.amax));
+    if (p.vec[k]) quads_split<true>(src, s.ld_src, hi, lo, s.ld_dst, (unsigned)s.rows, (unsigned)s.cols, S, id % blocks, blocks);
+    else quads_split<false>(src, s.ld_src, hi, lo, s.ld_dst, (unsigned)s.rows, (unsigned)s.cols, S, id % blocks, blocks);
 }
 
 // ---- host side --------------------------------------------------------------
@@ -723,46 +746,57 @@ int gemm_split3(const SplitOperand& A, const SplitOperand& B, float* C, const Ge
     return B.mn_major ? launch<0, 1>(maps, kp, grid, stream) : launch<0, 0>(maps, kp, grid, stream);
 }
 
-int split_f16(const float* src, long long ld_src, long long src_batch_stride, void* hi, void* lo, long long ld_dst,
-              long long dst_batch_stride, long long rows, long long cols, int batches, unsigned* amax,
-              cudaStream_t stream, bool have_amax) {
-    if (ld_dst % 8 || dst_batch_stride % 8 || ld_dst < (cols + 3) / 4 * 4 || !ok16(hi) || !ok16(lo) || !amax) {
-        set_error("split_f16: destination rows must be 16-byte aligned and hold whole quads (cols=%lld ld_dst=%lld)",
-                  cols, ld_dst);
-        return AUSSM_EINVAL;
-    }
-    const long long quads = (cols + 3) / 4, total = rows * quads;
-    if (total <= 0 || batches <= 0) return AUSSM_OK;
-    const bool vec = cols % 4 == 0 && ld_src % 4 == 0 && src_batch_stride % 4 == 0 && ok16(src);
-    cudaError_t e = have_amax ? cudaSuccess : cudaMemsetAsync(amax, 0, sizeof(unsigned), stream);
-    if (e == cudaSuccess) {
+int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream, bool have_amax) {
+    SplitLaunch p = {};
+    unsigned total_blocks = 0;
+    int used = 0;
+    for (int i = 0; i < count; ++i) {
+        const SplitSource& s = sources[i];
+        if (s.ld_dst % 8 || s.dst_batch_stride % 8 || s.ld_dst < (s.cols + 3) / 4 * 4 || !ok16(s.hi) || !ok16(s.lo) ||
+            !s.amax || used == kSplitSources) {
+            set_error("split_f16: destination rows must be 16-byte aligned and hold whole quads (cols=%lld ld_dst=%lld)",
+                      s.cols, s.ld_dst);
+            return AUSSM_EINVAL;
+        }
+        const long long total = s.rows * ((s.cols + 3) / 4);
+        if (total <= 0 || s.batches <= 0) continue;
         // eight resident blocks per SM over all batch entries (all of one wave), fewer when there is less than one
         // round of four quads per thread to do
         const long long want = (total + 256 * QUADS_IN_FLIGHT - 1) / (256 * QUADS_IN_FLIGHT);
-        const long long most = std::max<long long>(1, ((long long)sm_count() * 8 + batches - 1) / batches);
-        const dim3 g1((unsigned)std::min(want, most), 1, batches), g2 = g1;
-        const unsigned nr = (unsigned)rows, nc = (unsigned)cols;    // from 32-bit sizes
-        if (!have_amax) {
-            if (vec) absmax_kernel<true><<<g1, 256, 0, stream>>>(src, ld_src, src_batch_stride, nr, nc, amax);
-            else absmax_kernel<false><<<g1, 256, 0, stream>>>(src, ld_src, src_batch_stride, nr, nc, amax);
-            count_launch();
-        }
-        __half* h = static_cast<__half*>(hi);
-        __half* l = static_cast<__half*>(lo);
-        if (vec)
-            split_f16_kernel<true><<<g2, 256, 0, stream>>>(src, ld_src, src_batch_stride, h, l, ld_dst,
-                                                            dst_batch_stride, nr, nc, amax);
-        else
-            split_f16_kernel<false><<<g2, 256, 0, stream>>>(src, ld_src, src_batch_stride, h, l, ld_dst,
-                                                             dst_batch_stride, nr, nc, amax);
-        count_launch();
-        e = cudaGetLastError();
+        const long long most = std::max<long long>(1, ((long long)sm_count() * 8 + s.batches - 1) / s.batches);
+        p.s[used] = s;
+        p.blocks_of[used] = (unsigned)std::min(want, most);
+        p.vec[used] = s.cols % 4 == 0 && s.ld_src % 4 == 0 && s.src_batch_stride % 4 == 0 && ok16(s.src);
+        total_blocks += p.blocks_of[used] * (unsigned)s.batches;
+        if (++used == 1) p.second = total_blocks;
     }
+    if (used == 0) return AUSSM_OK;
+    if (!have_amax) {
+        absmax_kernel<<<total_blocks, 256, 0, stream>>>(p);
+        count_launch();
+    }
+    split_f16_kernel<<<total_blocks, 256, 0, stream>>>(p);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("split_f16 launch: %s", cudaGetErrorString(e));
         return AUSSM_ECUDA;
     }
     return AUSSM_OK;
+}
+
+int split_f16(const float* src, long long ld_src, long long src_batch_stride, void* hi, void* lo, long long ld_dst,
+              long long dst_batch_stride, long long rows, long long cols, int batches, unsigned* amax,
+              cudaStream_t stream, bool have_amax) {
+    const SplitSource s = {src, ld_src, src_batch_stride, hi, lo, ld_dst, dst_batch_stride, rows, cols, batches, amax};
+    if (amax && !have_amax) {
+        cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(unsigned), stream);
+        if (e != cudaSuccess) {
+            set_error("split_f16: clearing the maximum: %s", cudaGetErrorString(e));
+            return AUSSM_ECUDA;
+        }
+    }
+    return split_f16_many(&s, 1, stream, have_amax);
 }
 
 }  // namespace aussm

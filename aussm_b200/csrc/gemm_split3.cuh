@@ -61,6 +61,18 @@ bool gemm_split3_supported(const SplitOperand& A, const SplitOperand& B, const f
 // batched.  ld_dst / dst_batch_stride count halves and are multiples of 8, ld_dst >= cols rounded up to 4.
 // amax is a device word that receives the bit pattern of max|src|; have_amax: *amax already holds the maximum
 // (its producer computed it) and the pass over src that finds it is skipped.
+struct SplitSource {
+    const float* src;
+    long long ld_src, src_batch_stride;
+    void *hi, *lo;
+    long long ld_dst, dst_batch_stride, rows, cols;
+    int batches;
+    unsigned* amax;
+};
+// Several tensors (up to kSplitSources) with one launch for the maxima and one for the parts: on small operands the
+// launches are what a split costs.  The amax words must be zero (or hold the maxima: have_amax).
+constexpr int kSplitSources = 2;
+int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream, bool have_amax = false);
 int split_f16(const float* src, long long ld_src, long long src_batch_stride, void* hi, void* lo, long long ld_dst,
               long long dst_batch_stride, long long rows, long long cols, int batches, unsigned* amax,
               cudaStream_t stream, bool have_amax = false);

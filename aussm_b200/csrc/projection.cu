@@ -103,14 +103,21 @@ void proj_scratch_bind(ProjScratch& s, void* base, int B, int D, long long M_, l
     s.Dp = (long long)Dp;
 }
 
-int proj_begin(int D, long long M, const float* x, ProjScratch& s, cudaStream_t stream) {
-    return split_f16(x, D, 0, s.x_hi, s.x_lo, s.Dp, 0, M, D, 1, s.amax + 0, stream);
-}
+void proj_begin(const float* x, ProjScratch& s) { s.x = x; }
 
 int proj_split_u(const ProjDims& d, const float* u, ProjScratch& s, cudaStream_t stream) {
-    // rows r (D of them per batch entry), tl columns of this window
-    return split_f16(u + d.t0, d.L, (long long)d.D * d.L, s.u_hi, s.u_lo, d.ldw, (long long)d.D * d.ldw, d.D, d.tl, d.B,
-                     s.amax + 1, stream);
+    const int first = s.x ? 0 : 1;               // maxima to find anew: [x,] u, dtheta
+    cudaError_t e = cudaMemsetAsync(s.amax + first, 0, (3 - first) * sizeof(unsigned), stream);
+    if (e != cudaSuccess) {
+        set_error("projection: clearing the maxima: %s", cudaGetErrorString(e));
+        return AUSSM_ECUDA;
+    }
+    const SplitSource sources[2] = {
+        {s.x, d.D, 0, s.x_hi, s.x_lo, s.Dp, 0, d.M, d.D, 1, s.amax + 0},
+        // rows r (D of them per batch entry), tl columns of this window
+        {u + d.t0, d.L, (long long)d.D * d.L, s.u_hi, s.u_lo, d.ldw, (long long)d.D * d.ldw, d.D, d.tl, d.B, s.amax + 1}};
+    s.x = nullptr;
+    return split_f16_many(sources + first, 2 - first, stream);
 }
 
 int proj_theta(const ProjDims& d, const float* u, float* theta_w, ProjScratch& s, cudaStream_t stream) {

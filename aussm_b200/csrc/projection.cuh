@@ -39,6 +39,7 @@ struct ProjScratch {
     float* part;      // partial outputs of the adjoint products: (dx_runs, M, D), then (du_runs, B, D, ldw)
     int dx_runs, du_runs;
     unsigned* amax;   // bit patterns of max|x|, max|u window|, max|dtheta window|
+    const float* x;   // weight still to be split (together with the first window of u), or nullptr
     long long Dp;
 };
 
@@ -47,9 +48,10 @@ size_t proj_scratch_bytes(int B, int D, long long M, long long ldw);
 void proj_scratch_bind(ProjScratch& s, void* base, int B, int D, long long M, long long ldw);
 
 // returns 0 or a negative AUSSM_E* code (message set)
-// Splits x (once per operator call).
-int proj_begin(int D, long long M, const float* x, ProjScratch& s, cudaStream_t stream);
-// FP16 parts of the current window of u (proj_theta does this itself; proj_adjoints expects it done).
+// Notes x; its FP16 parts are made together with those of the first window of u (once per operator call).
+void proj_begin(const float* x, ProjScratch& s);
+// FP16 parts of the current window of u (proj_theta does this itself; proj_adjoints expects it done).  Clears the
+// maximum of dtheta, for a scan that collects it.
 int proj_split_u(const ProjDims& d, const float* u, ProjScratch& s, cudaStream_t stream);
 int proj_theta(const ProjDims& d, const float* u, float* theta_w, ProjScratch& s, cudaStream_t stream);
 // dx and du from dtheta_w; requires the split of u of the same window (proj_theta or proj_split_u).
