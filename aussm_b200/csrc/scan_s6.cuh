@@ -11,10 +11,7 @@
 
 namespace aussm {
 
-constexpr int kS6Tile = 32;      // steps per tile; the forward pass stores the state at every tile start
-// Channel-per-thread kernels (scan_s6_wide.cu) serve N <= kS6WideStates: 16-step tiles, record (nch, tiles, N)
-constexpr int kS6WideTile = 16;
-constexpr int kS6WideStates = 16;
+constexpr int kS6Tile = 16;      // steps per tile; the forward pass records the state at every tile start
 
 struct S6FwdParams {
     const float* u;           // (nch, L)
@@ -26,12 +23,11 @@ struct S6FwdParams {
     const float* z;           // (nch, L) or nullptr
     const float* delta_bias;  // (D,) or nullptr
     float* out;               // (nch, L)
-    float* ckpt;              // state at the start of every tile, or nullptr: (nch, N, tiles of 32 steps) for
-                              // N > 16, (nch, tiles of 16 steps, N) for N <= 16
+    float* ckpt;              // state at the start of every tile, (nch, tiles, N), or nullptr
     float* last_state;        // (nch, N) or nullptr
     int delta_softplus;
     int nch, Dmod, N, L;
-    // Time-axis split (N <= kS6WideStates, filled in by the launcher): nseg > 1 segments of seg_tiles tiles side by
+    // Time-axis split (filled in by the launcher): nseg > 1 segments of seg_tiles tiles side by
     // side.  The start state of a segment is the record's entry of its first tile.
     int nseg, seg_tiles;
 };
@@ -72,14 +68,10 @@ struct S6ReduceParams {
     int batch, D, N;
 };
 
-inline bool s6_wide(int N) { return N <= kS6WideStates; }
-// tiles of the state record (its size is nch * N * tiles floats in both layouts)
-inline long long s6_ntiles(long long L, int N) {
-    const int t = s6_wide(N) ? kS6WideTile : kS6Tile;
-    return (L + t - 1) / t;
-}
+// tiles of the state record
+inline long long s6_ntiles(long long L) { return (L + kS6Tile - 1) / kS6Tile; }
 
-// Time-axis split of the wide kernels' launches (nseg == 1: none)
+// Time-axis split of a launch (nseg == 1: none)
 struct S6Plan {
     int nseg, seg_tiles;
 };
@@ -88,8 +80,5 @@ S6Plan s6_split_plan(long long batches, int D, int N, int L, bool bwd);
 cudaError_t launch_s6_fwd(const S6FwdParams& p, cudaStream_t stream);
 cudaError_t launch_s6_bwd(const S6BwdParams& p, cudaStream_t stream);
 cudaError_t launch_s6_reduce(const S6ReduceParams& p, cudaStream_t stream);
-// N <= kS6WideStates
-cudaError_t launch_s6_wide_fwd(const S6FwdParams& p, cudaStream_t stream);
-cudaError_t launch_s6_wide_bwd(const S6BwdParams& p, cudaStream_t stream);
 
 }  // namespace aussm

@@ -1,4 +1,4 @@
-// Real selective scan ("S6") for sm_100a, several-states-per-thread kernels for up to 16 states per channel.
+// Real selective scan ("S6") for sm_100a, several-states-per-thread kernels for up to 32 states per channel.
 //
 // The S6 recurrence has a constant A, so unlike the unitary and complex scans it streams no per-state exponent:
 // per (b, i, t) it moves 16 bytes forward and 28 backward for N states of arithmetic, and what has to be cheap is
@@ -8,8 +8,7 @@
 // through a two-stage ring:
 //   * B_j(t), C_j(t) are the same for every channel of a batch entry: the lanes that own the same states read the
 //     same shared-memory address (one wavefront per distinct address, and the LPC addresses of an instruction
-//     fall into disjoint banks), against one wavefront per 2 channels in the thread-per-state kernels of
-//     scan_s6.cu, whose bound is the shared-memory pipe;
+//     fall into disjoint banks); with a thread per state and channel the shared-memory pipe was the bound;
 //   * the sum over states is a chain in the thread plus log2(LPC) shuffles: no column-sum tiles;
 //   * what depends on the channel and the step only (softplus, the gate and its derivative) is evaluated once per
 //     tile by a pass in which the lanes of a channel share the tile's steps;
@@ -22,8 +21,8 @@
 // the states at every fourth step in shared memory, and then walks the tile's four-step groups in reverse, each
 // group recomputed once more, state by state, with the state before every step held in registers.
 //
-// Same operator, arguments and gradients as scan_s6.cu (mamba_ssm.selective_scan_fn as called by
-// MambaBlock.ssm_mamba, ai-modules/wavesAI/model/aussm.py:771-805); that file serves 16 < N <= 32.
+// The operator is mamba_ssm.selective_scan_fn as called by MambaBlock.ssm_mamba (ai-modules/wavesAI/model/aussm.py:
+// 771-805).
 #include <stdint.h>
 
 #include <algorithm>
@@ -35,7 +34,7 @@
 namespace aussm {
 namespace {
 
-constexpr int WT = kS6WideTile;          // steps per tile = checkpoint interval
+constexpr int WT = kS6Tile;          // steps per tile = checkpoint interval
 constexpr int WTP = WT + 4;              // row pitch: a quarter-warp's 128-bit reads of eight rows hit disjoint banks
 constexpr int NQ = WT / 4;
 constexpr int WSTAGES = 2;
@@ -331,10 +330,16 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
 #pragma unroll
     for (int jj = 0; jj < SPT; ++jj)
         hn[jj] = jj * LPC + k < N ? ck[(long long)(last - 1) * N + jj * LPC + k] : 0.f;
-    // lane r of the channel-sum pass owns row r of the tile: dB of state r (r < NS) or dC of state r - NS
-    const int rj = lane % NS;
-    float* red_dst = (lane < NS ? p.dB : p.dC) + ((long long)b * N + min(rj, N - 1)) * L;
-    const bool red_on = lane < 2 * NS && rj < N;
+    // lane r of the channel-sum pass owns rows r, r + 32 of the tile: dB of state r (r < NS) or dC of state r - NS
+    constexpr int RROWS = (2 * NS + 31) / 32;
+    float* red_dst[RROWS];
+    bool red_on[RROWS];
+#pragma unroll
+    for (int x = 0; x < RROWS; ++x) {
+        const int row = x * 32 + lane, rj = row % NS;
+        red_dst[x] = (row < NS ? p.dB : p.dC) + ((long long)b * N + min(rj, N - 1)) * L;
+        red_on[x] = row < 2 * NS && rj < N;
+    }
 
     for (int r = 0; r < last - first; ++r) {
         const int tile = last - 1 - r;
@@ -453,14 +458,18 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
             }
             __syncwarp();
             // dB, dC: lane r adds row r over the warp's channels, one vector atomic per state and group
-            if (lane < 2 * NS) {
-                float4 acc = ld_shared_f4(red + (lane * RP) * 4);
 #pragma unroll
-                for (int l = 1; l < CPW; ++l) {
-                    const float4 v = ld_shared_f4(red + (lane * RP + l) * 4);
-                    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+            for (int x = 0; x < RROWS; ++x) {
+                const int row = x * 32 + lane;
+                if (row < 2 * NS) {
+                    float4 acc = ld_shared_f4(red + (row * RP) * 4);
+#pragma unroll
+                    for (int l = 1; l < CPW; ++l) {
+                        const float4 v = ld_shared_f4(red + (row * RP + l) * 4);
+                        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+                    }
+                    if (red_on[x]) red_add_v4w(red_dst[x] + t0 + 4 * q, acc);
                 }
-                if (red_on) red_add_v4w(red_dst + t0 + 4 * q, acc);
             }
             // the channel's d delta, du, dz of the group replace delta, u, z in the stage
             float dd[4], du[4], dz[4];
@@ -728,11 +737,32 @@ __global__ void __launch_bounds__(128) s6w_bwd_chain_kernel(const S6BwdParams p)
     }
 }
 
+// second stage of the parameter gradients: partials added over the batch entries (and segments) in a fixed order
+__global__ void __launch_bounds__(256) s6_reduce_kernel(const S6ReduceParams p) {
+    const long long o = (long long)blockIdx.x * 256 + threadIdx.x;
+    const long long DN = (long long)p.D * p.N;
+    if (o < DN) {
+        float acc = 0.f;
+        for (int b = 0; b < p.batch; ++b) acc += p.part_A[(long long)b * DN + o];
+        p.dA[o] = acc;
+    } else if (o < DN + p.D) {
+        const long long i = o - DN;
+        float aD = 0.f, ab = 0.f;
+        for (int b = 0; b < p.batch; ++b) {
+            aD += p.part_D[(long long)b * p.D + i];
+            ab += p.part_bias[(long long)b * p.D + i];
+        }
+        if (p.dD) p.dD[i] = aD;
+        if (p.dbias) p.dbias[i] = ab;
+    }
+}
+
 // Lanes per channel for a launch.  Forward: one is the cheapest per step; more when the channels alone give too few
 // warps (about three per scheduler hide the latencies of the dependent chains).  Backward: two measured best at
 // every size tried (batch 8 x 2048 channels x 4096 steps: 2.75 / 2.32 / 3.37 ms with 1 / 2 / 4 lanes; batch 32 x
 // 4096 x 1024: 4.83 / 4.14 / 4.64 ms) - one lane per channel needs every register there is, four repeat the
-// per-channel work of a group four times; four only when even two give less than one warp per scheduler.
+// per-channel work of a group four times; four only when even two give less than one warp per scheduler, and for more
+// than 16 states, where four keep the eight states per thread that two keep for 16.
 int lanes_per_channel(long long batches, int D, int NS, bool bwd) {
     static int sms = 0;                                     // the GPUs of a box are alike
     if (sms <= 0) {
@@ -774,26 +804,32 @@ cudaError_t launch_w_bwd(const S6BwdParams& p, cudaStream_t stream) {
     return launch_w<C>(s6w_bwd_kernel<NS, LPC>, p, p.nseg > 1 ? p.nseg : 1, stream);
 }
 
+// lanes per channel of a launch that is cut along the time axis: eight states per thread at most
+template <int NS>
+constexpr int split_lanes() { return NS > 16 ? 4 : 2; }
+
 template <int NS>
 cudaError_t launch_w_fwd_split(const S6FwdParams& p, cudaStream_t stream) {
-    using C = WCfg<NS, 2, false>;
-    cudaError_t e = launch_w<C>(s6w_fwd_summary_kernel<NS, 2>, p, p.nseg - 1, stream);
+    constexpr int LPC = split_lanes<NS>();
+    using C = WCfg<NS, LPC, false>;
+    cudaError_t e = launch_w<C>(s6w_fwd_summary_kernel<NS, LPC>, p, p.nseg - 1, stream);
     if (e != cudaSuccess) return e;
     s6w_fwd_chain_kernel<<<chain_blocks(p.nch, p.N), 128, 0, stream>>>(p, (p.L + WT - 1) / WT);
     count_launch();
     e = cudaGetLastError();
-    return e != cudaSuccess ? e : launch_w_fwd<NS, 2>(p, stream);
+    return e != cudaSuccess ? e : launch_w_fwd<NS, LPC>(p, stream);
 }
 
 template <int NS>
 cudaError_t launch_w_bwd_split(const S6BwdParams& p, cudaStream_t stream) {
-    using C = WCfg<NS, 2, false>;
-    cudaError_t e = launch_w<C>(s6w_bwd_summary_kernel<NS, 2>, p, p.nseg - 1, stream);
+    constexpr int LPC = split_lanes<NS>();
+    using C = WCfg<NS, LPC, false>;
+    cudaError_t e = launch_w<C>(s6w_bwd_summary_kernel<NS, LPC>, p, p.nseg - 1, stream);
     if (e != cudaSuccess) return e;
     s6w_bwd_chain_kernel<<<chain_blocks(p.nch, p.N), 128, 0, stream>>>(p);
     count_launch();
     e = cudaGetLastError();
-    return e != cudaSuccess ? e : launch_w_bwd<NS, 2>(p, stream);
+    return e != cudaSuccess ? e : launch_w_bwd<NS, LPC>(p, stream);
 }
 
 template <int NS>
@@ -809,8 +845,12 @@ cudaError_t launch_w_fwd_ns(const S6FwdParams& p, cudaStream_t stream) {
 template <int NS>
 cudaError_t launch_w_bwd_ns(const S6BwdParams& p, cudaStream_t stream) {
     if (p.nseg > 1) return launch_w_bwd_split<NS>(p, stream);
-    if (lanes_per_channel(p.nch / p.Dmod, p.Dmod, NS, true) == 4) return launch_w_bwd<NS, 4>(p, stream);
-    return launch_w_bwd<NS, 2>(p, stream);
+    if constexpr (NS > 16) {
+        return launch_w_bwd<NS, 4>(p, stream);
+    } else {
+        if (lanes_per_channel(p.nch / p.Dmod, p.Dmod, NS, true) == 4) return launch_w_bwd<NS, 4>(p, stream);
+        return launch_w_bwd<NS, 2>(p, stream);
+    }
 }
 
 }  // namespace
@@ -824,9 +864,10 @@ cudaError_t launch_w_bwd_ns(const S6BwdParams& p, cudaStream_t stream) {
 // 2067 -> 1863 us; B2 D256 N4 L300 216 -> 224 us (bound by the host).
 S6Plan s6_split_plan(long long batches, int D, int N, int L, bool bwd) {
     S6Plan plan = {1, (L + WT - 1) / WT};
-    if (!s6_wide(N) || L < 256 || !time_split_option()) return plan;
+    if (N > 32 || L < 512 || !time_split_option()) return plan;
     constexpr long long SMS = 148;                          // fixed: a workspace sized with the plan always fits
-    const long long warps = batches * ((D + 15) / 16);
+    const int per_warp = N > 16 ? 8 : 16;                   // channels
+    const long long warps = batches * ((D + per_warp - 1) / per_warp);
     if (warps >= (bwd ? 4 : 3) * SMS) return plan;
     const long long want = std::min<long long>((bwd ? 8 : 14) * SMS / warps, L / 64);
     if (want < 2) return plan;
@@ -836,7 +877,7 @@ S6Plan s6_split_plan(long long batches, int D, int N, int L, bool bwd) {
     return plan;
 }
 
-cudaError_t launch_s6_wide_fwd(const S6FwdParams& p_, cudaStream_t stream) {
+cudaError_t launch_s6_fwd(const S6FwdParams& p_, cudaStream_t stream) {
     if (p_.nch <= 0 || p_.L <= 0) return cudaSuccess;
     S6FwdParams p = p_;
     p.nseg = 1;
@@ -848,15 +889,24 @@ cudaError_t launch_s6_wide_fwd(const S6FwdParams& p_, cudaStream_t stream) {
     if (p.N <= 4) return launch_w_fwd_ns<4>(p, stream);
     if (p.N <= 8) return launch_w_fwd_ns<8>(p, stream);
     if (p.N <= 16) return launch_w_fwd_ns<16>(p, stream);
+    if (p.N <= 32) return launch_w_fwd_ns<32>(p, stream);
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_s6_wide_bwd(const S6BwdParams& p, cudaStream_t stream) {
+cudaError_t launch_s6_bwd(const S6BwdParams& p, cudaStream_t stream) {
     if (p.nch <= 0 || p.L <= 0) return cudaSuccess;
     if (p.N <= 4) return launch_w_bwd_ns<4>(p, stream);
     if (p.N <= 8) return launch_w_bwd_ns<8>(p, stream);
     if (p.N <= 16) return launch_w_bwd_ns<16>(p, stream);
+    if (p.N <= 32) return launch_w_bwd_ns<32>(p, stream);
     return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_s6_reduce(const S6ReduceParams& p, cudaStream_t stream) {
+    const long long total = (long long)p.D * p.N + p.D;
+    s6_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(p);
+    count_launch();
+    return cudaGetLastError();
 }
 
 }  // namespace aussm

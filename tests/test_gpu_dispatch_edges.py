@@ -113,7 +113,8 @@ S6_KEYS = ["u", "delta", "A", "B", "C", "D", "z", "delta_bias"]
 
 # A step of the contracting recurrence costs two roundings and the exponential's 2^-22; earlier errors decay, but at
 # worst (A near 0) stay.  Sums over states, channels and steps add an ulp per term at worst.
-@pytest.mark.parametrize("shape", [(1, 5, 16, 512), (2, 33, 4, 516), (1, 16, 7, 1028), (3, 40, 12, 516), (1, 1, 1, 4096)])
+@pytest.mark.parametrize("shape", [(1, 5, 16, 512), (2, 33, 4, 516), (1, 16, 7, 1028), (3, 40, 12, 516), (1, 1, 1, 4096),
+                                   (1, 9, 17, 520), (2, 3, 32, 1000), (40, 7, 24, 64)])
 @pytest.mark.parametrize("full", [True, False])
 def test_selective_scan_cut_into_segments(shape, full):
     b, d, n, l = shape
