@@ -530,8 +530,10 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
                 er[k] = sc[k].kr * gr + sc[k].ki * gi;
                 ei[k] = sc[k].kr * gi - sc[k].ki * gr;
                 // conj(h~_{L-1}) * gh
-                hlr[k] = hr[k] * gr + hi[k] * gi;
-                hli[k] = hr[k] * gi - hi[k] * gr;
+                if (wt.seg == wt.nseg - 1) {
+                    hlr[k] = hr[k] * gr + hi[k] * gi;
+                    hli[k] = hr[k] * gi - hi[k] * gr;
+                }
             } else {
                 hr[k] = ar; hi[k] = ai; er[k] = gr; ei[k] = gi;
             }
@@ -773,11 +775,15 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
             // dCc = conj(Bc) G_M
             dcr = kr * gmr[k] + ki * gmi[k];
             dci = kr * gmi[k] - ki * gmr[k];
-            // dBc = conj(Cc) G_M + conj(h~_{L-1}) gh - conj(h~_{-1} / Bc) carry
+            // dBc = conj(Cc) G_M + conj(h~_{L-1}) gh - conj(h~_{-1} / Bc) carry.  The boundary terms of neighbouring
+            // segments cancel; they are left out, because each is as large as the sum (with them dBc of B1 D200 N16
+            // L20001 was off by several times the error of an unsplit launch).
             float qr, qi;
             cdiv(hr[k], hi[k], kr, ki, qr, qi);
-            dbr = ccr[k] * gmr[k] + cci[k] * gmi[k] + hlr[k] - (qr * er[k] + qi * ei[k]);
-            dbi = ccr[k] * gmi[k] - cci[k] * gmr[k] + hli[k] - (qr * ei[k] - qi * er[k]);
+            dbr = ccr[k] * gmr[k] + cci[k] * gmi[k];
+            dbi = ccr[k] * gmi[k] - cci[k] * gmr[k];
+            if (wt.seg == wt.nseg - 1) { dbr += hlr[k]; dbi += hli[k]; }
+            if (wt.seg == 0) { dbr -= qr * er[k] + qi * ei[k]; dbi -= qr * ei[k] - qi * er[k]; }
             // dh0 = carry / conj(Bc) ;  h0 = Bc h~_{-1}
             cdiv(er[k], ei[k], kr, -ki, d0r, d0i);
             s0r = kr * hr[k] - ki * hi[k];
