@@ -157,11 +157,11 @@ class MambaBlock(nn.Module):
             z = z + b_in[di:, None]
         xs = stages.causal_conv_bias(xs, self.conv1d.weight, self.conv1d.bias)
         low = stages.project_channels(self.x_proj.weight, xs)       # (b, rank + 2n, l): dt, B, C rows
-        dt = stages.project_channels(self.dt_proj.weight, low[:, :r].contiguous()) + self.dt_proj.bias[:, None]
-        # dt_proj is applied with its bias, and the bias goes in once more as delta_bias (aussm.py:786-799)
+        dt = stages.project_channels(self.dt_proj.weight, low[:, :r].contiguous())
+        # dt_proj is applied with its bias, and the bias goes in once more as delta_bias (aussm.py:786-799): both here
         y = s6.selective_scan_fn(F.silu(xs), dt, (-torch.exp(self.A_log.float())).contiguous(),
                                  low[:, r:r + n].contiguous(), low[:, r + n:].contiguous(),
-                                 self.D.float().contiguous(), z=z, delta_bias=self.dt_proj.bias.float(),
+                                 self.D.float().contiguous(), z=z, delta_bias=2.0 * self.dt_proj.bias.float(),
                                  delta_softplus=True)
         return stages.project_back(self.out_proj.weight, y, self.out_proj.bias)
 

@@ -8,7 +8,7 @@ produces its result directly in ``(b, d, l)``:
 
 * ``project_tokens`` / ``project_channels`` / ``project_back``: the block's linear layers as matrix products
   whose output (or input) is channel-major, so no transposing copy exists.  Large products run on the
-  library's split GEMM (float32-accurate, tcgen05), small ones on ``torch.matmul`` over views;
+  library's split GEMM (float32-accurate, tcgen05), small ones as one batched product;
 * ``causal_conv_bias``: depthwise causal convolution + bias, one pass (``aussm_b200_conv_pre_fwd/_bwd``);
 * ``softplus_bias``: ``softplus(pre + scale * bias)``, one pass, in place (``aussm_b200_softplus_bias_fwd/_bwd``).
 
@@ -26,8 +26,7 @@ from .variants import _gemm
 __all__ = ["causal_conv_bias", "softplus_bias", "project_tokens", "project_channels", "project_back", "rms_norm",
            "rms_norm_residual"]
 
-# Below this many floating-point operations a product runs on torch.matmul (over views: still no copies); the
-# split GEMM spends two passes over each operand on its FP16 parts before the product starts.
+# Below this many floating-point operations a product runs as a batched library product over views; the split GEMM spends two passes over each operand on its FP16 parts before the product starts.
 MIN_FLOP = 2.0e10
 
 
@@ -203,6 +202,81 @@ def _big(flop: float, *dims: int) -> bool:
     return flop >= MIN_FLOP
 
 
+# Products below MIN_FLOP: one batched product per direction, in the layout the next stage reads.  torch.matmul folds
+# the batch of a shared weight into rows, which copies the channel-major side before or after the product (six to
+# eight transposing copies of a layer's training pass) and sums the weight's gradient over all b l tokens in the few
+# tiles of one output (117 us each at 46080 tokens of 128 channels).  Training pass of SSMTS, 64 x 720 steps of width 128:
+# 10.1 -> 6.9 ms of device time together with the row plans of block_stages.cu.  The gradients are ordinary operations, so
+# they can be differentiated again.
+class _BatchedTokens(torch.autograd.Function):
+    """out[b] (m, l) = W (m, k) x[b]^T"""
+
+    @staticmethod
+    def forward(ctx, W, x):
+        ctx.save_for_backward(W, x)
+        return torch.bmm(W.expand(x.shape[0], -1, -1), x.transpose(1, 2))
+
+    @staticmethod
+    def backward(ctx, g):
+        W, x = ctx.saved_tensors
+        dW = _token_product(g, x) if ctx.needs_input_grad[0] else None
+        dx = torch.bmm(g.transpose(1, 2), W.expand(x.shape[0], -1, -1)) if ctx.needs_input_grad[1] else None
+        return dW, dx
+
+
+class _BatchedChannels(torch.autograd.Function):
+    """out[b] (m, l) = W (m, k) u[b] (k, l)"""
+
+    @staticmethod
+    def forward(ctx, W, u):
+        ctx.save_for_backward(W, u)
+        return torch.bmm(W.expand(u.shape[0], -1, -1), u)
+
+    @staticmethod
+    def backward(ctx, g):
+        W, u = ctx.saved_tensors
+        dW = _token_product(g, u.transpose(1, 2)) if ctx.needs_input_grad[0] else None
+        du = torch.bmm(W.t().expand(u.shape[0], -1, -1), g) if ctx.needs_input_grad[1] else None
+        return dW, du
+
+
+class _BatchedBack(torch.autograd.Function):
+    """out[b] (l, m) = y[b]^T (l, k) W^T"""
+
+    @staticmethod
+    def forward(ctx, W, y):
+        ctx.save_for_backward(W, y)
+        return torch.bmm(y.transpose(1, 2), W.t().expand(y.shape[0], -1, -1))
+
+    @staticmethod
+    def backward(ctx, g):
+        W, y = ctx.saved_tensors
+        gt = g.transpose(1, 2)
+        dW = _token_product(gt, y.transpose(1, 2)) if ctx.needs_input_grad[0] else None
+        dy = torch.bmm(W.t().expand(y.shape[0], -1, -1), gt) if ctx.needs_input_grad[1] else None
+        return dW, dy
+
+
+def _token_product(g: Tensor, x: Tensor) -> Tensor:
+    """``sum_b g[b] x[b]`` for g (b, m, l), x (b, l, k): few tiles and a long contraction, so a single sequence is cut
+    into pieces that run as batch entries (views) and the partial products are added."""
+    b, m, l = g.shape
+    if b == 1:
+        pieces = 1
+        while pieces < 64 and l % (2 * pieces) == 0 and l // (2 * pieces) >= 256:
+            pieces *= 2
+        if pieces > 1:
+            return torch.bmm(g[0].unflatten(1, (pieces, -1)).transpose(0, 1), x[0].unflatten(0, (pieces, -1))).sum(0)
+    return torch.bmm(g, x).sum(0)
+
+
+def _batched(W: Tensor, x: Tensor, l: int) -> bool:
+    """Whether a small product runs batched: the weight's gradient then has a partial product per batch entry, which
+    may take twice the memory of the layer's input and output at most."""
+    m, k = W.shape
+    return x.is_cuda and x.dtype == W.dtype == torch.float32 and x.numel() > 0 and m * k <= 2 * l * (m + k) and _eager()
+
+
 def _weight_grad(A: Tensor, a_mn: int, B: Tensor, b_mn: int, m: int, k: int, l: int, b: int) -> Tensor:
     """``dW[m][k] = sum_b sum_t A_b(m, t) B_b(k, t)`` for batched operands whose contraction index is time.
 
@@ -269,6 +343,8 @@ def project_tokens(W: Tensor, x: Tensor) -> Tensor:
     b, l, _ = x.shape
     if _big(2.0 * b * l * m * k):
         return _ProjectTokens.apply(_f32c("W", W), _f32c("x", x, (b, l, k)))
+    if _batched(W, x, l):
+        return _BatchedTokens.apply(W, x)
     return torch.matmul(W, x.transpose(1, 2))
 
 
@@ -279,6 +355,8 @@ def project_channels(W: Tensor, u: Tensor) -> Tensor:
     if _big(2.0 * b * l * m * k):
         from .variants import _Projection
         return _Projection.apply(_f32c("W", W), _f32c("u", u, (b, k, l)))
+    if _batched(W, u, l):
+        return _BatchedChannels.apply(W, u)
     return torch.matmul(W, u)
 
 
@@ -321,6 +399,8 @@ def project_back(W: Tensor, y: Tensor, bias: Tensor = None) -> Tensor:
     b, _, l = y.shape
     if _big(2.0 * b * l * m * k):
         out = _ProjectBack.apply(_f32c("W", W), _f32c("y", y, (b, k, l)))
+    elif _batched(W, y, l):
+        out = _BatchedBack.apply(W, y)
     else:
         out = torch.matmul(y.transpose(1, 2), W.t())
     return out if bias is None else out + bias

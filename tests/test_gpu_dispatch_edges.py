@@ -241,3 +241,23 @@ def test_polar_parameters(n):
         results.append([*out, *(torch.stack([t.real, t.imag]) for t in torch.autograd.grad(loss, (b, c)))])
     for t, o in zip(*results):
         assert scaled_error(o.detach().cpu(), t.detach()) < 1e-6
+
+
+# Small products of the blocks, batched (one sequence: its weight gradient in pieces).  Sums of k or m products, the
+# weight's of b l products, an ulp each at worst.
+@pytest.mark.parametrize("b,l,m,k", [(1, 4096, 16, 24), (1, 1000, 8, 40), (3, 96, 40, 20), (64, 33, 12, 12), (2, 8, 300, 200)])
+def test_small_projections(b, l, m, k):
+    g = torch.Generator().manual_seed(8000 + b + l)
+    r = lambda *s: torch.randn(*s, generator=g)
+    cases = [(stages.project_tokens, r(b, l, k), "mk,blk->bml"), (stages.project_channels, r(b, k, l), "mk,bkl->bml"),
+             (stages.project_back, r(b, k, l), "mk,bkl->blm")]
+    for fn, x, formula in cases:
+        W, results = r(m, k), []
+        for dev, dtype in (("cpu", torch.float64), ("cuda", torch.float32)):
+            a = [t.to(dev, dtype).requires_grad_(True) for t in (W, x)]
+            y = torch.einsum(formula, *a) if dev == "cpu" else fn(*a)
+            grads = torch.autograd.grad(y.square().sum(), a, create_graph=True)
+            (second,) = torch.autograd.grad(grads[0].sum(), a[1])
+            results.append([y, *grads, second])
+        for t, o in zip(*results):
+            assert o.shape == t.shape and scaled_error(o.detach().cpu(), t.detach()) < 1.2e-7 * (m + k + b * l), fn.__name__
