@@ -26,6 +26,87 @@ namespace {
 constexpr int KMAX = AUSSM_MAX_CONV_TAPS;
 constexpr int ROW_THREADS = 256;
 
+// How a streaming kernel walks (rows, L): a row belongs to 32 to 256 threads (as many as it has quads), several short
+// rows share a block, and a long row is cut into chunks when there are too few rows to fill the GPU.  Threads take
+// whole quads, 128-bit where the rows are 16-byte aligned.
+constexpr int MAX_CHUNKS = 16;
+struct RowPlan {
+    long long rows;
+    int L, quads, vec;
+    int tpr;                 // threads per row (32, 64, 128, 256)
+    int chunks, qpc;         // chunks per row and quads per chunk (1 chunk when several rows share a block)
+    unsigned blocks;
+};
+inline int row_chunks_max(long long rows) { return rows < 148 * 16 ? MAX_CHUNKS : 1; }
+RowPlan row_plan(long long rows, int L, bool vec) {
+    RowPlan p;
+    p.rows = rows;
+    p.L = L;
+    p.quads = (int)(((long long)L + 3) / 4);
+    p.vec = vec ? 1 : 0;
+    p.tpr = 32;
+    while (p.tpr < ROW_THREADS && p.tpr < p.quads) p.tpr *= 2;
+    p.chunks = p.tpr < ROW_THREADS ? 1 : std::max(1, std::min(row_chunks_max(rows), p.quads / (2 * ROW_THREADS)));
+    p.qpc = (p.quads + p.chunks - 1) / p.chunks;
+    const long long rpb = ROW_THREADS / p.tpr;
+    p.blocks = (unsigned)((rows + rpb - 1) / rpb * p.chunks);
+    return p;
+}
+struct RowSlot {
+    long long row;
+    int chunk, lane;         // lane: thread of the row
+    int q0, q1;              // its first quad, end of the chunk (empty for a row that does not exist)
+    __device__ __forceinline__ explicit RowSlot(const RowPlan& p) {
+        chunk = (int)(blockIdx.x % (unsigned)p.chunks);
+        row = (long long)(blockIdx.x / (unsigned)p.chunks) * (ROW_THREADS / p.tpr) + threadIdx.x / p.tpr;
+        lane = threadIdx.x % p.tpr;
+        q0 = chunk * p.qpc + lane;
+        q1 = row < p.rows ? min(p.quads, (chunk + 1) * p.qpc) : 0;
+    }
+};
+
+// quad t .. t+3 of a row (t a multiple of 4), zero outside [0, L)
+__device__ __forceinline__ void load_quad(const float* row, int t, int L, int vec, float* v) {
+    if (t < 0 || t >= L) {
+        v[0] = v[1] = v[2] = v[3] = 0.f;
+    } else if (vec) {
+        const float4 f = *reinterpret_cast<const float4*>(row + t);
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = t + e < L ? row[t + e] : 0.f;
+    }
+}
+__device__ __forceinline__ void store_quad(float* row, int t, int L, int vec, const float* v) {
+    if (vec) {
+        *reinterpret_cast<float4*>(row + t) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (t + e < L) row[t + e] = v[e];
+    }
+}
+
+// Sums of n values over the threads of a row, in a fixed order; thread k < n of the row gets value k.
+template <int n>
+__device__ __forceinline__ float row_sums(float (&acc)[n], const RowPlan& p, const RowSlot& s) {
+    __shared__ float red[ROW_THREADS / 32][n];
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = acc[k];
+    }
+    __syncthreads();
+    float sum = 0.f;
+    if (s.lane < n) {
+        const int first = (threadIdx.x - s.lane) >> 5;
+        for (int w = 0; w < p.tpr / 32; ++w) sum += red[first + w][s.lane];
+    }
+    return sum;
+}
+
+// The filter right-aligned in a window of KMAX taps: u[t] = sum_m w[m] x[t - (KMAX-1) + m], m >= KMAX - K.
 struct Taps {
     float w[KMAX];
 };
@@ -33,114 +114,91 @@ struct Taps {
 __device__ __forceinline__ Taps load_taps(const float* w, int i, int K) {
     Taps t;
 #pragma unroll
-    for (int k = 0; k < KMAX; ++k) t.w[k] = k < K ? w[(long long)i * K + k] : 0.f;
+    for (int m = 0; m < KMAX; ++m) t.w[m] = m >= KMAX - K ? w[(long long)i * K + m - (KMAX - K)] : 0.f;
     return t;
 }
+static_assert(KMAX == 4, "a quad's window is the quad and its neighbour");
 
 // ---- forward: u = conv(xs) + bias -------------------------------------------------------------
-// one thread per four consecutive steps of a row
-__global__ void __launch_bounds__(256) conv_pre_fwd_kernel(const float* __restrict__ xs, const float* __restrict__ w,
-                                                           const float* __restrict__ bias, float* __restrict__ u,
-                                                           int D, int L, int K, long long quads_per_row,
-                                                           long long total_quads, int vec) {
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < total_quads;
-         q += (long long)gridDim.x * blockDim.x) {
-        const long long row = q / quads_per_row;
-        const int t0 = (int)(q % quads_per_row) * 4;
-        const int i = (int)(row % D);
-        const float* x = xs + row * L;
-        const Taps tp = load_taps(w, i, K);
-        const float bv = bias ? bias[i] : 0.f;
-        // window x[t0 - (KMAX-1) .. t0 + 3]
-        float win[KMAX + 3];
-#pragma unroll
-        for (int k = 0; k < KMAX + 3; ++k) {
-            const int t = t0 - (KMAX - 1) + k;
-            win[k] = (t >= 0 && t < L) ? x[t] : 0.f;
-        }
-        float out[4];
+__global__ void __launch_bounds__(ROW_THREADS) conv_pre_fwd_kernel(const float* __restrict__ xs, const float* __restrict__ w,
+                                                                   const float* __restrict__ bias, float* __restrict__ u,
+                                                                   int D, int K, const RowPlan p) {
+    const RowSlot s(p);
+    if (s.q0 >= s.q1) return;
+    const int i = (int)(s.row % D);
+    const float* x = xs + s.row * p.L;
+    const Taps tp = load_taps(w, i, K);
+    const float bv = bias ? bias[i] : 0.f;
+    for (int q = s.q0; q < s.q1; q += p.tpr) {
+        float win[8], out[4];                                   // x[t0 - 4 .. t0 + 3]
+        load_quad(x, 4 * q - 4, p.L, p.vec, win);
+        load_quad(x, 4 * q, p.L, p.vec, win + 4);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            float acc = bv;
-            // tap k of a K-tap filter reads x[t - (K-1) + k]; with the taps right-aligned in the KMAX window
-            // that is win[(KMAX - K) + k + e]
+            out[e] = bv;
 #pragma unroll
-            for (int k = 0; k < KMAX; ++k) {
-                const int src = (KMAX - K) + k + e;
-                if (k < K) acc = fmaf(tp.w[k], win[src < KMAX + 3 ? src : 0], acc);
-            }
-            out[e] = acc;
+            for (int m = 0; m < KMAX; ++m)
+                if (m >= KMAX - K) out[e] = fmaf(tp.w[m], win[1 + e + m], out[e]);
         }
-        float* dst = u + row * L + t0;
-        if (vec && t0 + 3 < L) {
-            *reinterpret_cast<float4*>(dst) = make_float4(out[0], out[1], out[2], out[3]);
-        } else {
-            for (int e = 0; e < 4; ++e)
-                if (t0 + e < L) dst[e] = out[e];
-        }
+        store_quad(u + s.row * p.L, 4 * q, p.L, p.vec, out);
     }
 }
 
 // ---- backward: dxs = conv^T(du); per-row partial sums of dw and dbias ---------------------------
-// one block per row; partial[(row) * (KMAX + 1) + k] = sum_t du[t] xs[t - (K-1) + k], [KMAX] = sum_t du[t]
+// partial[(row * chunks + chunk) * (KMAX + 1) + m] = sum_t du[t] xs[t - (KMAX-1) + m], [KMAX] = sum_t du[t].  Bound by HBM
+// (12 bytes a step): B1 D512 L65536 231 us with one block per row and scalar loads, 101 us now (4.0 TB/s).
 __global__ void __launch_bounds__(ROW_THREADS) conv_pre_bwd_kernel(const float* __restrict__ du,
                                                                    const float* __restrict__ xs,
                                                                    const float* __restrict__ w,
                                                                    float* __restrict__ dxs,
-                                                                   float* __restrict__ partial, int D, int L, int K) {
-    __shared__ float red[ROW_THREADS / 32][KMAX + 1];
-    const long long row = blockIdx.x;
-    const int i = (int)(row % D);
-    const float* g = du + row * L;
-    const float* x = xs + row * L;
-    float* dx = dxs + row * L;
-    const Taps tp = load_taps(w, i, K);
+                                                                   float* __restrict__ partial, int D, int K,
+                                                                   const RowPlan p) {
+    const RowSlot s(p);
+    const float* g = du + s.row * p.L;
+    const float* x = xs + s.row * p.L;
     float acc[KMAX + 1];
 #pragma unroll
     for (int k = 0; k <= KMAX; ++k) acc[k] = 0.f;
-    for (int t = threadIdx.x; t < L; t += ROW_THREADS) {
-        const float gt = g[t];
-        // dxs[t] = sum_k w[k] du[t + (K-1) - k]
-        float d = 0.f;
+    if (s.q0 < s.q1) {
+        const Taps tp = load_taps(w, (int)(s.row % D), K);
+        for (int q = s.q0; q < s.q1; q += p.tpr) {
+            float xw[8], gw[8], d[4];                           // x[t0 - 4 .. t0 + 3], du[t0 .. t0 + 7]
+            load_quad(x, 4 * q - 4, p.L, p.vec, xw);
+            load_quad(x, 4 * q, p.L, p.vec, xw + 4);
+            load_quad(g, 4 * q, p.L, p.vec, gw);
+            load_quad(g, 4 * q + 4, p.L, p.vec, gw + 4);
+            const bool inner = q > 0 && 4 * q + 7 < p.L;        // no term outside the row (nor a product with its zero)
 #pragma unroll
-        for (int k = 0; k < KMAX; ++k) {
-            if (k < K) {
-                const int tt = t + (K - 1) - k;
-                if (tt < L) d = fmaf(tp.w[k], g[tt], d);
-                const int ts = t - (K - 1) + k;
-                if (ts >= 0) acc[k] = fmaf(gt, x[ts], acc[k]);
+            for (int e = 0; e < 4; ++e) {
+                const int t = 4 * q + e;
+                d[e] = 0.f;
+#pragma unroll
+                for (int m = 0; m < KMAX; ++m) {
+                    if (m >= KMAX - K) {                        // dxs[t] = sum_m w[m] du[t + (KMAX-1) - m]
+                        if (inner || t + (KMAX - 1) - m < p.L) d[e] = fmaf(tp.w[m], gw[e + (KMAX - 1) - m], d[e]);
+                        if (inner || (t - (KMAX - 1) + m >= 0 && t < p.L)) acc[m] = fmaf(gw[e], xw[1 + e + m], acc[m]);
+                    }
+                }
+                acc[KMAX] += gw[e];
             }
+            store_quad(dxs + s.row * p.L, 4 * q, p.L, p.vec, d);
         }
-        dx[t] = d;
-        acc[KMAX] += gt;
     }
-#pragma unroll
-    for (int k = 0; k <= KMAX; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k <= KMAX; ++k) red[warp][k] = acc[k];
-    }
-    __syncthreads();
-    if (threadIdx.x <= KMAX) {
-        float s = 0.f;
-        for (int wv = 0; wv < ROW_THREADS / 32; ++wv) s += red[wv][threadIdx.x];
-        partial[row * (KMAX + 1) + threadIdx.x] = s;
-    }
+    const float sum = row_sums(acc, p, s);
+    if (s.row < p.rows && s.lane <= KMAX) partial[(s.row * p.chunks + s.chunk) * (KMAX + 1) + s.lane] = sum;
 }
 
-// dw[i][k] = sum_b partial[b][i][k], dbias[i] = sum_b partial[b][i][KMAX]
+// dw[i][k] and dbias[i] = sums of the partials over batch entries and chunks, in a fixed order
 __global__ void __launch_bounds__(256) conv_pre_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw,
-                                                              float* __restrict__ dbias, int B, int D, int K) {
+                                                              float* __restrict__ dbias, int B, int D, int K,
+                                                              int chunks) {
     const int o = blockIdx.x * 256 + threadIdx.x;
     if (o >= D * (K + 1)) return;
     const int i = o / (K + 1), k = o % (K + 1);
-    const int slot = k < K ? k : KMAX;
+    const int slot = k < K ? KMAX - K + k : KMAX;
     float s = 0.f;
-    for (int b = 0; b < B; ++b) s += partial[((long long)b * D + i) * (KMAX + 1) + slot];
+    for (int b = 0; b < B; ++b)
+        for (int c = 0; c < chunks; ++c) s += partial[(((long long)b * D + i) * chunks + c) * (KMAX + 1) + slot];
     if (k < K) dw[(long long)i * K + k] = s;
     else if (dbias) dbias[i] = s;
 }
@@ -149,65 +207,53 @@ __global__ void __launch_bounds__(256) conv_pre_reduce_kernel(const float* __res
 // torch.nn.functional.softplus with its defaults (beta 1, threshold 20): x above 20 passes through
 __device__ __forceinline__ float softplus_(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 
-__global__ void __launch_bounds__(256) softplus_bias_fwd_kernel(const float* __restrict__ pre,
-                                                                const float* __restrict__ bias, float scale,
-                                                                float* __restrict__ dt, int D, int L,
-                                                                long long quads_per_row, long long total_quads,
-                                                                int vec) {
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < total_quads;
-         q += (long long)gridDim.x * blockDim.x) {
-        const long long row = q / quads_per_row;
-        const int t0 = (int)(q % quads_per_row) * 4;
-        const float bv = bias ? scale * bias[row % D] : 0.f;
-        const float* src = pre + row * L + t0;
-        float* dst = dt + row * L + t0;
-        if (vec && t0 + 3 < L) {
-            const float4 v = *reinterpret_cast<const float4*>(src);
-            *reinterpret_cast<float4*>(dst) =
-                make_float4(softplus_(v.x + bv), softplus_(v.y + bv), softplus_(v.z + bv), softplus_(v.w + bv));
-        } else {
-            for (int e = 0; e < 4; ++e)
-                if (t0 + e < L) dst[e] = softplus_(src[e] + bv);
-        }
+__global__ void __launch_bounds__(ROW_THREADS) softplus_bias_fwd_kernel(const float* __restrict__ pre,
+                                                                        const float* __restrict__ bias, float scale,
+                                                                        float* __restrict__ dt, int D, const RowPlan p) {
+    const RowSlot s(p);
+    if (s.q0 >= s.q1) return;
+    const float bv = bias ? scale * bias[s.row % D] : 0.f;
+    for (int q = s.q0; q < s.q1; q += p.tpr) {
+        float v[4];
+        load_quad(pre + s.row * p.L, 4 * q, p.L, p.vec, v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = softplus_(v[e] + bv);
+        store_quad(dt + s.row * p.L, 4 * q, p.L, p.vec, v);
     }
 }
 
 // dpre = ddt * sigmoid(pre + scale bias), with sigmoid recovered from the output: 1 - exp(-dt) (exact also
 // above the threshold, where the forward passed x through and sigmoid(x) = 1 to float32 accuracy; expm1
 // keeps the relative accuracy for very negative arguments, where dt is tiny);
-// partial[row] = sum_t dpre
+// partial[row * chunks + chunk] = sum_t dpre
 __global__ void __launch_bounds__(ROW_THREADS) softplus_bias_bwd_kernel(const float* __restrict__ ddt,
                                                                         const float* __restrict__ dt,
                                                                         float* __restrict__ dpre,
-                                                                        float* __restrict__ partial, int L) {
-    __shared__ float red[ROW_THREADS / 32];
-    const long long row = blockIdx.x;
-    const float* g = ddt + row * L;
-    const float* y = dt + row * L;
-    float* d = dpre + row * L;
-    float acc = 0.f;
-    for (int t = threadIdx.x; t < L; t += ROW_THREADS) {
-        const float v = g[t] * -expm1f(-y[t]);
-        d[t] = v;
-        acc += v;
-    }
+                                                                        float* __restrict__ partial, const RowPlan p) {
+    const RowSlot s(p);
+    float acc[1] = {0.f};
+    for (int q = s.q0; q < s.q1; q += p.tpr) {
+        float g[4], y[4];
+        load_quad(ddt + s.row * p.L, 4 * q, p.L, p.vec, g);
+        load_quad(dt + s.row * p.L, 4 * q, p.L, p.vec, y);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.f;
-        for (int wv = 0; wv < ROW_THREADS / 32; ++wv) s += red[wv];
-        partial[row] = s;
+        for (int e = 0; e < 4; ++e) {
+            g[e] *= -expm1f(-y[e]);
+            acc[0] += g[e];
+        }
+        store_quad(dpre + s.row * p.L, 4 * q, p.L, p.vec, g);
     }
+    const float sum = row_sums(acc, p, s);
+    if (s.row < p.rows && s.lane == 0) partial[s.row * p.chunks + s.chunk] = sum;
 }
 
 __global__ void __launch_bounds__(256) bias_reduce_kernel(const float* __restrict__ partial, float scale,
-                                                          float* __restrict__ dbias, int B, int D) {
+                                                          float* __restrict__ dbias, int B, int D, int chunks) {
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= D) return;
     float s = 0.f;
-    for (int b = 0; b < B; ++b) s += partial[(long long)b * D + i];
+    for (int b = 0; b < B; ++b)
+        for (int c = 0; c < chunks; ++c) s += partial[((long long)b * D + i) * chunks + c];
     dbias[i] = scale * s;
 }
 
@@ -392,10 +438,6 @@ int launch_ok(const char* who) {
     return AUSSM_OK;
 }
 
-unsigned stream_blocks(long long items) {
-    return (unsigned)std::min<long long>((items + 255) / 256, 148LL * 32);
-}
-
 }  // namespace
 }  // namespace aussm
 
@@ -410,16 +452,16 @@ int aussm_b200_conv_pre_fwd(const float* xs, const float* w, const float* bias, 
         set_error("conv_pre_fwd: null pointer or unsupported filter length %d (1..%d)", K, KMAX);
         return AUSSM_EINVAL;
     }
-    const long long qpr = ((long long)L + 3) / 4, total = qpr * B * D;
-    const int vec = (L % 4 == 0 && al16(u)) ? 1 : 0;
-    conv_pre_fwd_kernel<<<stream_blocks(total), 256, 0, (cudaStream_t)stream>>>(xs, w, bias, u, D, L, K, qpr, total, vec);
+    const RowPlan p = row_plan((long long)B * D, L, L % 4 == 0 && al16(xs) && al16(u));
+    conv_pre_fwd_kernel<<<p.blocks, ROW_THREADS, 0, (cudaStream_t)stream>>>(xs, w, bias, u, D, K, p);
     count_launch();
     return launch_ok("conv_pre_fwd");
 }
 
 size_t aussm_b200_conv_pre_bwd_workspace_bytes(int B, int D) {
     if (B <= 0 || D <= 0) return 0;
-    return ((size_t)B * D * (KMAX + 1) * sizeof(float) + 255) / 256 * 256;
+    const long long rows = (long long)B * D;
+    return ((size_t)rows * row_chunks_max(rows) * (KMAX + 1) * sizeof(float) + 255) / 256 * 256;
 }
 
 int aussm_b200_conv_pre_bwd(const float* du, const float* xs, const float* w, float* dxs, float* dw, float* dbias,
@@ -437,10 +479,11 @@ int aussm_b200_conv_pre_bwd(const float* du, const float* xs, const float* w, fl
     }
     cudaStream_t stream = (cudaStream_t)stream_;
     float* partial = static_cast<float*>(workspace);
-    conv_pre_bwd_kernel<<<(unsigned)((long long)B * D), ROW_THREADS, 0, stream>>>(du, xs, w, dxs, partial, D, L, K);
+    const RowPlan p = row_plan((long long)B * D, L, L % 4 == 0 && al16(du) && al16(xs) && al16(dxs));
+    conv_pre_bwd_kernel<<<p.blocks, ROW_THREADS, 0, stream>>>(du, xs, w, dxs, partial, D, K, p);
     count_launch();
     if (int rc = launch_ok("conv_pre_bwd")) return rc;
-    conv_pre_reduce_kernel<<<(D * (K + 1) + 255) / 256, 256, 0, stream>>>(partial, dw, dbias, B, D, K);
+    conv_pre_reduce_kernel<<<(D * (K + 1) + 255) / 256, 256, 0, stream>>>(partial, dw, dbias, B, D, K, p.chunks);
     count_launch();
     return launch_ok("conv_pre_bwd reduction");
 }
@@ -452,17 +495,16 @@ int aussm_b200_softplus_bias_fwd(const float* pre, const float* bias, float scal
         set_error("softplus_bias_fwd: null pointer");
         return AUSSM_EINVAL;
     }
-    const long long qpr = ((long long)L + 3) / 4, total = qpr * B * D;
-    const int vec = (L % 4 == 0 && al16(pre) && al16(dt)) ? 1 : 0;
-    softplus_bias_fwd_kernel<<<stream_blocks(total), 256, 0, (cudaStream_t)stream>>>(pre, bias, scale, dt, D, L, qpr,
-                                                                                     total, vec);
+    const RowPlan p = row_plan((long long)B * D, L, L % 4 == 0 && al16(pre) && al16(dt));
+    softplus_bias_fwd_kernel<<<p.blocks, ROW_THREADS, 0, (cudaStream_t)stream>>>(pre, bias, scale, dt, D, p);
     count_launch();
     return launch_ok("softplus_bias_fwd");
 }
 
 size_t aussm_b200_softplus_bias_bwd_workspace_bytes(int B, int D) {
     if (B <= 0 || D <= 0) return 0;
-    return ((size_t)B * D * sizeof(float) + 255) / 256 * 256;
+    const long long rows = (long long)B * D;
+    return ((size_t)rows * row_chunks_max(rows) * sizeof(float) + 255) / 256 * 256;
 }
 
 int aussm_b200_softplus_bias_bwd(const float* ddt, const float* dt, float scale, float* dpre, float* dbias, int B,
@@ -479,11 +521,12 @@ int aussm_b200_softplus_bias_bwd(const float* ddt, const float* dt, float scale,
     }
     cudaStream_t stream = (cudaStream_t)stream_;
     float* partial = static_cast<float*>(workspace);
-    softplus_bias_bwd_kernel<<<(unsigned)((long long)B * D), ROW_THREADS, 0, stream>>>(ddt, dt, dpre, partial, L);
+    const RowPlan p = row_plan((long long)B * D, L, L % 4 == 0 && al16(ddt) && al16(dt) && al16(dpre));
+    softplus_bias_bwd_kernel<<<p.blocks, ROW_THREADS, 0, stream>>>(ddt, dt, dpre, partial, p);
     count_launch();
     if (int rc = launch_ok("softplus_bias_bwd")) return rc;
     if (dbias) {
-        bias_reduce_kernel<<<(D + 255) / 256, 256, 0, stream>>>(partial, scale, dbias, B, D);
+        bias_reduce_kernel<<<(D + 255) / 256, 256, 0, stream>>>(partial, scale, dbias, B, D, p.chunks);
         count_launch();
         return launch_ok("softplus_bias_bwd reduction");
     }

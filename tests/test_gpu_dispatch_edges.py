@@ -261,3 +261,25 @@ def test_small_projections(b, l, m, k):
             results.append([y, *grads, second])
         for t, o in zip(*results):
             assert o.shape == t.shape and scaled_error(o.detach().cpu(), t.detach()) < 1.2e-7 * (m + k + b * l), fn.__name__
+
+
+# Rows in chunks, several rows in a block, lengths that end inside a quad.  A gradient of the weight or the bias sums
+# b l terms.
+@pytest.mark.parametrize("b,d,l,taps", [(1, 3, 9001, 4), (1, 2, 4096, 2), (3, 5, 130, 3), (2, 9, 515, 4), (1, 1, 3, 4), (40, 70, 20, 1)])
+def test_conv_and_step_size_row_plans(b, d, l, taps):
+    g = torch.Generator().manual_seed(9000 + l)
+    r = lambda *s: torch.randn(*s, generator=g)
+    x, w, bias, gy = r(b, d, l), r(d, 1, taps), r(d), r(b, d, l)
+    results = []
+    for dev, dtype in (("cpu", torch.float64), ("cuda", torch.float32)):
+        a = [t.to(dev, dtype).requires_grad_(True) for t in (x, w, bias)]
+        if dev == "cpu":
+            u = F.conv1d(a[0], a[1], a[2], padding=taps - 1, groups=d)[..., :l]
+            dt = F.softplus(a[0] + 2.0 * a[2][:, None])
+        else:
+            u, dt = stages.causal_conv_bias(*a), stages.softplus_bias(a[0], a[2], 2.0)
+        gu = torch.autograd.grad((u * gy.to(dev, dtype)).sum(), a)
+        gd = torch.autograd.grad((dt * gy.to(dev, dtype)).sum(), (a[0], a[2]))
+        results.append([u, dt, *gu, *gd])
+    for t, o in zip(*results):
+        assert scaled_error(o.detach().cpu(), t.detach()) < 1e-6 + (1.2e-7 * b * l if t.numel() <= d * taps else 0.0)
