@@ -65,8 +65,6 @@ constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + EPI_BYTES;    // + slac
 // cost the big sum extra truncations).  The 512 columns hold such a pair for each 128-column half of the tile,
 // and the halves take turns: while the tensor core works on one half of a chunk, the epilogue warps drain the
 // other.
-// FP16 parts: the scaled low part is stored times 2^LO_SHIFT (see split_f16_kernel)
-constexpr int LO_SHIFT = 11;
 constexpr int MMA_N = 128;                           // the tile's two column halves take turns (see below)
 constexpr int TMEM_COLS = 2 * BN;                    // 512: per column half a main and a cross accumulator
 constexpr int NUM_THREADS = 32 * (2 + EPI_WARPS);
@@ -88,17 +86,6 @@ struct GemmKernelParams {
     int c_vec;                // 1: C rows are 16-byte aligned (vector stores), 0: scalar stores
     int tiles_m, tiles_n, ntiles;   // one-CTA kernel: a CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...
 };
-
-// Power-of-two scale that brings a tensor whose largest magnitude has the bit pattern `maxbits` to about 2^14
-// (FP16 overflows at 65504), and its exact inverse.
-__host__ __device__ __forceinline__ int scale_exponent(unsigned maxbits) {
-    const int e = (int)((maxbits >> 23) & 0xffu) - 127;      // floor(log2(max)); -127 for zero / subnormal
-    int k = 14 - e;
-    if (k > 100) k = 100;
-    if (k < -100) k = -100;
-    return k;
-}
-__device__ __forceinline__ float pow2f(int k) { return __uint_as_float((unsigned)(127 + k) << 23); }
 
 // ---- PTX wrappers ---------------------------------------------------------
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1,
@@ -531,7 +518,6 @@ template <bool VEC>
 __device__ __forceinline__ void quads_split(const float* __restrict__ src, long long ld_src, __half* __restrict__ hi,
                                             __half* __restrict__ lo, long long ld_dst, unsigned rows, unsigned cols,
                                             float S, unsigned block, unsigned blocks) {
-    const float up = pow2f(LO_SHIFT);
     for (QuadWalk w((cols + 3) / 4, block, blocks); w.r < rows;) {
         float4 v[QUADS_IN_FLIGHT];
         long long at[QUADS_IN_FLIGHT];
@@ -544,18 +530,8 @@ __device__ __forceinline__ void quads_split(const float* __restrict__ src, long 
         }
 #pragma unroll
         for (int k = 0; k < QUADS_IN_FLIGHT; ++k) {
-            const float a[4] = {v[k].x * S, v[k].y * S, v[k].z * S, v[k].w * S};
-            __half h[4], l[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                h[e] = __float2half_rn(a[e]);
-                l[e] = __float2half_rn((a[e] - __half2float(h[e])) * up);
-            }
             uint2 ph, pl;
-            ph.x = (uint32_t)__half_as_ushort(h[0]) | ((uint32_t)__half_as_ushort(h[1]) << 16);
-            ph.y = (uint32_t)__half_as_ushort(h[2]) | ((uint32_t)__half_as_ushort(h[3]) << 16);
-            pl.x = (uint32_t)__half_as_ushort(l[0]) | ((uint32_t)__half_as_ushort(l[1]) << 16);
-            pl.y = (uint32_t)__half_as_ushort(l[2]) | ((uint32_t)__half_as_ushort(l[3]) << 16);
+            split_f16x4(v[k], S, ph, pl);
             if (at[k] >= 0) {
                 *reinterpret_cast<uint2*>(hi + at[k]) = ph;
                 *reinterpret_cast<uint2*>(lo + at[k]) = pl;
@@ -746,7 +722,7 @@ int gemm_split3(const SplitOperand& A, const SplitOperand& B, float* C, const Ge
     return B.mn_major ? launch<0, 1>(maps, kp, grid, stream) : launch<0, 0>(maps, kp, grid, stream);
 }
 
-int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream, bool have_amax) {
+int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream) {
     SplitLaunch p = {};
     unsigned total_blocks = 0;
     int used = 0;
@@ -771,10 +747,8 @@ int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream, b
         if (++used == 1) p.second = total_blocks;
     }
     if (used == 0) return AUSSM_OK;
-    if (!have_amax) {
-        absmax_kernel<<<total_blocks, 256, 0, stream>>>(p);
-        count_launch();
-    }
+    absmax_kernel<<<total_blocks, 256, 0, stream>>>(p);
+    count_launch();
     split_f16_kernel<<<total_blocks, 256, 0, stream>>>(p);
     count_launch();
     cudaError_t e = cudaGetLastError();
@@ -787,16 +761,16 @@ int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream, b
 
 int split_f16(const float* src, long long ld_src, long long src_batch_stride, void* hi, void* lo, long long ld_dst,
               long long dst_batch_stride, long long rows, long long cols, int batches, unsigned* amax,
-              cudaStream_t stream, bool have_amax) {
+              cudaStream_t stream) {
     const SplitSource s = {src, ld_src, src_batch_stride, hi, lo, ld_dst, dst_batch_stride, rows, cols, batches, amax};
-    if (amax && !have_amax) {
+    if (amax) {
         cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(unsigned), stream);
         if (e != cudaSuccess) {
             set_error("split_f16: clearing the maximum: %s", cudaGetErrorString(e));
             return AUSSM_ECUDA;
         }
     }
-    return split_f16_many(&s, 1, stream, have_amax);
+    return split_f16_many(&s, 1, stream);
 }
 
 }  // namespace aussm

@@ -55,8 +55,8 @@ void proj_begin(const float* x, ProjScratch& s);
 int proj_split_u(const ProjDims& d, const float* u, ProjScratch& s, cudaStream_t stream);
 int proj_theta(const ProjDims& d, const float* u, float* theta_w, ProjScratch& s, cudaStream_t stream);
 // dx and du from dtheta_w; requires the split of u of the same window (proj_theta or proj_split_u).
-// dtheta_amax_known: s.amax[2] already holds the bit pattern of max|dtheta_w| (the scan kernel produced it)
+// dtheta_w == nullptr: its FP16 parts are already in s.dth_hi / s.dth_lo, scaled by s.amax[2] (the scan wrote them).
 int proj_adjoints(const ProjDims& d, const float* dtheta_w, float* dx, float* du, bool overwrite_dx, ProjScratch& s,
-                  cudaStream_t stream, bool dtheta_amax_known = false);
+                  cudaStream_t stream);
 
 }  // namespace aussm

@@ -71,8 +71,9 @@ def operator_bound(b, d, n, l):
     return scan_bound(b, d, n, l) + 2.4e-7 * math.sqrt(d) * l
 
 
-def operator_errors(b, d, n, l, seed):
+def operator_errors(b, d, n, l, seed, gain=1.0):
     inp = model_like_inputs(seed, b, d, n, l)
+    inp["gy"] = inp["gy"] * gain
     results = []
     for dev, real, cplx, fn in (("cpu", torch.float64, torch.complex128, O.interface_unitary),
                                 ("cuda", torch.float32, torch.complex64, aussm_b200.ssm_adaptive_interface)):
@@ -93,6 +94,16 @@ def test_operator_adjoints_summed_in_runs(shape):
     assert aussm_b200.device_status() == 0
     bound = operator_bound(*shape)
     assert max(errors.values()) < 10 * bound, (errors, bound)
+
+
+# The phase gradients leave the scan as FP16 parts scaled by a bound, not by their maximum: any magnitude of the
+# incoming gradient, and inputs whose bound is far too high (a long window, one large step).
+@pytest.mark.parametrize("gain", [1e-25, 1e-6, 1.0, 1e18])
+@pytest.mark.parametrize("shape", [(1, 9, 5, 1500), (2, 20, 16, 130)])
+def test_operator_gradients_of_any_magnitude(shape, gain):
+    errors = operator_errors(*shape, 3200 + sum(shape), gain)
+    assert aussm_b200.device_status() == 0
+    assert max(errors.values()) < operator_bound(*shape), errors
 
 
 @pytest.mark.parametrize("steps", [576, 640, 2000])
