@@ -137,6 +137,25 @@ __device__ __forceinline__ float channel_sum(float v) {
 }
 
 #define AUSSM_F4(v) {(v).x, (v).y, (v).z, (v).w}
+// four consecutive steps as two pairs: what does not run along the recurrence is done two steps at a time with the
+// packed float32x2 instructions (the kernels are bound by the instructions a few warps can issue, not by a pipe)
+#define AUSSM_F22(v) {make_float2((v).x, (v).y), make_float2((v).z, (v).w)}
+
+// multipliers exp(dlt A) of four steps
+__device__ __forceinline__ void multipliers(const float2 (&dlt)[2], float2 A2, float2 (&a)[2]) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const float2 x = __fmul2_rn(dlt[p], A2);
+        a[p] = make_float2(ex2_ftz(x.x), ex2_ftz(x.y));
+    }
+}
+// four steps of h_t = a_t h_{t-1} + x_t; h receives the states after each step
+__device__ __forceinline__ void four_steps(float h0, const float2 (&a)[2], const float2 (&x)[2], float2 (&h)[2]) {
+    h[0].x = fmaf(a[0].x, h0, x[0].x);
+    h[0].y = fmaf(a[0].y, h[0].x, x[0].y);
+    h[1].x = fmaf(a[1].x, h[0].y, x[1].x);
+    h[1].y = fmaf(a[1].y, h[1].x, x[1].y);
+}
 
 // ---------------------------------------------------------------------------
 // Forward
@@ -227,25 +246,25 @@ __global__ void __launch_bounds__(32) s6w_fwd_kernel(const S6FwdParams p) {
         for (int q = 0; q < NQ; ++q) {
             if (4 * q >= tlen) break;
             const float4 u4 = ld_shared_f4(urow + 4 * q), d4 = ld_shared_f4(drow + 4 * q);
-            const float uv[4] = AUSSM_F4(u4), dlt[4] = AUSSM_F4(d4);
-            float s[4], y[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                s[e] = dlt[e] * uv[e];
-                y[e] = 0.f;
-            }
+            const float uv[4] = AUSSM_F4(u4);
+            const float2 uv2[2] = AUSSM_F22(u4), dlt[2] = AUSSM_F22(d4);
+            const float2 s[2] = {__fmul2_rn(dlt[0], uv2[0]), __fmul2_rn(dlt[1], uv2[1])};
+            float2 y2[2] = {f2(0.f), f2(0.f)};
 #pragma unroll
             for (int jj = 0; jj < SPT; ++jj) {
                 const int j = jj * LPC + k;
                 const float4 b4 = ld_shared_f4(st + j * WTP + 4 * q);               // one address per value of k
                 const float4 c4 = ld_shared_f4(st + (NS + j) * WTP + 4 * q);
-                const float bv[4] = AUSSM_F4(b4), cv[4] = AUSSM_F4(c4);
+                const float2 bv[2] = AUSSM_F22(b4), cv[2] = AUSSM_F22(c4);
+                float2 a[2], ht[2];
+                multipliers(dlt, f2(A2[jj]), a);
+                const float2 x[2] = {__fmul2_rn(s[0], bv[0]), __fmul2_rn(s[1], bv[1])};
+                four_steps(h[jj], a, x, ht);
+                h[jj] = ht[1].y;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    h[jj] = fmaf(ex2_ftz(dlt[e] * A2[jj]), h[jj], s[e] * bv[e]);
-                    y[e] = fmaf(cv[e], h[jj], y[e]);
-                }
+                for (int p2 = 0; p2 < 2; ++p2) y2[p2] = __ffma2_rn(cv[p2], ht[p2], y2[p2]);
             }
+            float y[4] = {y2[0].x, y2[0].y, y2[1].x, y2[1].y};
 #pragma unroll
             for (int e = 0; e < 4; ++e) y[e] = fmaf(dskip, uv[e], channel_sum<LPC>(y[e]));
             if (gate) {
@@ -300,13 +319,14 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
     float* sub = smem + WSTAGES * C::STAGE_FLOATS;          // [NQ][SPT][32]
     float* red = sub + C::SUB_FLOATS;                       // [2 NS][RP] float4: gB rows, then gC rows
 
-    float A2[SPT], eps[SPT], dA[SPT];
+    float A2[SPT], eps[SPT];
+    float2 dA2[SPT];         // even and odd steps
 #pragma unroll
     for (int jj = 0; jj < SPT; ++jj) {
         const int j = jj * LPC + k;
         A2[jj] = j < N ? p.A[(long long)i * N + j] * kLog2e : 0.f;
         eps[jj] = (p.nseg > 1 && act && j < N) ? p.seg_grad[(ch * p.nseg + seg) * N + j] : 0.f;       // a_{t+1} eta_{t+1}
-        dA[jj] = 0.f;
+        dA2[jj] = f2(0.f);
     }
     const float dskip = p.Dskip ? p.Dskip[i] : 0.f;
     const float bias = p.delta_bias ? p.delta_bias[i] : 0.f;
@@ -403,14 +423,17 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
             for (int jj = 0; jj < SPT; ++jj) sub[(q * SPT + jj) * 32 + lane] = h[jj];
             if (q + 1 >= nq) break;                                   // the last group's end state is not needed
             const float4 u4 = ld_shared_f4(urow + 4 * q), d4 = ld_shared_f4(drow + 4 * q);
-            const float uv[4] = AUSSM_F4(u4), dlt[4] = AUSSM_F4(d4);
-            const float s[4] = {dlt[0] * uv[0], dlt[1] * uv[1], dlt[2] * uv[2], dlt[3] * uv[3]};
+            const float2 uv[2] = AUSSM_F22(u4), dlt[2] = AUSSM_F22(d4);
+            const float2 s[2] = {__fmul2_rn(dlt[0], uv[0]), __fmul2_rn(dlt[1], uv[1])};
 #pragma unroll
             for (int jj = 0; jj < SPT; ++jj) {
                 const float4 b4 = ld_shared_f4(st + (jj * LPC + k) * WTP + 4 * q);
-                const float bv[4] = AUSSM_F4(b4);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) h[jj] = fmaf(ex2_ftz(dlt[e] * A2[jj]), h[jj], s[e] * bv[e]);
+                const float2 bv[2] = AUSSM_F22(b4);
+                const float2 x[2] = {__fmul2_rn(s[0], bv[0]), __fmul2_rn(s[1], bv[1])};
+                float2 a[2], ht[2];
+                multipliers(dlt, f2(A2[jj]), a);
+                four_steps(h[jj], a, x, ht);
+                h[jj] = ht[1].y;
             }
         }
 
@@ -420,42 +443,50 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
             const float4 u4 = ld_shared_f4(urow + 4 * q), d4 = ld_shared_f4(drow + 4 * q);
             const float4 w4 = ld_shared_f4(grow + 4 * q);
             const float uv[4] = AUSSM_F4(u4), dlt[4] = AUSSM_F4(d4), w[4] = AUSSM_F4(w4);
-            float s[4], SQ[4], SY[4], SP[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                s[e] = dlt[e] * uv[e];
-                SQ[e] = SY[e] = SP[e] = 0.f;
-            }
+            const float2 uv2[2] = AUSSM_F22(u4), dlt2[2] = AUSSM_F22(d4), w2[2] = AUSSM_F22(w4);
+            const float2 s[2] = {__fmul2_rn(dlt2[0], uv2[0]), __fmul2_rn(dlt2[1], uv2[1])};
+            float2 SQ2[2] = {f2(0.f), f2(0.f)}, SY2[2] = {f2(0.f), f2(0.f)}, SP2[2] = {f2(0.f), f2(0.f)};
 #pragma unroll
             for (int jj = 0; jj < SPT; ++jj) {
                 const int j = jj * LPC + k;
                 const float4 b4 = ld_shared_f4(st + j * WTP + 4 * q);
                 const float4 c4 = ld_shared_f4(st + (NS + j) * WTP + 4 * q);
-                const float bv[4] = AUSSM_F4(b4), cv[4] = AUSSM_F4(c4);
-                float hp[4], av[4], gB[4], gC[4];
-                float hj = sub[(q * SPT + jj) * 32 + lane];
+                const float2 bv[2] = AUSSM_F22(b4), cv2[2] = AUSSM_F22(c4);
+                const float cv[4] = AUSSM_F4(c4);
+                const float2 x[2] = {__fmul2_rn(s[0], bv[0]), __fmul2_rn(s[1], bv[1])};
+                float2 a[2], ht[2];                    // multipliers; the states after each step of the group
+                multipliers(dlt2, f2(A2[jj]), a);
+                const float h0 = sub[(q * SPT + jj) * 32 + lane];
+                four_steps(h0, a, x, ht);
+                // eta_t = C_t w_t + a_{t+1} eta_{t+1}
+                float2 g[2], ag[2];
+                g[1].y = fmaf(cv[3], w[3], eps[jj]);
+                ag[1].y = a[1].y * g[1].y;
+                g[1].x = fmaf(cv[2], w[2], ag[1].y);
+                ag[1].x = a[1].x * g[1].x;
+                g[0].y = fmaf(cv[1], w[1], ag[1].x);
+                ag[0].y = a[0].y * g[0].y;
+                g[0].x = fmaf(cv[0], w[0], ag[0].y);
+                ag[0].x = a[0].x * g[0].x;
+                eps[jj] = ag[0].x;
+                const float2 hp[2] = {make_float2(h0, ht[0].x), make_float2(ht[0].y, ht[1].x)};   // before each step
+                float2 gB[2], gC[2];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {          // the state BEFORE each step of the group
-                    hp[e] = hj;
-                    av[e] = ex2_ftz(dlt[e] * A2[jj]);
-                    hj = fmaf(av[e], hj, s[e] * bv[e]);
+                for (int p2 = 0; p2 < 2; ++p2) {
+                    const float2 qa = __fmul2_rn(ag[p2], hp[p2]);                // a_t eta_t h_{t-1}
+                    dA2[jj] = __ffma2_rn(qa, dlt2[p2], dA2[jj]);
+                    SQ2[p2] = __ffma2_rn(qa, f2(A2[jj]), SQ2[p2]);               // times ln 2 below
+                    SY2[p2] = __ffma2_rn(g[p2], bv[p2], SY2[p2]);
+                    SP2[p2] = __ffma2_rn(cv2[p2], ht[p2], SP2[p2]);
+                    gB[p2] = __fmul2_rn(g[p2], s[p2]);
+                    gC[p2] = __fmul2_rn(w2[p2], ht[p2]);
                 }
-#pragma unroll
-                for (int e = 3; e >= 0; --e) {
-                    const float ht = fmaf(av[e], hp[e], s[e] * bv[e]);       // h_t
-                    const float g = fmaf(cv[e], w[e], eps[jj]);              // eta_t
-                    const float qa = g * hp[e] * av[e];                      // eta_t h_{t-1} a_t
-                    dA[jj] = fmaf(qa, dlt[e], dA[jj]);
-                    SQ[e] = fmaf(qa, A2[jj], SQ[e]);                         // times ln 2 below
-                    SY[e] = fmaf(g, bv[e], SY[e]);
-                    SP[e] = fmaf(cv[e], ht, SP[e]);
-                    gB[e] = g * s[e];
-                    gC[e] = w[e] * ht;
-                    eps[jj] = av[e] * g;
-                }
-                st_shared_f4(red + (j * RP + c) * 4, make_float4(gB[0], gB[1], gB[2], gB[3]));
-                st_shared_f4(red + ((NS + j) * RP + c) * 4, make_float4(gC[0], gC[1], gC[2], gC[3]));
+                st_shared_f4(red + (j * RP + c) * 4, make_float4(gB[0].x, gB[0].y, gB[1].x, gB[1].y));
+                st_shared_f4(red + ((NS + j) * RP + c) * 4, make_float4(gC[0].x, gC[0].y, gC[1].x, gC[1].y));
             }
+            const float SQ[4] = {SQ2[0].x, SQ2[0].y, SQ2[1].x, SQ2[1].y};
+            const float SY[4] = {SY2[0].x, SY2[0].y, SY2[1].x, SY2[1].y};
+            const float SP[4] = {SP2[0].x, SP2[0].y, SP2[1].x, SP2[1].y};
             __syncwarp();
             // dB, dC: lane r adds row r over the warp's channels, one vector atomic per state and group
 #pragma unroll
@@ -511,7 +542,7 @@ __global__ void __launch_bounds__(32) s6w_bwd_kernel(const S6BwdParams p) {
         const long long o = ((long long)b * max(1, p.nseg) + seg) * p.Dmod + i;
 #pragma unroll
         for (int jj = 0; jj < SPT; ++jj)
-            if (jj * LPC + k < N) p.part_A[o * N + jj * LPC + k] = dA[jj];
+            if (jj * LPC + k < N) p.part_A[o * N + jj * LPC + k] = dA2[jj].x + dA2[jj].y;
         if (k == 0) {
             p.part_D[o] = dD_acc;
             p.part_bias[o] = db_acc;
@@ -775,7 +806,7 @@ int lanes_per_channel(long long batches, int D, int NS, bool bwd) {
     }
     auto warps = [&](int lpc) { return batches * ((D + 32 / lpc - 1) / (32 / lpc)); };
     if (bwd) return warps(2) < 4LL * sms ? 4 : 2;
-    int lpc = 1;
+    int lpc = NS > 16 ? 2 : 1;                              // 32 states of one thread do not fit its registers
     while (lpc < 4 && lpc * 2 <= NS && warps(lpc) < 12LL * sms) lpc *= 2;
     return lpc;
 }
