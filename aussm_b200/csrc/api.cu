@@ -189,11 +189,10 @@ int run_unitary_fwd(const OpArgs& a, const float* h0_re, const float* h0_im, flo
         const int tl = (int)std::min<long long>(pl.window, a.L - t0);
         const ProjDims pd = {a.B, a.D, (long long)a.D * a.N, a.L, pl.ldw, t0, tl};
         if (keep) theta_w = keep + (size_t)w * pl.rows * pl.ldw;
-        if (int rc = proj_theta(pd, a.u, theta_w, ps, stream)) return rc;
+        if (int rc = proj_theta(pd, a.u, a.x_bias, theta_w, ps, stream)) return rc;
         const bool last = (w == nwin - 1);
         ScanFwdParams sp = {};
         sp.theta = theta_w;
-        sp.theta_bias = a.x_bias;
         sp.u = a.u + t0;
         sp.dt = a.dt + t0;
         sp.z = a.z + t0;
@@ -265,7 +264,7 @@ int aussm_b200_scan_unitary_fwd(const float* theta, const float* u, const float*
         return AUSSM_EINVAL;
     }
     ScanFwdParams p = {};
-    p.theta = theta; p.theta_bias = nullptr; p.u = u; p.dt = dt; p.z = z;
+    p.theta = theta; p.u = u; p.dt = dt; p.z = z;
     p.B_r = B_r; p.B_theta = B_theta; p.C_r = C_r; p.C_theta = C_theta; p.Dskip = Dskip;
     p.h0_re = h0_re; p.h0_im = h0_im; p.y = y; p.h1_re = h1_re; p.h1_im = h1_im;
     p.nch = B * D; p.Dmod = D; p.N = N; p.L = L; p.ld_theta = L; p.ld_row = L;
@@ -304,7 +303,7 @@ int aussm_b200_scan_unitary_fwd_ws(const float* theta, const float* u, const flo
         return AUSSM_EWORKSPACE;
     }
     ScanFwdParams p = {};
-    p.theta = theta; p.theta_bias = nullptr; p.u = u; p.dt = dt; p.z = z;
+    p.theta = theta; p.u = u; p.dt = dt; p.z = z;
     p.B_r = B_r; p.B_theta = B_theta; p.C_r = C_r; p.C_theta = C_theta; p.Dskip = Dskip;
     p.h0_re = h0_re; p.h0_im = h0_im; p.y = y; p.h1_re = h1_re; p.h1_im = h1_im;
     p.nch = B * D; p.Dmod = D; p.N = N; p.L = L; p.ld_theta = L; p.ld_row = L;
@@ -358,7 +357,7 @@ int aussm_b200_scan_unitary_bwd(const float* grad_y, const float* gh1_re, const 
     float* part_d = part_bc + nch * nseg * N * 4;
     float* split_scratch = reinterpret_cast<float*>(
         static_cast<char*>(workspace) + align_up(scan_bwd_partial_floats(nch * nseg, N) * sizeof(float), 256));
-    p.theta = theta; p.theta_bias = nullptr; p.u = u; p.dt = dt; p.z = z; p.gy = grad_y;
+    p.theta = theta; p.u = u; p.dt = dt; p.z = z; p.gy = grad_y;
     p.B_r = B_r; p.B_theta = B_theta; p.C_r = C_r; p.C_theta = C_theta; p.Dskip = Dskip;
     p.h1_re = h1_re; p.h1_im = h1_im; p.gh1_re = gh1_re; p.gh1_im = gh1_im;
     p.dtheta = dtheta; p.du = du; p.ddt = ddt; p.dz = dz; p.dh0_re = dh0_re; p.dh0_im = dh0_im;
@@ -597,11 +596,11 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
         if (keep) {
             theta_w = keep + (size_t)w * pl.rows * pl.ldw;    // phases of the forward call; dtheta replaces them
             if (int rc = proj_split_u(pd, u, ps, stream)) return rc;
-        } else if (int rc = proj_theta(pd, u, theta_w, ps, stream)) {
+        } else if (int rc = proj_theta(pd, u, x_bias, theta_w, ps, stream)) {
             return rc;
         }
         ScanBwdParams p = {};
-        p.theta = theta_w; p.theta_bias = x_bias;
+        p.theta = theta_w;
         p.u = u + t0; p.dt = dt + t0; p.z = z + t0; p.gy = grad_y + t0;
         p.B_r = B_r; p.B_theta = B_theta; p.C_r = C_r; p.C_theta = C_theta; p.Dskip = Dskip;
         p.h1_re = first ? hend_re : cur_re;

@@ -215,7 +215,7 @@ int aussm_b200_complex_fwd(const float* u, const float* dt, const float* x, int 
         const long long t0 = (long long)w * pl.window;
         const int tl = (int)std::min<long long>(pl.window, L - t0);
         const ProjDims pd = {B, D, pl.M, L, pl.ldw, t0, tl};
-        if (int rc = proj_theta(pd, u, lam, ps, stream)) return rc;
+        if (int rc = proj_theta(pd, u, nullptr, lam, ps, stream)) return rc;
         CplxFwdParams p = {};
         p.rho = lam; p.theta = has_theta ? lam + DN * pl.ldw : nullptr;
         p.u = u + t0; p.dt = dt + t0; p.z = z + t0;
@@ -274,7 +274,7 @@ int aussm_b200_complex_bwd(const float* gy, const float* gstates, const float* u
         const int tl = (int)std::min<long long>(pl.window, L - t0);
         const bool first = (w == nwin - 1);             // first processed = last in time
         const ProjDims pd = {B, D, pl.M, L, pl.ldw, t0, tl};
-        if (int rc = proj_theta(pd, u, lam, ps, stream)) return rc;     // recompute this window's exponents
+        if (int rc = proj_theta(pd, u, nullptr, lam, ps, stream)) return rc;     // recompute this window's exponents
         CplxBwdParams p = {};
         p.gy = gy + t0; p.rho = lam; p.theta = has_theta ? lam + DN * pl.ldw : nullptr;
         p.u = u + t0; p.dt = dt + t0; p.z = z + t0;

@@ -80,6 +80,7 @@ struct GemmKernelParams {
     int ksplit;        // partial outputs per output (runs of the contraction), c_part_stride floats apart
     long long c_part_stride;
     int beta;
+    const float* row_bias;
     int* status;
     const unsigned* amax_a;   // FP16 parts: bit patterns of max|a|, max|b| (the parts are scaled by a power of two)
     const unsigned* amax_b;
@@ -362,6 +363,8 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
         for (int t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
             const int zb = tile_batch(t), run = tile_run(t), total = run_begin(run + 1) - run_begin(run);
             const int m0 = ((t % tiles_mn) % p.tiles_m) * BM, n0 = ((t % tiles_mn) / p.tiles_m) * BN;
+            const int own_row = m0 + quarter * 32 + lane;
+            const float rb = (p.row_bias && own_row < p.M) ? p.row_bias[own_row] : 0.f;     // long before its use
 #pragma unroll
             for (int i = 0; i < MMA_N; ++i) acc[i] = 0.f;
             for (int it = 0; it < total; ++it) {
@@ -391,7 +394,7 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
 #pragma unroll
                 for (int blk = 0; blk < MMA_N / 32; ++blk) {
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) stg[lane * EPI_PITCH + c] = (acc[blk * 32 + c] * ua) * ub;
+                    for (int c = 0; c < 32; ++c) stg[lane * EPI_PITCH + c] = (acc[blk * 32 + c] * ua) * ub + rb;
                     __syncwarp();
                     const int col = n0 + h * MMA_N + blk * 32 + c4;
 #pragma unroll
@@ -704,6 +707,7 @@ int gemm_split3(const SplitOperand& A, const SplitOperand& B, float* C, const Ge
     kp.ksplit = std::max(1, std::min(s.ksplit, (s.K + BK - 1) / BK * kp.kbatches));
     kp.c_part_stride = s.c_part_stride;
     kp.beta = s.beta;
+    kp.row_bias = s.row_bias;
     kp.a_batched = A.batch_stride != 0;
     kp.b_batched = B.batch_stride != 0;
     kp.amax_a = A.amax;

@@ -66,6 +66,7 @@ struct GemmShape {
                           // batch entries) is cut into g nearly equal runs, each a partial output of its own at
                           // C + run * c_part_stride, to be added by the caller
     long long c_part_stride;
+    const float* row_bias;  // (M) added to every row of the result, or nullptr (with ksplit <= 1)
 };
 
 long long gemm_split3_blocks(const GemmShape& s);      // K blocks of one output: no more runs than these are made

@@ -105,7 +105,7 @@ extern "C" int aussm_b200_scan_unitary_bwd_static(
     float* part_bc = scratch;
     float* part_d = part_bc + nch * N * 4;
     ScanBwdParams p = {};
-    p.theta = theta; p.theta_bias = nullptr; p.u = u; p.dt = dt; p.z = z; p.gy = grad_y;
+    p.theta = theta; p.u = u; p.dt = dt; p.z = z; p.gy = grad_y;
     p.B_r = B_r; p.B_theta = B_theta; p.C_r = C_r; p.C_theta = C_theta; p.Dskip = Dskip;
     p.h1_re = h1_re; p.h1_im = h1_im; p.gh1_re = gh1_re; p.gh1_im = gh1_im;
     p.dtheta = dtheta; p.du = du; p.ddt = ddt; p.dz = dz; p.dh0_re = dh0_re; p.dh0_im = dh0_im;

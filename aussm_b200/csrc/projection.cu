@@ -120,13 +120,13 @@ int proj_split_u(const ProjDims& d, const float* u, ProjScratch& s, cudaStream_t
     return split_f16_many(sources + first, 2 - first, stream);
 }
 
-int proj_theta(const ProjDims& d, const float* u, float* theta_w, ProjScratch& s, cudaStream_t stream) {
+int proj_theta(const ProjDims& d, const float* u, const float* bias, float* theta_w, ProjScratch& s, cudaStream_t stream) {
     const int M = (int)d.M;
     if (int rc = proj_split_u(d, u, s, stream)) return rc;
     // theta_w[b] (M x tl) = x (M x D, K-major) * u_b (D x tl: K rows, N contiguous -> MN-major)
     const SplitOperand A = {s.x_hi, s.x_lo, 0, s.Dp, 0, s.amax + 0};
     const SplitOperand Bop = {s.u_hi, s.u_lo, 1, d.ldw, (long long)d.D * d.ldw, s.amax + 1};
-    const GemmShape shape = {M, d.tl, d.D, d.B, 0, 0, d.ldw, (long long)M * d.ldw, 1, 0};
+    const GemmShape shape = {M, d.tl, d.D, d.B, 0, 0, d.ldw, (long long)M * d.ldw, 1, 0, bias};
     return gemm_split3(A, Bop, theta_w, shape, stream);
 }
 

@@ -53,7 +53,8 @@ void proj_begin(const float* x, ProjScratch& s);
 // FP16 parts of the current window of u (proj_theta does this itself; proj_adjoints expects it done).  Clears the
 // maximum of dtheta, for a scan that collects it.
 int proj_split_u(const ProjDims& d, const float* u, ProjScratch& s, cudaStream_t stream);
-int proj_theta(const ProjDims& d, const float* u, float* theta_w, ProjScratch& s, cudaStream_t stream);
+// bias: (M) added to every row of theta_w, or nullptr
+int proj_theta(const ProjDims& d, const float* u, const float* bias, float* theta_w, ProjScratch& s, cudaStream_t stream);
 // dx and du from dtheta_w; requires the split of u of the same window (proj_theta or proj_split_u).
 // dtheta_w == nullptr: its FP16 parts are already in s.dth_hi / s.dth_lo, scaled by s.amax[2] (the scan wrote them).
 int proj_adjoints(const ProjDims& d, const float* dtheta_w, float* dx, float* du, bool overwrite_dx, ProjScratch& s,

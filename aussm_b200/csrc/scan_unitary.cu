@@ -108,18 +108,16 @@ struct StateConsts {
     float mr, mi;      // M: projection constant (Cc*Bc normalised, Cc otherwise)
     float br, bi;      // Bc
     float kr, ki;      // state scale kappa (Bc normalised, 1 otherwise)
-    float bias;        // phase offset
     bool act;
 };
 
-__device__ __forceinline__ void load_state_consts(StateConsts& sc, bool act, int j, int i, int N,
+__device__ __forceinline__ void load_state_consts(StateConsts& sc, bool act, int j,
                                                   const float* B_r, const float* B_theta, const float* C_r,
-                                                  const float* C_theta, const float* theta_bias, bool& norm_ok) {
+                                                  const float* C_theta, bool& norm_ok) {
     sc.act = act;
     sc.mr = sc.mi = sc.br = sc.bi = 0.f;
     sc.kr = 1.f;
     sc.ki = 0.f;
-    sc.bias = 0.f;
     norm_ok = true;
     if (!act) return;
     float brad = B_r[j], bth = B_theta[j], crad = C_r[j], cth = C_theta[j];
@@ -130,7 +128,6 @@ __device__ __forceinline__ void load_state_consts(StateConsts& sc, bool act, int
     sc.bi = brad * sb;
     sc.mr = crad * ccc;   // Cc for now
     sc.mi = crad * scc;
-    sc.bias = theta_bias ? theta_bias[(size_t)i * N + j] : 0.f;
     norm_ok = fabsf(brad) >= 1e-12f;
 }
 
@@ -284,7 +281,7 @@ __device__ __forceinline__ void issue_words(float* stage, const float* theta_war
 // Forward
 // ---------------------------------------------------------------------------
 // VEC: rows are 16-byte aligned and L is a multiple of 4 (16-byte copies and vector stores).
-template <class C, bool VEC, bool NORM, bool BIAS>
+template <class C, bool VEC, bool NORM>
 __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, const WarpTask& wt, int lane,
                                          StateConsts (&sc)[C::SPT]) {
     constexpr int NL = C::NL, SPT = C::SPT, T = C::T, TP = C::TP, STAGES = C::STAGES, AUX = C::AUX, VW = C::VW;
@@ -369,11 +366,7 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, con
 #pragma unroll
             for (int k = 0; k < SPT; ++k) {
                 const float4 t4 = ld_shared_f4(th + (k * 32 + lane) * TP + 4 * q);
-                float tv[4] = {t4.x, t4.y, t4.z, t4.w};
-                if (BIAS) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) tv[e] += sc[k].bias;
-                }
+                const float tv[4] = {t4.x, t4.y, t4.z, t4.w};
                 float sn[4], cs[4];
                 sincos4(tv, sn, cs);
 #pragma unroll
@@ -456,7 +449,7 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, con
     }
 }
 
-template <class C, bool VEC, bool BIAS>
+template <class C, bool VEC>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const ScanFwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -465,15 +458,13 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const S
     const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / C::NL, jl = lane % C::NL;
-    const int i = (int)((wt.ch0 + min(c, nvalid - 1)) % p.Dmod);
     StateConsts sc[C::SPT];
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < C::SPT; ++k) {
         const int j = jl + k * C::NL;
         bool okk;
-        load_state_consts(sc[k], c < nvalid && j < p.N, j, i, p.N, p.B_r, p.B_theta, p.C_r, p.C_theta,
-                          BIAS ? p.theta_bias : nullptr, okk);
+        load_state_consts(sc[k], c < nvalid && j < p.N, j, p.B_r, p.B_theta, p.C_r, p.C_theta, okk);
         ok = ok && okk;
     }
     if (__all_sync(0xffffffffu, ok)) {
@@ -482,17 +473,17 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const S
             float a, b;
             normalise_consts(sc[k], a, b);
         }
-        fwd_warp<C, VEC, true, BIAS>(p, wsm, wt, lane, sc);
+        fwd_warp<C, VEC, true>(p, wsm, wt, lane, sc);
     } else {
-        fwd_warp<C, VEC, false, BIAS>(p, wsm, wt, lane, sc);
+        fwd_warp<C, VEC, false>(p, wsm, wt, lane, sc);
     }
 }
 
 // ---------------------------------------------------------------------------
 // Backward
 // ---------------------------------------------------------------------------
-// PARTS: dtheta leaves as its FP16 parts.
-template <class C, bool VEC, bool NORM, bool BIAS, bool PARTS>
+// PARTS (the drop-in pipeline): dtheta leaves as its FP16 parts, and its sums over time are collected.
+template <class C, bool VEC, bool NORM, bool PARTS>
 __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, const WarpTask& wt, int lane,
                                          StateConsts (&sc)[C::SPT], const float (&ccr)[C::SPT],
                                          const float (&cci)[C::SPT]) {
@@ -624,11 +615,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
                 for (int k = 0; k < SPT; ++k) {
                     float* cell = th + (k * 32 + lane) * TP + sbeg + 4 * q;
                     const float4 t4 = ld_shared_f4(cell);
-                    float tv[4] = {t4.x, t4.y, t4.z, t4.w};
-                    if (BIAS) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) tv[e] += sc[k].bias;
-                    }
+                    const float tv[4] = {t4.x, t4.y, t4.z, t4.w};
                     float sn[4], cs[4];
                     sincos4(tv, sn, cs);
                     float dth[4];
@@ -650,7 +637,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
                         // dtheta_t = -Im(conj(eta) a)
                         const float d = fmaf(ni, ar, -nr * ai);
                         dth[e] = d;
-                        if (BIAS) rsum[k] += d;
+                        if (PARTS) rsum[k] += d;
                         const float pv = fmaf(sc[k].mr, hr[k], -sc[k].mi * hi[k]);
                         // gradient of the real drive s_t: Re(conj(eta) beta)
                         const float ev = NORM ? nr : fmaf(nr, sc[k].br, ni * sc[k].bi);
@@ -817,7 +804,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
             dbr += old.x; dbi += old.y; dcr += old.z; dci += old.w;
         }
         *pb = make_float4(dbr, dbi, dcr, dci);
-        if (BIAS && p.part_rowsum) p.part_rowsum[po] = rsum[k] + (p.accumulate ? p.part_rowsum[po] : 0.f);
+        if (PARTS) p.part_rowsum[po] = rsum[k] + (p.accumulate ? p.part_rowsum[po] : 0.f);
         if (p.dh0_re) { p.dh0_re[o] = d0r; p.dh0_im[o] = d0i; }
         if (p.h0_re) { p.h0_re[o] = s0r; p.h0_im[o] = s0i; }
     }
@@ -836,7 +823,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
     }
 }
 
-template <class C, bool VEC, bool BIAS, bool PARTS>
+template <class C, bool VEC, bool PARTS>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const ScanBwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -845,7 +832,6 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const S
     const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / C::NL, jl = lane % C::NL;
-    const int i = (int)((wt.ch0 + min(c, nvalid - 1)) % p.Dmod);
     StateConsts sc[C::SPT];
     float ccr[C::SPT], cci[C::SPT];
     bool ok = true;
@@ -853,8 +839,7 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const S
     for (int k = 0; k < C::SPT; ++k) {
         const int j = jl + k * C::NL;
         bool okk;
-        load_state_consts(sc[k], c < nvalid && j < p.N, j, i, p.N, p.B_r, p.B_theta, p.C_r, p.C_theta,
-                          BIAS ? p.theta_bias : nullptr, okk);
+        load_state_consts(sc[k], c < nvalid && j < p.N, j, p.B_r, p.B_theta, p.C_r, p.C_theta, okk);
         ccr[k] = sc[k].mr;
         cci[k] = sc[k].mi;
         ok = ok && okk;
@@ -862,9 +847,9 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const S
     if (__all_sync(0xffffffffu, ok)) {
 #pragma unroll
         for (int k = 0; k < C::SPT; ++k) normalise_consts(sc[k], ccr[k], cci[k]);
-        bwd_warp<C, VEC, true, BIAS, PARTS>(p, wsm, wt, lane, sc, ccr, cci);
+        bwd_warp<C, VEC, true, PARTS>(p, wsm, wt, lane, sc, ccr, cci);
     } else {
-        bwd_warp<C, VEC, false, BIAS, PARTS>(p, wsm, wt, lane, sc, ccr, cci);
+        bwd_warp<C, VEC, false, PARTS>(p, wsm, wt, lane, sc, ccr, cci);
     }
 }
 
@@ -878,7 +863,7 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const S
 // for the two passes of B1 D512 N16 L65536 (2 x 2.1 GB of phases, 0.62 of the copy bandwidth), where the two aggregate
 // passes and the adjoint pass took 1710 us.
 // ---------------------------------------------------------------------------
-template <class C, bool VEC, bool BIAS, bool BWD>
+template <class C, bool VEC, bool BWD>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_summary_kernel(const SegSummaryParams p) {
     constexpr int NL = C::NL, SPT = C::SPT, T = C::T, TP = C::TP, STAGES = C::STAGES, AUX = C::AUX, VW = C::VW;
     extern __shared__ __align__(128) float smem[];
@@ -888,15 +873,13 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_summary_kernel(con
     const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / NL, jl = lane % NL;
-    const int i = (int)((wt.ch0 + min(c, nvalid - 1)) % p.Dmod);
     const int N = p.N, L = wt.L;
     const int ntiles = (L + T - 1) / T;
     StateConsts sc[SPT];
 #pragma unroll
     for (int k = 0; k < SPT; ++k) {
         bool okk;
-        load_state_consts(sc[k], c < nvalid && jl + k * NL < N, jl + k * NL, i, N, p.B_r, p.B_theta, p.C_r, p.C_theta,
-                          BIAS ? p.theta_bias : nullptr, okk);      // mr, mi hold Cc
+        load_state_consts(sc[k], c < nvalid && jl + k * NL < N, jl + k * NL, p.B_r, p.B_theta, p.C_r, p.C_theta, okk);      // mr, mi hold Cc
     }
     const float* theta_warp = p.theta + wt.ch0 * N * p.ld_theta + wt.t0;
     const long long row0 = wt.ch0 * p.ld_row + wt.t0;
@@ -961,11 +944,7 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_summary_kernel(con
 #pragma unroll
             for (int k = 0; k < SPT; ++k) {
                 const float4 t4 = ld_shared_f4(th + (k * 32 + lane) * TP + 4 * q);
-                float tv[4] = {t4.x, t4.y, t4.z, t4.w};
-                if (BIAS) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) tv[e] += sc[k].bias;
-                }
+                const float tv[4] = {t4.x, t4.y, t4.z, t4.w};
                 float sn[4], cs[4];
                 sincos4(tv, sn, cs);
 #pragma unroll
@@ -1215,9 +1194,9 @@ long long warp_tasks(const P& p) {
     return (((long long)p.nch + C::CPW - 1) / C::CPW) * (p.nseg > 1 ? p.nseg : 1);
 }
 
-template <class C, bool VEC, bool BIAS>
+template <class C, bool VEC>
 cudaError_t launch_fwd_cfg(const ScanFwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_fwd_kernel<C, VEC, BIAS>;
+    auto kern = scan_unitary_fwd_kernel<C, VEC>;
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1227,9 +1206,9 @@ cudaError_t launch_fwd_cfg(const ScanFwdParams& p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template <class C, bool VEC, bool BIAS, bool PARTS>
+template <class C, bool VEC, bool PARTS>
 cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_bwd_kernel<C, VEC, BIAS, PARTS>;
+    auto kern = scan_unitary_bwd_kernel<C, VEC, PARTS>;
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1239,25 +1218,22 @@ cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-// Runtime properties -> template parameters.  The forward kernels for unaligned rows are instantiated with the phase
-// offset always on, to keep the build small.
+// Runtime properties -> template parameters.
 template <class C>
 cudaError_t launch_fwd_sel(const ScanFwdParams& p, bool vec, cudaStream_t s) {
-    if (!vec) return launch_fwd_cfg<C, false, true>(p, s);
-    return p.theta_bias != nullptr ? launch_fwd_cfg<C, true, true>(p, s) : launch_fwd_cfg<C, true, false>(p, s);
+    return vec ? launch_fwd_cfg<C, true>(p, s) : launch_fwd_cfg<C, false>(p, s);
 }
 
 template <class C>
 cudaError_t launch_bwd_sel(const ScanBwdParams& p, bool vec, cudaStream_t s) {
-    // the drop-in pipeline has the phase offset and takes the FP16 parts, the scan core neither
-    if (p.parts_hi) return vec ? launch_bwd_cfg<C, true, true, true>(p, s) : launch_bwd_cfg<C, false, true, true>(p, s);
-    if (p.theta_bias || p.part_rowsum) return cudaErrorInvalidValue;
-    return vec ? launch_bwd_cfg<C, true, false, false>(p, s) : launch_bwd_cfg<C, false, false, false>(p, s);
+    if ((p.parts_hi != nullptr) != (p.part_rowsum != nullptr)) return cudaErrorInvalidValue;
+    if (p.parts_hi) return vec ? launch_bwd_cfg<C, true, true>(p, s) : launch_bwd_cfg<C, false, true>(p, s);
+    return vec ? launch_bwd_cfg<C, true, false>(p, s) : launch_bwd_cfg<C, false, false>(p, s);
 }
 
-template <class C, bool VEC, bool BIAS, bool BWD>
+template <class C, bool VEC, bool BWD>
 cudaError_t launch_summary_cfg(const SegSummaryParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_summary_kernel<C, VEC, BIAS, BWD>;
+    auto kern = scan_unitary_summary_kernel<C, VEC, BWD>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     const long long blocks = (warp_tasks<C>(p) + C::WARPS - 1) / C::WARPS;
@@ -1271,8 +1247,8 @@ template <int NL, int SPT, int T, int STAGES, int WARPS>
 cudaError_t launch_summary_sel(const SegSummaryParams& p, bool vec, cudaStream_t s) {
     using F = Cfg<NL, SPT, T, T, STAGES, WARPS, 2, false>;
     using B = Cfg<NL, SPT, T, T, STAGES, WARPS, 4, false>;
-    if (p.gy) return vec ? launch_summary_cfg<B, true, true, true>(p, s) : launch_summary_cfg<B, false, true, true>(p, s);
-    return vec ? launch_summary_cfg<F, true, true, false>(p, s) : launch_summary_cfg<F, false, true, false>(p, s);
+    if (p.gy) return vec ? launch_summary_cfg<B, true, true>(p, s) : launch_summary_cfg<B, false, true>(p, s);
+    return vec ? launch_summary_cfg<F, true, false>(p, s) : launch_summary_cfg<F, false, false>(p, s);
 }
 
 // a warp's rows must be addressable with 32-bit byte offsets from its first row
@@ -1389,7 +1365,7 @@ cudaError_t scan_unitary_fwd_split(const ScanFwdParams& p, const SegPlan& plan, 
     const long long VN = (long long)p.nch * plan.nseg * p.N;
     float *e_re = scratch, *e_im = e_re + VN, *a_re = e_im + VN, *a_im = a_re + VN, *b_re = a_im + VN,
           *b_im = b_re + VN;
-    const SegSummaryParams sum = {p.theta, p.theta_bias, p.u, p.dt, nullptr, nullptr, p.B_r, p.B_theta, p.C_r, p.C_theta,
+    const SegSummaryParams sum = {p.theta, p.u, p.dt, nullptr, nullptr, p.B_r, p.B_theta, p.C_r, p.C_theta,
                                   e_re, e_im, a_re, a_im, nullptr, nullptr, p.nch, p.Dmod, p.N, p.L, p.ld_theta,
                                   p.ld_row, plan.nseg, plan.seg_len};
     cudaError_t err = launch_summary(sum, stream);
@@ -1415,7 +1391,7 @@ cudaError_t scan_unitary_bwd_split(const ScanBwdParams& p, const SegPlan& plan, 
     const long long VN = (long long)p.nch * plan.nseg * p.N;
     float *e_re = scratch, *e_im = e_re + VN, *a_re = e_im + VN, *a_im = a_re + VN, *s_re = a_im + VN,
           *s_im = s_re + VN, *l_re = s_im + VN, *l_im = l_re + VN, *g_re = l_im + VN, *g_im = g_re + VN;
-    const SegSummaryParams sum = {p.theta, p.theta_bias, p.u, p.dt, p.z, p.gy, p.B_r, p.B_theta, p.C_r, p.C_theta,
+    const SegSummaryParams sum = {p.theta, p.u, p.dt, p.z, p.gy, p.B_r, p.B_theta, p.C_r, p.C_theta,
                                   e_re, e_im, a_re, a_im, l_re, l_im, p.nch, p.Dmod, p.N, p.L, p.ld_theta, p.ld_row,
                                   plan.nseg, plan.seg_len};
     cudaError_t err = launch_summary(sum, stream);

@@ -14,7 +14,6 @@ namespace aussm {
 // longer sequence, or on a packed workspace).
 struct ScanFwdParams {
     const float* theta;        // (nch, N, L) rows, ld_theta apart
-    const float* theta_bias;   // (D, N) added to every phase, or nullptr
     const float* u;            // (nch, L) rows, ld_row apart
     const float* dt;
     const float* z;
@@ -43,7 +42,6 @@ struct ScanFwdParams {
 
 struct ScanBwdParams {
     const float* theta;
-    const float* theta_bias;
     const float* u;
     const float* dt;
     const float* z;
@@ -67,7 +65,7 @@ struct ScanBwdParams {
     float* h0_im;
     float* part_bc;            // (nch, N, 4): grad of Bc (re, im), grad of Cc (re, im)
     float* part_d;             // (nch,)
-    float* part_rowsum;        // (nch, N) sum over t of dtheta, or nullptr
+    float* part_rowsum;        // (nch, N) sum over t of dtheta; with parts_hi only
     // Instead of dtheta its FP16 parts (the drop-in pipeline; see gemm_split3.cuh): same rows and pitch, in halves,
     // scaled by the power of two that the bit pattern of a bound of |dtheta| at *parts_max gives.  nullptr: dtheta.
     __half* parts_hi;
@@ -85,7 +83,7 @@ struct ScanBwdParams {
 
 // What every segment of a launch does to the state and to the adjoint (see scan_unitary_summary_kernel)
 struct SegSummaryParams {
-    const float *theta, *theta_bias, *u, *dt, *z, *gy;      // z, gy only for the backward pass (gy == nullptr: forward)
+    const float *theta, *u, *dt, *z, *gy;      // z, gy only for the backward pass (gy == nullptr: forward)
     const float *B_r, *B_theta, *C_r, *C_theta;
     float *e_re, *e_im, *a_re, *a_im, *l_re, *l_im;         // (nch, nseg, N)
     int nch, Dmod, N, L;
