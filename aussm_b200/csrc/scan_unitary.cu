@@ -1068,8 +1068,8 @@ __global__ void __launch_bounds__(256) dtheta_bound_kernel(const ScanBwdParams p
     const long long ch = blockIdx.x, row = ch * p.ld_row;
     float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};       // sum |s|, sum |w|; max |h|^2, |g|^2, |B|, |C|
     auto add = [&](float u, float dt, float z, float gy) {
-        v[0] += fabsf(dt * siluf_(u));
-        v[1] += fabsf(gy * siluf_(z));
+        v[0] += fmaxf(fabsf(dt * siluf_(u)), 0.f);       // a NaN counts as zero: it spoils its own channel, no other's scale
+        v[1] += fmaxf(fabsf(gy * siluf_(z)), 0.f);
     };
     if (VEC) {
         for (int q = threadIdx.x; q < p.L / 4; q += 256) {
@@ -1109,9 +1109,9 @@ __global__ void __launch_bounds__(256) dtheta_bound_kernel(const ScanBwdParams p
 #pragma unroll
             for (int k = 0; k < 6; ++k) v[k] = k < 2 ? v[k] + sums[w][k] : fmaxf(v[k], sums[w][k]);
         }
-        // 1 % for the roundings of the sums and of the scan itself; a product out of range or a NaN counts as the largest
+        // 1 % for the roundings of the sums and of the scan itself; a product out of range counts as the largest
         const float b = 1.01f * (sqrtf(v[2]) + v[4] * v[0]) * (sqrtf(v[3]) + v[5] * v[1]);
-        if (!(b <= 0.f)) atomicMax(bound, __float_as_uint(fminf(b, 3.0e38f)));
+        if (b > 0.f) atomicMax(bound, __float_as_uint(fminf(b, 3.0e38f)));
     }
 }
 

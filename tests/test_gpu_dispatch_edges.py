@@ -106,6 +106,23 @@ def test_operator_gradients_of_any_magnitude(shape, gain):
     assert max(errors.values()) < operator_bound(*shape), errors
 
 
+def test_a_nan_spoils_its_own_channel_only():
+    """A NaN in one channel's incoming gradient must not reach the other channels' rows of dx nor other batch entries."""
+    b, d, n, l = 2, 6, 4, 200
+    inp = model_like_inputs(3300, b, d, n, l)
+    results = []
+    for bad in (0.0, float("nan")):
+        a = {k: inp[k].cuda().requires_grad_(True) for k in NAMES}
+        gy = inp["gy"].cuda()
+        gy[0, 2, 77] = bad
+        results.append(torch.autograd.grad(aussm_b200.ssm_adaptive_interface(**a), (a["x"], a["u"]), gy))
+    (dx, du), (dx_nan, du_nan) = results
+    others = [i for i in range(d) if i != 2]
+    assert torch.isnan(dx_nan[2]).any() and torch.isnan(du_nan[0]).any()
+    assert scaled_error(dx_nan[others], dx[others]) < operator_bound(b, d, n, l)
+    assert scaled_error(du_nan[1], du[1]) < operator_bound(b, d, n, l)
+
+
 @pytest.mark.parametrize("steps", [576, 640, 2000])
 def test_operator_windows_of_unequal_length_split_in_time(steps):
     """2000 steps in windows of 576 (the last one shorter than a segment), 640 and one: same result."""
