@@ -142,7 +142,7 @@ void keep_note_layout(const void* keep, const Plan& pl) {
     g_keep_layouts[keep] = KeepLayout{pl.window, pl.ldw, pl.rows};
 }
 
-// consumes the note (the backward call overwrites the phases: a buffer serves one backward call)
+// consumes the note (a buffer serves one backward call)
 int keep_check_layout(const void* keep, const Plan& pl) {
     std::lock_guard<std::mutex> lock(g_keep_mutex);
     auto it = g_keep_layouts.find(keep);

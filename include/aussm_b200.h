@@ -66,7 +66,7 @@ unsigned long long aussm_b200_kernel_launches(void);
  * that was written under another value, and a call given a workspace sized
  * under another value returns AUSSM_EWORKSPACE; neither computes with a wrong
  * layout.  "time_split" (default 1): 0 turns the time-axis split of under-filled
- * scans off (see aussm_b200_scan_unitary_fwd_ws); it changes workspace sizes
+ * scans (unitary, selective, complex) off (see aussm_b200_scan_unitary_fwd_ws); it changes workspace sizes
  * too.  Returns AUSSM_EINVAL for an unknown name. */
 int aussm_b200_set_option(const char* name, int value);
 
@@ -84,9 +84,10 @@ int aussm_b200_scan_unitary_fwd(const float* theta, const float* u, const float*
 /* Time-axis split.  The scans walk time sequentially and get their parallelism
  * from the B*D channels (the reference gets it from block scans over time,
  * ssm_adaptive_unitary_forward.cu:122-144, reverse_scan.h:152-302).  When the
- * channels fill less than a quarter of the GPU, the launch is cut into equal
- * time segments per channel: an aggregate pass gives every segment's end state
- * from zero and the product of its rotations, a short chain over the segments
+ * channels fill less than a quarter of the GPU (and L is at least 1024), the
+ * launch is cut into time segments per channel: a summary pass gives every
+ * segment's end state from zero, the product of its rotations and (backward) the
+ * gradient it sends to its start, a short chain over the segments
  * gives every segment its true initial state (backward: its end state and the
  * incoming gradient, the rotations being invertible), and the real pass then
  * runs all segments side by side.  Same results up to float32 rounding.  The
@@ -216,9 +217,9 @@ int aussm_b200_unitary_bwd(const float* grad_y, const float* gh1_re, const float
  * counterpart in the reference, whose backward recomputes every intermediate
  * from the 12 inputs: ssm_adaptive_unitary_backward.cu:50-141).  The forward
  * writes every window's phases into `theta_keep` (aussm_b200_unitary_keep_bytes
- * bytes, 256-byte aligned: about 4*B*D*N*L); the backward reads them instead
- * of running the projection again and overwrites them with their gradient, so
- * the buffer is consumed by one backward call.  The final state h1_* of the
+ * bytes, 256-byte aligned: about 4*B*D*N*L; x_bias included); the backward reads
+ * them instead of running the projection again.  The buffer serves one backward
+ * call.  The final state h1_* of the
  * forward call is required.  Results are bit-identical to the plain pair. */
 size_t aussm_b200_unitary_keep_bytes(int B, int D, int N, int L);
 
@@ -248,8 +249,9 @@ int aussm_b200_unitary_bwd_kept(const float* grad_y, const float* gh1_re, const 
  * u, delta, z, out: (B, D, L); A: (D, N); Bm, Cm: (B, N, L).  L must be a
  * multiple of 4 and N <= 32.  `ckpt` (aussm_b200_selective_scan_ckpt_floats
  * floats; its layout belongs to the library) receives the state at every 16th
- * step (every 32nd for N > 16) and is what the backward pass restarts from
- * (NULL when no backward pass will follow).  dB and dC are summed
+ * step and is what the backward pass restarts from (NULL when no backward pass
+ * will follow; launches with few channels hand states between time segments
+ * through it and run whole without it).  dB and dC are summed
  * over the channels with float atomics (as in mamba-ssm), so they are
  * reproducible only up to rounding; everything else is deterministic. */
 size_t aussm_b200_selective_scan_ckpt_floats(int B, int D, int N, int L);
