@@ -34,6 +34,8 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(d_model))
 
     def forward(self, x):
+        if torch.jit.is_scripting():
+            return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + self.eps) * self.weight
         return stages.rms_norm(x, self.weight, self.eps)
 
 

@@ -299,6 +299,9 @@ def _backward(ctx, grad_y, grad_next_hid_real, grad_next_hid_imag):
 torch.library.register_autograd("extension_cpp::ssm_adaptive_unitary", _backward, setup_context=_setup_context)
 
 
+_PLAIN = (Tensor, torch.nn.Parameter)          # no subclass that has to see the operations
+
+
 class _PolarParams(torch.autograd.Function):
     @staticmethod
     def forward(ctx, B, C):
@@ -315,7 +318,7 @@ class _PolarParams(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *g):
         B, C = ctx.saved_tensors
-        if torch.is_grad_enabled():                    # a graph of the gradient is wanted: differentiable operations
+        if torch.is_grad_enabled() or not _eager():    # a graph of the gradient is wanted: differentiable operations
             zero = torch.zeros_like(B.real)
             gBr, gBt, gCr, gCt = (zero if t is None else t for t in g)
             return (torch.complex(gBr * torch.sigmoid(B.real), gBt), torch.complex(gCr * torch.sigmoid(C.real), gCt))
@@ -330,15 +333,18 @@ class _PolarParams(torch.autograd.Function):
 
 
 def _eager() -> bool:
-    """No function transform, forward-mode differentiation or tracing around this call."""
+    """No function transform, forward-mode differentiation, tracer or dispatch mode around this call.  A kernel that
+    writes through raw pointers is invisible to a tracer (the graph would hold the empty outputs only), and a fake
+    tensor has no memory to point to."""
     return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
-                or torch.compiler.is_compiling())
+                or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() > 0
+                or torch._ops._len_torch_dispatch_stack_pre_dispatch() > 0 or torch._C._is_tracing())
 
 
 def _polar_params(B: Tensor, C: Tensor):
     """(B_r, B_theta, C_r, C_theta) with radius softplus(real part) and angle imaginary part."""
-    if (B.is_cuda and C.device == B.device and B.dtype == C.dtype == torch.complex64 and B.dim() == 1
-            and B.shape == C.shape and B.numel() > 0 and _eager()):
+    if (type(B) in _PLAIN and type(C) in _PLAIN and _eager() and B.is_cuda and C.device == B.device
+            and B.dtype == C.dtype == torch.complex64 and B.dim() == 1 and B.shape == C.shape and B.numel() > 0):
         return _PolarParams.apply(B, C)
     return (F.softplus(B.real).contiguous(), B.imag.contiguous(), F.softplus(C.real).contiguous(), C.imag.contiguous())
 

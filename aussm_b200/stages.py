@@ -20,7 +20,7 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from .ops import _eager, _f32c, _ptr, _stream, _workspace
+from .ops import _PLAIN, _eager, _f32c, _ptr, _stream, _workspace
 from .variants import _gemm
 
 __all__ = ["causal_conv_bias", "softplus_bias", "project_tokens", "project_channels", "project_back", "rms_norm",
@@ -124,12 +124,11 @@ def _rms_norm_ops(x: Tensor, weight: Tensor, eps: float) -> Tensor:
 
 def _norm_kernel_takes(x: Tensor, weight: Tensor) -> bool:
     """The kernels serve whole rows of quads in eager mode; everything else (other types and devices, odd widths,
-    function transforms, forward-mode differentiation, tracing) takes the plain operations."""
-    return (x.is_cuda and x.dtype == torch.float32 and weight.dtype == torch.float32 and weight.device == x.device
+    function transforms, forward-mode differentiation, tracers and dispatch modes) takes the plain operations."""
+    return (type(x) in _PLAIN and type(weight) in _PLAIN and _eager()
+            and x.is_cuda and x.dtype == torch.float32 and weight.dtype == torch.float32 and weight.device == x.device
             and weight.dim() == 1 and x.dim() >= 1 and x.shape[-1] == weight.shape[0] and x.numel() > 0
-            and x.shape[-1] % 4 == 0 and x.shape[-1] <= MAX_NORM_CHANNELS
-            and type(x) is Tensor and isinstance(weight, Tensor)
-            and _eager())
+            and x.shape[-1] % 4 == 0 and x.shape[-1] <= MAX_NORM_CHANNELS)
 
 
 def _aligned(t: Tensor) -> Tensor:
@@ -160,7 +159,7 @@ class _RMSNorm(torch.autograd.Function):
         x, weight, rstd = ctx.saved_tensors
         if g is None:
             return extra, None, None
-        if torch.is_grad_enabled():                    # a graph of the gradient is wanted: differentiable operations
+        if torch.is_grad_enabled() or not _eager():    # a graph of the gradient is wanted: differentiable operations
             r = torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + ctx.eps)
             gw = g * weight
             dx = r * gw - x * r.pow(3) * (gw * x).mean(-1, keepdim=True)
