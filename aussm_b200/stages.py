@@ -271,9 +271,11 @@ def _token_product(g: Tensor, x: Tensor) -> Tensor:
 
 def _batched(W: Tensor, x: Tensor, l: int) -> bool:
     """Whether a small product runs batched: the weight's gradient then has a partial product per batch entry, which
-    may take twice the memory of the layer's input and output at most."""
+    may take twice the memory of the layer's input and output at most.  Under autocast the product's type is not its
+    operands', which the gradients above do not undo: torch.matmul."""
     m, k = W.shape
-    return x.is_cuda and x.dtype == W.dtype == torch.float32 and x.numel() > 0 and m * k <= 2 * l * (m + k) and _eager()
+    return (x.is_cuda and x.dtype == W.dtype == torch.float32 and x.numel() > 0 and m * k <= 2 * l * (m + k)
+            and not torch.is_autocast_enabled("cuda") and _eager())
 
 
 def _weight_grad(A: Tensor, a_mn: int, B: Tensor, b_mn: int, m: int, k: int, l: int, b: int) -> Tensor:

@@ -91,3 +91,22 @@ def test_a_jit_traced_norm_can_be_saved():
     torch.jit.save(torch.jit.trace(norm, x), buffer)
     buffer.seek(0)
     assert (torch.jit.load(buffer)(x) - norm(x)).abs().max() < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,shape,product", [
+    ("project_tokens", (2, 24, 8), lambda W, x: torch.matmul(W, x.transpose(1, 2))),
+    ("project_channels", (2, 8, 24), lambda W, x: torch.matmul(W, x)),
+    ("project_back", (2, 8, 24), lambda W, x: torch.matmul(x.transpose(1, 2), W.t()))])
+def test_small_projections_under_autocast(name, shape, product):
+    """Forward and backward, as torch.matmul does them; the backward pass runs outside of the context, as is usual."""
+    W, x = (torch.randn(s, device="cuda", requires_grad=True) for s in ((12, 8), shape))
+    results = []
+    for fn in (getattr(stages, name), product):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = fn(W, x)
+        results.append((y, *torch.autograd.grad(y.float().square().sum(), (W, x))))
+    for got, expected in zip(*results):
+        assert got.dtype == expected.dtype
+        # products of up to 48 bf16 values in another order, rounded to bf16
+        assert (got.float() - expected.float()).abs().max() < 2.0 ** -7 * expected.float().abs().max()
