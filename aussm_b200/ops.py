@@ -201,12 +201,24 @@ def _fake_backward(grad_y, g_re, g_im, u, dt, x, x_bias, B_r, B_theta, C_r, C_th
 keep_phases = "auto"
 
 
+# Buffers below this size may be granted on the allocator's word.  A call of this size takes a workspace at least as
+# large from the same allocator, so a wrong answer cannot cost more than the call itself on a card that is full.
+_SMALL_KEEP = 256 << 20
+
+
 def _fits_a_quarter(nbytes: int, device) -> bool:
-    """True when ``nbytes`` are at most a quarter of the memory that is free for this process.  The allocator's own
-    count answers when the blocks it holds unused are room enough (8 us); the driver is asked otherwise (75 to 110 us)."""
-    stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
-    if stats and nbytes <= (stats["reserved_bytes"]["all"]["current"] - stats["active_bytes"]["all"]["current"]) // 4:
-        return True
+    """True when ``nbytes`` are at most a quarter of the memory that is free for this process.  The driver knows (75 to
+    110 us); for a small buffer the allocator's segments without any used block answer first (8 us).  Its fragments do
+    not count: no contiguous request can rely on them, nor are they given back to the driver."""
+    if nbytes < _SMALL_KEEP:
+        try:
+            stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
+            reserved, active, fragments = (stats[k]["all"]["current"] for k in
+                                           ("reserved_bytes", "active_bytes", "inactive_split_bytes"))
+            if nbytes <= (reserved - active - fragments) // 4:
+                return True
+        except Exception:                       # an allocator without statistics
+            pass
     free, _total = torch.cuda.mem_get_info(device)
     return nbytes <= free // 4
 
@@ -223,16 +235,25 @@ def _want_keep(inputs, b, d, n, l) -> int:
     return nbytes if _fits_a_quarter(nbytes, inputs[0].device) else 0
 
 
+def _keep_buffer(nbytes: int, device) -> Optional[Tensor]:
+    """The phase buffer, or None (recompute) when it was only expected to fit."""
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        if keep_phases is True:
+            raise
+        return None
+
+
 class _UnitaryKeep(torch.autograd.Function):
     """extension_cpp::ssm_adaptive_unitary with the phases kept for the backward pass."""
 
     @staticmethod
-    def forward(ctx, keep_bytes, *inputs):
+    def forward(ctx, keep, *inputs):
         (b, d, n, l, u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, D, z, h_re, h_im) = _check_op_inputs(*inputs)
         lib = _lib.load()
         y = torch.empty_like(u)
         o_re, o_im = (torch.empty(b, d, n, device=u.device, dtype=torch.float32) for _ in range(2))
-        keep = torch.empty(keep_bytes, dtype=torch.uint8, device=u.device)
         with torch.cuda.device(u.device):
             ws = _workspace(lib.aussm_b200_unitary_workspace_bytes(b, d, n, l), u.device)
             rc = lib.aussm_b200_unitary_fwd_keep(
@@ -264,8 +285,9 @@ def ssm_adaptive_unitary(u: Tensor, dt: Tensor, x: Tensor, x_bias: Tensor, B_r: 
     inputs = (u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, D, z, prev_hidden_state_real, prev_hidden_state_imag)
     if u.is_cuda and u.dim() == 3 and x.dim() == 3:
         keep_bytes = _want_keep(inputs, u.shape[0], u.shape[1], x.shape[1], u.shape[2])
-        if keep_bytes:
-            return _UnitaryKeep.apply(keep_bytes, *inputs)
+        keep = _keep_buffer(keep_bytes, u.device) if keep_bytes else None
+        if keep is not None:
+            return _UnitaryKeep.apply(keep, *inputs)
     if prev_hidden_state_real is None and prev_hidden_state_imag is None:      # the op's schema has no optional state
         zeros = torch.zeros((u.shape[0], u.shape[1], x.shape[1]), device=u.device, dtype=torch.float32)
         inputs = inputs[:10] + (zeros, zeros.clone())

@@ -1,0 +1,71 @@
+"""Whether a differentiable operator call keeps its phases: the memory that may be counted as free, without a GPU."""
+import pytest
+import torch
+
+from aussm_b200 import ops
+
+MB = 1 << 20
+
+
+def _stats(reserved, active, fragments):
+    return {k + "_bytes": {"all": {"current": v * MB}} for k, v in
+            (("reserved", reserved), ("active", active), ("inactive_split", fragments))}
+
+
+@pytest.fixture
+def memory(monkeypatch):
+    """memory(statistics or an exception, free megabytes) -> list that counts the questions to the driver"""
+    def setup(stats, free_mb):
+        asked = []
+
+        def statistics(device=None):
+            if isinstance(stats, Exception):
+                raise stats
+            return stats
+
+        def driver(device=None):
+            asked.append(device)
+            return free_mb * MB, 180_000 * MB
+
+        monkeypatch.setattr(torch.cuda.memory, "memory_stats_as_nested_dict", statistics)
+        monkeypatch.setattr(torch.cuda, "mem_get_info", driver)
+        return asked
+    return setup
+
+
+def test_whole_unused_segments_answer_for_a_small_buffer(memory):
+    asked = memory(_stats(1000, 200, 300), 0)
+    assert ops._fits_a_quarter(125 * MB, "cuda") and not asked          # a quarter of 500 MB
+    assert not ops._fits_a_quarter(126 * MB, "cuda") and asked
+
+
+def test_fragments_are_not_free_memory(memory):
+    """A reserve in pieces serves no contiguous request and cannot be given back: the driver's answer stands."""
+    asked = memory(_stats(100_000, 20_000, 79_990), 20)
+    assert not ops._fits_a_quarter(50 * MB, "cuda") and asked
+
+
+def test_a_large_buffer_asks_the_driver(memory):
+    """Unused blocks of other streams and of graphs' pools are in the allocator's count too."""
+    asked = memory(_stats(100_000, 0, 0), 500)
+    assert not ops._fits_a_quarter(1024 * MB, "cuda") and asked
+    memory(_stats(100_000, 0, 0), 4096)
+    assert ops._fits_a_quarter(1024 * MB, "cuda")
+
+
+@pytest.mark.parametrize("stats", [{}, RuntimeError("this allocator has no statistics")])
+def test_an_allocator_without_statistics_asks_the_driver(memory, stats):
+    asked = memory(stats, 100)
+    assert ops._fits_a_quarter(25 * MB, "cuda") and not ops._fits_a_quarter(26 * MB, "cuda") and len(asked) == 2
+
+
+def test_a_buffer_that_does_not_fit_after_all(monkeypatch):
+    """The call falls back to recomputing the phases, unless keeping them was asked for."""
+    def full(*args, **kwargs):
+        raise torch.cuda.OutOfMemoryError("full")
+
+    monkeypatch.setattr(torch, "empty", full)
+    assert ops._keep_buffer(MB, "cuda") is None
+    monkeypatch.setattr(ops, "keep_phases", True)
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        ops._keep_buffer(MB, "cuda")
