@@ -97,6 +97,8 @@ def _check_op_inputs(u, dt, x, x_bias, B_r, B_theta, C_r, C_theta, D, z, h_re, h
         raise RuntimeError(f"x must be (d, n, d) with d={d}, got {tuple(x.shape)}")
     n = x.shape[1]
     u = _f32c("u", u)
+    if (h_re is None) != (h_im is None):
+        raise RuntimeError("prev_hid_real and prev_hid_imag: both tensors or both None")
     return (b, d, n, l,
             u, _f32c("dt", dt, (b, d, l)), _f32c("x", x, (d, n, d)), _f32c("x_bias", x_bias, (d, n)),
             _f32c("B_r", B_r, (n,)), _f32c("B_theta", B_theta, (n,)), _f32c("C_r", C_r, (n,)),

@@ -1,6 +1,7 @@
-"""Whether a differentiable operator call keeps its phases: the memory that may be counted as free, without a GPU."""
+"""Host side of a differentiable operator call, without a GPU: what it refuses, whether it keeps its phases."""
 import pytest
 import torch
+from torch._subclasses import FakeTensorMode
 
 from aussm_b200 import ops
 
@@ -69,3 +70,14 @@ def test_a_buffer_that_does_not_fit_after_all(monkeypatch):
     monkeypatch.setattr(ops, "keep_phases", True)
     with pytest.raises(torch.cuda.OutOfMemoryError):
         ops._keep_buffer(MB, "cuda")
+
+
+@pytest.mark.parametrize("given", [10, 11])
+def test_half_of_a_state_is_refused(given):
+    b, d, n, l = 2, 8, 4, 16
+    with FakeTensorMode():
+        shapes = [(b, d, l), (b, d, l), (d, n, d), (d, n)] + [(n,)] * 4 + [(d,), (b, d, l), None, None]
+        shapes[given] = (b, d, n)
+        inputs = [None if s is None else torch.empty(s, device="cuda") for s in shapes]
+        with pytest.raises(RuntimeError, match="both"):
+            ops._check_op_inputs(*inputs)
