@@ -618,13 +618,10 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
         p.part_nseg = nseg_b;
         p.nch = (int)nch; p.Dmod = D; p.N = N; p.L = tl;
         p.ld_theta = pl.ldw; p.ld_dtheta = pl.ldw; p.ld_row = L;
-        // the scan writes the FP16 parts of dtheta that the adjoint GEMMs take, scaled by a bound (cleared with the
+        // the scan leaves max|dtheta| of the window behind for the FP16 split of the adjoint GEMMs (cleared with the
         // split of u)
-        p.parts_hi = static_cast<__half*>(ps.dth_hi);
-        p.parts_lo = static_cast<__half*>(ps.dth_lo);
-        p.parts_max = ps.amax + 2;
-        cudaError_t e = launch_dtheta_bound(p, ps.amax + 2, stream);
-        if (e != cudaSuccess) return cuda_fail(e, "dtheta bound launch");
+        p.dtheta_amax = ps.amax + 2;
+        cudaError_t e;
         const SegPlan seg = window_segments(pl.seg_bwd, tl);
         if (seg.nseg > 1) {
             e = scan_unitary_bwd_split(p, seg, reinterpret_cast<float*>(ws + pl.off_split), stream);
@@ -632,7 +629,7 @@ static int unitary_bwd_impl(const float* grad_y, const float* gh1_re, const floa
             e = launch_scan_unitary_bwd(p, stream);
         }
         if (e != cudaSuccess) return cuda_fail(e, "unitary scan backward launch");
-        if (int rc = proj_adjoints(pd, nullptr, dx, du, first, ps, stream)) return rc;
+        if (int rc = proj_adjoints(pd, theta_w, dx, du, first, ps, stream, true)) return rc;
     }
     ReduceParams r = {};
     r.part_bc = part_bc; r.part_d = part_d; r.part_rowsum = part_rowsum;

@@ -88,6 +88,33 @@ struct GemmKernelParams {
     int tiles_m, tiles_n, ntiles;   // one-CTA kernel: a CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...
 };
 
+// FP16 parts: the scaled low part is stored times 2^LO_SHIFT (see split_f16x4)
+constexpr int LO_SHIFT = 11;
+
+// Power-of-two scale that brings a tensor whose largest magnitude has the bit pattern `maxbits` to about 2^14
+// (FP16 overflows at 65504), and its exact inverse.
+__device__ __forceinline__ int scale_exponent(unsigned maxbits) {
+    const int e = (int)((maxbits >> 23) & 0xffu) - 127;      // floor(log2(max)); -127 for zero / subnormal
+    int k = 14 - e;
+    if (k > 100) k = 100;
+    if (k < -100) k = -100;
+    return k;
+}
+__device__ __forceinline__ float pow2f(int k) { return __uint_as_float((unsigned)(127 + k) << 23); }
+
+// The parts of four consecutive values, as the 8-byte words that are stored.  S = 2^k brings the tensor's largest
+// magnitude to about 2^14:  hi = fp16(S a),  lo = fp16((S a - hi) 2^LO_SHIFT).
+__device__ __forceinline__ void split_f16x4(const float4& v, float S, uint2& hi, uint2& lo) {
+    constexpr float up = (float)(1 << LO_SHIFT);
+    const float2 a = make_float2(v.x * S, v.y * S), b = make_float2(v.z * S, v.w * S);
+    const __half2 ha = __float22half2_rn(a), hb = __float22half2_rn(b);
+    const float2 fa = __half22float2(ha), fb = __half22float2(hb);
+    const __half2 la = __float22half2_rn(make_float2((a.x - fa.x) * up, (a.y - fa.y) * up));
+    const __half2 lb = __float22half2_rn(make_float2((b.x - fb.x) * up, (b.y - fb.y) * up));
+    hi = make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hb));
+    lo = make_uint2(*reinterpret_cast<const uint32_t*>(&la), *reinterpret_cast<const uint32_t*>(&lb));
+}
+
 // ---- PTX wrappers ---------------------------------------------------------
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1,
                                             int c2, int c3) {
@@ -726,7 +753,7 @@ int gemm_split3(const SplitOperand& A, const SplitOperand& B, float* C, const Ge
     return B.mn_major ? launch<0, 1>(maps, kp, grid, stream) : launch<0, 0>(maps, kp, grid, stream);
 }
 
-int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream) {
+int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream, bool have_amax) {
     SplitLaunch p = {};
     unsigned total_blocks = 0;
     int used = 0;
@@ -751,8 +778,10 @@ int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream) {
         if (++used == 1) p.second = total_blocks;
     }
     if (used == 0) return AUSSM_OK;
-    absmax_kernel<<<total_blocks, 256, 0, stream>>>(p);
-    count_launch();
+    if (!have_amax) {
+        absmax_kernel<<<total_blocks, 256, 0, stream>>>(p);
+        count_launch();
+    }
     split_f16_kernel<<<total_blocks, 256, 0, stream>>>(p);
     count_launch();
     cudaError_t e = cudaGetLastError();
@@ -765,16 +794,16 @@ int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream) {
 
 int split_f16(const float* src, long long ld_src, long long src_batch_stride, void* hi, void* lo, long long ld_dst,
               long long dst_batch_stride, long long rows, long long cols, int batches, unsigned* amax,
-              cudaStream_t stream) {
+              cudaStream_t stream, bool have_amax) {
     const SplitSource s = {src, ld_src, src_batch_stride, hi, lo, ld_dst, dst_batch_stride, rows, cols, batches, amax};
-    if (amax) {
+    if (amax && !have_amax) {
         cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(unsigned), stream);
         if (e != cudaSuccess) {
             set_error("split_f16: clearing the maximum: %s", cudaGetErrorString(e));
             return AUSSM_ECUDA;
         }
     }
-    return split_f16_many(&s, 1, stream);
+    return split_f16_many(&s, 1, stream, have_amax);
 }
 
 }  // namespace aussm

@@ -5,7 +5,6 @@
 // magnitude to about 2^14,  hi = fp16(S a),  lo = fp16((S a - hi) 2^11).
 #pragma once
 
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -13,33 +12,6 @@
 #include "host_common.cuh"
 
 namespace aussm {
-
-// FP16 parts: the scaled low part is stored times 2^LO_SHIFT (see split_f16x4)
-constexpr int LO_SHIFT = 11;
-
-// Power-of-two scale that brings a tensor whose largest magnitude has the bit pattern `maxbits` to about 2^14
-// (FP16 overflows at 65504), and its exact inverse.
-__device__ __forceinline__ int scale_exponent(unsigned maxbits) {
-    const int e = (int)((maxbits >> 23) & 0xffu) - 127;      // floor(log2(max)); -127 for zero / subnormal
-    int k = 14 - e;
-    if (k > 100) k = 100;
-    if (k < -100) k = -100;
-    return k;
-}
-__device__ __forceinline__ float pow2f(int k) { return __uint_as_float((unsigned)(127 + k) << 23); }
-
-// The parts of four consecutive values, as the 8-byte words that are stored.  S = 2^k brings the tensor's largest
-// magnitude to about 2^14:  hi = fp16(S a),  lo = fp16((S a - hi) 2^LO_SHIFT).
-__device__ __forceinline__ void split_f16x4(const float4& v, float S, uint2& hi, uint2& lo) {
-    constexpr float up = (float)(1 << LO_SHIFT);
-    const float2 a = make_float2(v.x * S, v.y * S), b = make_float2(v.z * S, v.w * S);
-    const __half2 ha = __float22half2_rn(a), hb = __float22half2_rn(b);
-    const float2 fa = __half22float2(ha), fb = __half22float2(hb);
-    const __half2 la = __float22half2_rn(make_float2((a.x - fa.x) * up, (a.y - fa.y) * up));
-    const __half2 lb = __float22half2_rn(make_float2((b.x - fb.x) * up, (b.y - fb.y) * up));
-    hi = make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hb));
-    lo = make_uint2(*reinterpret_cast<const uint32_t*>(&la), *reinterpret_cast<const uint32_t*>(&lb));
-}
 
 // One operand, already split into its two FP16 parts by split_f16.  `mn_major == 0`: stored as [rows][K] with K
 // contiguous; `mn_major == 1`: stored as [K][rows] with the row (M or N) index contiguous.  `ld` is the pitch of
@@ -99,11 +71,12 @@ struct SplitSource {
     unsigned* amax;
 };
 // Several tensors (up to kSplitSources) with one launch for the maxima and one for the parts: on small operands the
-// launches are what a split costs.  The amax words must be zero.
+// launches are what a split costs.  The amax words must be zero.  have_amax: they hold the maxima already (the
+// producers found them) and the pass over the sources that does is skipped.
 constexpr int kSplitSources = 2;
-int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream);
+int split_f16_many(const SplitSource* sources, int count, cudaStream_t stream, bool have_amax = false);
 int split_f16(const float* src, long long ld_src, long long src_batch_stride, void* hi, void* lo, long long ld_dst,
               long long dst_batch_stride, long long rows, long long cols, int batches, unsigned* amax,
-              cudaStream_t stream);
+              cudaStream_t stream, bool have_amax = false);
 
 }  // namespace aussm

@@ -131,13 +131,11 @@ int proj_theta(const ProjDims& d, const float* u, const float* bias, float* thet
 }
 
 int proj_adjoints(const ProjDims& d, const float* dtheta_w, float* dx, float* du, bool overwrite_dx, ProjScratch& s,
-                  cudaStream_t stream) {
+                  cudaStream_t stream, bool dtheta_amax_known) {
     const int M = (int)d.M;
-    if (dtheta_w) {
-        if (int rc = split_f16(dtheta_w, d.ldw, (long long)M * d.ldw, s.dth_hi, s.dth_lo, d.ldw, (long long)M * d.ldw, M,
-                               d.tl, d.B, s.amax + 2, stream))
-            return rc;
-    }
+    if (int rc = split_f16(dtheta_w, d.ldw, (long long)M * d.ldw, s.dth_hi, s.dth_lo, d.ldw, (long long)M * d.ldw, M,
+                           d.tl, d.B, s.amax + 2, stream, dtheta_amax_known))
+        return rc;
     {
         // dx (M x D) (+)= sum_b dtheta_b (M x tl, K-major) * u_b^T (u_b: D rows x tl, K-major)
         const SplitOperand A = {s.dth_hi, s.dth_lo, 0, d.ldw, (long long)M * d.ldw, s.amax + 2};

@@ -56,8 +56,8 @@ int proj_split_u(const ProjDims& d, const float* u, ProjScratch& s, cudaStream_t
 // bias: (M) added to every row of theta_w, or nullptr
 int proj_theta(const ProjDims& d, const float* u, const float* bias, float* theta_w, ProjScratch& s, cudaStream_t stream);
 // dx and du from dtheta_w; requires the split of u of the same window (proj_theta or proj_split_u).
-// dtheta_w == nullptr: its FP16 parts are already in s.dth_hi / s.dth_lo, scaled by s.amax[2] (the scan wrote them).
+// dtheta_amax_known: s.amax[2] already holds the bit pattern of max|dtheta_w| (the scan kernel found it).
 int proj_adjoints(const ProjDims& d, const float* dtheta_w, float* dx, float* du, bool overwrite_dx, ProjScratch& s,
-                  cudaStream_t stream);
+                  cudaStream_t stream, bool dtheta_amax_known = false);
 
 }  // namespace aussm

@@ -43,7 +43,6 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "gemm_split3.cuh"
 #include "scan_unitary.cuh"
 
 namespace aussm {
@@ -482,8 +481,8 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const S
 // ---------------------------------------------------------------------------
 // Backward
 // ---------------------------------------------------------------------------
-// PARTS (the drop-in pipeline): dtheta leaves as its FP16 parts, and its sums over time are collected.
-template <class C, bool VEC, bool NORM, bool PARTS>
+// SUMS (the drop-in pipeline): the sums of dtheta over time and its largest magnitude are collected.
+template <class C, bool VEC, bool NORM, bool SUMS>
 __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, const WarpTask& wt, int lane,
                                          StateConsts (&sc)[C::SPT], const float (&ccr)[C::SPT],
                                          const float (&cci)[C::SPT]) {
@@ -496,9 +495,6 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
     const float* theta_warp = p.theta + wt.ch0 * N * p.ld_theta + wt.t0;
     float* dtheta_warp = p.dtheta + wt.ch0 * N * p.ld_theta + wt.t0;      // launcher guarantees equal pitches
     const long long row0 = wt.ch0 * p.ld_row + wt.t0;
-    __half* hi_warp = PARTS ? p.parts_hi + wt.ch0 * N * p.ld_theta + wt.t0 : nullptr;
-    __half* lo_warp = PARTS ? p.parts_lo + wt.ch0 * N * p.ld_theta + wt.t0 : nullptr;
-    const float parts_scale = PARTS ? pow2f(scale_exponent(*p.parts_max)) : 1.f;
 
     float* scratch = wsm + STAGES * C::STAGE_FLOATS;
     float* pt = scratch;                    // [32][TSP] projections, summed over a thread's states
@@ -509,6 +505,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
     float er[SPT], ei[SPT];     // exp(-i theta_{t+1}) eta_{t+1}
     float gmr[SPT], gmi[SPT];   // sum_t w_t conj(h_t)
     float sbr[SPT], sbi[SPT];   // sum_t eta_t s_t              (general representation only)
+    float amax = 0.f;           // max |dtheta| seen by this thread (spares the split of dtheta a pass of its own)
     float rsum[SPT];            // sum_t dtheta_t
     float hlr[SPT], hli[SPT];   // conj(h_{L-1}) . gh   (boundary term of the Bc gradient)
 #pragma unroll
@@ -637,7 +634,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
                         // dtheta_t = -Im(conj(eta) a)
                         const float d = fmaf(ni, ar, -nr * ai);
                         dth[e] = d;
-                        if (PARTS) rsum[k] += d;
+                        if (SUMS) { rsum[k] += d; amax = fmaxf(amax, fabsf(d)); }
                         const float pv = fmaf(sc[k].mr, hr[k], -sc[k].mi * hi[k]);
                         // gradient of the real drive s_t: Re(conj(eta) beta)
                         const float ev = NORM ? nr : fmaf(nr, sc[k].br, ni * sc[k].bi);
@@ -721,17 +718,10 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
             constexpr int CPR = C::CHUNKS_PER_ROW, RPI = 32 / CPR;
             const int col = lane % CPR;
             const float* src0 = th + (lane / CPR) * TP + col * 4;
-            // 16 bytes of dtheta, or 8 bytes of each part at half the distance
+            float* dst0 = dtheta_warp + t0;
             auto leave = [&](const int i) {
-                const float4 v = ld_shared_f4(src0 + i * RPI * TP);
-                if (PARTS) {
-                    uint2 hi, lo;
-                    split_f16x4(v, parts_scale, hi, lo);
-                    *reinterpret_cast<uint2*>(reinterpret_cast<char*>(hi_warp + t0) + map.theta_off[i] / 2) = hi;
-                    *reinterpret_cast<uint2*>(reinterpret_cast<char*>(lo_warp + t0) + map.theta_off[i] / 2) = lo;
-                } else {
-                    *reinterpret_cast<float4*>(reinterpret_cast<char*>(dtheta_warp + t0) + map.theta_off[i]) = v;
-                }
+                *reinterpret_cast<float4*>(reinterpret_cast<char*>(dst0) + map.theta_off[i]) =
+                    ld_shared_f4(src0 + i * RPI * TP);
             };
             if (nvalid == C::CPW && N == NL * SPT && tlen == T) {      // whole tile, every row real: no per-piece test
 #pragma unroll
@@ -746,20 +736,12 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
                 }
             }
         } else if (lane < tlen) {                       // one row of 32 steps per instruction
+            float* dst = dtheta_warp + t0 + lane;
             const float* src = th + lane;
 #pragma unroll
             for (int slot = 0; slot < C::NROWS; ++slot) {
                 const int cc = (slot % 32) / NL, j = slot % NL + (slot / 32) * NL;
-                if (cc >= nvalid || j >= N) continue;
-                const long long at = (long long)(cc * N + j) * p.ld_theta + t0 + lane;
-                if (PARTS) {
-                    const float v = src[slot * TP] * parts_scale;
-                    const __half hi = __float2half_rn(v);
-                    hi_warp[at] = hi;
-                    lo_warp[at] = __float2half_rn((v - __half2float(hi)) * (float)(1 << LO_SHIFT));
-                } else {
-                    dtheta_warp[at] = src[slot * TP];
-                }
+                if (cc < nvalid && j < N) dst[(long long)(cc * N + j) * p.ld_theta] = src[slot * TP];
             }
         }
         __syncwarp();
@@ -804,9 +786,14 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
             dbr += old.x; dbi += old.y; dcr += old.z; dci += old.w;
         }
         *pb = make_float4(dbr, dbi, dcr, dci);
-        if (PARTS) p.part_rowsum[po] = rsum[k] + (p.accumulate ? p.part_rowsum[po] : 0.f);
+        if (SUMS) p.part_rowsum[po] = rsum[k] + (p.accumulate ? p.part_rowsum[po] : 0.f);
         if (p.dh0_re) { p.dh0_re[o] = d0r; p.dh0_im[o] = d0i; }
         if (p.h0_re) { p.h0_re[o] = s0r; p.h0_im[o] = s0i; }
+    }
+    if (SUMS) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if (lane == 0 && amax > 0.f) atomicMax(p.dtheta_amax, __float_as_uint(fminf(amax, 3.0e38f)));
     }
     // dD: add the lanes' partial sums channel by channel through the scratch tile
     __syncwarp();
@@ -823,7 +810,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
     }
 }
 
-template <class C, bool VEC, bool PARTS>
+template <class C, bool VEC, bool SUMS>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const ScanBwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -847,9 +834,9 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const S
     if (__all_sync(0xffffffffu, ok)) {
 #pragma unroll
         for (int k = 0; k < C::SPT; ++k) normalise_consts(sc[k], ccr[k], cci[k]);
-        bwd_warp<C, VEC, true, PARTS>(p, wsm, wt, lane, sc, ccr, cci);
+        bwd_warp<C, VEC, true, SUMS>(p, wsm, wt, lane, sc, ccr, cci);
     } else {
-        bwd_warp<C, VEC, false, PARTS>(p, wsm, wt, lane, sc, ccr, cci);
+        bwd_warp<C, VEC, false, SUMS>(p, wsm, wt, lane, sc, ccr, cci);
     }
 }
 
@@ -1056,66 +1043,6 @@ __global__ void __launch_bounds__(128) segment_states_bwd_kernel(const SegChainP
 }
 
 // ---------------------------------------------------------------------------
-// Bound of |dtheta|, one block per channel.  The FP16 parts need a common scale before the first of them is written; a
-// bound does instead of the maximum (which needed dtheta in float32 first, and a pass that read it again): the parts
-// resolve 2^-50 of the scale's top, so even a bound 2^20 too high leaves the pair finer than 2^-30 of the
-// true maximum (random inputs: about the length of the window too high).  Reads u, dt, z and gy once: 134 MB against
-// the 1074 MB it saves at B1 D512 N16 and a window of 16384 steps.
-// ---------------------------------------------------------------------------
-template <bool VEC>
-__global__ void __launch_bounds__(256) dtheta_bound_kernel(const ScanBwdParams p, unsigned* bound) {
-    __shared__ float sums[8][6];
-    const long long ch = blockIdx.x, row = ch * p.ld_row;
-    float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};       // sum |s|, sum |w|; max |h|^2, |g|^2, |B|, |C|
-    auto add = [&](float u, float dt, float z, float gy) {
-        v[0] += fmaxf(fabsf(dt * siluf_(u)), 0.f);       // a NaN counts as zero: it spoils its own channel, no other's scale
-        v[1] += fmaxf(fabsf(gy * siluf_(z)), 0.f);
-    };
-    if (VEC) {
-        for (int q = threadIdx.x; q < p.L / 4; q += 256) {
-            const float4 u = reinterpret_cast<const float4*>(p.u + row)[q], d = reinterpret_cast<const float4*>(p.dt + row)[q];
-            const float4 z = reinterpret_cast<const float4*>(p.z + row)[q], g = reinterpret_cast<const float4*>(p.gy + row)[q];
-            add(u.x, d.x, z.x, g.x);
-            add(u.y, d.y, z.y, g.y);
-            add(u.z, d.z, z.z, g.z);
-            add(u.w, d.w, z.w, g.w);
-        }
-    } else {
-        for (int t = threadIdx.x; t < p.L; t += 256) add(p.u[row + t], p.dt[row + t], p.z[row + t], p.gy[row + t]);
-    }
-    for (int j = threadIdx.x; j < p.N; j += 256) {
-        const float hr = p.h1_re[ch * p.N + j], hi = p.h1_im[ch * p.N + j];
-        v[2] = fmaxf(v[2], fmaf(hr, hr, hi * hi));
-        if (p.gh1_re) {
-            const float gr = p.gh1_re[ch * p.N + j], gi = p.gh1_im[ch * p.N + j];
-            v[3] = fmaxf(v[3], fmaf(gr, gr, gi * gi));
-        }
-        v[4] = fmaxf(v[4], fabsf(p.B_r[j]));
-        v[5] = fmaxf(v[5], fabsf(p.C_r[j]));
-    }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float other = __shfl_xor_sync(0xffffffffu, v[k], o);
-            v[k] = k < 2 ? v[k] + other : fmaxf(v[k], other);
-        }
-        if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5][k] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int w = 1; w < 8; ++w) {
-#pragma unroll
-            for (int k = 0; k < 6; ++k) v[k] = k < 2 ? v[k] + sums[w][k] : fmaxf(v[k], sums[w][k]);
-        }
-        // 1 % for the roundings of the sums and of the scan itself; a product out of range counts as the largest
-        const float b = 1.01f * (sqrtf(v[2]) + v[4] * v[0]) * (sqrtf(v[3]) + v[5] * v[1]);
-        if (b > 0.f) atomicMax(bound, __float_as_uint(fminf(b, 3.0e38f)));
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Second stage: fixed-order sums of the per-channel partials (deterministic)
 // and the polar chain rule  dr = Re(conj(G) e^{i phi}),  dphi = -Im(conj(G) w).
 // ---------------------------------------------------------------------------
@@ -1206,9 +1133,9 @@ cudaError_t launch_fwd_cfg(const ScanFwdParams& p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template <class C, bool VEC, bool PARTS>
+template <class C, bool VEC, bool SUMS>
 cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_bwd_kernel<C, VEC, PARTS>;
+    auto kern = scan_unitary_bwd_kernel<C, VEC, SUMS>;
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1226,8 +1153,8 @@ cudaError_t launch_fwd_sel(const ScanFwdParams& p, bool vec, cudaStream_t s) {
 
 template <class C>
 cudaError_t launch_bwd_sel(const ScanBwdParams& p, bool vec, cudaStream_t s) {
-    if ((p.parts_hi != nullptr) != (p.part_rowsum != nullptr)) return cudaErrorInvalidValue;
-    if (p.parts_hi) return vec ? launch_bwd_cfg<C, true, true>(p, s) : launch_bwd_cfg<C, false, true>(p, s);
+    if ((p.dtheta_amax != nullptr) != (p.part_rowsum != nullptr)) return cudaErrorInvalidValue;
+    if (p.part_rowsum) return vec ? launch_bwd_cfg<C, true, true>(p, s) : launch_bwd_cfg<C, false, true>(p, s);
     return vec ? launch_bwd_cfg<C, true, false>(p, s) : launch_bwd_cfg<C, false, false>(p, s);
 }
 
@@ -1411,15 +1338,6 @@ cudaError_t scan_unitary_bwd_split(const ScanBwdParams& p, const SegPlan& plan, 
     q.h1_re = s_re; q.h1_im = s_im; q.gh1_re = g_re; q.gh1_im = g_im;
     q.dh0_re = q.dh0_im = nullptr; q.h0_re = q.h0_im = nullptr;
     return launch_scan_unitary_bwd(q, stream);
-}
-
-cudaError_t launch_dtheta_bound(const ScanBwdParams& p, unsigned* bound, cudaStream_t stream) {
-    if (p.nch <= 0 || p.L <= 0) return cudaSuccess;
-    const bool vec = p.L % 4 == 0 && p.ld_row % 4 == 0 && aligned16(p.u) && aligned16(p.dt) && aligned16(p.z) && aligned16(p.gy);
-    if (vec) dtheta_bound_kernel<true><<<(unsigned)p.nch, 256, 0, stream>>>(p, bound);
-    else dtheta_bound_kernel<false><<<(unsigned)p.nch, 256, 0, stream>>>(p, bound);
-    count_launch();
-    return cudaGetLastError();
 }
 
 cudaError_t launch_reduce_param_grads(const ReduceParams& p, cudaStream_t stream) {

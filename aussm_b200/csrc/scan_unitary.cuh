@@ -1,7 +1,6 @@
 // Parameter blocks and launchers of the unitary scan-core kernels.
 #pragma once
 
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 
@@ -65,12 +64,9 @@ struct ScanBwdParams {
     float* h0_im;
     float* part_bc;            // (nch, N, 4): grad of Bc (re, im), grad of Cc (re, im)
     float* part_d;             // (nch,)
-    float* part_rowsum;        // (nch, N) sum over t of dtheta; with parts_hi only
-    // Instead of dtheta its FP16 parts (the drop-in pipeline; see gemm_split3.cuh): same rows and pitch, in halves,
-    // scaled by the power of two that the bit pattern of a bound of |dtheta| at *parts_max gives.  nullptr: dtheta.
-    __half* parts_hi;
-    __half* parts_lo;
-    const unsigned* parts_max;
+    float* part_rowsum;        // (nch, N) sum over t of dtheta, or nullptr
+    unsigned* dtheta_amax;     // receives (atomic max) the bit pattern of max|dtheta| of this launch; given together
+                               // with part_rowsum (the drop-in pipeline)
     int accumulate;            // 1: add to the partial buffers instead of overwriting them
     int nch, Dmod, N, L;
     long long ld_theta;
@@ -111,9 +107,6 @@ struct ReduceParams {
 
 cudaError_t launch_scan_unitary_fwd(const ScanFwdParams& p, cudaStream_t stream);
 cudaError_t launch_scan_unitary_bwd(const ScanBwdParams& p, cudaStream_t stream);
-// Writes (atomic max; *bound must be zero) the bit pattern of an upper bound of |dtheta| over the whole launch that `p`
-// describes: |dtheta_t| = |Im(conj(eta_t) lambda_t h_{t-1})| <= (|h_L| + |Bc| sum|s|) (|g_L| + |Cc| sum|w|).
-cudaError_t launch_dtheta_bound(const ScanBwdParams& p, unsigned* bound, cudaStream_t stream);
 cudaError_t launch_reduce_param_grads(const ReduceParams& p, cudaStream_t stream);
 
 // floats of scratch behind part_bc / part_d / part_rowsum for a launch

@@ -275,7 +275,7 @@ class _UnitaryKeep(torch.autograd.Function):
         inputs, f_re, f_im = saved[:12], saved[12], saved[13]
         if grad_y is None:
             grad_y = torch.zeros_like(inputs[0])
-        keep, ctx.keep = ctx.keep, None        # a phase buffer serves one backward call
+        keep, ctx.keep = ctx.keep, None        # the backward call overwrites the phases: usable once
         return (None,) + tuple(_unitary_backward(grad_y, g_re, g_im, *inputs, final_state=(f_re, f_im), keep=keep))
 
 

@@ -218,8 +218,8 @@ int aussm_b200_unitary_bwd(const float* grad_y, const float* gh1_re, const float
  * from the 12 inputs: ssm_adaptive_unitary_backward.cu:50-141).  The forward
  * writes every window's phases into `theta_keep` (aussm_b200_unitary_keep_bytes
  * bytes, 256-byte aligned: about 4*B*D*N*L; x_bias included); the backward reads
- * them instead of running the projection again.  The buffer serves one backward
- * call.  The final state h1_* of the
+ * them instead of running the projection again and overwrites them with their
+ * gradient, so the buffer serves one backward call.  The final state h1_* of the
  * forward call is required.  Results are bit-identical to the plain pair. */
 size_t aussm_b200_unitary_keep_bytes(int B, int D, int N, int L);
 

@@ -96,14 +96,40 @@ def test_operator_adjoints_summed_in_runs(shape):
     assert max(errors.values()) < 10 * bound, (errors, bound)
 
 
-# The phase gradients leave the scan as FP16 parts scaled by a bound, not by their maximum: any magnitude of the
-# incoming gradient, and inputs whose bound is far too high (a long window, one large step).
+# The phase gradients are split into FP16 parts scaled by their maximum: any magnitude of the incoming gradient.
 @pytest.mark.parametrize("gain", [1e-25, 1e-6, 1.0, 1e18])
 @pytest.mark.parametrize("shape", [(1, 9, 5, 1500), (2, 20, 16, 130)])
 def test_operator_gradients_of_any_magnitude(shape, gain):
     errors = operator_errors(*shape, 3200 + sum(shape), gain)
     assert aussm_b200.device_status() == 0
     assert max(errors.values()) < operator_bound(*shape), errors
+
+
+# Channels far apart in magnitude: every row of dx has to be right on its own scale.  The FP16 parts resolve 2^-50 of the
+# largest |dtheta|, so a channel 2^-s below it (its rows' norm up to 8 times below its maximum) has its values to 2^(s-47);
+# the scan itself is held to four times the 4e-7 sqrt(l) measured for the operator.
+@pytest.mark.parametrize("l", [300, 4096])
+@pytest.mark.parametrize("how", ["gradient", "large step"])
+def test_operator_rows_of_small_channels(l, how):
+    b, d, n = 1, 6, 4
+    inp = model_like_inputs(3250 + l, b, d, n, l)
+    below = torch.zeros(d)
+    if how == "gradient":
+        below = torch.tensor([0.0, 12.0, 20.0, 26.0, 30.0, 34.0])
+        inp["gy"] = inp["gy"] * (0.5 ** below)[:, None]
+    else:                                            # one step of one channel drives its state and dtheta far up
+        inp["dt"][0, 0, l // 2] *= 1e7
+        below[1:] = 24.0
+    dx = []
+    for dev, real, cplx, fn in (("cpu", torch.float64, torch.complex128, O.interface_unitary),
+                                ("cuda", torch.float32, torch.complex64, aussm_b200.ssm_adaptive_interface)):
+        a = {k: inp[k].to(dev, cplx if inp[k].is_complex() else real).requires_grad_(k == "x") for k in NAMES}
+        dx.append(torch.autograd.grad(fn(*(a[k] for k in NAMES)), a["x"], inp["gy"].to(dev, real))[0].double().cpu())
+    truth, got = dx
+    assert aussm_b200.device_status() == 0
+    error = (got - truth).flatten(1).norm(dim=1) / truth.flatten(1).norm(dim=1)
+    bound = 1.6e-6 * math.sqrt(l) + 2.0 ** (below.double() - 47)
+    assert (error < bound).all(), (error, bound)
 
 
 def test_a_nan_spoils_its_own_channel_only():
