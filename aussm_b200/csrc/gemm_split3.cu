@@ -518,8 +518,12 @@ __device__ __forceinline__ float quads_absmax(const float* __restrict__ src, lon
             w.next();
         }
 #pragma unroll
-        for (int k = 0; k < QUADS_IN_FLIGHT; ++k)
-            m = fmaxf(fmaxf(fmaxf(m, fabsf(v[k].x)), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
+        for (int k = 0; k < QUADS_IN_FLIGHT; ++k) {
+            const float a[4] = {fabsf(v[k].x), fabsf(v[k].y), fabsf(v[k].z), fabsf(v[k].w)};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)                  // no infinity, no NaN: these spoil their own rows and columns
+                if (a[e] <= 3.402823466e38f) m = fmaxf(m, a[e]);
+        }
     }
     return m;
 }
@@ -539,7 +543,7 @@ __global__ void __launch_bounds__(256) absmax_kernel(const SplitLaunch p) {
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int w = 1; w < 8; ++w) m = fmaxf(m, warp_max[w]);
-        // non-negative floats order like their bit patterns; NaN / inf would only spoil a result that is spoilt anyway
+        // non-negative floats order like their bit patterns
         if (m > 0.f) atomicMax(s.amax, __float_as_uint(fminf(m, 3.0e38f)));
     }
 }

@@ -69,6 +69,8 @@ cudaError_t read_and_clear_device_status(cudaStream_t stream, int* value) {
 
 namespace {
 
+constexpr float kFloatMax = 3.402823466e38f;
+
 constexpr int cmin(int a, int b) { return a < b ? a : b; }
 
 // Shape of one warp's work.  NL lanes per channel, SPT states per thread,
@@ -505,7 +507,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
     float er[SPT], ei[SPT];     // exp(-i theta_{t+1}) eta_{t+1}
     float gmr[SPT], gmi[SPT];   // sum_t w_t conj(h_t)
     float sbr[SPT], sbi[SPT];   // sum_t eta_t s_t              (general representation only)
-    float amax = 0.f;           // max |dtheta| seen by this thread (spares the split of dtheta a pass of its own)
+    float amax = 0.f;           // largest finite |dtheta| seen by this thread (spares its split a pass of its own)
     float rsum[SPT];            // sum_t dtheta_t
     float hlr[SPT], hli[SPT];   // conj(h_{L-1}) . gh   (boundary term of the Bc gradient)
 #pragma unroll
@@ -602,6 +604,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
             __syncwarp();
 
             // reverse scan
+            float tmax = 0.f;
             auto quad = [&](const int q, auto whole) {
                 const float4 s4 = ld_shared_f4(sw + (c * 3 + 0) * TS + 4 * q);
                 const float4 w4 = ld_shared_f4(sw + (c * 3 + 1) * TS + 4 * q);
@@ -634,7 +637,7 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
                         // dtheta_t = -Im(conj(eta) a)
                         const float d = fmaf(ni, ar, -nr * ai);
                         dth[e] = d;
-                        if (SUMS) { rsum[k] += d; amax = fmaxf(amax, fabsf(d)); }
+                        if (SUMS) { rsum[k] += d; tmax = fmaxf(tmax, fabsf(d)); }
                         const float pv = fmaf(sc[k].mr, hr[k], -sc[k].mi * hi[k]);
                         // gradient of the real drive s_t: Re(conj(eta) beta)
                         const float ev = NORM ? nr : fmaf(nr, sc[k].br, ni * sc[k].bi);
@@ -659,6 +662,20 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
                 for (int q = TS / 4 - 1; q >= 0; --q) quad(q, std::true_type{});
             } else {
                 for (int q = nq - 1; q >= 0; --q) quad(q, std::false_type{});
+            }
+            if (SUMS) {
+                // an infinity (like a NaN, which fmaxf passes over) spoils its own row, not the scale of all others
+                if (tmax > kFloatMax) {
+                    tmax = 0.f;
+#pragma unroll 1
+                    for (int k = 0; k < SPT; ++k)
+#pragma unroll 1
+                        for (int t = 0; t < slen; ++t) {
+                            const float d = fabsf(th[(k * 32 + lane) * TP + sbeg + t]);
+                            if (d <= kFloatMax) tmax = fmaxf(tmax, d);
+                        }
+                }
+                amax = fmaxf(amax, tmax);
             }
             __syncwarp();
 

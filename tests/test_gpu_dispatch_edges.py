@@ -149,6 +149,32 @@ def test_a_nan_spoils_its_own_channel_only():
     assert scaled_error(du_nan[1], du[1]) < operator_bound(b, d, n, l)
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf")])
+@pytest.mark.parametrize("l", [200, 1100])
+def test_an_infinity_does_not_reach_the_scale_of_the_others(bad, l):
+    """In one channel's incoming gradient: the other channels' rows of dx, the other batch entries' du.  In one batch
+    entry's u: the other entries' outputs and du."""
+    b, d, n = 2, 6, 4
+    inp = model_like_inputs(3350, b, d, n, l)
+    results = []
+    for which in (None, "gy", "u"):
+        a = {k: inp[k].cuda() for k in NAMES}
+        gy = inp["gy"].cuda()
+        if which == "gy":
+            gy[0, 2, 77] = bad
+        elif which == "u":
+            a["u"][0, 2, 77] = bad
+        a = {k: t.requires_grad_(True) for k, t in a.items()}
+        y = aussm_b200.ssm_adaptive_interface(**a)
+        results.append((y.detach(), *torch.autograd.grad(y, (a["x"], a["u"]), gy)))
+    (y, dx, du), (_, dx_gy, du_gy), (y_u, _, du_u) = results
+    others = [i for i in range(d) if i != 2]
+    bound = operator_bound(b, d, n, l)
+    assert not torch.isfinite(dx_gy[2]).all() and not torch.isfinite(y_u[0]).all()
+    assert scaled_error(dx_gy[others], dx[others]) < bound and scaled_error(du_gy[1], du[1]) < bound
+    assert scaled_error(y_u[1], y[1]) < bound and scaled_error(du_u[1], du[1]) < bound
+
+
 @pytest.mark.parametrize("steps", [576, 640, 2000])
 def test_operator_windows_of_unequal_length_split_in_time(steps):
     """2000 steps in windows of 576 (the last one shorter than a segment), 640 and one: same result."""
