@@ -156,6 +156,17 @@ __device__ __forceinline__ void cdiv(float ar, float ai, float kr, float ki, flo
 
 // A warp's work: CPW consecutive channels and, when the time axis is split, one segment of it.  The segments are
 // seg_len steps (a multiple of the tile), the last one what is left; all channels of a warp share the segment.
+// SEG = false: a launch without segments.  Length and start then come from the parameters and not from the warp's
+// index, so loop bounds and addresses stay uniform.  It is compiled (FOLD at the launchers) for the tile shapes whose
+// whole launches it makes faster; what it does to the others is the register allocation (N <= 4 forward: 114 -> 96, N <=
+// 8 backward 110 -> 80, with fewer loads in flight).  Calls with / without the segment form, us:
+//     N, B D L             forward      backward
+//     4,  8 512 4096       168 / 191    308 / 284
+//     8,  8 512 4096       191 / 200    345 / 365
+//     16, 2 1024 8192      396 / 361    598 / 613
+//     32, 8 512 2048       298 / 288    546 / 531
+//     64, 8 256 2048       324 / 312    750 / 732
+//     128, 4 256 2048      416 / 474    978 / 957
 struct WarpTask {
     long long ch0;      // first channel
     int nvalid;         // channels that exist
@@ -165,9 +176,19 @@ struct WarpTask {
     // entry of the per-segment state arrays that belongs to channel ch0 + c
     __device__ __forceinline__ long long entry(int c) const { return (ch0 + c) * nseg + seg; }
 };
-template <int CPW, class P>
+template <int CPW, bool SEG, class P>
 __device__ __forceinline__ bool warp_task(const P& p, long long task, WarpTask& w) {
     const long long groups = ((long long)p.nch + CPW - 1) / CPW;
+    if (!SEG) {
+        if (task >= groups) return false;
+        w.seg = 0;
+        w.nseg = 1;
+        w.ch0 = task * CPW;
+        w.nvalid = (int)min((long long)CPW, (long long)p.nch - w.ch0);
+        w.t0 = 0;
+        w.L = p.L;
+        return true;
+    }
     w.nseg = p.nseg > 1 ? p.nseg : 1;
     if (task >= groups * w.nseg) return false;
     w.seg = w.nseg > 1 ? (int)(task / groups) : 0;
@@ -450,12 +471,12 @@ __device__ __forceinline__ void fwd_warp(const ScanFwdParams& p, float* wsm, con
     }
 }
 
-template <class C, bool VEC>
+template <class C, bool VEC, bool SEG>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_fwd_kernel(const ScanFwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpTask wt;
-    if (!warp_task<C::CPW>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;   // no block barriers
+    if (!warp_task<C::CPW, SEG>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;   // no block barriers
     const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / C::NL, jl = lane % C::NL;
@@ -827,12 +848,12 @@ __device__ __forceinline__ void bwd_warp(const ScanBwdParams& p, float* wsm, con
     }
 }
 
-template <class C, bool VEC, bool SUMS>
+template <class C, bool VEC, bool SUMS, bool SEG>
 __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_bwd_kernel(const ScanBwdParams p) {
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpTask wt;
-    if (!warp_task<C::CPW>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;
+    if (!warp_task<C::CPW, SEG>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;
     const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / C::NL, jl = lane % C::NL;
@@ -873,7 +894,7 @@ __global__ void __launch_bounds__(C::WARPS * 32) scan_unitary_summary_kernel(con
     extern __shared__ __align__(128) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpTask wt;
-    if (!warp_task<C::CPW>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;
+    if (!warp_task<C::CPW, true>(p, (long long)blockIdx.x * C::WARPS + warp, wt)) return;
     const int nvalid = wt.nvalid;
     float* wsm = smem + (size_t)warp * C::WARP_FLOATS;
     const int c = lane / NL, jl = lane % NL;
@@ -1138,9 +1159,9 @@ long long warp_tasks(const P& p) {
     return (((long long)p.nch + C::CPW - 1) / C::CPW) * (p.nseg > 1 ? p.nseg : 1);
 }
 
-template <class C, bool VEC>
+template <class C, bool VEC, bool SEG>
 cudaError_t launch_fwd_cfg(const ScanFwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_fwd_kernel<C, VEC>;
+    auto kern = scan_unitary_fwd_kernel<C, VEC, SEG>;
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1150,9 +1171,9 @@ cudaError_t launch_fwd_cfg(const ScanFwdParams& p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template <class C, bool VEC, bool SUMS>
+template <class C, bool VEC, bool SUMS, bool SEG>
 cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
-    auto kern = scan_unitary_bwd_kernel<C, VEC, SUMS>;
+    auto kern = scan_unitary_bwd_kernel<C, VEC, SUMS, SEG>;
     const size_t smem = C::SMEM_BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1162,17 +1183,29 @@ cudaError_t launch_bwd_cfg(const ScanBwdParams& p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-// Runtime properties -> template parameters.
-template <class C>
+// Runtime properties -> template parameters.  FOLD: whole launches have a form of their own (see warp_task).
+template <class C, bool FOLD>
 cudaError_t launch_fwd_sel(const ScanFwdParams& p, bool vec, cudaStream_t s) {
-    return vec ? launch_fwd_cfg<C, true>(p, s) : launch_fwd_cfg<C, false>(p, s);
+    if (!vec) return launch_fwd_cfg<C, false, true>(p, s);
+    if constexpr (FOLD) {
+        if (p.nseg <= 1) return launch_fwd_cfg<C, true, false>(p, s);
+    }
+    return launch_fwd_cfg<C, true, true>(p, s);
 }
 
-template <class C>
+template <class C, bool FOLD, bool SUMS>
+cudaError_t launch_bwd_sums(const ScanBwdParams& p, bool vec, cudaStream_t s) {
+    if (!vec) return launch_bwd_cfg<C, false, SUMS, true>(p, s);
+    if constexpr (FOLD) {
+        if (p.nseg <= 1) return launch_bwd_cfg<C, true, SUMS, false>(p, s);
+    }
+    return launch_bwd_cfg<C, true, SUMS, true>(p, s);
+}
+
+template <class C, bool FOLD>
 cudaError_t launch_bwd_sel(const ScanBwdParams& p, bool vec, cudaStream_t s) {
     if ((p.dtheta_amax != nullptr) != (p.part_rowsum != nullptr)) return cudaErrorInvalidValue;
-    if (p.part_rowsum) return vec ? launch_bwd_cfg<C, true, true>(p, s) : launch_bwd_cfg<C, false, true>(p, s);
-    return vec ? launch_bwd_cfg<C, true, false>(p, s) : launch_bwd_cfg<C, false, false>(p, s);
+    return p.part_rowsum ? launch_bwd_sums<C, FOLD, true>(p, vec, s) : launch_bwd_sums<C, FOLD, false>(p, vec, s);
 }
 
 template <class C, bool VEC, bool BWD>
@@ -1211,12 +1244,12 @@ cudaError_t launch_scan_unitary_fwd(const ScanFwdParams& p_, cudaStream_t stream
                        aligned16(p.u) && aligned16(p.dt) && aligned16(p.z) && (p.y == nullptr || aligned16(p.y)) &&
                        offsets_fit(p.ld_theta, 128);
     const int N = p.N;
-    if (N <= 4) return launch_fwd_sel<FwdCfg<4, 1, 32, 2, 4>>(p, vec, stream);
-    if (N <= 8) return launch_fwd_sel<FwdCfg<8, 1, 32, 2, 4>>(p, vec, stream);
-    if (N <= 16) return launch_fwd_sel<FwdCfg<16, 1, 32, 2, 4>>(p, vec, stream);
-    if (N <= 32) return launch_fwd_sel<FwdCfg<32, 1, 32, 2, 4>>(p, vec, stream);
-    if (N <= 64) return launch_fwd_sel<FwdCfg<32, 2, 32, 2, 4>>(p, vec, stream);
-    if (N <= 128) return launch_fwd_sel<FwdCfg<32, 4, 32, 2, 2>>(p, vec, stream);
+    if (N <= 4) return launch_fwd_sel<FwdCfg<4, 1, 32, 2, 4>, false>(p, vec, stream);
+    if (N <= 8) return launch_fwd_sel<FwdCfg<8, 1, 32, 2, 4>, false>(p, vec, stream);
+    if (N <= 16) return launch_fwd_sel<FwdCfg<16, 1, 32, 2, 4>, true>(p, vec, stream);
+    if (N <= 32) return launch_fwd_sel<FwdCfg<32, 1, 32, 2, 4>, true>(p, vec, stream);
+    if (N <= 64) return launch_fwd_sel<FwdCfg<32, 2, 32, 2, 4>, true>(p, vec, stream);
+    if (N <= 128) return launch_fwd_sel<FwdCfg<32, 4, 32, 2, 2>, false>(p, vec, stream);
     return cudaErrorInvalidValue;
 }
 
@@ -1232,13 +1265,13 @@ cudaError_t launch_scan_unitary_bwd(const ScanBwdParams& p_, cudaStream_t stream
                        aligned16(p.gy) && aligned16(p.du) && aligned16(p.ddt) && aligned16(p.dz) &&
                        offsets_fit(p.ld_theta, 128);
     const int N = p.N;
-    if (N <= 4) return launch_bwd_sel<BwdCfg<4, 1, 32, 32, 2, 2>>(p, vec, stream);
-    if (N <= 8) return launch_bwd_sel<BwdCfg<8, 1, 32, 32, 2, 2>>(p, vec, stream);
+    if (N <= 4) return launch_bwd_sel<BwdCfg<4, 1, 32, 32, 2, 2>, true>(p, vec, stream);
+    if (N <= 8) return launch_bwd_sel<BwdCfg<8, 1, 32, 32, 2, 2>, false>(p, vec, stream);
     // one-warp blocks: a finished warp is replaced at once (measured 9.55 ms against 10.2 ms with two-warp blocks)
-    if (N <= 16) return launch_bwd_sel<BwdCfg<16, 1, 32, 32, 2, 1>>(p, vec, stream);
-    if (N <= 32) return launch_bwd_sel<BwdCfg<32, 1, 32, 32, 2, 2>>(p, vec, stream);
-    if (N <= 64) return launch_bwd_sel<BwdCfg<32, 2, 32, 32, 2, 2>>(p, vec, stream);
-    if (N <= 128) return launch_bwd_sel<BwdCfg<32, 4, 32, 32, 2, 2>>(p, vec, stream);
+    if (N <= 16) return launch_bwd_sel<BwdCfg<16, 1, 32, 32, 2, 1>, false>(p, vec, stream);
+    if (N <= 32) return launch_bwd_sel<BwdCfg<32, 1, 32, 32, 2, 2>, true>(p, vec, stream);
+    if (N <= 64) return launch_bwd_sel<BwdCfg<32, 2, 32, 32, 2, 2>, true>(p, vec, stream);
+    if (N <= 128) return launch_bwd_sel<BwdCfg<32, 4, 32, 32, 2, 2>, true>(p, vec, stream);
     return cudaErrorInvalidValue;
 }
 

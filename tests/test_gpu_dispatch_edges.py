@@ -56,6 +56,16 @@ def test_scan_rows_that_start_anywhere(n, l):
     check_scan(errors, b, d, n, l)
 
 
+@pytest.mark.parametrize("n", [1, 4, 5, 8, 9, 16, 20, 32, 33, 64, 100, 128])
+@pytest.mark.parametrize("l", [4, 28, 32, 36, 132])
+def test_scan_whole_launches_of_aligned_rows(n, l):
+    """Every tile shape in the form that whole launches take: warps with missing channels and states, short last tiles."""
+    b, d = 2, 5
+    errors = scan_errors(b, d, n, l, 1500 + 10 * n + l)
+    assert aussm_b200.device_status() == 0
+    check_scan(errors, b, d, n, l)
+
+
 @pytest.mark.parametrize("shape", [(1, 3, 16, 1024), (1, 2, 5, 1029), (2, 5, 4, 1533), (1, 2, 33, 1280),
                                    (1, 1, 128, 1100), (1, 1, 1, 2047), (3, 7, 10, 1027)])
 def test_scan_cut_into_unequal_segments(shape):
