@@ -203,21 +203,24 @@ def _fake_backward(grad_y, g_re, g_im, u, dt, x, x_bias, B_r, B_theta, C_r, C_th
 keep_phases = "auto"
 
 
-# Buffers below this size may be granted on the allocator's word.  A call of this size takes a workspace at least as
-# large from the same allocator, so a wrong answer cannot cost more than the call itself on a card that is full.
+# Buffers below the first size may be granted on the allocator's word.  A call of this size takes a workspace at least
+# as large from the same allocator, so a wrong answer cannot cost more than the call itself on a card that is full.
+# Requests below the second are carved out of the allocator's shared segments of 2 and 20 MB.
 _SMALL_KEEP = 256 << 20
+_SHARED_KEEP = 10 << 20
 
 
 def _fits_a_quarter(nbytes: int, device) -> bool:
     """True when ``nbytes`` are at most a quarter of the memory that is free for this process.  The driver knows (75 to
-    110 us); for a small buffer the allocator's segments without any used block answer first (8 us).  Its fragments do
-    not count: no contiguous request can rely on them, nor are they given back to the driver."""
+    110 us); for a small buffer the allocator's segments without any used block answer first (8 us).  Its fragments
+    count only for a buffer that is carved out of shared segments anyway: no larger contiguous request can rely on
+    them, nor are they given back to the driver."""
     if nbytes < _SMALL_KEEP:
         try:
             stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
             reserved, active, fragments = (stats[k]["all"]["current"] for k in
                                            ("reserved_bytes", "active_bytes", "inactive_split_bytes"))
-            if nbytes <= (reserved - active - fragments) // 4:
+            if nbytes <= (reserved - active - (fragments if nbytes >= _SHARED_KEEP else 0)) // 4:
                 return True
         except Exception:                       # an allocator without statistics
             pass

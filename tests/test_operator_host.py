@@ -46,6 +46,12 @@ def test_fragments_are_not_free_memory(memory):
     assert not ops._fits_a_quarter(50 * MB, "cuda") and asked
 
 
+def test_fragments_serve_requests_of_the_shared_segments(memory):
+    asked = memory(_stats(1000, 980, 20), 0)
+    assert ops._fits_a_quarter(5 * MB, "cuda") and not asked
+    assert not ops._fits_a_quarter(6 * MB, "cuda") and asked
+
+
 def test_a_large_buffer_asks_the_driver(memory):
     """Unused blocks of other streams and of graphs' pools are in the allocator's count too."""
     asked = memory(_stats(100_000, 0, 0), 500)
