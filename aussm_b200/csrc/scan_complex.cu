@@ -378,14 +378,6 @@ __device__ __forceinline__ void add_channels(float (&b)[4], const float (&c)[4])
         for (int e = 0; e < 4; ++e) b[e] += __shfl_xor_sync(0xffffffffu, b[e], off);
     }
 }
-// a warp with fewer channels than lanes for them: the missing ones add nothing to dB and dC
-__device__ __forceinline__ void drop_if(bool drop, float (&a)[4], float (&b)[4]) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        if (drop) a[e] = b[e] = 0.f;
-    }
-}
-
 template <int NL, bool REAL>
 __global__ void __launch_bounds__(CCfg<NL, true>::WARPS * 32)
 cplx_bwd_kernel(const CplxBwdParams p) {
@@ -463,6 +455,7 @@ cplx_bwd_kernel(const CplxBwdParams p) {
     const bool upper = (lane & 16) != 0;
     const bool grad_lane = (NL == 32 || (lane & 15) < NL) && j < N && nvalid > 0;
     const long long grad_off = bo + (long long)j * p.ld_row;
+    float* const grad_ptr = (upper ? p.dC_re : p.dB_re) + grad_off;
 
     for (int r = 0; r < last - first; ++r) {
         const int tile = last - 1 - r;
@@ -478,7 +471,8 @@ cplx_bwd_kernel(const CplxBwdParams p) {
         block_sync<C>();                                    // every warp's share of the B / C tile has landed
 
         // pre-pass: every activation once.  s = dt silu(u) and w = gy silu(z) feed the scan; silu(u) and
-        // d silu(z)/dz replace the u and z cells, d silu(u)/du gets a row of its own.
+        // d silu(z)/dz replace the u and z cells, d silu(u)/du gets a row of its own.  A missing channel's s and w are
+        // zero: it then adds nothing to dB and dC, without a test or select in the step loops.
 #pragma unroll
         for (int it = 0; it < C::ITERS; ++it) {
             const int e0 = (lane + 32 * it) * VW;
@@ -493,8 +487,9 @@ cplx_bwd_kernel(const CplxBwdParams p) {
                 for (int e = 0; e < VW; ++e) {
                     float gz;
                     u.v[e] = silu_and_grad(u.v[e], gu.v[e]);
-                    d.v[e] *= u.v[e];
-                    g.v[e] *= silu_and_grad(z.v[e], gz);
+                    d.v[e] = cc < nvalid ? d.v[e] * u.v[e] : 0.f;
+                    const float sz = silu_and_grad(z.v[e], gz);
+                    g.v[e] = cc < nvalid ? g.v[e] * sz : 0.f;
                     z.v[e] = gz;
                 }
                 u.st(aux + (cc * AUX + 0) * T + t);
@@ -570,7 +565,6 @@ cplx_bwd_kernel(const CplxBwdParams p) {
             st_shared_f4(st + lane * TP + 4 * q, make_float4(dr[0], dr[1], dr[2], dr[3]));
             st_shared_f4(et + lane * TP + 4 * q, make_float4(E[0], E[1], E[2], E[3]));
             st_shared_f4(pt + lane * TP + 4 * q, make_float4(P[0], P[1], P[2], P[3]));
-            if (nvalid < CPW) drop_if(!act, gBr, gCr);
             add_channels<NL>(gBr, gCr);
             const long long o = grad_off + t0 + 4 * q;
             if (NL == 32) {
@@ -579,7 +573,7 @@ cplx_bwd_kernel(const CplxBwdParams p) {
                     red_add_v4c(p.dC_re + o, gCr);
                 }
             } else if (grad_lane) {
-                red_add_v4c((upper ? p.dC_re : p.dB_re) + o, gBr);
+                red_add_v4c(grad_ptr + t0 + 4 * q, gBr);
             }
         };
         // reverse pass
@@ -627,10 +621,6 @@ cplx_bwd_kernel(const CplxBwdParams p) {
                                                                   : make_float4(0.f, 0.f, 0.f, 0.f));
             st_shared_f4(et + lane * TP + 4 * q, make_float4(E[0], E[1], E[2], E[3]));
             st_shared_f4(pt + lane * TP + 4 * q, make_float4(P[0], P[1], P[2], P[3]));
-            if (nvalid < CPW) {
-                drop_if(!act, gBr, gCr);
-                drop_if(!act, gBi, gCi);
-            }
             add_channels<NL>(gBr, gCr);
             const bool imag = p.dB_im || p.dC_im;
             if (imag) add_channels<NL>(gBi, gCi);
