@@ -44,13 +44,13 @@ namespace {
 
 constexpr int BM = 128, BN = 256;
 constexpr int BK = 64;                               // K values per block
-constexpr int KROW_BYTES = BK * 2;                   // a K-major row of a block: one swizzle row (128 or 64 bytes)
+constexpr int KROW_BYTES = BK * 2;                   // a K-major row of a block: one swizzle row of 128 bytes
 constexpr int MNBOX = 64;                            // row elements per MN-major TMA box (128-byte swizzle rows)
-constexpr int MNBOX_BYTES = MNBOX * 2 * BK;          // 4 KB: BK rows of 128 bytes
-constexpr int STAGES = BK == 64 ? 2 : 4;
-constexpr int A_TILE_BYTES = BM * BK * 2;            // one part of the A tile: 8 KB
-constexpr int B_HALF_BYTES = 128 * BK * 2;           // one part of one 128-column half: 8 KB
-constexpr int STAGE_BYTES = 2 * A_TILE_BYTES + 4 * B_HALF_BYTES;   // hi + lo of both operands: 48 KB
+constexpr int MNBOX_BYTES = MNBOX * 2 * BK;          // 8 KB: BK rows of 128 bytes
+constexpr int STAGES = 2;
+constexpr int A_TILE_BYTES = BM * BK * 2;            // one part of the A tile: 16 KB
+constexpr int B_HALF_BYTES = 128 * BK * 2;           // one part of one 128-column half: 16 KB
+constexpr int STAGE_BYTES = 2 * A_TILE_BYTES + 4 * B_HALF_BYTES;   // hi + lo of both operands: 96 KB
 // Epilogue staging: every accumulate warp turns its 32 x 32 blocks through shared memory (pitch 33 floats, free
 // of bank conflicts both ways) so that C leaves - and, with beta, enters - as whole 128-byte row pieces.
 constexpr int EPI_PITCH = 33;
@@ -59,7 +59,7 @@ constexpr int EPI_WARPS = 8;                         // per column half one warp
 constexpr int EPI_BYTES = EPI_WARPS * EPI_WARP_FLOATS * 4;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + EPI_BYTES;    // + slack for 1024-byte alignment
 // Tensor-memory accumulation truncates instead of rounding, so a long K loop drifts (measured 3.5e-5 relative
-// at K = 4096).  The K loop is therefore cut into chunks of 64 K values: each chunk accumulates from zero in
+// at K = 4096).  The K loop is therefore cut into chunks of 256 K values: each chunk accumulates from zero in
 // tensor memory and the epilogue warps add the finished chunk into float32 registers (round-to-nearest).  The
 // hi*hi products and the two small cross terms go to separate accumulators (adding the tiny terms must not
 // cost the big sum extra truncations).  The 512 columns hold such a pair for each 128-column half of the tile,
@@ -134,7 +134,7 @@ __device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* m
         : "memory");
 }
 
-// One copy = both parts (hi then lo) of 128 rows of an operand for one K block: 16 KB.
+// One copy = both parts (hi then lo) of 128 rows of an operand for one K block: 32 KB.
 template <int MN_MAJOR>
 __device__ __forceinline__ void load_rows128(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int row0, int k0,
                                              int batch) {
@@ -216,13 +216,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
 template <int MN_MAJOR>
 __device__ __forceinline__ uint64_t operand_desc(uint32_t tile_saddr, int kk) {
     if (MN_MAJOR) {
-        // MN-major, 128-byte swizzle (type 2): TMA boxes of BK K-rows x 64 row-elements (4 KB) placed 4096 B
+        // MN-major, 128-byte swizzle (type 2): TMA boxes of BK K-rows x 64 row-elements (8 KB) placed 8192 B
         // apart along the row index, groups of 8 K-rows 1024 B apart; a K = 16 slice is two groups
         return smem_desc(tile_saddr + kk * 2048, MNBOX_BYTES, 1024, 2);
     }
-    // K-major, 64-byte swizzle (type 4): rows of 64 B (32 halves of K), 8-row groups 512 B apart; a K = 16
+    // K-major, 128-byte swizzle (type 2): rows of 128 B (64 halves of K), 8-row groups 1024 B apart; a K = 16
     // slice starts 32 B further into the row
-    return smem_desc(tile_saddr + kk * 32, 16, 8 * KROW_BYTES, KROW_BYTES == 128 ? 2 : 4);
+    return smem_desc(tile_saddr + kk * 32, 16, 8 * KROW_BYTES, 2);
 }
 
 // Accumulation chunks.  A chunk is KC consecutive K blocks accumulated in tensor memory before the epilogue warps
@@ -468,7 +468,8 @@ gemm_split3_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
 // B1 D512 N16 L65536, took 6.18 ms in 112 launches, now 1.61 ms).  VEC: rows of the
 // source are 16-byte aligned and whole quads (one 128-bit load per thread); otherwise scalar loads with a bound check
 // per column.  The destination pitch is always a multiple of 8 halves, so every thread stores its four halves as one
-// 8-byte word; columns between `cols` and the pitch receive zeros (the tensor maps never read them).
+// 8-byte word, zeros after `cols`; what lies between that quad and the pitch stays undefined (the K extent of a
+// K-major tensor map ends before it, and in an MN-major operand it meets columns of C that are never stored).
 template <bool VEC>
 __device__ __forceinline__ float4 load_quad(const float* row, long long c, long long cols) {
     if (VEC) return *reinterpret_cast<const float4*>(row + c);
@@ -606,7 +607,7 @@ EncodeTiledFn encode_fn() {
 }
 
 // Tensor map of a split operand (halves), both parts.  `part_stride` is the distance from the hi to the lo part
-// in bytes.  K-major: dims (K, rows, part, batch), box (BK, 128, 2, 1), 64-byte swizzle.  MN-major: dims (64, K,
+// in bytes.  K-major: dims (K, rows, part, batch), box (BK, 128, 2, 1), 128-byte swizzle.  MN-major: dims (64, K,
 // rows / 64, part, batch), box (64, BK, 2, 2, 1), 128-byte swizzle: the row index is cut into the 64-element
 // boxes the MMA descriptors expect, so one copy fills two boxes of each part.  Out-of-range K rows and boxes read
 // as zero; the last box of an MN-major operand may reach up to 63 elements past `rows` (into the next row, or
@@ -644,7 +645,7 @@ int make_map(CUtensorMap* map, const void* base, long long part_stride, int mn_m
     }
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box,
                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    (mn_major || KROW_BYTES == 128) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                    CU_TENSOR_MAP_SWIZZLE_128B,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled failed with code %d (rows=%lld K=%lld ld=%lld batches=%d mn_major=%d)", (int)r,

@@ -1,10 +1,9 @@
 // General complex / positive-real diagonal selective scan for sm_100a.
 //
-// Same decomposition as scan_unitary.cu and scan_s6.cu: one thread per state
-// and channel, sequential in time; one warp per 32/NL channels of one batch
+// Same decomposition as scan_unitary.cu: one thread per state and channel, sequential in time; one warp per 32/NL channels of one batch
 // entry; 16-step tiles staged by coalesced 16-byte asynchronous copies in a
 // two-stage ring.  A thread consumes its own rho and theta rows (like the
-// unitary scan) and the B_j, C_j rows of its batch entry (like the S6 scan).
+// unitary scan) and the B_j, C_j rows of its batch entry.
 // The B / C rows are the same for every channel of a batch entry, so the warps
 // of a block (all of one batch entry) share one copy of them: each warp fetches
 // its share, two block barriers per tile make the copy visible and protect it

@@ -1291,7 +1291,9 @@ cudaError_t launch_summary(const SegSummaryParams& p, cudaStream_t stream) {
 
 unsigned chain_blocks(long long total) { return (unsigned)((total + 127) / 128); }
 
-// warps of a kernel that an SM holds: shared memory limits them (228 KB, 1 KB of it per block reserved)
+// Warps of a kernel that an SM holds by its shared memory (228 KB, 1 KB of it per block reserved), which is the limit for
+// aligned rows.  The forward kernel for unaligned rows (128 registers at N = 16) and the summary for N > 64 hold fewer, 16
+// instead of 20 warps; the plan must not depend on the rows' alignment, which a workspace query does not know.
 template <class C>
 constexpr long long warps_per_sm() {
     return (228 * 1024 / (long long)(C::SMEM_BYTES + 1024)) * C::WARPS;

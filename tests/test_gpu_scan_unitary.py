@@ -240,7 +240,7 @@ def test_full_size_properties():
 
 @pytest.mark.parametrize("shape", [(1, 6, 16, 4096), (2, 3, 4, 2048), (1, 2, 32, 8192), (1, 40, 16, 1024)])
 def test_time_axis_split_agrees_with_the_sequential_scan(shape):
-    """Few channels: the launch is cut into time segments (aggregate pass, chain over the segments, real pass).
+    """Few channels: the launch is cut into time segments (summary pass, chain over the segments, real pass).
     Forward and backward must agree with the unsplit kernels to float32 rounding, and with the float64 oracle."""
     b, d, n, l = shape
     lib = _lib.load()
