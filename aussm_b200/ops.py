@@ -211,16 +211,19 @@ _SHARED_KEEP = 10 << 20
 
 
 def _fits_a_quarter(nbytes: int, device) -> bool:
-    """True when ``nbytes`` are at most a quarter of the memory that is free for this process.  The driver knows (75 to
-    110 us); for a small buffer the allocator's segments without any used block answer first (8 us).  Its fragments
-    count only for a buffer that is carved out of shared segments anyway: no larger contiguous request can rely on
-    them, nor are they given back to the driver."""
+    """True when ``nbytes`` are at most a quarter of the memory that is free for this process.  The driver knows, but
+    takes 75 to 110 us and several times that while other processes of the machine ask it; for a small buffer the
+    allocator's count of what it holds unused answers first (8 us).  Its fragments, on which no contiguous request can
+    rely, are part of that only where a new segment in their place does no harm: for a buffer that is carved out of
+    shared segments, and while the allocator holds less than half of the card (the driver then has room for the
+    buffer four times over unless another process fills it)."""
     if nbytes < _SMALL_KEEP:
         try:
             stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
             reserved, active, fragments = (stats[k]["all"]["current"] for k in
                                            ("reserved_bytes", "active_bytes", "inactive_split_bytes"))
-            if nbytes <= (reserved - active - (fragments if nbytes >= _SHARED_KEEP else 0)) // 4:
+            roomy = reserved <= torch.cuda.get_device_properties(device).total_memory // 2
+            if nbytes <= (reserved - active - (0 if roomy or nbytes < _SHARED_KEEP else fragments)) // 4:
                 return True
         except Exception:                       # an allocator without statistics
             pass

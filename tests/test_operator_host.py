@@ -1,4 +1,6 @@
 """Host side of a differentiable operator call, without a GPU: what it refuses, whether it keeps its phases."""
+import types
+
 import pytest
 import torch
 from torch._subclasses import FakeTensorMode
@@ -16,7 +18,7 @@ def _stats(reserved, active, fragments):
 @pytest.fixture
 def memory(monkeypatch):
     """memory(statistics or an exception, free megabytes) -> list that counts the questions to the driver"""
-    def setup(stats, free_mb):
+    def setup(stats, free_mb, total_mb=1500):
         asked = []
 
         def statistics(device=None):
@@ -30,6 +32,8 @@ def memory(monkeypatch):
 
         monkeypatch.setattr(torch.cuda.memory, "memory_stats_as_nested_dict", statistics)
         monkeypatch.setattr(torch.cuda, "mem_get_info", driver)
+        monkeypatch.setattr(torch.cuda, "get_device_properties",
+                            lambda device=None: types.SimpleNamespace(total_memory=total_mb * MB))
         return asked
     return setup
 
@@ -50,6 +54,15 @@ def test_fragments_serve_requests_of_the_shared_segments(memory):
     asked = memory(_stats(1000, 980, 20), 0)
     assert ops._fits_a_quarter(5 * MB, "cuda") and not asked
     assert not ops._fits_a_quarter(6 * MB, "cuda") and asked
+
+
+def test_fragments_count_while_the_card_has_room_for_a_new_segment(memory):
+    stats = _stats(1000, 600, 400)
+    asked = memory(stats, 0, total_mb=2000)
+    assert ops._fits_a_quarter(100 * MB, "cuda") and not asked
+    assert not ops._fits_a_quarter(101 * MB, "cuda") and asked
+    asked = memory(stats, 0, total_mb=1999)
+    assert not ops._fits_a_quarter(100 * MB, "cuda") and asked
 
 
 def test_a_large_buffer_asks_the_driver(memory):
