@@ -138,7 +138,7 @@ __device__ __forceinline__ float channel_sum(float v) {
 
 #define AUSSM_F4(v) {(v).x, (v).y, (v).z, (v).w}
 // four consecutive steps as two pairs: what does not run along the recurrence is done two steps at a time with the
-// packed float32x2 instructions (the kernels are bound by the instructions a few warps can issue, not by a pipe)
+// packed float32x2 instructions (the kernels are bound by the shared-memory pipe and by what a few warps can issue, not by the FP32 pipe)
 #define AUSSM_F22(v) {make_float2((v).x, (v).y), make_float2((v).z, (v).w)}
 
 // multipliers exp(dlt A) of four steps
