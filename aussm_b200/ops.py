@@ -222,8 +222,10 @@ def _fits_a_quarter(nbytes: int, device) -> bool:
             stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
             reserved, active, fragments = (stats[k]["all"]["current"] for k in
                                            ("reserved_bytes", "active_bytes", "inactive_split_bytes"))
-            roomy = reserved <= torch.cuda.get_device_properties(device).total_memory // 2
-            if nbytes <= (reserved - active - (0 if roomy or nbytes < _SHARED_KEEP else fragments)) // 4:
+            if (nbytes >= _SHARED_KEEP
+                    and reserved > torch.cuda.get_device_properties(device).total_memory // 2):
+                active += fragments
+            if nbytes <= (reserved - active) // 4:
                 return True
         except Exception:                       # an allocator without statistics
             pass
